@@ -83,8 +83,10 @@ typedef struct qcs_cuda_op {
 
 /* How qcs_cuda_run executes a gate list. */
 typedef struct qcs_cuda_run_options {
-  int fusion_k;  /* 0 or 1: one kernel per gate; 2..7: greedy fusion into
-                    dense blocks of at most fusion_k qubits               */
+  int fusion_k;  /* 0 or 1: gate by gate (several gates to a pass over the
+                    state, with the results of one sweep per gate);
+                    2..7: greedy fusion into dense blocks of at most
+                    fusion_k qubits                                       */
   int fusion_engine; /* QCS_FUSE_AUTO, QCS_FUSE_SIMT or QCS_FUSE_TENSOR    */
   int partitioner;   /* QCS_PARTITION_GREEDY or QCS_PARTITION_LEARNED     */
   int flags;         /* QCS_RUN_* bits, 0 by default                      */
@@ -94,7 +96,7 @@ typedef struct qcs_cuda_run_options {
  * exact bytes of the op list and on the options (and, for the learned
  * partitioner, the cost model and its current parameters); running the same
  * list again skips planning.  Any change (one angle) plans afresh.  A plain
- * run (one kernel per op) of a state of at most 26 qubits and at least 16
+ * run (no fusion) of a state of at most 26 qubits and at least 16
  * ops is captured into a CUDA graph when the same list runs twice in a row,
  * and replayed from then on (not while profiling).  This bit plans
  * afresh every time, launches kernel by kernel, and leaves what is kept
@@ -210,7 +212,8 @@ int qcs_cuda_plan(const qcs_cuda_op *ops, int count, int num_qubits, int kmax,
 #define QCS_KCLASS_SAMPLE 9     /* shot sampling                          */
 #define QCS_KCLASS_OTHER 10     /* set-basis, phase flip, finalisers      */
 #define QCS_KCLASS_BLOCK_TC7 11 /* fused 7-qubit block, tensor cores      */
-#define QCS_KCLASS_COUNT 12
+#define QCS_KCLASS_TILE 12      /* plain gates, several to a pass         */
+#define QCS_KCLASS_COUNT 13
 /* enable != 0: from now on bracket every kernel with CUDA events on the
  * state's stream and accumulate device time and algorithmic bytes per
  * class (counters are cleared); enable == 0 stops recording. */

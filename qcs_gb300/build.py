@@ -25,7 +25,7 @@ LIB = os.path.join(PKG, "libqcs_gb300.so")
 INCLUDE = os.path.join(ROOT, "include")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-CU_SOURCES = ["state.cu", "gates.cu", "readout.cu", "blocks.cu", "blocks_tc.cu",
+CU_SOURCES = ["state.cu", "gates.cu", "readout.cu", "blocks.cu", "blocks_tc.cu", "tiles.cu",
               "batch.cu", "mlp.cu", "noalloc.cu"]
 CPP_SOURCES = ["fusion.cpp", "costmodel.cpp"]
 C_SOURCES = ["qcs_api.c"]

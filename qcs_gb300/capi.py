@@ -30,7 +30,8 @@ FUSE_AUTO, FUSE_SIMT, FUSE_TENSOR = 0, 1, 2
 PARTITION_GREEDY, PARTITION_LEARNED = 0, 1
 # QCS_KCLASS_* order (include/qcs_cuda.h)
 KCLASS_NAMES = ("dense1q", "diag1q", "phase_mask", "ctrl1q", "block_simt", "block_tc",
-                "reduce", "diffuse", "collapse", "sample", "other", "block_tc7")
+                "reduce", "diffuse", "collapse", "sample", "other", "block_tc7",
+                "tile")
 
 
 class QcsCudaError(RuntimeError):

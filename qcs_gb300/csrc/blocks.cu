@@ -22,6 +22,7 @@
 #include "common.cuh"
 #include "costmodel.h"
 #include "fusion.h"
+#include "tiles.h"
 
 namespace qcs {
 
@@ -274,7 +275,7 @@ static int validate_ops(const qcs_cuda_state *s, const qcs_cuda_op *ops, int cou
   return QCS_CUDA_OK;
 }
 
-static int apply_op(qcs_cuda_state *s, const qcs_cuda_op &o) {
+int apply_op(qcs_cuda_state *s, const qcs_cuda_op &o) {
   if (o.kind == QCS_OP_PHASE_FLIP) return phase_flip(s, o.index);
   if (o.kind == QCS_OP_DIFFUSION) return diffusion(s);
   double m[8];
@@ -478,9 +479,23 @@ static int execute_plan(qcs_cuda_state *s, const qcs_cuda_op *ops,
   return QCS_CUDA_OK;
 }
 
+// Runs of gates between phase flips and diffusions go through the tile
+// engine, everything else op by op.  REFERENCE semantics leave the state
+// before the last gate in the second buffer, which a phase flip brings back:
+// the last gate of a run is a sweep of its own there.
 static int run_plain(qcs_cuda_state *s, const qcs_cuda_op *ops, int count) {
-  for (int i = 0; i < count; i++) {
-    int rc = apply_op(s, ops[i]);
+  const bool ref = s->sem == QCS_CUDA_REFERENCE;
+  for (int i = 0; i < count;) {
+    int j = i;
+    while (j < count && gate_kind_valid(ops[j].kind)) j++;
+    const int last = ref ? j - 1 : j;  // the tile engine takes ops[i .. last)
+    int rc;
+    if (last - i >= 2 && tiles_supported(s)) {
+      rc = run_tiles(s, ops + i, last - i);
+      i = last;
+    } else {
+      rc = apply_op(s, ops[i++]);
+    }
     if (rc) return rc;
   }
   return QCS_CUDA_OK;

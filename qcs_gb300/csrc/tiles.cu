@@ -1,0 +1,779 @@
+// tiles.cu -- runs of gates applied tile by tile in shared memory.
+//
+// The sweeps of gates.cu read and write the whole state once per gate.  A
+// plain gate list (no fusion asked for) runs here in passes instead: a pass
+// takes the longest stretch of consecutive gates whose non-diagonal targets
+// fit one set of tile qubits, and for every tile (one setting of the other
+// qubits) a CTA reads the 2^nt amplitudes into shared memory, applies the
+// stretch there and writes them back.  A diagonal gate, and the control of a
+// controlled one, needs no tile qubit: outside the tile its bit is a constant
+// of the tile.
+//
+// The gates keep their order and each amplitude goes through the same
+// products and sums as in the sweeps, so the results are the sweeps' bit for
+// bit; only products with an entry that is exactly 0 or 1 are left out, which
+// changes no finite value (at most the sign of a zero).  A tile that holds an
+// infinity or a NaN takes every product the sweeps take (general_tile).
+//
+// Inside a tile the gates run in register groups: the stretch is cut, again
+// in order, into groups whose targets lie on at most 4 tile bits; a thread
+// holds the 16 amplitudes of one setting of the other bits in registers and
+// takes them through the group's gates, so shared memory is read and written
+// once per group.
+//
+// X and CNOT move amplitudes without arithmetic, and they are not even moved
+// here: the shared-memory position of tile index l is an affine map over
+// GF(2), A l + c, such a gate changes A or c (on the host; a CNOT whose
+// control lies outside the tile changes c for half of the tiles), and the
+// groups and the final store read through the map.
+//
+// Measured against one sweep per gate: 27 qubits complex64, brick, 752 gates
+// 240.7 -> 31.1 ms; 13 qubits, QFT and 200 random gates 201 -> 36 us a run;
+// complex128, 20 qubits, the same circuit 3.88 -> 1.74 ms.  What bounds it:
+// on large complex64 states the instructions of the gate loop (a 24-qubit
+// pass of 36 rotations issues 0.55 of the slots, DRAM at 0.13; a pass of
+// CNOTs alone runs at 0.9 of HBM); on complex128 the FP64 pipe (84 % busy); on
+// small states the latency of a pass.
+#include <stddef.h>
+#include <string.h>
+
+#include <algorithm>
+#include <vector>
+
+#include "common.cuh"
+#include "fusion.h"
+#include "tiles.h"
+
+namespace qcs {
+
+int apply_op(qcs_cuda_state *s, const qcs_cuda_op &o);
+
+constexpr int kTileMaxBits = 11;    // tile amplitudes: 2^11 at most
+constexpr int kTileMaxGates = 128;  // per pass (they ride in the kernel parameters)
+constexpr int kTileMaxGroups = 32;
+constexpr int kTileMaxFlips = 32;
+
+// How the register code applies a gate.  The first five take a register
+// target t; TF_DIAG_OUT is chosen by a bit outside the registers.
+enum TileForm {
+  TF_REAL,      // [[p0, p1], [p2, p3]], all real (RY)
+  TF_HAD,       // p0 * [[1, 1], [1, -1]]
+  TF_RX,        // [[p0, i p1], [i p1, p0]]
+  TF_Y,
+  TF_DIAG,      // p0 + i p1 on bit 0, p2 + i p3 on bit 1 of a register target
+  TF_DIAG_OUT,  // the same, target bit outside the registers
+  TF_NONE,      // leaves finite amplitudes as they are
+  TF_PHASE,     // p2 + i p3 where every condition bit is set
+  TF_SIGN,      // -1 where every condition bit is set
+  TF_COPY,      // the reference's CNOT: v0 := v1 where the control is set
+  TF_SWAP       // X, CNOT: in the maps, never in a group
+};
+
+// One gate of a pass.  `general`: which products the sweep takes, 1: m00 v0,
+// 2: m01 v1, 4: m10 v0, 8: m11 v1; an output without a product keeps its
+// value.
+template <typename R> struct TileGate {
+  R p[4];
+  uint32_t id_cond;       // bits of the tile's id that must be set
+  uint32_t id_tgt;        // the target, where it is a bit of the tile's id
+  unsigned short t_cond;  // bits of the thread index that must be set
+  unsigned short t_tgt;   // the target, where it is a bit of the thread index
+  unsigned short l_tgt, l_ctl;  // target and control as tile bits
+  uint32_t id_ctl;              // control as a bit of the tile's id
+  unsigned char r_cond;   // register bits that must be set
+  unsigned char op;       // TileForm * 8 + register target
+  unsigned char general;
+  unsigned char pad;
+};
+
+// A group: gates seq[gate0 .. gate1) on registers e, where bit j of e adds
+// reg[j], bit j of the thread index col[j], to the shared-memory position
+// (XOR).  Before it, flips [flip0, flip1) change the constant.
+struct TileGroup {
+  unsigned char gate0, gate1, flip0, flip1;
+  unsigned short reg[4];
+  unsigned short col[kTileMaxBits - 4];
+};
+struct TileFlip {
+  unsigned short mask;  // XORed into the constant
+  short id_bit;         // where this bit of the tile's id is set (-1: always)
+};
+
+template <typename R> struct TilePass {
+  i64 n_tiles;
+  R minus_zero;  // see scale2
+  int nt, nout, ngroups, ngates;
+  unsigned char flip0, flip1;       // flips before the store
+  signed char q[kTileMaxBits];      // tile bit -> qubit, ascending
+  signed char out[36];              // bit of the tile id -> qubit, ascending
+  unsigned short store[kTileMaxBits];  // tile bit -> position, after the last gate
+  TileFlip flip[kTileMaxFlips];
+  TileGroup group[kTileMaxGroups];
+  unsigned char seq[kTileMaxGates];
+  TileGate<R> gate[kTileMaxGates];
+};
+
+// ---------------------------------------------------------------------------
+// device
+// ---------------------------------------------------------------------------
+
+// Shared-memory position of tile amplitude i: its place in the 128-byte row
+// is XORed with the row's number, so that whichever tile bits are held in
+// registers a warp's lanes spread over the banks.  Linear over XOR.
+__host__ __device__ __forceinline__ int tile_pos(int i, float2) {
+  return i ^ ((i >> 4) & 15) ^ ((i >> 8) & 15);
+}
+__host__ __device__ __forceinline__ int tile_pos(int i, double2) {
+  return i ^ ((i >> 3) & 7) ^ ((i >> 6) & 7) ^ ((i >> 9) & 7);
+}
+
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
+
+// Collects whether an amplitude was an infinity or a NaN: 0 * x is NaN for
+// those alone (and FP32 products cost no integer slot); FP64, whose products
+// are dear, looks at the exponent.
+struct FiniteF32 {
+  float z = 0.f;
+  __device__ __forceinline__ void see(float2 a) { z = fmaf(a.x, 0.f, fmaf(a.y, 0.f, z)); }
+  __device__ __forceinline__ bool bad() const { return z != 0.f; }
+};
+struct FiniteF64 {
+  bool b = false;
+  __device__ __forceinline__ void see(double2 a) {
+    b = b || (__double2hiint(a.x) & 0x7ff00000) == 0x7ff00000 ||
+        (__double2hiint(a.y) & 0x7ff00000) == 0x7ff00000;
+  }
+  __device__ __forceinline__ bool bad() const { return b; }
+};
+
+// regs: amplitudes a thread holds.  16 measured against 32 (complex64, 27-qubit
+// brick, 752 gates): 32.6 ms and 32.5 ms, but 98 us against 116 us on 13
+// qubits, where the tile's threads are all the parallelism there is.
+// max_bits: a tile's qubits; 11 against 12 (complex64): 32.6 and 33.4 ms on 27
+// qubits, 98 and 114 us on 13; 10 against 11 (complex128, 20 qubits, 417
+// gates): 2.13 and 2.32 ms.
+// low: qubits every tile holds, so that it is read in runs of 128 bytes.
+constexpr int kTileRegBits = 4;
+constexpr int kTileRegs = 1 << kTileRegBits;
+template <typename C> struct TileTraits;
+template <> struct TileTraits<float2> {
+  typedef float R;
+  typedef FiniteF32 Finite;
+  static constexpr int max_bits = 11, low = 4, blocks = 6;
+};
+template <> struct TileTraits<double2> {
+  typedef double R;
+  typedef FiniteF64 Finite;
+  static constexpr int max_bits = 10, low = 3, blocks = 8;
+};
+
+// s * v and v + w, v - w, both parts at once (one packed FP32 instruction).
+// The packed product is written as s * v + z with z = -0 that only the host
+// knows: of a plain packed product and a packed sum the assembler makes one
+// fused operation, with one rounding instead of two, .rn or not.
+__device__ __forceinline__ u64 pack2(float x, float y) {
+  return ((u64)__float_as_uint(y) << 32) | __float_as_uint(x);
+}
+__device__ __forceinline__ float2 unpack2(u64 v) {
+  return make_float2(__uint_as_float((uint32_t)v), __uint_as_float((uint32_t)(v >> 32)));
+}
+__device__ __forceinline__ float2 scale2(float s, float2 v, float z) {
+  u64 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(r) : "l"(pack2(s, s)), "l"(pack2(v.x, v.y)), "l"(pack2(z, z)));
+  return unpack2(r);
+}
+__device__ __forceinline__ float2 add2(float2 v, float2 w) {
+  u64 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(v.x, v.y)), "l"(pack2(w.x, w.y)));
+  return unpack2(r);
+}
+__device__ __forceinline__ double2 scale2(double s, double2 v, double) {
+  return make_double2(__dmul_rn(s, v.x), __dmul_rn(s, v.y));
+}
+__device__ __forceinline__ double2 add2(double2 v, double2 w) { return cadd(v, w); }
+
+// d * v.  FP32: the fused multiply-adds the compiler makes of cmul in the
+// sweeps, written out so that no other contraction can change a bit.
+__device__ __forceinline__ float2 turn(float2 d, float2 v) {
+  return make_float2(__fmaf_rn(d.x, v.x, -__fmul_rn(d.y, v.y)),
+                     __fmaf_rn(d.y, v.x, __fmul_rn(d.x, v.y)));
+}
+__device__ __forceinline__ double2 turn(double2 d, double2 v) { return cmul(d, v); }
+
+// A non-diagonal gate on register bit TB.
+template <int FORM, int TB, typename C, typename R>
+__device__ __forceinline__ void tile_gate(C (&a)[kTileRegs], const TileGate<R> &g, R z) {
+#pragma unroll
+  for (int e = 0; e < kTileRegs; e++) {
+    if (e & (1 << TB)) continue;
+    const int f = e | (1 << TB);
+    const C v0 = a[e], v1 = a[f];
+    if constexpr (FORM == TF_REAL) {
+      a[e] = add2(scale2(g.p[0], v0, z), scale2(g.p[1], v1, z));
+      a[f] = add2(scale2(g.p[2], v0, z), scale2(g.p[3], v1, z));
+    } else if constexpr (FORM == TF_HAD) {
+      const C x0 = scale2(g.p[0], v0, z), x1 = scale2(g.p[0], v1, z);
+      a[e] = add2(x0, x1);
+      a[f].x = sub_rn(x0.x, x1.x);
+      a[f].y = sub_rn(x0.y, x1.y);
+    } else if constexpr (FORM == TF_RX) {
+      a[e].x = sub_rn(mul_rn(g.p[0], v0.x), mul_rn(g.p[1], v1.y));
+      a[e].y = add_rn(mul_rn(g.p[0], v0.y), mul_rn(g.p[1], v1.x));
+      a[f].x = sub_rn(mul_rn(g.p[0], v1.x), mul_rn(g.p[1], v0.y));
+      a[f].y = add_rn(mul_rn(g.p[0], v1.y), mul_rn(g.p[1], v0.x));
+    } else if constexpr (FORM == TF_COPY) {
+      if ((e & g.r_cond) == g.r_cond) a[e] = v1;
+    } else {  // TF_Y
+      a[e].x = v1.y;
+      a[e].y = -v1.x;
+      a[f].x = -v0.y;
+      a[f].y = v0.x;
+    }
+  }
+}
+
+template <int TB, typename C, typename R>
+__device__ __forceinline__ void tile_diag(C (&a)[kTileRegs], const TileGate<R> &g) {
+  C d0, d1;
+  d0.x = g.p[0];
+  d0.y = g.p[1];
+  d1.x = g.p[2];
+  d1.y = g.p[3];
+#pragma unroll
+  for (int e = 0; e < kTileRegs; e++) a[e] = turn((e & (1 << TB)) ? d1 : d0, a[e]);
+}
+
+// The phase on the registers with every bit of COND set (at most two bits).
+// The condition is static: a product that is only predicated off would still
+// take its slot in the FP64 pipe.
+template <int COND, typename C, typename R>
+__device__ __forceinline__ void tile_phase(C (&a)[kTileRegs], const TileGate<R> &g) {
+  C d;
+  d.x = g.p[2];
+  d.y = g.p[3];
+#pragma unroll
+  for (int e = 0; e < kTileRegs; e++)
+    if ((e & COND) == COND) a[e] = turn(d, a[e]);
+}
+
+#define QCS_TILE_FORM(FORM)                                \
+  case FORM * 8 + 0: tile_gate<FORM, 0>(a, g, z); break;       \
+  case FORM * 8 + 1: tile_gate<FORM, 1>(a, g, z); break;       \
+  case FORM * 8 + 2: tile_gate<FORM, 2>(a, g, z); break;       \
+  case FORM * 8 + 3: tile_gate<FORM, 3>(a, g, z); break;
+#define QCS_TILE_PHASE(COND) \
+  case COND: tile_phase<COND>(a, g); break;
+
+// One gate on the amplitudes of thread t.
+template <typename C, typename R>
+__device__ __forceinline__ void tile_apply(C (&a)[kTileRegs], const TileGate<R> &g, uint32_t t,
+                                           uint32_t tile, R z) {
+  switch (g.op) {
+    QCS_TILE_FORM(TF_REAL)
+    QCS_TILE_FORM(TF_HAD)
+    QCS_TILE_FORM(TF_RX)
+    QCS_TILE_FORM(TF_Y)
+    case TF_DIAG * 8 + 0: tile_diag<0>(a, g); break;
+    case TF_DIAG * 8 + 1: tile_diag<1>(a, g); break;
+    case TF_DIAG * 8 + 2: tile_diag<2>(a, g); break;
+    case TF_DIAG * 8 + 3: tile_diag<3>(a, g); break;
+    case TF_DIAG_OUT * 8: {
+      const bool one = (t & g.t_tgt) || (tile & g.id_tgt);
+      C d;
+      d.x = one ? g.p[2] : g.p[0];
+      d.y = one ? g.p[3] : g.p[1];
+#pragma unroll
+      for (int e = 0; e < kTileRegs; e++) a[e] = turn(d, a[e]);
+      break;
+    }
+    default: {  // the forms with conditions
+      if ((t & g.t_cond) != g.t_cond || (tile & g.id_cond) != g.id_cond) break;
+      switch (g.op) {
+        QCS_TILE_FORM(TF_COPY)
+        case TF_PHASE * 8:
+          switch (g.r_cond) {
+            QCS_TILE_PHASE(0) QCS_TILE_PHASE(1) QCS_TILE_PHASE(2) QCS_TILE_PHASE(3)
+            QCS_TILE_PHASE(4) QCS_TILE_PHASE(5) QCS_TILE_PHASE(6) QCS_TILE_PHASE(8)
+            QCS_TILE_PHASE(9) QCS_TILE_PHASE(10) QCS_TILE_PHASE(12)
+          }
+          break;
+        default:  // TF_SIGN
+#pragma unroll
+          for (int e = 0; e < kTileRegs; e++)
+            if ((e & g.r_cond) == g.r_cond) {
+              a[e].x = -a[e].x;
+              a[e].y = -a[e].y;
+            }
+      }
+    }
+  }
+}
+#undef QCS_TILE_PHASE
+#undef QCS_TILE_FORM
+
+// The gates of a pass on a tile with an infinity or a NaN in it: one at a
+// time, with the products the sweep of each gate takes (TileGate::general),
+// so that what spreads, and where to, is the same.
+__device__ __forceinline__ float2 sum2(float2 v, float2 w) {
+  return make_float2(__fadd_rn(v.x, w.x), __fadd_rn(v.y, w.y));
+}
+__device__ __forceinline__ double2 sum2(double2 v, double2 w) { return cadd(v, w); }
+
+template <typename C, typename R>
+__device__ __noinline__ void general_tile(C *S, const TilePass<R> &P, uint32_t tile) {
+  const C kind = {};
+  for (int gi = 0; gi < P.ngates; gi++) {
+    const TileGate<R> &g = P.gate[gi];
+    C m[4] = {};
+    const int form = g.op >> 3;
+    if (form == TF_REAL || form == TF_HAD) {
+      for (int i = 0; i < 4; i++) m[i].x = g.p[i];
+    } else if (form == TF_RX) {
+      m[0].x = m[3].x = g.p[0];
+      m[1].y = m[2].y = g.p[1];
+    } else if (form == TF_SWAP || form == TF_COPY) {
+      m[1].x = m[2].x = 1;
+    } else if (form == TF_Y) {
+      m[1].y = -1;
+      m[2].y = 1;
+    } else {  // diagonal
+      m[0].x = g.p[0];
+      m[0].y = g.p[1];
+      m[3].x = g.p[2];
+      m[3].y = g.p[3];
+    }
+    if ((tile & g.id_ctl) == g.id_ctl) {
+      for (int l = threadIdx.x; l < (1 << P.nt); l += blockDim.x) {
+        if ((l & g.l_ctl) != g.l_ctl) continue;
+        C *x = S + tile_pos(l, kind);
+        if (!g.l_tgt) {  // a diagonal on a qubit outside the tile
+          const bool one = tile & g.id_tgt;
+          if (g.general & (one ? 8 : 1)) *x = turn(one ? m[3] : m[0], *x);
+          continue;
+        }
+        if (l & g.l_tgt) continue;
+        C *y = S + tile_pos(l | g.l_tgt, kind);
+        const C v0 = *x, v1 = *y;
+        const int u = g.general & 3, w = g.general >> 2;
+        if (u) *x = u == 3 ? sum2(turn(m[0], v0), turn(m[1], v1))
+                           : u == 1 ? turn(m[0], v0) : turn(m[1], v1);
+        if (w) *y = w == 3 ? sum2(turn(m[2], v0), turn(m[3], v1))
+                           : w == 1 ? turn(m[2], v0) : turn(m[3], v1);
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// One thread per TileTraits::regs amplitudes of the tile; CTAs are persistent
+// over their tiles.
+template <typename C>
+__global__ void __launch_bounds__(1 << (TileTraits<C>::max_bits - kTileRegBits),
+                                  TileTraits<C>::blocks)
+    k_tile(C *v, const __grid_constant__ TilePass<typename TileTraits<C>::R> P) {
+  constexpr int RB = kTileRegBits, REGS = kTileRegs;
+  constexpr int UNIT = 16 / sizeof(C);  // amplitudes per 16-byte access
+  constexpr int STEPS = REGS / UNIT;    // accesses per thread and tile
+  constexpr int STEP_BITS = UNIT == 2 ? RB - 1 : RB;
+  const C kind = {};
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C *S = reinterpret_cast<C *>(smem_raw);
+  const int t = threadIdx.x;
+  const int sb = P.nt - STEP_BITS;  // the tile bits from sb up count a thread's accesses
+  // this thread's first unit: its offset in memory, its position on loading
+  // and (by the map left by the last gate) on storing
+  i64 toff = 0;
+  int tstore = 0;
+  for (int m = 0; m < sb; m++)
+    if ((t * UNIT >> m) & 1) {
+      toff |= 1LL << P.q[m];
+      tstore ^= P.store[m];
+    }
+  const int tload = tile_pos(t * UNIT, kind);
+  auto step_off = [&](int k) {
+    i64 o = 0;
+#pragma unroll
+    for (int j = 0; j < STEP_BITS; j++)
+      if ((k >> j) & 1) o |= 1LL << P.q[sb + j];
+    return o;
+  };
+  auto step_store = [&](int k) {
+    int o = 0;
+#pragma unroll
+    for (int j = 0; j < STEP_BITS; j++)
+      if ((k >> j) & 1) o ^= P.store[sb + j];
+    return o;
+  };
+  for (i64 tile = blockIdx.x; tile < P.n_tiles; tile += gridDim.x) {
+    i64 base = 0;
+    for (int j = 0; j < P.nout; j++) base |= ((tile >> j) & 1LL) << P.out[j];
+    C *const vt = v + base + toff;
+    const uint32_t id = (uint32_t)tile;
+    typename TileTraits<C>::Finite fin;
+    {
+      uint4 x[STEPS];
+#pragma unroll
+      for (int k = 0; k < STEPS; k++) x[k] = *reinterpret_cast<const uint4 *>(vt + step_off(k));
+#pragma unroll
+      for (int k = 0; k < STEPS; k++) {
+        const C *y = reinterpret_cast<const C *>(&x[k]);
+        const int at = tload ^ tile_pos(k << sb, kind);
+#pragma unroll
+        for (int j = 0; j < UNIT; j++) {
+          fin.see(y[j]);
+          S[at ^ j] = y[j];
+        }
+      }
+    }
+    const bool bad = __syncthreads_or(fin.bad());
+    int c = 0;  // the map's constant
+    auto flips = [&](int f0, int f1) {
+      for (int f = f0; f < f1; f++)
+        if (P.flip[f].id_bit < 0 || ((id >> P.flip[f].id_bit) & 1)) c ^= P.flip[f].mask;
+    };
+    if (bad) {
+      general_tile(S, P, id);
+      for (int k = 0; k < STEPS; k++) {
+        uint4 x;
+        C *y = reinterpret_cast<C *>(&x);
+        for (int j = 0; j < UNIT; j++) y[j] = S[tload ^ tile_pos((k << sb) | j, kind)];
+        *reinterpret_cast<uint4 *>(vt + step_off(k)) = x;
+      }
+    } else {
+      for (int gr = 0; gr < P.ngroups; gr++) {
+        const TileGroup &G = P.group[gr];
+        flips(G.flip0, G.flip1);
+        int at = c;
+#pragma unroll
+        for (int j = 0; j < TileTraits<C>::max_bits - RB; j++)
+          if ((t >> j) & 1) at ^= G.col[j];
+        int pos[REGS];
+#pragma unroll
+        for (int e = 0; e < REGS; e++) {  // e's highest bit, then the rest
+          int hb = 0;
+          while ((e >> hb) > 1) hb++;
+          pos[e] = e == 0 ? at : pos[e ^ (1 << hb)] ^ G.reg[hb];
+        }
+        C a[REGS];
+#pragma unroll
+        for (int e = 0; e < REGS; e++) a[e] = S[pos[e]];
+        for (int i = G.gate0; i < G.gate1; i++) tile_apply(a, P.gate[P.seq[i]], (uint32_t)t, id, P.minus_zero);
+#pragma unroll
+        for (int e = 0; e < REGS; e++) S[pos[e]] = a[e];
+        __syncthreads();
+      }
+      flips(P.flip0, P.flip1);
+#pragma unroll
+      for (int k = 0; k < STEPS; k++) {
+        uint4 x;
+        C *y = reinterpret_cast<C *>(&x);
+        const int at = c ^ tstore ^ step_store(k);
+#pragma unroll
+        for (int j = 0; j < UNIT; j++) y[j] = S[j ? at ^ P.store[0] : at];
+        *reinterpret_cast<uint4 *>(vt + step_off(k)) = x;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// ---------------------------------------------------------------------------
+// host: the plan
+// ---------------------------------------------------------------------------
+
+// The qubit a gate needs in the tile: the target of a non-diagonal gate; -1
+// for a diagonal one.
+static int needed_qubit(const qcs_cuda_op &o) {
+  switch (o.kind) {
+    case QCS_GATE_H: case QCS_GATE_X: case QCS_GATE_Y: case QCS_GATE_RX: case QCS_GATE_RY:
+    case QCS_GATE_CNOT: return o.target;
+    default: return -1;
+  }
+}
+
+static bool moves_only(const qcs_cuda_op &o, bool reference) {
+  return o.kind == QCS_GATE_X || (o.kind == QCS_GATE_CNOT && !reference);
+}
+
+// The register groups of a stretch.  A move (X, CNOT) waits for the end of
+// the current group; a later gate may still join the group if it commutes
+// with the waiting moves exactly: on other qubits, or diagonal on their
+// controls.  Stops early (s.last) when the pass is full.
+static void cut_groups(const qcs_cuda_op *ops, bool reference, TileStretch &s) {
+  typedef unsigned long long Mask;
+  Mask moved = 0, ctl = 0;  // targets and controls of the waiting moves
+  TileStretch::Group g;
+  int flips = 0;
+  auto close = [&](int at) {
+    if (g.gates.empty() && g.moves.empty()) return true;
+    if ((int)s.groups.size() == kTileMaxGroups - 1 || flips > kTileMaxFlips - 2) {
+      s.last = at;
+      return false;
+    }
+    s.groups.push_back(g);
+    g = TileStretch::Group();
+    moved = ctl = 0;
+    return true;
+  };
+  for (int i = s.first; i < s.last; i++) {
+    const qcs_cuda_op &o = ops[i];
+    const Mask t = 1ULL << o.target;
+    const Mask c = gate_is_controlled(o.kind) ? 1ULL << o.control : 0;
+    if (moves_only(o, reference)) {
+      if (flips > kTileMaxFlips - 2) {
+        s.last = i;
+        break;
+      }
+      if (!c || !(s.qubits & c)) flips++;  // at most one flip each
+      g.moves.push_back(i);
+      moved |= t;
+      ctl |= c;
+      continue;
+    }
+    const int q = needed_qubit(o);
+    const bool held = q < 0 || ((g.qubits >> q) & 1);
+    const bool full = !held && __builtin_popcountll(g.qubits) == kTileRegBits;
+    // a condition of the gate on a moved qubit, or its target on a control
+    const bool clash = ((t | c) & moved) || (q >= 0 && (t & ctl));
+    if ((full || clash) && !close(i)) break;
+    if (q >= 0) g.qubits |= 1ULL << q;
+    g.gates.push_back(i);
+  }
+  s.groups.push_back(g);
+}
+
+std::vector<TileStretch> tile_stretches(const qcs_cuda_op *ops, int count, int n, int nt, int low,
+                                        bool reference) {
+  std::vector<TileStretch> plan;
+  for (int i = 0; i < count;) {
+    TileStretch s;
+    s.first = i;
+    unsigned long long set = (1ULL << low) - 1;
+    int room = nt - low;
+    for (; i < count && i - s.first < kTileMaxGates; i++) {
+      const int q = needed_qubit(ops[i]);
+      if (q < 0 || ((set >> q) & 1)) continue;
+      if (room == 0) break;
+      set |= 1ULL << q;
+      room--;
+    }
+    for (int q = low; q < n && room > 0; q++)
+      if (!((set >> q) & 1)) {
+        set |= 1ULL << q;
+        room--;
+      }
+    s.last = i;
+    s.qubits = set;
+    cut_groups(ops, reference, s);
+    i = s.last;
+    plan.push_back(s);
+  }
+  return plan;
+}
+
+// Which products the sweep of this gate takes (gates.cu), as TileGate::general.
+static int sweep_products(const qcs_cuda_state *s, const double m[8], bool controlled) {
+  auto zero = [&](int i) { return m[2 * i] == 0.0 && m[2 * i + 1] == 0.0; };
+  auto one = [&](int i) { return m[2 * i] == 1.0 && m[2 * i + 1] == 0.0; };
+  const bool diag = zero(1) && zero(2), exch = zero(0) && zero(3);
+  if (s->sem == QCS_CUDA_REFERENCE) {
+    if (controlled) return zero(1) ? 1 : zero(0) ? 2 : 3;
+    return diag ? 1 | 8 : exch ? 2 | 4 : 15;
+  }
+  if (diag && one(0)) return one(3) ? 0 : 8;
+  if (!controlled && diag) return 1 | 8;
+  if (exch && s->prec == QCS_CUDA_C128) return 2 | 4;
+  return 15;
+}
+
+// Gate record; bit_of: qubit -> tile bit (-1: outside), id_of: qubit -> bit of
+// the tile's id, reg_of and thread_of: tile bit -> register or thread bit of
+// the gate's group (-1: the other).
+template <typename R>
+static void fill_gate(const qcs_cuda_state *s, const qcs_cuda_op &o, const int *bit_of,
+                      const int *id_of, const int *reg_of, const int *thread_of, TileGate<R> &g) {
+  memset(&g, 0, sizeof(g));
+  double m[8];
+  gate_matrix(o.kind, o.angle, m);
+  const bool ctl = gate_is_controlled(o.kind);
+  const bool ref = s->sem == QCS_CUDA_REFERENCE;
+  g.general = (unsigned char)sweep_products(s, m, ctl);
+  if (bit_of[o.target] >= 0) g.l_tgt = (unsigned short)(1 << bit_of[o.target]);
+  else g.id_tgt = 1u << id_of[o.target];
+  if (ctl) {
+    if (bit_of[o.control] >= 0) g.l_ctl = (unsigned short)(1 << bit_of[o.control]);
+    else g.id_ctl = 1u << id_of[o.control];
+  }
+  auto place = [&](int q, unsigned char &r, unsigned short &t, uint32_t &id) {
+    if (bit_of[q] < 0) id |= 1u << id_of[q];
+    else if (reg_of[bit_of[q]] >= 0) r |= (unsigned char)(1 << reg_of[bit_of[q]]);
+    else t |= (unsigned short)(1 << thread_of[bit_of[q]]);
+  };
+  int form = TF_NONE;
+  bool cond_tgt = false;  // the target bit is a condition too (phases)
+  switch (o.kind) {
+    case QCS_GATE_H: form = TF_HAD; break;
+    case QCS_GATE_RY: form = TF_REAL; break;
+    case QCS_GATE_RX: form = TF_RX; break;
+    case QCS_GATE_X: form = TF_SWAP; break;
+    case QCS_GATE_Y: form = TF_Y; break;
+    case QCS_GATE_CNOT: form = ref ? TF_COPY : TF_SWAP; break;
+    case QCS_GATE_RZ: form = TF_DIAG; break;
+    case QCS_GATE_Z: form = TF_SIGN; cond_tgt = true; break;
+    case QCS_GATE_P: form = TF_PHASE; cond_tgt = true; break;
+    // under the reference's rule a CPHASE multiplies by its U00 = 1 only
+    case QCS_GATE_CPHASE: form = ref ? TF_NONE : TF_PHASE; cond_tgt = true; break;
+    default: form = TF_NONE; break;  // identity
+  }
+  if (form == TF_RX) {
+    g.p[0] = (R)m[0];
+    g.p[1] = (R)m[3];
+  } else if (form == TF_REAL || form == TF_HAD) {
+    for (int i = 0; i < 4; i++) g.p[i] = (R)m[2 * i];
+  } else {
+    g.p[0] = (R)m[0];
+    g.p[1] = (R)m[1];
+    g.p[2] = (R)m[6];
+    g.p[3] = (R)m[7];
+  }
+  if (ctl) place(o.control, g.r_cond, g.t_cond, g.id_cond);
+  if (cond_tgt) place(o.target, g.r_cond, g.t_cond, g.id_cond);
+  int reg = bit_of[o.target] >= 0 ? reg_of[bit_of[o.target]] : -1;
+  if (form == TF_DIAG && reg < 0) {
+    form = TF_DIAG_OUT;
+    unsigned char none = 0;
+    uint32_t id = 0;  // id_tgt is set above
+    place(o.target, none, g.t_tgt, id);
+  }
+  const bool on_reg = form <= TF_DIAG || form == TF_COPY;
+  g.op = (unsigned char)(form * 8 + (on_reg ? reg : 0));
+}
+
+template <typename C>
+static int launch_pass(qcs_cuda_state *s, const qcs_cuda_op *ops, const TileStretch &st) {
+  typedef typename TileTraits<C>::R R;
+  constexpr int RB = kTileRegBits;
+  const C kind = {};
+  TilePass<R> P;
+  memset(&P, 0, offsetof(TilePass<R>, gate));
+  int bit_of[36], id_of[36];
+  for (int q = 0; q < s->n; q++) {
+    bit_of[q] = id_of[q] = -1;
+    if ((st.qubits >> q) & 1) {
+      bit_of[q] = P.nt;
+      P.q[P.nt++] = (signed char)q;
+    } else {
+      id_of[q] = P.nout;
+      P.out[P.nout++] = (signed char)q;
+    }
+  }
+  P.n_tiles = 1LL << P.nout;
+  P.minus_zero = (R)-0.0;
+  P.ngates = st.last - st.first;
+  int map[kTileMaxBits];  // column b: what tile bit b adds to the position
+  for (int b = 0; b < P.nt; b++) map[b] = tile_pos(1 << b, kind);
+  int nseq = 0, nflip = 0, flip0 = 0;
+  auto move = [&](const qcs_cuda_op &o) {  // X or CNOT: see the head of the file
+    const int t = bit_of[o.target];
+    if (o.kind == QCS_GATE_CNOT && bit_of[o.control] >= 0) {
+      map[bit_of[o.control]] ^= map[t];
+    } else {
+      TileFlip &f = P.flip[nflip++];
+      f.mask = (unsigned short)map[t];
+      f.id_bit = (short)(o.kind == QCS_GATE_CNOT ? id_of[o.control] : -1);
+    }
+  };
+  int none[kTileMaxBits];
+  std::fill(none, none + kTileMaxBits, 0);
+  for (const TileStretch::Group &gr : st.groups) {
+    if (!gr.gates.empty()) {
+      TileGroup &G = P.group[P.ngroups++];
+      G.flip0 = (unsigned char)flip0;
+      G.flip1 = (unsigned char)nflip;
+      flip0 = nflip;
+      // Which tile bits the registers take besides the group's targets, and
+      // which the lanes of a warp: a condition on a register bit costs the
+      // other registers nothing and one on the upper thread bits skips whole
+      // warps, but one on a lane leaves half of the warp idle, so the bits
+      // that most gates depend on come first.
+      int uses[kTileMaxBits] = {0}, order[kTileMaxBits];
+      for (int i : gr.gates) {
+        const qcs_cuda_op &o = ops[i];
+        if (bit_of[o.target] >= 0) uses[bit_of[o.target]]++;
+        if (gate_is_controlled(o.kind) && bit_of[o.control] >= 0) uses[bit_of[o.control]]++;
+      }
+      for (int b = 0; b < P.nt; b++) {
+        order[b] = P.nt - 1 - b;
+        if ((gr.qubits >> P.q[b]) & 1) uses[b] += 1 << 16;  // a target: in a register
+      }
+      std::stable_sort(order, order + P.nt, [&](int x, int y) { return uses[x] > uses[y]; });
+      int reg_of[kTileMaxBits], thread_of[kTileMaxBits];
+      std::fill(reg_of, reg_of + kTileMaxBits, -1);
+      std::fill(thread_of, thread_of + kTileMaxBits, -1);
+      for (int j = 0; j < P.nt; j++) {
+        const int b = order[j];
+        if (j < RB) {
+          G.reg[j] = (unsigned short)map[b];
+          reg_of[b] = j;
+        } else {
+          const int t = P.nt - 1 - j;  // the last, least used ones are the lanes
+          G.col[t] = (unsigned short)map[b];
+          thread_of[b] = t;
+        }
+      }
+      G.gate0 = (unsigned char)nseq;
+      for (int i : gr.gates) {
+        P.seq[nseq] = (unsigned char)(i - st.first);
+        TileGate<R> &g = P.gate[i - st.first];
+        fill_gate<R>(s, ops[i], bit_of, id_of, reg_of, thread_of, g);
+        if (g.op != TF_NONE * 8) nseq++;
+      }
+      G.gate1 = (unsigned char)nseq;
+    }
+    for (int i : gr.moves) {
+      fill_gate<R>(s, ops[i], bit_of, id_of, none, none, P.gate[i - st.first]);
+      move(ops[i]);
+    }
+  }
+  P.flip0 = (unsigned char)flip0;
+  P.flip1 = (unsigned char)nflip;
+  for (int b = 0; b < P.nt; b++) P.store[b] = (unsigned short)map[b];
+  const int threads = 1 << (P.nt - RB);
+  const size_t smem = sizeof(C) << P.nt;
+  const i64 cap = (i64)s->dev.num_sms * std::min(32, TileTraits<C>::blocks
+                                                         << (TileTraits<C>::max_bits - P.nt));
+  const int grid = (int)std::min<i64>(P.n_tiles, cap);
+  s->h2d_bytes += (long long)(offsetof(TilePass<R>, gate) + P.ngates * sizeof(TileGate<R>));
+  prof_begin(s);
+  k_tile<C><<<grid, threads, smem, s->stream>>>((C *)s->vec, P);
+  invalidate_sum(s);
+  return launched(s, KC_TILE, 2.0 * s->size * sizeof(C), "gate tile pass");
+}
+
+template <typename C>
+static int run_tiles_t(qcs_cuda_state *s, const qcs_cuda_op *ops, int count) {
+  const int nt = std::min(TileTraits<C>::max_bits, s->n);
+  for (const TileStretch &st : tile_stretches(ops, count, s->n, nt, TileTraits<C>::low,
+                                              s->sem == QCS_CUDA_REFERENCE)) {
+    const int rc = st.last - st.first == 1 ? apply_op(s, ops[st.first])
+                                           : launch_pass<C>(s, ops, st);
+    if (rc) return rc;
+  }
+  return QCS_CUDA_OK;
+}
+
+int run_tiles(qcs_cuda_state *s, const qcs_cuda_op *ops, int count) {
+  return s->prec == QCS_CUDA_C128 ? run_tiles_t<double2>(s, ops, count)
+                                  : run_tiles_t<float2>(s, ops, count);
+}
+
+// A state smaller than one thread's registers stays with the sweeps.
+bool tiles_supported(const qcs_cuda_state *s) { return s->n >= kTileRegBits; }
+
+}  // namespace qcs
