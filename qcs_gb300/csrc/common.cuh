@@ -85,19 +85,21 @@ struct qcs_cuda_state {
   qcs::DeviceInfo dev;
   // reductions: per-block partials, a final result slot, pinned host mirror
   qcs::ReduceSlot *d_partials;
+  unsigned *d_count;   // blocks of the running reduction that are done
   double *d_result;    // 8 doubles
   double *h_result;    // pinned, 8 doubles
+  double *h_result_dev;  // its device address: kernels write results there
   // cached sum of amplitudes (complex, FP64) for Grover iterations; valid
   // while sum_valid != 0 (kept on the device in d_result[4..5])
   int sum_valid;
   // sampling scratch (grown on demand)
   double *d_tile_prefix;  // n_tiles + 1 (exclusive prefix, then total)
   qcs::i64 n_tiles;
-  double *d_draws;
-  qcs::i64 *d_samples;
   int sample_cap;
-  double *h_draws;        // pinned staging
-  qcs::i64 *h_samples;    // pinned staging
+  double *h_draws;        // pinned, read and written by the sampler in place
+  qcs::i64 *h_samples;
+  double *h_draws_dev;    // their device addresses
+  qcs::i64 *h_samples_dev;
   // measurement support
   long long launches;
   qcs::ProfData *prof;    // non-null while profiling

@@ -87,7 +87,8 @@ static int na_launch(const C *v, i64 count, const double *draws, int shots, i64 
   i64 per = 1;
   smp_ranges(n_tiles, sms, kNoAllocMaxRanges, &G, &per);
   double *in = prefix, *boff = prefix + n_tiles;
-  k_smp_tile_sums<C><<<G, kSampleThreads, 0, st>>>(v, tile, n_tiles, per, in, boff);
+  k_smp_tile_sums<C><<<G, kSampleThreads, 0, st>>>(v, tile, n_tiles, per, in, boff,
+                                                     nullptr);
   rc = check_launch("sample_noalloc tile sums");
   if (rc) return rc;
   k_smp_prefix<<<1, 1024, 0, st>>>(boff, G);

@@ -9,8 +9,17 @@
 // Precision plan (GB300 has little FP64 throughput): for complex64 states a
 // thread forms |a|^2 (or re, im) in FP32 over 8 amplitudes, then adds that
 // partial into FP64 accumulators; block and grid combination are FP64.  The
-// grid is fixed per device, so every reduction is deterministic.  complex128
-// states use FP64 throughout.
+// grid is fixed per state size, so every reduction is deterministic.
+// complex128 states use FP64 throughout.
+//
+// The last block of a reduction to finish combines the blocks' partials (in a
+// fixed order) and leaves the result where it is wanted: in device memory, or
+// straight in the state's pinned host buffer.  A call is then one kernel and
+// one wait; a second kernel of one warp (10 us for 608 slots; 169 us where
+// one thread walked them, for the argmax) and a copy back took longer than
+// the reduction of a small state.
+#include <type_traits>
+
 #include "common.cuh"
 #include "sampler.cuh"
 
@@ -22,6 +31,23 @@ __device__ __forceinline__ double warp_sum(double x) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
   return x;
+}
+
+// Called by every thread of every block, after thread 0 has written the
+// block's partial: true in the block that gets here last, which then sees
+// every block's.  Leaves the counter at zero for the next launch.
+__device__ __forceinline__ bool last_block(unsigned *count) {
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(count, 1u) == gridDim.x - 1;
+    if (last) {
+      *count = 0;
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  return last;
 }
 
 // Sum four FP64 values over the block; thread 0 writes `out`.
@@ -58,6 +84,35 @@ __device__ void block_sum4(double a, double b, double c, double d, ReduceSlot *o
   }
 }
 
+// The block adds nblocks partials in a fixed order; thread 0 writes four sums.
+__device__ void sum_slots(const ReduceSlot *p, int nblocks, double *result) {
+  double a = 0.0, b = 0.0, c = 0.0, d = 0.0;
+  for (int i = threadIdx.x; i < nblocks; i += blockDim.x) {
+    const double2 *s = reinterpret_cast<const double2 *>(p + i);
+    const double2 x = __ldcg(s), y = __ldcg(s + 1);
+    a += x.x;
+    b += x.y;
+    c += y.x;
+    d += y.y;
+  }
+  __syncthreads();
+  ReduceSlot r;
+  block_sum4(a, b, c, d, &r);
+  if (threadIdx.x == 0) {
+    result[0] = r.a;
+    result[1] = r.b;
+    result[2] = r.c;
+    result[3] = r.d;
+  }
+}
+
+// Ends a reduction: the block's partial, then (last block) the total.
+__device__ __forceinline__ void reduce_end(double a, double b, ReduceSlot *slots, unsigned *count,
+                                           double *result) {
+  block_sum4(a, b, 0.0, 0.0, slots + blockIdx.x);
+  if (last_block(count)) sum_slots(slots, gridDim.x, result);
+}
+
 template <int OP, typename R>
 __device__ __forceinline__ void accum(i64 idx, R re, R im, int q, R &pa, R &pb) {
   if (OP == OP_NORM) {
@@ -76,7 +131,8 @@ __device__ __forceinline__ void accum(i64 idx, R re, R im, int q, R &pa, R &pb) 
 // step, FP32 within a step, FP64 across steps.
 template <int OP>
 __global__ void __launch_bounds__(kReduceThreads)
-    k_reduce_c64(const float4 *v, i64 units, int q, ReduceSlot *out) {
+    k_reduce_c64(const float4 *v, i64 units, int q, ReduceSlot *slots, unsigned *count,
+                 double *result) {
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   double A = 0.0, B = 0.0;
   for (i64 u = (i64)blockIdx.x * blockDim.x + threadIdx.x; u < units; u += 4 * nthr) {
@@ -103,47 +159,34 @@ __global__ void __launch_bounds__(kReduceThreads)
     A += (double)pa;
     B += (double)pb;
   }
-  block_sum4(A, B, 0.0, 0.0, out + blockIdx.x);
+  reduce_end(A, B, slots, count, result);
 }
 
 template <int OP>
 __global__ void __launch_bounds__(kReduceThreads)
-    k_reduce_c128(const double2 *v, i64 size, int q, ReduceSlot *out) {
+    k_reduce_c128(const double2 *v, i64 size, int q, ReduceSlot *slots, unsigned *count,
+                  double *result) {
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   double A = 0.0, B = 0.0;
   for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < size; i += nthr) {
     double2 x = v[i];
     accum<OP, double>(i, x.x, x.y, q, A, B);
   }
-  block_sum4(A, B, 0.0, 0.0, out + blockIdx.x);
+  reduce_end(A, B, slots, count, result);
 }
 
-// One warp combines the per-block partials in a fixed order.
-__global__ void k_finalize(const ReduceSlot *p, int nblocks, double *result) {
-  double a = 0.0, b = 0.0, c = 0.0, d = 0.0;
-  for (int i = threadIdx.x; i < nblocks; i += 32) {
-    a += p[i].a;
-    b += p[i].b;
-    c += p[i].c;
-    d += p[i].d;
-  }
-  a = warp_sum(a);
-  b = warp_sum(b);
-  c = warp_sum(c);
-  d = warp_sum(d);
-  if (threadIdx.x == 0) {
-    result[0] = a;
-    result[1] = b;
-    result[2] = c;
-    result[3] = d;
-  }
+// One block combines partials that another kernel left.
+__global__ void __launch_bounds__(kReduceThreads)
+    k_finalize(const ReduceSlot *p, int nblocks, double *result) {
+  sum_slots(p, nblocks, result);
 }
 
 // Physical diffusion psi := 2*(S/N) - psi, fused with the sum of the new
 // amplitudes (the sum is invariant in exact arithmetic; carrying the real
 // sum of what was stored keeps a following phase flip's cached sum exact).
 __global__ void __launch_bounds__(kReduceThreads)
-    k_diffuse_c64(float4 *v, i64 units, const double *S, double inv_n, ReduceSlot *out) {
+    k_diffuse_c64(float4 *v, i64 units, double *S, double inv_n, ReduceSlot *slots,
+                  unsigned *count) {
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   const float tr = (float)(2.0 * (S[0] * inv_n));
   const float ti = (float)(2.0 * (S[1] * inv_n));
@@ -169,11 +212,12 @@ __global__ void __launch_bounds__(kReduceThreads)
     A += (double)pa;
     B += (double)pb;
   }
-  block_sum4(A, B, 0.0, 0.0, out + blockIdx.x);
+  reduce_end(A, B, slots, count, S);  // every block has read S by now
 }
 
 __global__ void __launch_bounds__(kReduceThreads)
-    k_diffuse_c128(double2 *v, i64 size, const double *S, double inv_n, ReduceSlot *out) {
+    k_diffuse_c128(double2 *v, i64 size, double *S, double inv_n, ReduceSlot *slots,
+                   unsigned *count) {
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   const double tr = 2.0 * (S[0] * inv_n);
   const double ti = 2.0 * (S[1] * inv_n);
@@ -185,7 +229,7 @@ __global__ void __launch_bounds__(kReduceThreads)
     A += y.x;
     B += y.y;
   }
-  block_sum4(A, B, 0.0, 0.0, out + blockIdx.x);
+  reduce_end(A, B, slots, count, S);
 }
 
 // The reference's diffusion (src/q_gates.c:334-355): mean := S/|S| when
@@ -285,24 +329,13 @@ __device__ __forceinline__ bool better(R v, i64 i, R bv, i64 bi) {
   return v > bv || (v == bv && i < bi);
 }
 
-template <typename C, typename R>
-__global__ void __launch_bounds__(kReduceThreads)
-    k_argmax(const C *v, i64 size, ReduceSlot *out) {
-  const i64 nthr = (i64)gridDim.x * blockDim.x;
-  R bv = (R)-1;
-  i64 bi = size;
-  for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < size; i += nthr) {
-    C x = v[i];
-    R p = (x.x * x.x) + (x.y * x.y);
-    if (better(p, i, bv, bi)) {
-      bv = p;
-      bi = i;
-    }
-  }
+// The best (value, index) pair over the block, in thread 0.
+template <typename R>
+__device__ __forceinline__ void block_best(R &bv, i64 &bi) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
-    R ov = __shfl_xor_sync(0xffffffffu, bv, o);
-    i64 oi = __shfl_xor_sync(0xffffffffu, bi, o);
+    const R ov = __shfl_xor_sync(0xffffffffu, bv, o);
+    const i64 oi = __shfl_xor_sync(0xffffffffu, bi, o);
     if (better(ov, oi, bv, bi)) {
       bv = ov;
       bi = oi;
@@ -310,7 +343,7 @@ __global__ void __launch_bounds__(kReduceThreads)
   }
   __shared__ R sv[kReduceThreads / 32];
   __shared__ i64 si[kReduceThreads / 32];
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   if (l == 0) {
     sv[w] = bv;
     si[w] = bi;
@@ -322,16 +355,58 @@ __global__ void __launch_bounds__(kReduceThreads)
         bv = sv[k];
         bi = si[k];
       }
-    out[blockIdx.x].a = (double)bv;
-    out[blockIdx.x].b = (double)bi;
   }
+}
+
+// Ends an argmax: the block's best, then (last block) the best of all.
+template <typename R>
+__device__ __forceinline__ void argmax_end(R bv, i64 bi, ReduceSlot *slots, unsigned *count,
+                                           double *result) {
+  block_best(bv, bi);
+  if (threadIdx.x == 0) {
+    slots[blockIdx.x].a = (double)bv;
+    slots[blockIdx.x].b = (double)bi;
+  }
+  if (!last_block(count)) return;
+  double v = -1.0;
+  i64 at = 1LL << 62;
+  for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
+    const double2 x = __ldcg(reinterpret_cast<const double2 *>(slots + k));
+    if (better(x.x, (i64)x.y, v, at)) {
+      v = x.x;
+      at = (i64)x.y;
+    }
+  }
+  block_best(v, at);
+  if (threadIdx.x == 0) {
+    result[0] = v;
+    result[1] = (double)at;
+  }
+}
+
+template <typename C, typename R>
+__global__ void __launch_bounds__(kReduceThreads)
+    k_argmax(const C *v, i64 size, ReduceSlot *slots, unsigned *count, double *result) {
+  const i64 nthr = (i64)gridDim.x * blockDim.x;
+  R bv = (R)-1;
+  i64 bi = size;
+  for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < size; i += nthr) {
+    C x = v[i];
+    R p = (x.x * x.x) + (x.y * x.y);
+    if (better(p, i, bv, bi)) {
+      bv = p;
+      bi = i;
+    }
+  }
+  argmax_end(bv, bi, slots, count, result);
 }
 
 // complex64: units of two amplitudes (one 16-byte load), four in flight per
 // thread; the same order (larger |a|^2, then smaller index) makes the result
 // independent of which thread saw which amplitude.
 __global__ void __launch_bounds__(kReduceThreads)
-    k_argmax_c64(const float4 *v, i64 units, ReduceSlot *out) {
+    k_argmax_c64(const float4 *v, i64 units, ReduceSlot *slots, unsigned *count,
+                 double *result) {
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   float bv = -1.f;
   i64 bi = 2 * units;
@@ -358,77 +433,52 @@ __global__ void __launch_bounds__(kReduceThreads)
       }
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-    const i64 oi = __shfl_xor_sync(0xffffffffu, bi, o);
-    if (better(ov, oi, bv, bi)) {
-      bv = ov;
-      bi = oi;
-    }
-  }
-  __shared__ float sv[kReduceThreads / 32];
-  __shared__ i64 si[kReduceThreads / 32];
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) {
-    sv[w] = bv;
-    si[w] = bi;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 1; k < (int)(blockDim.x >> 5); k++)
-      if (better(sv[k], si[k], bv, bi)) {
-        bv = sv[k];
-        bi = si[k];
-      }
-    out[blockIdx.x].a = (double)bv;
-    out[blockIdx.x].b = (double)bi;
-  }
-}
-
-__global__ void k_argmax_finalize(const ReduceSlot *p, int nblocks, double *result) {
-  if (threadIdx.x != 0) return;
-  double bv = -1.0, bi = 9.0e18;
-  for (int k = 0; k < nblocks; k++)
-    if (p[k].a > bv || (p[k].a == bv && p[k].b < bi)) {
-      bv = p[k].a;
-      bi = p[k].b;
-    }
-  result[0] = bv;
-  result[1] = bi;
+  argmax_end(bv, bi, slots, count, result);
 }
 
 // ---- shot sampling: sampler.cuh -------------------------------------------------
 
 // ---- host side -----------------------------------------------------------------
 
+// Blocks of a reduction over `work` items, one per thread and step: the
+// device's fixed reduction grid, or as many as have work.  (A grid that small
+// gives each thread one item, so the partial sums are those of the full grid.)
+static int reduce_grid(const qcs_cuda_state *s, i64 work) {
+  const i64 need = (work + kReduceThreads - 1) / kReduceThreads;
+  return (int)(need < 1 ? 1 : need < s->dev.reduce_blocks ? need : s->dev.reduce_blocks);
+}
+
+// Waits for a result that a kernel wrote to the pinned host buffer.
+static int wait_result(qcs_cuda_state *s, size_t bytes, const char *what) {
+  s->d2h_bytes += (long long)bytes;
+  return check_cuda(cudaStreamSynchronize(s->stream), what);
+}
+
+// Result in the pinned buffer (res != null), or, for the sum, on the device.
 static int reduce(qcs_cuda_state *s, int op, int q, double *res, int nres) {
-  const DeviceInfo &d = s->dev;
-  const double Ns = (double)s->size * (s->prec == QCS_CUDA_C128 ? 16 : 8);
+  const bool c128 = s->prec == QCS_CUDA_C128;
+  const double Ns = (double)s->size * (c128 ? 16 : 8);
+  double *dst = op == OP_SUM ? s->d_result + 4 : s->h_result_dev;
+  const i64 work = c128 ? s->size : s->size / 2;
+  const int grid = reduce_grid(s, work);
   prof_begin(s);
-  if (s->prec == QCS_CUDA_C128) {
-    const double2 *v = (const double2 *)s->vec;
-    if (op == OP_NORM) k_reduce_c128<OP_NORM><<<d.reduce_blocks, kReduceThreads, 0, s->stream>>>(v, s->size, q, s->d_partials);
-    else if (op == OP_MASK) k_reduce_c128<OP_MASK><<<d.reduce_blocks, kReduceThreads, 0, s->stream>>>(v, s->size, q, s->d_partials);
-    else k_reduce_c128<OP_SUM><<<d.reduce_blocks, kReduceThreads, 0, s->stream>>>(v, s->size, q, s->d_partials);
-  } else {
-    const float4 *v = (const float4 *)s->vec;
-    i64 units = s->size / 2;
-    if (op == OP_NORM) k_reduce_c64<OP_NORM><<<d.reduce_blocks, kReduceThreads, 0, s->stream>>>(v, units, q, s->d_partials);
-    else if (op == OP_MASK) k_reduce_c64<OP_MASK><<<d.reduce_blocks, kReduceThreads, 0, s->stream>>>(v, units, q, s->d_partials);
-    else k_reduce_c64<OP_SUM><<<d.reduce_blocks, kReduceThreads, 0, s->stream>>>(v, units, q, s->d_partials);
-  }
+  auto go = [&](auto opc) {
+    constexpr int OP = decltype(opc)::value;
+    if (c128)
+      k_reduce_c128<OP><<<grid, kReduceThreads, 0, s->stream>>>(
+          (const double2 *)s->vec, work, q, s->d_partials, s->d_count, dst);
+    else
+      k_reduce_c64<OP><<<grid, kReduceThreads, 0, s->stream>>>(
+          (const float4 *)s->vec, work, q, s->d_partials, s->d_count, dst);
+  };
+  if (op == OP_NORM) go(std::integral_constant<int, OP_NORM>());
+  else if (op == OP_MASK) go(std::integral_constant<int, OP_MASK>());
+  else go(std::integral_constant<int, OP_SUM>());
   int rc = launched(s, KC_REDUCE, Ns, "reduce");
-  if (rc) return rc;
-  double *dst = (op == OP_SUM) ? s->d_result + 4 : s->d_result;
-  prof_begin(s);
-  k_finalize<<<1, 32, 0, s->stream>>>(s->d_partials, d.reduce_blocks, dst);
-  rc = launched(s, KC_OTHER, d.reduce_blocks * 32.0, "reduce finalize");
   if (rc || !res) return rc;
-  rc = copy_d2h(s, s->h_result, s->d_result, 8 * sizeof(double), "reduce readback");
-  if (!rc) rc = check_cuda(cudaStreamSynchronize(s->stream), "reduce sync");
+  rc = wait_result(s, 4 * sizeof(double), "reduce sync");
   if (rc) return rc;
-  for (int i = 0; i < nres; i++) res[i] = s->h_result[(op == OP_SUM ? 4 : 0) + i];
+  for (int i = 0; i < nres; i++) res[i] = s->h_result[i];
   return QCS_CUDA_OK;
 }
 
@@ -471,16 +521,12 @@ int diffusion(qcs_cuda_state *s) {
   double inv_n = ldexp(1.0, -s->n);
   prof_begin(s);
   if (s->prec == QCS_CUDA_C128)
-    k_diffuse_c128<<<d.reduce_blocks, kReduceThreads, 0, s->stream>>>(
-        (double2 *)s->vec, s->size, s->d_result + 4, inv_n, s->d_partials);
+    k_diffuse_c128<<<reduce_grid(s, s->size), kReduceThreads, 0, s->stream>>>(
+        (double2 *)s->vec, s->size, s->d_result + 4, inv_n, s->d_partials, s->d_count);
   else
-    k_diffuse_c64<<<d.reduce_blocks, kReduceThreads, 0, s->stream>>>(
-        (float4 *)s->vec, s->size / 2, s->d_result + 4, inv_n, s->d_partials);
+    k_diffuse_c64<<<reduce_grid(s, s->size / 2), kReduceThreads, 0, s->stream>>>(
+        (float4 *)s->vec, s->size / 2, s->d_result + 4, inv_n, s->d_partials, s->d_count);
   rc = launched(s, KC_DIFFUSE, 2 * Ns, "diffusion");
-  if (rc) return rc;
-  prof_begin(s);
-  k_finalize<<<1, 32, 0, s->stream>>>(s->d_partials, d.reduce_blocks, s->d_result + 4);
-  rc = launched(s, KC_OTHER, d.reduce_blocks * 32.0, "diffusion finalize");
   if (rc) return rc;
   s->sum_valid = 1;
   return QCS_CUDA_OK;
@@ -500,7 +546,7 @@ int ensure_sum(qcs_cuda_state *s) {
 // combine them (fixed order) into the cached sum.
 int finalize_sum(qcs_cuda_state *s, int nslots) {
   prof_begin(s);
-  k_finalize<<<1, 32, 0, s->stream>>>(s->d_partials, nslots, s->d_result + 4);
+  k_finalize<<<1, kReduceThreads, 0, s->stream>>>(s->d_partials, nslots, s->d_result + 4);
   int rc = launched(s, KC_OTHER, nslots * 32.0, "sum finalize");
   if (!rc) s->sum_valid = 1;
   return rc;
@@ -568,10 +614,10 @@ int qcs_cuda_measure(qcs_cuda_state *s, int qubit, double random_val, int *outco
   double inv = do_scale ? 1.0 / sqrt(kept) : 1.0;
   prof_begin(s);
   if (s->prec == QCS_CUDA_C128)
-    k_collapse_c128<<<s->dev.reduce_blocks, kReduceThreads, 0, s->stream>>>(
+    k_collapse_c128<<<reduce_grid(s, s->size), kReduceThreads, 0, s->stream>>>(
         (double2 *)s->vec, s->size, qubit, o, inv, do_scale);
   else
-    k_collapse_c64<<<s->dev.reduce_blocks, kReduceThreads, 0, s->stream>>>(
+    k_collapse_c64<<<reduce_grid(s, s->size / 2), kReduceThreads, 0, s->stream>>>(
         (float4 *)s->vec, s->size / 2, qubit, o, (float)inv, do_scale);
   invalidate_sum(s);
   rc = launched(s, KC_COLLAPSE, 1.5 * s->size * (s->prec == QCS_CUDA_C128 ? 16 : 8),
@@ -606,25 +652,18 @@ int qcs_cuda_probability(qcs_cuda_state *s, long long index, double *p) {
 int qcs_cuda_argmax(qcs_cuda_state *s, long long *index, double *prob) {
   QCS_CHECK_STATE(s);
   if (!index) return set_error(QCS_CUDA_EINVAL, "null out");
-  const DeviceInfo &d = s->dev;
+  const bool pairs = s->prec == QCS_CUDA_C64;  // n >= 1: at least one pair
+  const int grid = reduce_grid(s, pairs ? s->size / 2 : s->size);
   prof_begin(s);
-  if (s->prec == QCS_CUDA_C128)
-    k_argmax<double2, double><<<d.reduce_blocks, kReduceThreads, 0, s->stream>>>(
-        (const double2 *)s->vec, s->size, s->d_partials);
-  else if (s->size >= 2)
-    k_argmax_c64<<<d.reduce_blocks, kReduceThreads, 0, s->stream>>>(
-        (const float4 *)s->vec, s->size / 2, s->d_partials);
+  if (pairs)
+    k_argmax_c64<<<grid, kReduceThreads, 0, s->stream>>>(
+        (const float4 *)s->vec, s->size / 2, s->d_partials, s->d_count, s->h_result_dev);
   else
-    k_argmax<float2, float><<<d.reduce_blocks, kReduceThreads, 0, s->stream>>>(
-        (const float2 *)s->vec, s->size, s->d_partials);
+    k_argmax<double2, double><<<grid, kReduceThreads, 0, s->stream>>>(
+        (const double2 *)s->vec, s->size, s->d_partials, s->d_count, s->h_result_dev);
   int rc = launched(s, KC_REDUCE, (double)s->size * (s->prec == QCS_CUDA_C128 ? 16 : 8),
                     "argmax");
-  if (rc) return rc;
-  prof_begin(s);
-  k_argmax_finalize<<<1, 32, 0, s->stream>>>(s->d_partials, d.reduce_blocks, s->d_result);
-  rc = launched(s, KC_OTHER, d.reduce_blocks * 32.0, "argmax finalize");
-  if (!rc) rc = copy_d2h(s, s->h_result, s->d_result, 2 * sizeof(double), "argmax readback");
-  if (!rc) rc = check_cuda(cudaStreamSynchronize(s->stream), "argmax sync");
+  if (!rc) rc = wait_result(s, 2 * sizeof(double), "argmax sync");
   if (rc) return rc;
   *index = (long long)s->h_result[1];
   if (prob) return qcs_cuda_probability(s, *index, prob);
@@ -649,35 +688,30 @@ int qcs_cuda_sample(qcs_cuda_state *s, const double *random_vals, int shots,
   prof_begin(s);
   if (s->prec == QCS_CUDA_C128)
     k_smp_tile_sums<double2><<<G, kSampleThreads, 0, s->stream>>>(
-        (const double2 *)s->vec, tile, s->n_tiles, per, in, boff);
+        (const double2 *)s->vec, tile, s->n_tiles, per, in, boff, s->d_count);
   else
     k_smp_tile_sums<float2><<<G, kSampleThreads, 0, s->stream>>>(
-        (const float2 *)s->vec, tile, s->n_tiles, per, in, boff);
+        (const float2 *)s->vec, tile, s->n_tiles, per, in, boff, s->d_count);
   rc = launched(s, KC_SAMPLE, s->size * sb, "sample tile sums");
   if (rc) return rc;
-  prof_begin(s);
-  k_smp_prefix<<<1, 1024, 0, s->stream>>>(boff, G);
-  rc = launched(s, KC_SAMPLE, 16.0 * G, "sample prefix");
-  if (rc) return rc;
+  // the kernel reads the draws from, and writes the samples to, pinned host
+  // memory: 8 bytes a shot beside the 64 KB it scans for it
   memcpy(s->h_draws, random_vals, (size_t)shots * sizeof(double));
-  rc = copy_h2d(s, s->d_draws, s->h_draws, (size_t)shots * sizeof(double), "sample draws upload");
-  if (rc) return rc;
+  s->h2d_bytes += (long long)((size_t)shots * sizeof(double));
   int threads = 256;
   int blocks = (int)(((i64)shots * 32 + threads - 1) / threads);
   if (blocks > d.num_sms * 16) blocks = d.num_sms * 16;
   prof_begin(s);
   if (s->prec == QCS_CUDA_C128)
     k_smp_sample<double2><<<blocks, threads, 0, s->stream>>>(
-        (const double2 *)s->vec, tile, s->n_tiles, per, in, boff, G, s->d_draws, shots,
-        s->d_samples);
+        (const double2 *)s->vec, tile, s->n_tiles, per, in, boff, G, s->h_draws_dev, shots,
+        s->h_samples_dev);
   else
     k_smp_sample<float2><<<blocks, threads, 0, s->stream>>>(
-        (const float2 *)s->vec, tile, s->n_tiles, per, in, boff, G, s->d_draws, shots,
-        s->d_samples);
+        (const float2 *)s->vec, tile, s->n_tiles, per, in, boff, G, s->h_draws_dev, shots,
+        s->h_samples_dev);
   rc = launched(s, KC_SAMPLE, (double)shots * tile * sb, "sample");
-  if (!rc) rc = copy_d2h(s, s->h_samples, s->d_samples, (size_t)shots * sizeof(i64),
-                         "sample readback");
-  if (!rc) rc = check_cuda(cudaStreamSynchronize(s->stream), "sample sync");
+  if (!rc) rc = wait_result(s, (size_t)shots * sizeof(i64), "sample sync");
   if (rc) return rc;
   memcpy(out_index, s->h_samples, (size_t)shots * sizeof(i64));
   return QCS_CUDA_OK;

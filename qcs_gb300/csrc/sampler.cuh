@@ -100,43 +100,15 @@ __device__ __forceinline__ double smp_small_tile_mass<float2>(const float2 *v, i
   return (double)a;
 }
 
-// Tile masses: block b takes tiles [b per, (b + 1) per) one after another
-// (FP64 across its threads in a fixed order), writes each tile's exclusive
-// prefix within the range to in[t] and the range total to bsum[b].
-template <typename C>
-__global__ void __launch_bounds__(kSampleThreads)
-    k_smp_tile_sums(const C *v, i64 tile, i64 n_tiles, i64 per, double *in, double *bsum) {
-  __shared__ double part[kSampleThreads / 32];
-  const i64 t0 = (i64)blockIdx.x * per;
-  const i64 t1 = t0 + per < n_tiles ? t0 + per : n_tiles;
-  double run = 0.0;  // thread 0: the range's running total
-  for (i64 t = t0; t < t1; t++) {
-    const double a = tile == kSampleTile ? smp_full_tile_mass<C>(v, t * kSampleTile)
-                                         : smp_warp_sum(smp_small_tile_mass<C>(v, tile));
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = a;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      double b = threadIdx.x < kSampleThreads / 32 ? part[threadIdx.x] : 0.0;
-      b = smp_warp_sum(b);
-      if (threadIdx.x == 0) {
-        in[t] = run;
-        run += b;
-      }
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) bsum[blockIdx.x] = run;
-}
-
 // In-place exclusive prefix of x[0 .. n) in FP64, the total into x[n] (the
 // range totals bsum[0 .. G) into the offsets boff[0 .. G]): one
-// block of 1024 threads walks x in chunks of 8192 entries with a running
+// block walks x in chunks of 8 entries a thread with a running
 // carry.  Thread t owns the 8 adjacent entries 8t .. 8t+7 of a chunk (moved
 // in 16-byte pieces, so a warp reads and writes 2 KB contiguous); the
-// block scans the threads' totals (warp shuffles, then the 32 warp totals),
+// block scans the threads' totals (warp shuffles, then the warp totals),
 // and each thread adds its entries one after another to its offset.  The
 // order of the additions is fixed, so the prefix is deterministic.
-__global__ void __launch_bounds__(1024) k_smp_prefix(double *x, i64 n) {
+__device__ void smp_prefix(double *x, i64 n) {
   constexpr int E = 8;
   __shared__ double wtot[32];
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
@@ -148,13 +120,13 @@ __global__ void __launch_bounds__(1024) k_smp_prefix(double *x, i64 n) {
       const double2 *p = reinterpret_cast<const double2 *>(x + i0);
 #pragma unroll
       for (int k = 0; k < E / 2; k++) {
-        const double2 d = p[k];
+        const double2 d = __ldcg(p + k);
         v[2 * k] = d.x;
         v[2 * k + 1] = d.y;
       }
     } else {
 #pragma unroll
-      for (int k = 0; k < E; k++) v[k] = i0 + k < n ? x[i0 + k] : 0.0;
+      for (int k = 0; k < E; k++) v[k] = i0 + k < n ? __ldcg(x + i0 + k) : 0.0;
     }
     double s = 0.0;
 #pragma unroll
@@ -170,7 +142,7 @@ __global__ void __launch_bounds__(1024) k_smp_prefix(double *x, i64 n) {
     if (lane == 31) wtot[w] = incl;
     __syncthreads();
     if (w == 0) {  // inclusive scan of the warp totals
-      double wt = lane < (int)(blockDim.x >> 5) ? wtot[lane] : 0.0;
+      double wt = lane < (int)(blockDim.x >> 5) ? wtot[lane] : 0.0;  // fewer warps: zeros
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const double y = __shfl_up_sync(0xffffffffu, wt, o);
@@ -201,17 +173,81 @@ __global__ void __launch_bounds__(1024) k_smp_prefix(double *x, i64 n) {
   if (t == 0) x[n] = carry;
 }
 
+// Tile masses: block b takes tiles [b per, (b + 1) per) one after another
+// (FP64 across its threads in a fixed order), writes each tile's exclusive
+// prefix within the range to in[t] and the range total to bsum[b].  With a
+// `count` (zero before and after), the block that finishes last turns the
+// totals into the offsets; without, k_smp_prefix does.
+template <typename C>
+__global__ void __launch_bounds__(kSampleThreads)
+    k_smp_tile_sums(const C *v, i64 tile, i64 n_tiles, i64 per, double *in, double *bsum,
+                    unsigned *count) {
+  __shared__ double part[kSampleThreads / 32];
+  const i64 t0 = (i64)blockIdx.x * per;
+  const i64 t1 = t0 + per < n_tiles ? t0 + per : n_tiles;
+  double run = 0.0;  // thread 0: the range's running total
+  for (i64 t = t0; t < t1; t++) {
+    const double a = tile == kSampleTile ? smp_full_tile_mass<C>(v, t * kSampleTile)
+                                         : smp_warp_sum(smp_small_tile_mass<C>(v, tile));
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = a;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      double b = threadIdx.x < kSampleThreads / 32 ? part[threadIdx.x] : 0.0;
+      b = smp_warp_sum(b);
+      if (threadIdx.x == 0) {
+        in[t] = run;
+        run += b;
+      }
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) bsum[blockIdx.x] = run;
+  if (!count) return;
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(count, 1u) == gridDim.x - 1;
+    if (last) {
+      *count = 0;
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  if (last) smp_prefix(bsum, gridDim.x);
+}
+
+__global__ void __launch_bounds__(1024) k_smp_prefix(double *x, i64 n) { smp_prefix(x, n); }
+
 // One warp per draw r: the tile whose inclusive prefix first exceeds r (a
 // binary search over the range offsets, then one over the tiles of that
-// range), then an FP64 scan of that tile 32 amplitudes at a time (four
-// groups' loads in flight together).  Result: the first index with
-// r < running sum (strict, as src/qcs.c:600), or -1 when r is not below the
-// total.  When r falls in a tile by its total but not by the element scan
-// (rounding at the tile's upper edge), the tile's last nonzero index.
+// range), then an FP64 scan of that tile 128 amplitudes at a time, four
+// adjacent ones a lane.  Result: the first index with r < running sum
+// (strict, as src/qcs.c:600), or -1 when r is not below the total.  When r
+// falls in a tile by its total but not by the element scan (rounding at the
+// tile's upper edge), the tile's last nonzero index.
+// The FP64 pipe bounds the scan (2 lanes an SM and clock): four amplitudes a
+// lane share one warp scan and one comparison, 19 FP64 instructions for 128
+// amplitudes where a scan of each 32 took 44.
+template <typename C>
+__device__ __forceinline__ void smp_load4(const C *v, C (&x)[4]);
+template <>
+__device__ __forceinline__ void smp_load4<float2>(const float2 *v, float2 (&x)[4]) {
+  const float4 a = reinterpret_cast<const float4 *>(v)[0];
+  const float4 b = reinterpret_cast<const float4 *>(v)[1];
+  x[0] = make_float2(a.x, a.y);
+  x[1] = make_float2(a.z, a.w);
+  x[2] = make_float2(b.x, b.y);
+  x[3] = make_float2(b.z, b.w);
+}
+template <>
+__device__ __forceinline__ void smp_load4<double2>(const double2 *v, double2 (&x)[4]) {
+#pragma unroll
+  for (int k = 0; k < 4; k++) x[k] = v[k];
+}
+
 template <typename C>
 __global__ void k_smp_sample(const C *v, i64 tile, i64 n_tiles, i64 per, const double *in,
                              const double *boff, int G, const double *draws, int shots, i64 *out) {
-  constexpr int G4 = 4;  // 32-amplitude groups loaded together
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -236,34 +272,53 @@ __global__ void k_smp_sample(const C *v, i64 tile, i64 n_tiles, i64 per, const d
         else lo = mid + 1;
       }
       double cum = off + in[lo];
-      i64 last_nonzero = lo * tile;
-      const i64 end = (lo + 1) * tile;
-      for (i64 base = lo * tile; base < end && result < 0; base += 32 * G4) {
-        double p[G4];
+      const i64 first = lo * tile, end = first + tile;
+      C next[4];  // the group after this one, in flight
+      auto load = [&](i64 base, C (&x)[4]) {
+        const i64 i = base + 4 * lane;
+        if (i + 4 <= end) {
+          smp_load4(v + i, x);
+        } else {
 #pragma unroll
-        for (int k = 0; k < G4; k++) {
-          const i64 i = base + 32 * k + lane;
-          p[k] = i < end ? smp_prob(v[i]) : 0.0;
+          for (int k = 0; k < 4; k++) x[k] = i + k < end ? v[i + k] : make_c<C>(0.0, 0.0);
         }
+      };
+      load(first, next);
+      for (i64 base = first; base < end && result < 0; base += 128) {
+        C x[4];
 #pragma unroll
-        for (int k = 0; k < G4; k++) {
-          const i64 gb = base + 32 * k;
-          if (result >= 0 || gb >= end) break;  // warp-uniform
-          double incl = p[k];
+        for (int k = 0; k < 4; k++) x[k] = next[k];
+        if (base + 128 < end) load(base + 128, next);
+        double sum[4];  // running sums of the lane's amplitudes
+        sum[0] = smp_prob(x[0]);
 #pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const double y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-          }
-          const bool valid = gb + lane < end;
-          const unsigned hit = __ballot_sync(0xffffffffu, valid && r < cum + incl);
-          const unsigned nz = __ballot_sync(0xffffffffu, valid && p[k] > 0.0);
-          if (hit) result = gb + __ffs(hit) - 1;
-          else if (nz) last_nonzero = gb + 31 - __clz(nz);
-          cum += __shfl_sync(0xffffffffu, incl, 31);
+        for (int k = 1; k < 4; k++) sum[k] = sum[k - 1] + smp_prob(x[k]);
+        double incl = sum[3];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const double y = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += y;
+        }
+        const unsigned hit = __ballot_sync(0xffffffffu, r < cum + incl);
+        if (hit) {  // in the first lane whose running sum exceeds r
+          const int at = __ffs(hit) - 1;
+          double before = __shfl_up_sync(0xffffffffu, incl, 1);
+          before = lane == 0 ? cum : cum + before;
+          int k = 0;
+          while (k < 3 && !(r < before + sum[k])) k++;
+          while (k > 0 && sum[k] == sum[k - 1]) k--;  // not one of no mass
+          result = base + 4 * at + __shfl_sync(0xffffffffu, k, at);
+        }
+        cum += __shfl_sync(0xffffffffu, incl, 31);
+      }
+      if (result < 0) {  // the tile's last nonzero amplitude
+        result = first;
+        for (i64 base = first; base < end; base += 32) {
+          const bool nz = base + lane < end && smp_prob(v[base + lane]) > 0.0;
+          const unsigned m = __ballot_sync(0xffffffffu, nz);
+          if (m) result = base + 31 - __clz(m);
         }
       }
-      if (result < 0) result = last_nonzero;
     }
     if (lane == 0) out[s] = result;
   }

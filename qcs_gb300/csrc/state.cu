@@ -86,6 +86,19 @@ __global__ void k_set_one(C *v, i64 index) {
   v[index] = make_c<C>(1.0, 0.0);
 }
 
+// |index> in one kernel: 16-byte units of zeros but for the one that holds
+// the index.
+template <typename C>
+__global__ void __launch_bounds__(kSweepThreads) k_basis(float4 *v, i64 units, i64 index) {
+  constexpr int UNIT = 16 / sizeof(C);
+  const i64 nthr = (i64)gridDim.x * blockDim.x;
+  for (i64 u = (i64)blockIdx.x * blockDim.x + threadIdx.x; u < units; u += nthr) {
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (u == index / UNIT) reinterpret_cast<C *>(&x)[index % UNIT] = make_c<C>(1.0, 0.0);
+    v[u] = x;
+  }
+}
+
 static int dmalloc(void **p, size_t bytes, const char *what) {
   *p = nullptr;
   if (inject_alloc_failure())
@@ -93,9 +106,23 @@ static int dmalloc(void **p, size_t bytes, const char *what) {
   return check_cuda(cudaMalloc(p, bytes), what);
 }
 
+// Pinned host memory that kernels read and write, and its device address.
+static int host_buffer(void **host, void **dev, size_t bytes, const char *what) {
+  *host = *dev = nullptr;
+  if (inject_alloc_failure())
+    return set_error(QCS_CUDA_ENOMEM, "%s: injected allocation failure", what);
+  int rc = check_cuda(cudaHostAlloc(host, bytes, cudaHostAllocMapped), what);
+  return rc ? rc : check_cuda(cudaHostGetDevicePointer(dev, *host, 0), what);
+}
+
 static size_t amp_bytes(const qcs_cuda_state *s) {
   return s->prec == QCS_CUDA_C128 ? 16 : 8;
 }
+
+// A state up to this size is reset by k_basis, one launch; beyond it the two
+// operations of a memset and a store cost nothing beside the bytes, and the
+// copy engine's fill needs no tuning.
+constexpr size_t kBasisKernelBytes = 16u << 20;
 
 static int launch_set_one(qcs_cuda_state *s, void *buf, i64 index) {
   prof_begin(s);
@@ -212,8 +239,7 @@ static void free_state(qcs_cuda_state *s) {
   cudaFree(s->d_partials);
   cudaFree(s->d_result);
   cudaFree(s->d_tile_prefix);
-  cudaFree(s->d_draws);
-  cudaFree(s->d_samples);
+  cudaFree(s->d_count);
   if (s->h_result) cudaFreeHost(s->h_result);
   if (s->h_draws) cudaFreeHost(s->h_draws);
   if (s->h_samples) cudaFreeHost(s->h_samples);
@@ -235,24 +261,16 @@ int ensure_sample_scratch(qcs_cuda_state *s, int shots) {
   }
   if (shots > s->sample_cap) {
     int cap = shots < 1024 ? 1024 : shots;
-    cudaFree(s->d_draws);
-    cudaFree(s->d_samples);
     if (s->h_draws) cudaFreeHost(s->h_draws);
     if (s->h_samples) cudaFreeHost(s->h_samples);
-    s->d_draws = nullptr;
-    s->d_samples = nullptr;
     s->h_draws = nullptr;
     s->h_samples = nullptr;
     s->sample_cap = 0;
-    rc = dmalloc((void **)&s->d_draws, (size_t)cap * sizeof(double), "cudaMalloc(draws)");
+    rc = host_buffer((void **)&s->h_draws, (void **)&s->h_draws_dev, (size_t)cap * sizeof(double),
+                     "cudaMallocHost(draws)");
     if (rc) return rc;
-    rc = dmalloc((void **)&s->d_samples, (size_t)cap * sizeof(i64), "cudaMalloc(samples)");
-    if (rc) return rc;
-    rc = check_cuda(cudaMallocHost((void **)&s->h_draws, (size_t)cap * sizeof(double)),
-                    "cudaMallocHost(draws)");
-    if (rc) return rc;
-    rc = check_cuda(cudaMallocHost((void **)&s->h_samples, (size_t)cap * sizeof(i64)),
-                    "cudaMallocHost(samples)");
+    rc = host_buffer((void **)&s->h_samples, (void **)&s->h_samples_dev,
+                     (size_t)cap * sizeof(i64), "cudaMallocHost(samples)");
     if (rc) return rc;
     s->sample_cap = cap;
   }
@@ -347,8 +365,11 @@ int qcs_cuda_state_create(int num_qubits, int precision, int semantics,
   if (!rc) rc = dmalloc((void **)&s->d_result, 8 * sizeof(double), "cudaMalloc(result)");
   if (!rc) rc = dmalloc((void **)&s->d_err, sizeof(int), "cudaMalloc(error flag)");
   if (!rc) rc = check_cuda(cudaMemsetAsync(s->d_err, 0, sizeof(int), s->stream), "cudaMemset(err)");
-  if (!rc) rc = check_cuda(cudaMallocHost((void **)&s->h_result, 8 * sizeof(double)),
-                           "cudaMallocHost(result)");
+  if (!rc) rc = host_buffer((void **)&s->h_result, (void **)&s->h_result_dev, 8 * sizeof(double),
+                            "cudaMallocHost(result)");
+  if (!rc) rc = dmalloc((void **)&s->d_count, sizeof(unsigned), "cudaMalloc(block counter)");
+  if (!rc) rc = check_cuda(cudaMemsetAsync(s->d_count, 0, sizeof(unsigned), s->stream),
+                           "cudaMemset(block counter)");
   if (!rc) rc = check_cuda(cudaMemsetAsync(s->vec, 0, bytes, s->stream), "cudaMemset(state)");
   if (!rc && s->scratch)
     rc = check_cuda(cudaMemsetAsync(s->scratch, 0, bytes, s->stream), "cudaMemset(scratch)");
@@ -416,10 +437,20 @@ int qcs_cuda_set_basis(qcs_cuda_state *s, long long index) {
   QCS_CHECK_STATE(s);
   if (index < 0 || index >= s->size)
     return set_error(QCS_CUDA_EINVAL, "basis index %lld outside [0, %lld)", index, s->size);
-  int rc = check_cuda(cudaMemsetAsync(s->vec, 0, (size_t)s->size * amp_bytes(s), s->stream),
-                      "cudaMemset(state)");
-  if (rc) return rc;
+  const size_t bytes = (size_t)s->size * amp_bytes(s);
   invalidate_sum(s);
+  if (bytes <= kBasisKernelBytes) {
+    const i64 units = (i64)(bytes / 16);
+    const int grid = grid_for(units, kSweepThreads, s->dev, 8);
+    prof_begin(s);
+    if (s->prec == QCS_CUDA_C128)
+      k_basis<double2><<<grid, kSweepThreads, 0, s->stream>>>((float4 *)s->vec, units, index);
+    else
+      k_basis<float2><<<grid, kSweepThreads, 0, s->stream>>>((float4 *)s->vec, units, index);
+    return launched(s, KC_OTHER, (double)bytes, "set_basis");
+  }
+  int rc = check_cuda(cudaMemsetAsync(s->vec, 0, bytes, s->stream), "cudaMemset(state)");
+  if (rc) return rc;
   return launch_set_one(s, s->vec, index);
 }
 
