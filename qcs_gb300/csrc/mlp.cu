@@ -2,13 +2,18 @@
 // GPU.
 //
 // Network: F input features -> 64 -> 64 -> 64 (ReLU) -> 1 (linear), FP32,
-// trained on squared error of log2(kernel milliseconds).  A CTA takes 64
-// samples; the three weight matrices stay in shared memory and every layer is
-// a small tiled product (256 threads, 16 outputs each).  The backward pass
-// writes each CTA's gradient sum to its own slot and a second kernel adds the
-// slots in a fixed order, so gradients are deterministic.  There is nothing
+// trained on squared error of log2(kernel milliseconds).  There is nothing
 // like it in the reference (its only optimisation is the gate-history
 // peephole of qc_optimize, src/qcs.c:650-698).
+//
+// A training step is two kernels.  k_mlp_rows takes 8 rows a CTA forward and
+// back (a batch of 256 rows is 32 CTAs) and leaves every layer's activations
+// and errors; k_mlp_grad forms the weight gradients, 8 weight rows a CTA, and
+// takes the Adam step in place.  A gradient is summed over the rows in slots
+// of 64, each in row order, and over the slots in order, so it does not
+// depend on how the work is cut.  Latency bounds both: 64 steps on 256 rows
+// take 1.3 ms, where one CTA per 64 rows for everything, a kernel for the sum
+// of the slots and one for Adam took 21.7 ms.
 #include <atomic>
 #include <math.h>
 #include <string.h>
@@ -20,8 +25,15 @@
 
 namespace qcs {
 
-constexpr int kMlpRows = 64;      // samples per CTA
-constexpr int kMlpThreads = 256;
+constexpr int kMlpSlot = 64;         // rows of a gradient slot
+constexpr int kMlpRows = 8;          // rows per CTA, forward and back
+constexpr int kMlpRowThreads = 128;  // a row's 64 units on 16 threads, 4 each
+constexpr int kMlpGradRows = 8;      // weight rows per CTA of k_mlp_grad
+constexpr int kMlpGradThreads = 16 * kMlpGradRows;
+constexpr int kMlpPitch = 68;        // floats per 64-wide row in shared memory
+// Batches up to this size go through k_mlp_grad in one piece; larger ones are
+// cut into slots, summed afterwards.
+constexpr int kMlpDirectRows = 1024;
 
 struct MlpShape {
   int F;
@@ -39,141 +51,328 @@ struct MlpShape {
   }
 };
 
-// out[s][j] = act(b[j] + sum_i in[s][i] * w[i][j]) for s < rows, j < 64;
-// in is [rows][K] with row stride ld_in.
-__device__ __forceinline__ void layer(const float *in, int ld_in, int K, const float *w,
-                                      const float *b, float *out, bool relu) {
-  for (int e = threadIdx.x; e < kMlpRows * kMlpHidden; e += kMlpThreads) {
-    const int s = e / kMlpHidden, j = e % kMlpHidden;
-    float acc = b[j];
-    for (int i = 0; i < K; i++) acc += in[s * ld_in + i] * w[i * kMlpHidden + j];
-    out[e] = relu ? fmaxf(acc, 0.f) : acc;
-  }
+// What a row leaves for the gradients: h1, h2, h3, then dL/d(pre-activation)
+// of layers 1, 2, 3 (64 each), then the output's error.
+constexpr int kMlpActs = 6 * kMlpHidden + 1;
+struct MlpActs {
+  float *p;
+  size_t rows;
+  __host__ __device__ float *h(int l) const { return p + (size_t)l * rows * kMlpHidden; }
+  __host__ __device__ float *g(int l) const { return p + (size_t)(3 + l) * rows * kMlpHidden; }
+  __host__ __device__ float *d() const { return p + (size_t)6 * rows * kMlpHidden; }
+};
+
+// Asynchronous copies to shared memory (16 or 4 bytes): a CTA has its whole
+// working set in flight at once, where loops of plain loads waited on one L2
+// access after another (k_mlp_rows 25
+// us instead of 8 on 256 rows, k_mlp_grad 34 instead of 11).
+__device__ __forceinline__ void copy16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
+}
+__device__ __forceinline__ void copy4(void *dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;"); }
+template <int PENDING>
+__device__ __forceinline__ void copy_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING));
 }
 
-// Forward (and, with y != nullptr, backward) for samples [r0, r0 + 64).
-__global__ void __launch_bounds__(kMlpThreads)
-    k_mlp(const float *params, int F, const float *X, const float *Y, int n, float inv_n,
-          float *grad_slots, double *loss_slots, float *pred) {
-  extern __shared__ float sm[];
+// Four outputs j .. j+3 of one row: act(b[j] + sum_i in[i] * w[i][j]), the
+// sum in the order of i.
+__device__ __forceinline__ float4 mlp_layer(const float *in, int K, const float *w, int ldw,
+                                            const float *b, int j, bool relu) {
+  float4 acc = *reinterpret_cast<const float4 *>(b + j);
+#pragma unroll 16
+  for (int i = 0; i < K; i++) {
+    const float x = in[i];
+    const float4 v = *reinterpret_cast<const float4 *>(w + i * ldw + j);
+    acc.x = fmaf(x, v.x, acc.x);
+    acc.y = fmaf(x, v.y, acc.y);
+    acc.z = fmaf(x, v.z, acc.z);
+    acc.w = fmaf(x, v.w, acc.w);
+  }
+  if (relu) {
+    acc.x = fmaxf(acc.x, 0.f);
+    acc.y = fmaxf(acc.y, 0.f);
+    acc.z = fmaxf(acc.z, 0.f);
+    acc.w = fmaxf(acc.w, 0.f);
+  }
+  return acc;
+}
+
+// Rows [8 b, 8 b + 8) of a batch: forward; with Y the squared error and, with
+// acts.p, back to every layer's pre-activations.
+__global__ void __launch_bounds__(kMlpRowThreads)
+    k_mlp_rows(const float *params, int F, const float *X, const float *Y, int n, float inv_n,
+               MlpActs acts, double *loss_rows, float *pred) {
+  extern __shared__ __align__(16) float sm[];
+  constexpr int H = kMlpHidden, LD = kMlpPitch;
   const MlpShape S(F);
-  float *w = sm;                                  // all parameters
-  float *x = w + S.count;                         // [64][F]
-  float *h1 = x + kMlpRows * F;                   // [64][64] activations
-  float *h2 = h1 + kMlpRows * kMlpHidden;
-  float *h3 = h2 + kMlpRows * kMlpHidden;
-  float *d = h3 + kMlpRows * kMlpHidden;          // [64] output error
-  float *g = d + kMlpRows;                        // [64][64] back-propagated error
-  float *g2 = g + kMlpRows * kMlpHidden;
-  __shared__ double lsum[kMlpThreads / 32];
+  float *w1 = sm;               // [F][LD]
+  float *w2 = w1 + F * LD;      // [H][LD]
+  float *w3 = w2 + H * LD;
+  float *b1 = w3 + H * LD;      // [H] each
+  float *b2 = b1 + H;
+  float *b3 = b2 + H;
+  float *w4 = b3 + H;
+  float *x = w4 + H;            // [rows][F]
+  float *h1 = x + kMlpRows * ((F + 3) & ~3);  // [rows][LD]
+  float *h2 = h1 + kMlpRows * LD;
+  float *h3 = h2 + kMlpRows * LD;
+  float *g = h3 + kMlpRows * LD;
+  __shared__ float err[kMlpRows];
+  const int tid = threadIdx.x;
   const int r0 = blockIdx.x * kMlpRows;
-  const int rows = n - r0 < kMlpRows ? n - r0 : kMlpRows;
-  for (int i = threadIdx.x; i < S.count; i += kMlpThreads) w[i] = params[i];
-  for (int e = threadIdx.x; e < kMlpRows * F; e += kMlpThreads) {
-    const int s = e / F;
-    x[e] = s < rows ? X[(size_t)(r0 + s) * F + e % F] : 0.f;
+  const int s = tid >> 4, j = 4 * (tid & 15), row = r0 + s;
+  for (int e = tid; e < (F + 2 * H) * (H / 4); e += kMlpRowThreads) {
+    const int i = e / (H / 4), c = 4 * (e % (H / 4));  // rows of w1, w2, w3
+    const int off = i < F ? S.off_w1 + i * H : i < F + H ? S.off_w2 + (i - F) * H
+                                                         : S.off_w3 + (i - F - H) * H;
+    copy16(w1 + i * LD + c, params + off + c);
   }
+  for (int e = tid; e < 4 * H / 4; e += kMlpRowThreads) {  // b1, b2, b3, w4
+    const int k = e / (H / 4), c = 4 * (e % (H / 4));
+    const int off = k == 0 ? S.off_b1 : k == 1 ? S.off_b2 : k == 2 ? S.off_b3 : S.off_w4;
+    copy16(b1 + k * H + c, params + off + c);
+  }
+  for (int e = tid; e < kMlpRows * F; e += kMlpRowThreads) {
+    if (r0 + e / F < n) copy4(x + e, X + (size_t)r0 * F + e);
+    else x[e] = 0.f;
+  }
+  const float b4 = params[S.off_b4];
+  const float yr = Y && row < n ? Y[row] : 0.f;
+  copy_commit();
+  copy_wait<0>();
   __syncthreads();
-  layer(x, F, F, w + S.off_w1, w + S.off_b1, h1, true);
+  auto put = [&](float *m, float4 v) { *reinterpret_cast<float4 *>(m + s * LD + j) = v; };
+  put(h1, mlp_layer(x + s * F, F, w1, LD, b1, j, true));
   __syncthreads();
-  layer(h1, kMlpHidden, kMlpHidden, w + S.off_w2, w + S.off_b2, h2, true);
+  put(h2, mlp_layer(h1 + s * LD, H, w2, LD, b2, j, true));
   __syncthreads();
-  layer(h2, kMlpHidden, kMlpHidden, w + S.off_w3, w + S.off_b3, h3, true);
+  put(h3, mlp_layer(h2 + s * LD, H, w3, LD, b3, j, true));
   __syncthreads();
-  if (threadIdx.x < kMlpRows) {
-    const int s = threadIdx.x;
-    float o = w[S.off_b4];
-    for (int i = 0; i < kMlpHidden; i++) o += h3[s * kMlpHidden + i] * w[S.off_w4 + i];
-    if (pred && s < rows) pred[r0 + s] = o;
+  if ((tid & 15) == 0) {
+    float o = b4;
+#pragma unroll 16
+    for (int i = 0; i < H; i++) o = fmaf(h3[s * LD + i], w4[i], o);
+    const bool in = row < n;
+    if (pred && in) pred[row] = o;
+    const float off = Y && in ? o - yr : 0.f;
     // dLoss/dout for loss = (1/n) sum (out - y)^2
-    d[s] = (Y && s < rows) ? 2.f * (o - Y[r0 + s]) * inv_n : 0.f;
-    double l = (Y && s < rows) ? (double)(o - Y[r0 + s]) * (o - Y[r0 + s]) : 0.0;
+    err[s] = 2.f * off * inv_n;
+    if (loss_rows && in) loss_rows[row] = (double)off * off;
+  }
+  if (!acts.p) return;
+  __syncthreads();
+  const float d = err[s];
+  const bool in = row < n;
+  auto keep = [&](float *m, float4 v) {
+    if (in) *reinterpret_cast<float4 *>(m + (size_t)row * H + j) = v;
+  };
+  auto at = [&](const float *m) { return *reinterpret_cast<const float4 *>(m + s * LD + j); };
+  keep(acts.h(0), at(h1));
+  keep(acts.h(1), at(h2));
+  keep(acts.h(2), at(h3));
+  if (in && (tid & 15) == 0) acts.d()[row] = d;
+  {  // dL/d(pre-activation 3)
+    const float4 h = at(h3);
+    const float4 v = make_float4(h.x > 0.f ? d * w4[j] : 0.f, h.y > 0.f ? d * w4[j + 1] : 0.f,
+                                 h.z > 0.f ? d * w4[j + 2] : 0.f, h.w > 0.f ? d * w4[j + 3] : 0.f);
+    keep(acts.g(2), v);
+    put(g, v);
+  }
+  __syncthreads();
+  // back through w3, then w2: units u, u + 16, u + 32, u + 48 of the row below,
+  // each a dot product with a row of the weights
+  const int u = tid & 15;
+  for (int L = 1; L >= 0; L--) {
+    const float *w = L == 1 ? w3 : w2, *below = L == 1 ? h2 : h1;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int c = 0; c < H; c += 4) {
+      const float4 e = *reinterpret_cast<const float4 *>(g + s * LD + c);
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
-    if ((threadIdx.x & 31) == 0) lsum[threadIdx.x >> 5] = l;
-  }
-  __syncthreads();
-  if (!Y) return;
-  if (threadIdx.x == 0) loss_slots[blockIdx.x] = lsum[0] + lsum[1];
-  float *gs = grad_slots + (size_t)blockIdx.x * S.count;
-  // ---- output layer
-  for (int i = threadIdx.x; i < kMlpHidden; i += kMlpThreads) {
-    float a = 0.f;
-    for (int s = 0; s < kMlpRows; s++) a += d[s] * h3[s * kMlpHidden + i];
-    gs[S.off_w4 + i] = a;
-  }
-  if (threadIdx.x == 0) {
-    float a = 0.f;
-    for (int s = 0; s < kMlpRows; s++) a += d[s];
-    gs[S.off_b4] = a;
-  }
-  for (int e = threadIdx.x; e < kMlpRows * kMlpHidden; e += kMlpThreads) {
-    const int s = e / kMlpHidden, i = e % kMlpHidden;
-    g[e] = h3[e] > 0.f ? d[s] * w[S.off_w4 + i] : 0.f;  // dL/d(pre-act 3)
-  }
-  __syncthreads();
-  // ---- hidden layers: g holds dL/d(pre-activation) of the layer above
-  const float *acts[3] = {x, h1, h2};
-  const int widths[3] = {F, kMlpHidden, kMlpHidden};
-  const int woff[3] = {S.off_w1, S.off_w2, S.off_w3};
-  const int boff[3] = {S.off_b1, S.off_b2, S.off_b3};
-  float *cur = g, *nxt = g2;
-  for (int L = 2; L >= 0; L--) {
-    const float *a = acts[L];
-    const int K = widths[L];
-    for (int e = threadIdx.x; e < K * kMlpHidden; e += kMlpThreads) {
-      const int i = e / kMlpHidden, j = e % kMlpHidden;
-      float acc = 0.f;
-      for (int s = 0; s < kMlpRows; s++) acc += a[s * K + i] * cur[s * kMlpHidden + j];
-      gs[woff[L] + e] = acc;
-    }
-    for (int j = threadIdx.x; j < kMlpHidden; j += kMlpThreads) {
-      float acc = 0.f;
-      for (int s = 0; s < kMlpRows; s++) acc += cur[s * kMlpHidden + j];
-      gs[boff[L] + j] = acc;
-    }
-    if (L > 0) {
-      const float *wl = w + woff[L];
-      for (int e = threadIdx.x; e < kMlpRows * kMlpHidden; e += kMlpThreads) {
-        const int s = e / kMlpHidden, i = e % kMlpHidden;
-        float acc = 0.f;
-        for (int j = 0; j < kMlpHidden; j++) acc += cur[s * kMlpHidden + j] * wl[i * kMlpHidden + j];
-        nxt[e] = a[e] > 0.f ? acc : 0.f;
+      for (int k = 0; k < 4; k++) {
+        const float4 v = *reinterpret_cast<const float4 *>(w + (u + 16 * k) * LD + c);
+        acc[k] = fmaf(e.x, v.x, acc[k]);
+        acc[k] = fmaf(e.y, v.y, acc[k]);
+        acc[k] = fmaf(e.z, v.z, acc[k]);
+        acc[k] = fmaf(e.w, v.w, acc[k]);
       }
-      __syncthreads();
-      float *t = cur;
-      cur = nxt;
-      nxt = t;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int i = u + 16 * k;
+      const float v = below[s * LD + i] > 0.f ? acc[k] : 0.f;
+      g[s * LD + i] = v;
+      if (in) acts.g(L)[(size_t)row * H + i] = v;
+    }
+    __syncthreads();
+  }
+}
+
+struct MlpAdam {
+  float *params, *m, *v;
+  float lr, b1, b2, c1, c2;
+};
+
+// One Adam step of a parameter from its state (m, v, p).
+__device__ __forceinline__ void adam_step(const MlpAdam &A, int i, float3 mvp, float gp) {
+  const float mp = A.b1 * mvp.x + (1.f - A.b1) * gp;
+  const float vp = A.b2 * mvp.y + (1.f - A.b2) * gp * gp;
+  A.m[i] = mp;
+  A.v[i] = vp;
+  A.params[i] = mvp.z - A.lr * (mp / A.c1) / (sqrtf(vp / A.c2) + 1e-8f);
+}
+__device__ __forceinline__ float3 adam_state(const MlpAdam &A, int i) {
+  return make_float3(A.m[i], A.v[i], A.params[i]);
+}
+
+// Gradients of 8 rows of one layer's weights, its bias being one row more
+// whose input is 1: for weight row i, unit j the sum over the batch of
+// in[s][i] * err[s][j].  blockIdx.x counts the CTAs of layers 1, 2, 3, then
+// one for the output layer, whose weights are one row with the output's error
+// for input and h3 for error.  Rows [64 blockIdx.y ..) with gridDim.y > 1,
+// else all of them.  A gradient goes to out[blockIdx.y * count + p], or into
+// an Adam step (adam.params).
+struct MlpChunk {  // one slot of rows: errors, and inputs of 8 weight rows
+  float err[kMlpSlot][kMlpHidden];
+  float in[kMlpSlot][kMlpGradRows + 1];
+};
+constexpr int kMlpStages = 4;  // chunks in flight
+
+__global__ void __launch_bounds__(kMlpGradThreads)
+    k_mlp_grad(int F, const float *X, int n, MlpActs acts, float *out, MlpAdam adam) {
+  constexpr int H = kMlpHidden;
+  extern __shared__ __align__(16) float sm[];
+  MlpChunk *ring = reinterpret_cast<MlpChunk *>(sm);
+  const MlpShape S(F);
+  const int tid = threadIdx.x, ti = tid >> 4, j = 4 * (tid & 15);
+  int b = blockIdx.x, layer = 0, K = F;
+  while (layer < 3 && b >= (K + kMlpGradRows) / kMlpGradRows) {
+    b -= (K + kMlpGradRows) / kMlpGradRows;  // ceil((K + 1) / 8)
+    layer++;
+    K = H;
+  }
+  const int i0 = b * kMlpGradRows, i = i0 + ti;
+  const bool last = layer == 3;  // the output layer: row 0 alone
+  const float *src = layer == 0 ? X : last ? acts.d() : acts.h(layer - 1);
+  const float *e = last ? acts.h(2) : acts.g(layer);
+  const int r_begin = gridDim.y > 1 ? blockIdx.y * kMlpSlot : 0;
+  const int r_end = gridDim.y > 1 && r_begin + kMlpSlot < n ? r_begin + kMlpSlot : n;
+  const int chunks = (r_end - r_begin + kMlpSlot - 1) / kMlpSlot;
+  auto load = [&](int c) {
+    if (c < chunks) {
+      MlpChunk &M = ring[c % kMlpStages];
+      const int r = r_begin + c * kMlpSlot;
+      const int rows = r_end - r < kMlpSlot ? r_end - r : kMlpSlot;
+      for (int q = tid; q < kMlpSlot * H / 4; q += kMlpGradThreads) {
+        const int s = q / (H / 4), u = 4 * (q % (H / 4));
+        if (s < rows) copy16(&M.err[s][u], e + (size_t)(r + s) * H + u);
+      }
+      for (int q = tid; q < kMlpSlot * kMlpGradRows; q += kMlpGradThreads) {
+        const int s = q / kMlpGradRows, k = q % kMlpGradRows;
+        if (s >= rows) continue;
+        if (last) {
+          if (k == 0) copy4(&M.in[s][0], src + r + s);
+          else M.in[s][k] = 0.f;
+        } else if (i0 + k < K) {
+          copy4(&M.in[s][k], src + (size_t)(r + s) * K + i0 + k);
+        } else {
+          M.in[s][k] = i0 + k == K ? 1.f : 0.f;
+        }
+      }
+    }
+    copy_commit();
+  };
+  for (int c = 0; c < kMlpStages - 1; c++) load(c);
+  const int off_w = layer == 0 ? S.off_w1 : layer == 1 ? S.off_w2 : layer == 2 ? S.off_w3 : S.off_w4;
+  const bool mine = last ? i == 0 : i <= K;  // a layer's bias follows its weights
+  const bool mine4 = last && tid == 0;       // and the output bias
+  const int p = off_w + i * H + j;
+  float3 state[4], state4;  // Adam's state, in flight with the rows
+  if (adam.params && mine)
+#pragma unroll
+    for (int k = 0; k < 4; k++) state[k] = adam_state(adam, p + k);
+  if (adam.params && mine4) state4 = adam_state(adam, S.off_b4);
+  float4 total = make_float4(0.f, 0.f, 0.f, 0.f);
+  float bias4 = 0.f;  // of the output layer
+  for (int c = 0; c < chunks; c++) {
+    copy_wait<kMlpStages - 2>();
+    __syncthreads();  // chunk c is here, and the ring slot of chunk c - 1 is free
+    load(c + kMlpStages - 1);
+    const MlpChunk &M = ring[c % kMlpStages];
+    const int left = r_end - r_begin - c * kMlpSlot;
+    const int rows = left < kMlpSlot ? left : kMlpSlot;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int s = 0; s < rows; s++) {
+      const float x = M.in[s][ti];
+      const float4 v = *reinterpret_cast<const float4 *>(&M.err[s][j]);
+      acc.x = fmaf(x, v.x, acc.x);
+      acc.y = fmaf(x, v.y, acc.y);
+      acc.z = fmaf(x, v.z, acc.z);
+      acc.w = fmaf(x, v.w, acc.w);
+    }
+    total.x += acc.x;
+    total.y += acc.y;
+    total.z += acc.z;
+    total.w += acc.w;
+    if (mine4) {
+      float a = 0.f;
+      for (int s = 0; s < rows; s++) a += M.in[s][0];
+      bias4 += a;
     }
   }
-}
-
-// Sum the per-CTA slots in a fixed order.
-__global__ void k_mlp_reduce(const float *slots, const double *loss_slots, int nslots, int count,
-                             float *grad, double *loss) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < count) {
-    float a = 0.f;
-    for (int k = 0; k < nslots; k++) a += slots[(size_t)k * count + p];
-    grad[p] = a;
+  if (mine) {
+    const float g[4] = {total.x, total.y, total.z, total.w};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (adam.params) adam_step(adam, p + k, state[k], g[k]);
+      else out[(size_t)blockIdx.y * S.count + p + k] = g[k];
+    }
   }
-  if (p == 0) {
-    double l = 0.0;
-    for (int k = 0; k < nslots; k++) l += loss_slots[k];
-    *loss = l;
+  if (mine4) {
+    if (adam.params) adam_step(adam, S.off_b4, state4, bias4);
+    else out[(size_t)blockIdx.y * S.count + S.off_b4] = bias4;
   }
 }
 
-__global__ void k_adam(float *params, const float *grad, float *m, float *v, int count, float lr,
-                       float b1, float b2, float c1, float c2) {
+static int mlp_grad_blocks(int F) {
+  return (F + kMlpGradRows) / kMlpGradRows + 2 * ((kMlpHidden + kMlpGradRows) / kMlpGradRows) + 1;
+}
+
+// Sum the slots of a large batch in order.
+__global__ void k_mlp_reduce(const float *slots, int nslots, int count, float *grad) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= count) return;
-  const float gp = grad[p];
-  const float mp = b1 * m[p] + (1.f - b1) * gp;
-  const float vp = b2 * v[p] + (1.f - b2) * gp * gp;
-  m[p] = mp;
-  v[p] = vp;
-  params[p] -= lr * (mp / c1) / (sqrtf(vp / c2) + 1e-8f);
+  float a = 0.f;
+  for (int k = 0; k < nslots; k++) a += slots[(size_t)k * count + p];
+  grad[p] = a;
+}
+
+// Sum of the rows' squared errors, in a fixed order.
+__global__ void __launch_bounds__(256) k_mlp_loss(const double *loss_rows, int n, double *loss) {
+  __shared__ double part[8];
+  double a = 0.0;
+  for (int i = threadIdx.x; i < n; i += 256) a += loss_rows[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = a;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < 8; k++) a += part[k];
+    *loss = a;
+  }
+}
+
+__global__ void k_adam(const float *grad, int count, MlpAdam adam) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < count) adam_step(adam, p, adam_state(adam, p), grad[p]);
 }
 
 }  // namespace qcs
@@ -181,10 +380,12 @@ __global__ void k_adam(float *params, const float *grad, float *m, float *v, int
 struct qcs_cuda_costmodel {
   int F;
   int count;
-  float *d_params, *d_grad, *d_m, *d_v, *d_slots;
-  double *d_loss_slots, *d_loss;
+  float *d_params, *d_grad, *d_m, *d_v;
+  double *d_loss_rows, *d_loss;
   float *d_x, *d_y, *d_pred;
   int cap_rows;
+  float *d_acts, *d_slots;  // for gradients of up to cap_grad rows
+  int cap_grad;
   int step;
   std::vector<float> host_params;  // mirror for planning on the host
   unsigned long long generation;   // bumped whenever host_params change
@@ -195,8 +396,8 @@ struct qcs_cuda_costmodel {
 namespace qcs {
 
 static size_t mlp_smem(int F) {
-  MlpShape S(F);
-  return sizeof(float) * ((size_t)S.count + kMlpRows * F + 5 * kMlpRows * kMlpHidden + kMlpRows);
+  return sizeof(float) * ((size_t)(F + 2 * kMlpHidden + 4 * kMlpRows) * kMlpPitch +
+                          4 * kMlpHidden + (size_t)kMlpRows * ((F + 3) & ~3));
 }
 
 static int cm_reserve(qcs_cuda_costmodel *m, int rows) {
@@ -204,29 +405,89 @@ static int cm_reserve(qcs_cuda_costmodel *m, int rows) {
   cudaFree(m->d_x);
   cudaFree(m->d_y);
   cudaFree(m->d_pred);
-  cudaFree(m->d_slots);
-  cudaFree(m->d_loss_slots);
-  const int nblk = (rows + kMlpRows - 1) / kMlpRows;
+  cudaFree(m->d_loss_rows);
+  m->d_x = m->d_y = m->d_pred = nullptr;
+  m->d_loss_rows = nullptr;
+  m->cap_rows = 0;
   int rc = check_cuda(cudaMalloc((void **)&m->d_x, (size_t)rows * m->F * sizeof(float)), "cudaMalloc(mlp)");
   if (!rc) rc = check_cuda(cudaMalloc((void **)&m->d_y, (size_t)rows * sizeof(float)), "cudaMalloc(mlp)");
   if (!rc) rc = check_cuda(cudaMalloc((void **)&m->d_pred, (size_t)rows * sizeof(float)), "cudaMalloc(mlp)");
-  if (!rc) rc = check_cuda(cudaMalloc((void **)&m->d_slots, (size_t)nblk * m->count * sizeof(float)), "cudaMalloc(mlp)");
-  if (!rc) rc = check_cuda(cudaMalloc((void **)&m->d_loss_slots, (size_t)nblk * sizeof(double)), "cudaMalloc(mlp)");
+  if (!rc) rc = check_cuda(cudaMalloc((void **)&m->d_loss_rows, (size_t)rows * sizeof(double)), "cudaMalloc(mlp)");
   if (!rc) m->cap_rows = rows;
   return rc;
 }
 
-// Loss (sum of squares) and gradient of the mean loss over rows [0, n) of
-// the device arrays d_x/d_y; results stay on the device.
-static int cm_grad_device(qcs_cuda_costmodel *m, const float *x, const float *y, int n) {
-  const int nblk = (n + kMlpRows - 1) / kMlpRows;
-  k_mlp<<<nblk, kMlpThreads, mlp_smem(m->F), m->stream>>>(m->d_params, m->F, x, y, n, 1.f / n,
-                                                          m->d_slots, m->d_loss_slots, nullptr);
-  int rc = check_launch("cost model backward");
+static int cm_reserve_grad(qcs_cuda_costmodel *m, int rows) {
+  if (rows <= m->cap_grad) return QCS_CUDA_OK;
+  cudaFree(m->d_acts);
+  cudaFree(m->d_slots);
+  m->d_acts = m->d_slots = nullptr;
+  m->cap_grad = 0;
+  const size_t nslots = rows > kMlpDirectRows ? (rows + kMlpSlot - 1) / kMlpSlot : 0;
+  int rc = check_cuda(cudaMalloc((void **)&m->d_acts, (size_t)rows * kMlpActs * sizeof(float)), "cudaMalloc(mlp)");
+  if (!rc && nslots)
+    rc = check_cuda(cudaMalloc((void **)&m->d_slots, nslots * m->count * sizeof(float)), "cudaMalloc(mlp)");
+  if (!rc) m->cap_grad = rows;
+  return rc;
+}
+
+// Forward over rows [0, n) of the device arrays x/y, keeping the rows' squared
+// errors, and the gradient of their mean: into d_grad, or into an Adam step.
+static int cm_grad_device(qcs_cuda_costmodel *m, const float *x, const float *y, int n,
+                          const MlpAdam *adam) {
+  MlpActs acts;
+  acts.p = m->d_acts;
+  acts.rows = (size_t)m->cap_grad;
+  k_mlp_rows<<<(n + kMlpRows - 1) / kMlpRows, kMlpRowThreads, mlp_smem(m->F), m->stream>>>(
+      m->d_params, m->F, x, y, n, 1.f / n, acts, m->d_loss_rows, nullptr);
+  int rc = check_launch("cost model rows");
   if (rc) return rc;
-  k_mlp_reduce<<<(m->count + 255) / 256, 256, 0, m->stream>>>(m->d_slots, m->d_loss_slots, nblk,
-                                                              m->count, m->d_grad, m->d_loss);
-  return check_launch("cost model gradient sum");
+  MlpAdam none;
+  memset(&none, 0, sizeof(none));
+  if (n <= kMlpDirectRows) {
+    k_mlp_grad<<<mlp_grad_blocks(m->F), kMlpGradThreads, kMlpStages * sizeof(MlpChunk), m->stream>>>(
+        m->F, x, n, acts, m->d_grad, adam ? *adam : none);
+    return check_launch("cost model gradient");
+  }
+  const int nslots = (n + kMlpSlot - 1) / kMlpSlot;
+  k_mlp_grad<<<dim3(mlp_grad_blocks(m->F), nslots), kMlpGradThreads,
+               kMlpStages * sizeof(MlpChunk), m->stream>>>(
+      m->F, x, n, acts, m->d_slots, none);
+  rc = check_launch("cost model gradient");
+  if (rc) return rc;
+  k_mlp_reduce<<<(m->count + 255) / 256, 256, 0, m->stream>>>(m->d_slots, nslots, m->count,
+                                                              m->d_grad);
+  rc = check_launch("cost model gradient sum");
+  if (rc || !adam) return rc;
+  k_adam<<<(m->count + 255) / 256, 256, 0, m->stream>>>(m->d_grad, m->count, *adam);
+  return check_launch("adam");
+}
+
+// Mean squared error over rows already on the device.
+static int cm_loss(qcs_cuda_costmodel *m, int n, double *loss) {
+  k_mlp_loss<<<1, 256, 0, m->stream>>>(m->d_loss_rows, n, m->d_loss);
+  int rc = check_launch("cost model loss");
+  double l = 0.0;
+  if (!rc) rc = check_cuda(cudaMemcpyAsync(&l, m->d_loss, sizeof(double), cudaMemcpyDeviceToHost, m->stream), "loss");
+  if (!rc) rc = check_cuda(cudaStreamSynchronize(m->stream), "sync");
+  if (!rc && loss) *loss = l / n;
+  return rc;
+}
+
+static int cm_upload(qcs_cuda_costmodel *m, const float *x, const float *y, int n) {
+  int rc = cm_reserve(m, n);
+  if (!rc) rc = check_cuda(cudaMemcpyAsync(m->d_x, x, (size_t)n * m->F * 4, cudaMemcpyHostToDevice, m->stream), "upload");
+  if (!rc && y) rc = check_cuda(cudaMemcpyAsync(m->d_y, y, (size_t)n * 4, cudaMemcpyHostToDevice, m->stream), "upload");
+  return rc;
+}
+
+// Forward only: predictions, or (with y) the rows' squared errors.
+static int cm_forward(qcs_cuda_costmodel *m, const float *x, const float *y, int n) {
+  MlpActs none = {nullptr, 0};
+  k_mlp_rows<<<(n + kMlpRows - 1) / kMlpRows, kMlpRowThreads, mlp_smem(m->F), m->stream>>>(
+      m->d_params, m->F, x, y, n, 1.f / n, none, y ? m->d_loss_rows : nullptr,
+      y ? nullptr : m->d_pred);
+  return check_launch("cost model forward");
 }
 
 // Generations are unique across models, so a plan kept for a destroyed model
@@ -305,8 +566,12 @@ int qcs_cuda_costmodel_create(int num_features, unsigned long long seed, qcs_cud
     if (!rc) rc = check_cuda(cudaMalloc((void **)&m->d_v, pb), "cudaMalloc(mlp)");
     if (!rc) rc = check_cuda(cudaMalloc((void **)&m->d_loss, sizeof(double)), "cudaMalloc(mlp)");
     if (!rc)
-      rc = check_cuda(cudaFuncSetAttribute(k_mlp, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      rc = check_cuda(cudaFuncSetAttribute(k_mlp_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)mlp_smem(64)),
+                      "cudaFuncSetAttribute(mlp)");
+    if (!rc)
+      rc = check_cuda(cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)(kMlpStages * sizeof(MlpChunk))),
                       "cudaFuncSetAttribute(mlp)");
     if (rc) {
       qcs_cuda_costmodel_destroy(m);
@@ -362,8 +627,9 @@ int qcs_cuda_costmodel_destroy(qcs_cuda_costmodel *m) {
   cudaFree(m->d_x);
   cudaFree(m->d_y);
   cudaFree(m->d_pred);
+  cudaFree(m->d_acts);
   cudaFree(m->d_slots);
-  cudaFree(m->d_loss_slots);
+  cudaFree(m->d_loss_rows);
   if (m->stream) cudaStreamDestroy(m->stream);
   delete m;
   return QCS_CUDA_OK;
@@ -402,17 +668,15 @@ int qcs_cuda_costmodel_loss_grad(qcs_cuda_costmodel *m, const float *x, const fl
                                  double *loss, float *grad) {
   if (!m || !x || !y || n < 1) return set_error(QCS_CUDA_EINVAL, "bad arguments");
   if (m->host_only) return set_error(QCS_CUDA_ENODEV, "cost model without a device: planning only");
-  int rc = cm_reserve(m, n);
-  if (!rc) rc = check_cuda(cudaMemcpyAsync(m->d_x, x, (size_t)n * m->F * 4, cudaMemcpyHostToDevice, m->stream), "upload");
-  if (!rc) rc = check_cuda(cudaMemcpyAsync(m->d_y, y, (size_t)n * 4, cudaMemcpyHostToDevice, m->stream), "upload");
-  if (!rc) rc = cm_grad_device(m, m->d_x, m->d_y, n);
-  double l = 0.0;
-  if (!rc) rc = check_cuda(cudaMemcpyAsync(&l, m->d_loss, sizeof(double), cudaMemcpyDeviceToHost, m->stream), "loss");
-  if (!rc && grad)
-    rc = check_cuda(cudaMemcpyAsync(grad, m->d_grad, m->count * sizeof(float), cudaMemcpyDeviceToHost, m->stream), "grad");
-  if (!rc) rc = check_cuda(cudaStreamSynchronize(m->stream), "sync");
-  if (!rc && loss) *loss = l / n;
-  return rc;
+  int rc = cm_upload(m, x, y, n);
+  if (!rc && !grad) rc = cm_forward(m, m->d_x, m->d_y, n);
+  if (!rc && grad) {
+    rc = cm_reserve_grad(m, n);
+    if (!rc) rc = cm_grad_device(m, m->d_x, m->d_y, n, nullptr);
+    if (!rc)
+      rc = check_cuda(cudaMemcpyAsync(grad, m->d_grad, m->count * sizeof(float), cudaMemcpyDeviceToHost, m->stream), "grad");
+  }
+  return rc ? rc : cm_loss(m, n, loss);
 }
 
 int qcs_cuda_costmodel_train(qcs_cuda_costmodel *m, const float *x, const float *y, int n,
@@ -420,23 +684,28 @@ int qcs_cuda_costmodel_train(qcs_cuda_costmodel *m, const float *x, const float 
   if (!m || !x || !y || n < 1 || epochs < 1 || batch < 1) return set_error(QCS_CUDA_EINVAL, "bad arguments");
   if (m->host_only) return set_error(QCS_CUDA_ENODEV, "cost model without a device: planning only");
   if (batch > n) batch = n;
-  int rc = cm_reserve(m, n);
-  if (!rc) rc = check_cuda(cudaMemcpyAsync(m->d_x, x, (size_t)n * m->F * 4, cudaMemcpyHostToDevice, m->stream), "upload");
-  if (!rc) rc = check_cuda(cudaMemcpyAsync(m->d_y, y, (size_t)n * 4, cudaMemcpyHostToDevice, m->stream), "upload");
-  const float b1 = 0.9f, b2 = 0.999f;
+  int rc = cm_upload(m, x, y, n);
+  if (!rc) rc = cm_reserve_grad(m, batch);
+  MlpAdam adam;
+  adam.params = m->d_params;
+  adam.m = m->d_m;
+  adam.v = m->d_v;
+  adam.lr = lr;
+  adam.b1 = 0.9f;
+  adam.b2 = 0.999f;
   for (int e = 0; !rc && e < epochs; e++) {
     for (int r = 0; !rc && r < n; r += batch) {
       const int rows = n - r < batch ? n - r : batch;
-      rc = cm_grad_device(m, m->d_x + (size_t)r * m->F, m->d_y + r, rows);
-      if (rc) break;
       m->step++;
-      const float c1 = 1.f - powf(b1, (float)m->step), c2 = 1.f - powf(b2, (float)m->step);
-      k_adam<<<(m->count + 255) / 256, 256, 0, m->stream>>>(m->d_params, m->d_grad, m->d_m, m->d_v,
-                                                            m->count, lr, b1, b2, c1, c2);
-      rc = check_launch("adam");
+      adam.c1 = 1.f - powf(adam.b1, (float)m->step);
+      adam.c2 = 1.f - powf(adam.b2, (float)m->step);
+      rc = cm_grad_device(m, m->d_x + (size_t)r * m->F, m->d_y + r, rows, &adam);
     }
   }
-  if (!rc && final_loss) rc = qcs_cuda_costmodel_loss_grad(m, x, y, n, final_loss, nullptr);
+  if (!rc && final_loss) {
+    rc = cm_forward(m, m->d_x, m->d_y, n);
+    if (!rc) rc = cm_loss(m, n, final_loss);
+  }
   if (!rc) rc = cm_sync_host(m);
   return rc;
 }
@@ -444,13 +713,8 @@ int qcs_cuda_costmodel_train(qcs_cuda_costmodel *m, const float *x, const float 
 int qcs_cuda_costmodel_predict(qcs_cuda_costmodel *m, const float *x, int n, float *out) {
   if (!m || !x || !out || n < 1) return set_error(QCS_CUDA_EINVAL, "bad arguments");
   if (m->host_only) return set_error(QCS_CUDA_ENODEV, "cost model without a device: planning only");
-  int rc = cm_reserve(m, n);
-  if (!rc) rc = check_cuda(cudaMemcpyAsync(m->d_x, x, (size_t)n * m->F * 4, cudaMemcpyHostToDevice, m->stream), "upload");
-  if (rc) return rc;
-  const int nblk = (n + kMlpRows - 1) / kMlpRows;
-  k_mlp<<<nblk, kMlpThreads, mlp_smem(m->F), m->stream>>>(m->d_params, m->F, m->d_x, nullptr, n,
-                                                          1.f / n, nullptr, nullptr, m->d_pred);
-  rc = check_launch("cost model forward");
+  int rc = cm_upload(m, x, nullptr, n);
+  if (!rc) rc = cm_forward(m, m->d_x, nullptr, n);
   if (!rc) rc = check_cuda(cudaMemcpyAsync(out, m->d_pred, (size_t)n * 4, cudaMemcpyDeviceToHost, m->stream), "predict");
   return rc ? rc : check_cuda(cudaStreamSynchronize(m->stream), "sync");
 }
