@@ -28,12 +28,12 @@
 // groups and the final store read through the map.
 //
 // Measured against one sweep per gate: 27 qubits complex64, brick, 752 gates
-// 240.7 -> 31.1 ms; 13 qubits, QFT and 200 random gates 201 -> 36 us a run;
-// complex128, 20 qubits, the same circuit 3.88 -> 1.74 ms.  What bounds it:
-// on large complex64 states the instructions of the gate loop (a 24-qubit
-// pass of 36 rotations issues 0.55 of the slots, DRAM at 0.13; a pass of
-// CNOTs alone runs at 0.9 of HBM); on complex128 the FP64 pipe (84 % busy); on
-// small states the latency of a pass.
+// 241 -> 24.5 ms; 13 qubits, QFT and 200 random gates 212 -> 34 us a run;
+// complex128, 20 qubits, the same circuit 3.98 -> 1.78 ms.  What bounds it:
+// on large complex64 states the instructions of the gate loop (a pass of 36
+// rotations issues 0.57 of the slots, two fifths of them packed arithmetic,
+// with DRAM at 0.19; a pass of CNOTs alone runs at 0.9 of HBM); on complex128
+// the FP64 pipe (84 % busy); on small states the latency of a pass.
 #include <stddef.h>
 #include <string.h>
 
@@ -42,31 +42,34 @@
 
 #include "common.cuh"
 #include "fusion.h"
+#include "tile_regs.cuh"
 #include "tiles.h"
 
 namespace qcs {
 
 int apply_op(qcs_cuda_state *s, const qcs_cuda_op &o);
 
+constexpr int kTileRegBits = 4;     // 16 amplitudes a thread
 constexpr int kTileMaxBits = 11;    // tile amplitudes: 2^11 at most
 constexpr int kTileMaxGates = 128;  // per pass (they ride in the kernel parameters)
 constexpr int kTileMaxGroups = 32;
 constexpr int kTileMaxFlips = 32;
 
-// How the register code applies a gate.  The first five take a register
-// target t; TF_DIAG_OUT is chosen by a bit outside the registers.
-enum TileForm {
-  TF_REAL,      // [[p0, p1], [p2, p3]], all real (RY)
-  TF_HAD,       // p0 * [[1, 1], [1, -1]]
-  TF_RX,        // [[p0, i p1], [i p1, p0]]
-  TF_Y,
-  TF_DIAG,      // p0 + i p1 on bit 0, p2 + i p3 on bit 1 of a register target
-  TF_DIAG_OUT,  // the same, target bit outside the registers
-  TF_NONE,      // leaves finite amplitudes as they are
-  TF_PHASE,     // p2 + i p3 where every condition bit is set
-  TF_SIGN,      // -1 where every condition bit is set
-  TF_COPY,      // the reference's CNOT: v0 := v1 where the control is set
-  TF_SWAP       // X, CNOT: in the maps, never in a group
+// How the register code applies a gate: TileGate::op.  Forms with a register
+// target t come as four numbers, the phase as one for each set of register
+// bits that must be set (at most two of the four).
+enum TileOp {
+  TO_DIAG = 0,       // + t: p0 + i p1 on bit 0, p2 + i p3 on bit 1
+  TO_REAL = 4,       // + t: [[p0, p1], [p2, p3]], all real (RY; complex64: H)
+  TO_PHASE = 8,      // + index of r_cond: p2 + i p3 where every condition bit is set
+  TO_DIAG_OUT = 19,  // TO_DIAG with the target bit outside the registers
+  TO_RX = 20,        // + t: [[p0, i p1], [i p1, p0]]
+  TO_Y = 24,         // + t
+  TO_HAD = 28,       // + t: p0 * [[1, 1], [1, -1]] (complex128)
+  TO_SIGN = 32,      // -1 where every condition bit is set
+  TO_COPY = 36,      // + t, the reference's CNOT: v0 := v1 where the control is set
+  TO_NONE = 40,      // leaves finite amplitudes as they are: in no group
+  TO_SWAP = 41       // X, CNOT: in the maps, never in a group
 };
 
 // One gate of a pass.  `general`: which products the sweep takes, 1: m00 v0,
@@ -81,18 +84,18 @@ template <typename R> struct TileGate {
   unsigned short l_tgt, l_ctl;  // target and control as tile bits
   uint32_t id_ctl;              // control as a bit of the tile's id
   unsigned char r_cond;   // register bits that must be set
-  unsigned char op;       // TileForm * 8 + register target
+  unsigned char op;       // TileOp
   unsigned char general;
   unsigned char pad;
 };
 
-// A group: gates seq[gate0 .. gate1) on registers e, where bit j of e adds
+// A group: gates [gate0, gate1) on registers e, where bit j of e adds
 // reg[j], bit j of the thread index col[j], to the shared-memory position
 // (XOR).  Before it, flips [flip0, flip1) change the constant.
 struct TileGroup {
   unsigned char gate0, gate1, flip0, flip1;
-  unsigned short reg[4];
-  unsigned short col[kTileMaxBits - 4];
+  unsigned short reg[kTileRegBits];
+  unsigned short col[kTileMaxBits - kTileRegBits];
 };
 struct TileFlip {
   unsigned short mask;  // XORed into the constant
@@ -101,7 +104,7 @@ struct TileFlip {
 
 template <typename R> struct TilePass {
   i64 n_tiles;
-  R minus_zero;  // see scale2
+  R minus_zero;  // see tile_regs.cuh
   int nt, nout, ngroups, ngates;
   unsigned char flip0, flip1;       // flips before the store
   signed char q[kTileMaxBits];      // tile bit -> qubit, ascending
@@ -109,7 +112,9 @@ template <typename R> struct TilePass {
   unsigned short store[kTileMaxBits];  // tile bit -> position, after the last gate
   TileFlip flip[kTileMaxFlips];
   TileGroup group[kTileMaxGroups];
-  unsigned char seq[kTileMaxGates];
+  // the gates of the groups, one group after another, then the others;
+  // order: all of them as the list has them
+  unsigned char order[kTileMaxGates];
   TileGate<R> gate[kTileMaxGates];
 };
 
@@ -120,19 +125,24 @@ template <typename R> struct TilePass {
 // Shared-memory position of tile amplitude i: its place in the 128-byte row
 // is XORed with the row's number, so that whichever tile bits are held in
 // registers a warp's lanes spread over the banks.  Linear over XOR.
+// (complex64: of a real or imaginary part.)
 __host__ __device__ __forceinline__ int tile_pos(int i, float2) {
-  return i ^ ((i >> 4) & 15) ^ ((i >> 8) & 15);
+  return i ^ ((i >> 5) & 31) ^ ((i >> 10) & 31);
 }
 __host__ __device__ __forceinline__ int tile_pos(int i, double2) {
   return i ^ ((i >> 3) & 7) ^ ((i >> 6) & 7) ^ ((i >> 9) & 7);
 }
 
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
+// One amplitude of a tile of L in shared memory.
+__device__ __forceinline__ float2 tile_get(const float *S, int L, int at) {
+  return make_float2(S[at], S[L + at]);
+}
+__device__ __forceinline__ void tile_put(float *S, int L, int at, float2 v) {
+  S[at] = v.x;
+  S[L + at] = v.y;
+}
+__device__ __forceinline__ double2 tile_get(const double2 *S, int, int at) { return S[at]; }
+__device__ __forceinline__ void tile_put(double2 *S, int, int at, double2 v) { S[at] = v; }
 
 // Collects whether an amplitude was an infinity or a NaN: 0 * x is NaN for
 // those alone (and FP32 products cost no integer slot); FP64, whose products
@@ -151,171 +161,115 @@ struct FiniteF64 {
   __device__ __forceinline__ bool bad() const { return b; }
 };
 
-// regs: amplitudes a thread holds.  16 measured against 32 (complex64, 27-qubit
-// brick, 752 gates): 32.6 ms and 32.5 ms, but 98 us against 116 us on 13
-// qubits, where the tile's threads are all the parallelism there is.
-// max_bits: a tile's qubits; 11 against 12 (complex64): 32.6 and 33.4 ms on 27
-// qubits, 98 and 114 us on 13; 10 against 11 (complex128, 20 qubits, 417
-// gates): 2.13 and 2.32 ms.
+// max_bits: a tile's qubits.  Measured, 11 against 12 (complex64): 27.0 and 29.2
+// ms on 27 qubits (brick, 752 gates), 87 and 101 us on 13, where the threads
+// of the tiles are all the parallelism there is; 10 against 11 (complex128,
+// 20 qubits, 417 gates): 2.13 and 2.32 ms.  Likewise 16 amplitudes a thread
+// against 32: 27.7 and 28.9 ms, 87 and 122 us.
 // low: qubits every tile holds, so that it is read in runs of 128 bytes.
-constexpr int kTileRegBits = 4;
-constexpr int kTileRegs = 1 << kTileRegBits;
+// blocks: CTAs an SM holds (72 registers a thread for complex64).
 template <typename C> struct TileTraits;
 template <> struct TileTraits<float2> {
   typedef float R;
+  typedef float Elem;  // of the tile in shared memory
   typedef FiniteF32 Finite;
-  static constexpr int max_bits = 11, low = 4, blocks = 6;
+  typedef RegsF32<kTileRegBits> Regs;
+  static constexpr int max_bits = 11, low = 4, blocks = 7;
 };
 template <> struct TileTraits<double2> {
   typedef double R;
+  typedef double2 Elem;
   typedef FiniteF64 Finite;
+  typedef RegsF64<kTileRegBits> Regs;
   static constexpr int max_bits = 10, low = 3, blocks = 8;
 };
 
-// s * v and v + w, v - w, both parts at once (one packed FP32 instruction).
-// The packed product is written as s * v + z with z = -0 that only the host
-// knows: of a plain packed product and a packed sum the assembler makes one
-// fused operation, with one rounding instead of two, .rn or not.
-__device__ __forceinline__ u64 pack2(float x, float y) {
-  return ((u64)__float_as_uint(y) << 32) | __float_as_uint(x);
-}
-__device__ __forceinline__ float2 unpack2(u64 v) {
-  return make_float2(__uint_as_float((uint32_t)v), __uint_as_float((uint32_t)(v >> 32)));
-}
-__device__ __forceinline__ float2 scale2(float s, float2 v, float z) {
-  u64 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(r) : "l"(pack2(s, s)), "l"(pack2(v.x, v.y)), "l"(pack2(z, z)));
-  return unpack2(r);
-}
-__device__ __forceinline__ float2 add2(float2 v, float2 w) {
-  u64 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(v.x, v.y)), "l"(pack2(w.x, w.y)));
-  return unpack2(r);
-}
-__device__ __forceinline__ double2 scale2(double s, double2 v, double) {
-  return make_double2(__dmul_rn(s, v.x), __dmul_rn(s, v.y));
-}
-__device__ __forceinline__ double2 add2(double2 v, double2 w) { return cadd(v, w); }
+#define QCS_TILE_TARGET(CALL)                                               \
+  if (op & 2) {                                                             \
+    if (op & 1) { constexpr int TB = 3; CALL; }                             \
+    else { constexpr int TB = 2; CALL; }                                    \
+  } else {                                                                  \
+    if (op & 1) { constexpr int TB = 1; CALL; }                             \
+    else { constexpr int TB = 0; CALL; }                                    \
+  }
+#define QCS_TILE_PHASE(I, COND) \
+  case TO_PHASE + I: a.template phase<COND>(g.p); break;
 
-// d * v.  FP32: the fused multiply-adds the compiler makes of cmul in the
-// sweeps, written out so that no other contraction can change a bit.
+// One gate on the amplitudes of thread t.  (The compiler makes no jump table of
+// a switch here but a tree of comparisons over all the forms, seven branches
+// a gate; asking for the common classes first takes four.)
+template <typename Regs, typename R>
+__device__ __forceinline__ void tile_apply(Regs &a, const TileGate<R> &g, uint32_t t,
+                                           uint32_t tile, u64 z) {
+  const int op = g.op;
+  if (op < TO_REAL) {
+    QCS_TILE_TARGET((a.template diag<TB>(g.p)))
+  } else if (op < TO_PHASE) {
+    QCS_TILE_TARGET((a.template real<TB>(g.p, z)))
+  } else if (op == TO_DIAG_OUT) {
+    const bool one = (t & g.t_tgt) || (tile & g.id_tgt);
+    const R f[2] = {one ? g.p[2] : g.p[0], one ? g.p[3] : g.p[1]};
+    a.template phase<0>(f);
+  } else if ((t & g.t_cond) != g.t_cond || (tile & g.id_cond) != g.id_cond) {
+    // a form with a condition that is not met (the others have none)
+  } else if (op < TO_DIAG_OUT) {
+    switch (op) {
+      QCS_TILE_PHASE(0, 0) QCS_TILE_PHASE(1, 1) QCS_TILE_PHASE(2, 2) QCS_TILE_PHASE(3, 3)
+      QCS_TILE_PHASE(4, 4) QCS_TILE_PHASE(5, 5) QCS_TILE_PHASE(6, 6) QCS_TILE_PHASE(7, 8)
+      QCS_TILE_PHASE(8, 9) QCS_TILE_PHASE(9, 10) QCS_TILE_PHASE(10, 12)
+    }
+  } else if (op < TO_Y) {
+    QCS_TILE_TARGET((a.template rx<TB>(g.p, z)))
+  } else if (op < TO_HAD) {
+    QCS_TILE_TARGET((a.template y<TB>()))
+  } else if (op < TO_SIGN) {
+    if constexpr (sizeof(R) == 8) QCS_TILE_TARGET((a.template had<TB>(g.p)))
+  } else if (op < TO_COPY) {
+    a.sign(g.r_cond);
+  } else {
+    QCS_TILE_TARGET((a.template copy<TB>(g.r_cond)))
+  }
+}
+#undef QCS_TILE_PHASE
+#undef QCS_TILE_TARGET
+
+// d * v with the sweeps' rounding (tile_regs.cuh).
 __device__ __forceinline__ float2 turn(float2 d, float2 v) {
   return make_float2(__fmaf_rn(d.x, v.x, -__fmul_rn(d.y, v.y)),
                      __fmaf_rn(d.y, v.x, __fmul_rn(d.x, v.y)));
 }
 __device__ __forceinline__ double2 turn(double2 d, double2 v) { return cmul(d, v); }
 
-// A non-diagonal gate on register bit TB.
-template <int FORM, int TB, typename C, typename R>
-__device__ __forceinline__ void tile_gate(C (&a)[kTileRegs], const TileGate<R> &g, R z) {
-#pragma unroll
-  for (int e = 0; e < kTileRegs; e++) {
-    if (e & (1 << TB)) continue;
-    const int f = e | (1 << TB);
-    const C v0 = a[e], v1 = a[f];
-    if constexpr (FORM == TF_REAL) {
-      a[e] = add2(scale2(g.p[0], v0, z), scale2(g.p[1], v1, z));
-      a[f] = add2(scale2(g.p[2], v0, z), scale2(g.p[3], v1, z));
-    } else if constexpr (FORM == TF_HAD) {
-      const C x0 = scale2(g.p[0], v0, z), x1 = scale2(g.p[0], v1, z);
-      a[e] = add2(x0, x1);
-      a[f].x = sub_rn(x0.x, x1.x);
-      a[f].y = sub_rn(x0.y, x1.y);
-    } else if constexpr (FORM == TF_RX) {
-      a[e].x = sub_rn(mul_rn(g.p[0], v0.x), mul_rn(g.p[1], v1.y));
-      a[e].y = add_rn(mul_rn(g.p[0], v0.y), mul_rn(g.p[1], v1.x));
-      a[f].x = sub_rn(mul_rn(g.p[0], v1.x), mul_rn(g.p[1], v0.y));
-      a[f].y = add_rn(mul_rn(g.p[0], v1.y), mul_rn(g.p[1], v0.x));
-    } else if constexpr (FORM == TF_COPY) {
-      if ((e & g.r_cond) == g.r_cond) a[e] = v1;
-    } else {  // TF_Y
-      a[e].x = v1.y;
-      a[e].y = -v1.x;
-      a[f].x = -v0.y;
-      a[f].y = v0.x;
-    }
-  }
-}
-
-template <int TB, typename C, typename R>
-__device__ __forceinline__ void tile_diag(C (&a)[kTileRegs], const TileGate<R> &g) {
-  C d0, d1;
-  d0.x = g.p[0];
-  d0.y = g.p[1];
-  d1.x = g.p[2];
-  d1.y = g.p[3];
-#pragma unroll
-  for (int e = 0; e < kTileRegs; e++) a[e] = turn((e & (1 << TB)) ? d1 : d0, a[e]);
-}
-
-// The phase on the registers with every bit of COND set (at most two bits).
-// The condition is static: a product that is only predicated off would still
-// take its slot in the FP64 pipe.
-template <int COND, typename C, typename R>
-__device__ __forceinline__ void tile_phase(C (&a)[kTileRegs], const TileGate<R> &g) {
-  C d;
-  d.x = g.p[2];
-  d.y = g.p[3];
-#pragma unroll
-  for (int e = 0; e < kTileRegs; e++)
-    if ((e & COND) == COND) a[e] = turn(d, a[e]);
-}
-
-#define QCS_TILE_FORM(FORM)                                \
-  case FORM * 8 + 0: tile_gate<FORM, 0>(a, g, z); break;       \
-  case FORM * 8 + 1: tile_gate<FORM, 1>(a, g, z); break;       \
-  case FORM * 8 + 2: tile_gate<FORM, 2>(a, g, z); break;       \
-  case FORM * 8 + 3: tile_gate<FORM, 3>(a, g, z); break;
-#define QCS_TILE_PHASE(COND) \
-  case COND: tile_phase<COND>(a, g); break;
-
-// One gate on the amplitudes of thread t.
+// A gate's 2x2 from its record.
 template <typename C, typename R>
-__device__ __forceinline__ void tile_apply(C (&a)[kTileRegs], const TileGate<R> &g, uint32_t t,
-                                           uint32_t tile, R z) {
-  switch (g.op) {
-    QCS_TILE_FORM(TF_REAL)
-    QCS_TILE_FORM(TF_HAD)
-    QCS_TILE_FORM(TF_RX)
-    QCS_TILE_FORM(TF_Y)
-    case TF_DIAG * 8 + 0: tile_diag<0>(a, g); break;
-    case TF_DIAG * 8 + 1: tile_diag<1>(a, g); break;
-    case TF_DIAG * 8 + 2: tile_diag<2>(a, g); break;
-    case TF_DIAG * 8 + 3: tile_diag<3>(a, g); break;
-    case TF_DIAG_OUT * 8: {
-      const bool one = (t & g.t_tgt) || (tile & g.id_tgt);
-      C d;
-      d.x = one ? g.p[2] : g.p[0];
-      d.y = one ? g.p[3] : g.p[1];
-#pragma unroll
-      for (int e = 0; e < kTileRegs; e++) a[e] = turn(d, a[e]);
-      break;
-    }
-    default: {  // the forms with conditions
-      if ((t & g.t_cond) != g.t_cond || (tile & g.id_cond) != g.id_cond) break;
-      switch (g.op) {
-        QCS_TILE_FORM(TF_COPY)
-        case TF_PHASE * 8:
-          switch (g.r_cond) {
-            QCS_TILE_PHASE(0) QCS_TILE_PHASE(1) QCS_TILE_PHASE(2) QCS_TILE_PHASE(3)
-            QCS_TILE_PHASE(4) QCS_TILE_PHASE(5) QCS_TILE_PHASE(6) QCS_TILE_PHASE(8)
-            QCS_TILE_PHASE(9) QCS_TILE_PHASE(10) QCS_TILE_PHASE(12)
-          }
-          break;
-        default:  // TF_SIGN
-#pragma unroll
-          for (int e = 0; e < kTileRegs; e++)
-            if ((e & g.r_cond) == g.r_cond) {
-              a[e].x = -a[e].x;
-              a[e].y = -a[e].y;
-            }
-      }
-    }
+__device__ void tile_matrix(const TileGate<R> &g, C (&m)[4]) {
+  const int op = g.op;
+  if (op < TO_REAL || op == TO_DIAG_OUT) {
+    m[0].x = g.p[0];
+    m[0].y = g.p[1];
+    m[3].x = g.p[2];
+    m[3].y = g.p[3];
+  } else if (op < TO_PHASE || (op >= TO_HAD && op < TO_SIGN)) {
+    for (int i = 0; i < 4; i++) m[i].x = g.p[i];
+  } else if (op < TO_DIAG_OUT) {
+    m[0].x = 1;
+    m[3].x = g.p[0];
+    m[3].y = g.p[1];
+  } else if (op < TO_Y) {
+    m[0].x = m[3].x = g.p[0];
+    m[1].y = m[2].y = g.p[1];
+  } else if (op < TO_HAD) {
+    m[1].y = -1;
+    m[2].y = 1;
+  } else if (op < TO_COPY) {
+    m[0].x = 1;
+    m[3].x = -1;
+  } else if (op == TO_NONE) {  // the identity; the reference's CPHASE takes its 1 alone
+    m[0].x = m[3].x = 1;
+  } else {
+    m[1].x = m[2].x = 1;
   }
 }
-#undef QCS_TILE_PHASE
-#undef QCS_TILE_FORM
 
 // The gates of a pass on a tile with an infinity or a NaN in it: one at a
 // time, with the products the sweep of each gate takes (TileGate::general),
@@ -325,46 +279,34 @@ __device__ __forceinline__ float2 sum2(float2 v, float2 w) {
 }
 __device__ __forceinline__ double2 sum2(double2 v, double2 w) { return cadd(v, w); }
 
-template <typename C, typename R>
-__device__ __noinline__ void general_tile(C *S, const TilePass<R> &P, uint32_t tile) {
+template <typename C, typename E, typename R>
+__device__ __noinline__ void general_tile(E *S, const TilePass<R> &P, uint32_t tile) {
   const C kind = {};
+  const int L = 1 << P.nt;
   for (int gi = 0; gi < P.ngates; gi++) {
-    const TileGate<R> &g = P.gate[gi];
+    const TileGate<R> &g = P.gate[P.order[gi]];
     C m[4] = {};
-    const int form = g.op >> 3;
-    if (form == TF_REAL || form == TF_HAD) {
-      for (int i = 0; i < 4; i++) m[i].x = g.p[i];
-    } else if (form == TF_RX) {
-      m[0].x = m[3].x = g.p[0];
-      m[1].y = m[2].y = g.p[1];
-    } else if (form == TF_SWAP || form == TF_COPY) {
-      m[1].x = m[2].x = 1;
-    } else if (form == TF_Y) {
-      m[1].y = -1;
-      m[2].y = 1;
-    } else {  // diagonal
-      m[0].x = g.p[0];
-      m[0].y = g.p[1];
-      m[3].x = g.p[2];
-      m[3].y = g.p[3];
-    }
+    tile_matrix(g, m);
     if ((tile & g.id_ctl) == g.id_ctl) {
-      for (int l = threadIdx.x; l < (1 << P.nt); l += blockDim.x) {
+      for (int l = threadIdx.x; l < L; l += blockDim.x) {
         if ((l & g.l_ctl) != g.l_ctl) continue;
-        C *x = S + tile_pos(l, kind);
+        const int x = tile_pos(l, kind);
         if (!g.l_tgt) {  // a diagonal on a qubit outside the tile
           const bool one = tile & g.id_tgt;
-          if (g.general & (one ? 8 : 1)) *x = turn(one ? m[3] : m[0], *x);
+          if (g.general & (one ? 8 : 1))
+            tile_put(S, L, x, turn(one ? m[3] : m[0], tile_get(S, L, x)));
           continue;
         }
         if (l & g.l_tgt) continue;
-        C *y = S + tile_pos(l | g.l_tgt, kind);
-        const C v0 = *x, v1 = *y;
+        const int y = tile_pos(l | g.l_tgt, kind);
+        const C v0 = tile_get(S, L, x), v1 = tile_get(S, L, y);
         const int u = g.general & 3, w = g.general >> 2;
-        if (u) *x = u == 3 ? sum2(turn(m[0], v0), turn(m[1], v1))
-                           : u == 1 ? turn(m[0], v0) : turn(m[1], v1);
-        if (w) *y = w == 3 ? sum2(turn(m[2], v0), turn(m[3], v1))
-                           : w == 1 ? turn(m[2], v0) : turn(m[3], v1);
+        if (u)
+          tile_put(S, L, x, u == 3 ? sum2(turn(m[0], v0), turn(m[1], v1))
+                                   : u == 1 ? turn(m[0], v0) : turn(m[1], v1));
+        if (w)
+          tile_put(S, L, y, w == 3 ? sum2(turn(m[2], v0), turn(m[3], v1))
+                                   : w == 1 ? turn(m[2], v0) : turn(m[3], v1));
       }
     }
     __syncthreads();
@@ -377,13 +319,17 @@ template <typename C>
 __global__ void __launch_bounds__(1 << (TileTraits<C>::max_bits - kTileRegBits),
                                   TileTraits<C>::blocks)
     k_tile(C *v, const __grid_constant__ TilePass<typename TileTraits<C>::R> P) {
-  constexpr int RB = kTileRegBits, REGS = kTileRegs;
+  typedef typename TileTraits<C>::Elem E;
+  constexpr int RB = kTileRegBits, REGS = 1 << RB;
   constexpr int UNIT = 16 / sizeof(C);  // amplitudes per 16-byte access
   constexpr int STEPS = REGS / UNIT;    // accesses per thread and tile
   constexpr int STEP_BITS = UNIT == 2 ? RB - 1 : RB;
   const C kind = {};
+  if constexpr (sizeof(C) == 8) QCS_REGS_F32_DECLARE(8);
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C *S = reinterpret_cast<C *>(smem_raw);
+  E *S = reinterpret_cast<E *>(smem_raw);
+  const int L = 1 << P.nt;
+  const u64 z = both2((float)P.minus_zero);
   const int t = threadIdx.x;
   const int sb = P.nt - STEP_BITS;  // the tile bits from sb up count a thread's accesses
   // this thread's first unit: its offset in memory, its position on loading
@@ -427,7 +373,7 @@ __global__ void __launch_bounds__(1 << (TileTraits<C>::max_bits - kTileRegBits),
 #pragma unroll
         for (int j = 0; j < UNIT; j++) {
           fin.see(y[j]);
-          S[at ^ j] = y[j];
+          tile_put(S, L, at ^ j, y[j]);
         }
       }
     }
@@ -438,11 +384,12 @@ __global__ void __launch_bounds__(1 << (TileTraits<C>::max_bits - kTileRegBits),
         if (P.flip[f].id_bit < 0 || ((id >> P.flip[f].id_bit) & 1)) c ^= P.flip[f].mask;
     };
     if (bad) {
-      general_tile(S, P, id);
+      general_tile<C>(S, P, id);
       for (int k = 0; k < STEPS; k++) {
         uint4 x;
         C *y = reinterpret_cast<C *>(&x);
-        for (int j = 0; j < UNIT; j++) y[j] = S[tload ^ tile_pos((k << sb) | j, kind)];
+        for (int j = 0; j < UNIT; j++)
+          y[j] = tile_get(S, L, tload ^ tile_pos((k << sb) | j, kind));
         *reinterpret_cast<uint4 *>(vt + step_off(k)) = x;
       }
     } else {
@@ -453,19 +400,29 @@ __global__ void __launch_bounds__(1 << (TileTraits<C>::max_bits - kTileRegBits),
 #pragma unroll
         for (int j = 0; j < TileTraits<C>::max_bits - RB; j++)
           if ((t >> j) & 1) at ^= G.col[j];
-        int pos[REGS];
+        auto place = [&](int (&pos)[REGS]) {  // register e: its bits' columns
+          int lo[4], hi[4];
 #pragma unroll
-        for (int e = 0; e < REGS; e++) {  // e's highest bit, then the rest
-          int hb = 0;
-          while ((e >> hb) > 1) hb++;
-          pos[e] = e == 0 ? at : pos[e ^ (1 << hb)] ^ G.reg[hb];
+          for (int k = 0; k < 4; k++) {
+            lo[k] = at ^ ((k & 1) ? G.reg[0] : 0) ^ ((k & 2) ? G.reg[1] : 0);
+            hi[k] = ((k & 1) ? G.reg[2] : 0) ^ ((k & 2) ? G.reg[3] : 0);
+          }
+#pragma unroll
+          for (int e = 0; e < REGS; e++) pos[e] = lo[e & 3] ^ hi[e >> 2];
+        };
+        typename TileTraits<C>::Regs a;
+        {
+          int pos[REGS];
+          place(pos);
+          a.load(S, L, pos);
         }
-        C a[REGS];
-#pragma unroll
-        for (int e = 0; e < REGS; e++) a[e] = S[pos[e]];
-        for (int i = G.gate0; i < G.gate1; i++) tile_apply(a, P.gate[P.seq[i]], (uint32_t)t, id, P.minus_zero);
-#pragma unroll
-        for (int e = 0; e < REGS; e++) S[pos[e]] = a[e];
+        for (int i = G.gate0; i < G.gate1; i++) tile_apply(a, P.gate[i], (uint32_t)t, id, z);
+        asm volatile("" : "+r"(at));  // the positions are formed anew, not kept
+        {
+          int pos[REGS];
+          place(pos);
+          a.store(S, L, pos);
+        }
         __syncthreads();
       }
       flips(P.flip0, P.flip1);
@@ -475,7 +432,7 @@ __global__ void __launch_bounds__(1 << (TileTraits<C>::max_bits - kTileRegBits),
         C *y = reinterpret_cast<C *>(&x);
         const int at = c ^ tstore ^ step_store(k);
 #pragma unroll
-        for (int j = 0; j < UNIT; j++) y[j] = S[j ? at ^ P.store[0] : at];
+        for (int j = 0; j < UNIT; j++) y[j] = tile_get(S, L, j ? at ^ P.store[0] : at);
         *reinterpret_cast<uint4 *>(vt + step_off(k)) = x;
       }
     }
@@ -592,6 +549,25 @@ static int sweep_products(const qcs_cuda_state *s, const double m[8], bool contr
   return 15;
 }
 
+// The constants of a record from the gate's 2x2.
+template <typename R>
+static void fill_const(TileGate<R> &g, int op, const double m[8]) {
+  if (op == TO_DIAG || op == TO_DIAG_OUT) {
+    for (int i = 0; i < 2; i++) {
+      g.p[i] = (R)m[i];
+      g.p[2 + i] = (R)m[6 + i];
+    }
+  } else if (op == TO_REAL || op == TO_HAD) {
+    for (int i = 0; i < 4; i++) g.p[i] = (R)m[2 * i];
+  } else if (op == TO_RX) {
+    g.p[0] = (R)m[0];
+    g.p[1] = (R)m[3];
+  } else if (op == TO_PHASE) {
+    g.p[0] = (R)m[6];
+    g.p[1] = (R)m[7];
+  }
+}
+
 // Gate record; bit_of: qubit -> tile bit (-1: outside), id_of: qubit -> bit of
 // the tile's id, reg_of and thread_of: tile bit -> register or thread bit of
 // the gate's group (-1: the other).
@@ -615,44 +591,37 @@ static void fill_gate(const qcs_cuda_state *s, const qcs_cuda_op &o, const int *
     else if (reg_of[bit_of[q]] >= 0) r |= (unsigned char)(1 << reg_of[bit_of[q]]);
     else t |= (unsigned short)(1 << thread_of[bit_of[q]]);
   };
-  int form = TF_NONE;
+  int op = TO_NONE;
   bool cond_tgt = false;  // the target bit is a condition too (phases)
   switch (o.kind) {
-    case QCS_GATE_H: form = TF_HAD; break;
-    case QCS_GATE_RY: form = TF_REAL; break;
-    case QCS_GATE_RX: form = TF_RX; break;
-    case QCS_GATE_X: form = TF_SWAP; break;
-    case QCS_GATE_Y: form = TF_Y; break;
-    case QCS_GATE_CNOT: form = ref ? TF_COPY : TF_SWAP; break;
-    case QCS_GATE_RZ: form = TF_DIAG; break;
-    case QCS_GATE_Z: form = TF_SIGN; cond_tgt = true; break;
-    case QCS_GATE_P: form = TF_PHASE; cond_tgt = true; break;
+    case QCS_GATE_H: op = sizeof(R) == 8 ? TO_HAD : TO_REAL; break;
+    case QCS_GATE_RY: op = TO_REAL; break;
+    case QCS_GATE_RX: op = TO_RX; break;
+    case QCS_GATE_X: op = TO_SWAP; break;
+    case QCS_GATE_Y: op = TO_Y; break;
+    case QCS_GATE_CNOT: op = ref ? TO_COPY : TO_SWAP; break;
+    case QCS_GATE_RZ: op = TO_DIAG; break;
+    case QCS_GATE_Z: op = TO_SIGN; cond_tgt = true; break;
+    case QCS_GATE_P: op = TO_PHASE; cond_tgt = true; break;
     // under the reference's rule a CPHASE multiplies by its U00 = 1 only
-    case QCS_GATE_CPHASE: form = ref ? TF_NONE : TF_PHASE; cond_tgt = true; break;
-    default: form = TF_NONE; break;  // identity
-  }
-  if (form == TF_RX) {
-    g.p[0] = (R)m[0];
-    g.p[1] = (R)m[3];
-  } else if (form == TF_REAL || form == TF_HAD) {
-    for (int i = 0; i < 4; i++) g.p[i] = (R)m[2 * i];
-  } else {
-    g.p[0] = (R)m[0];
-    g.p[1] = (R)m[1];
-    g.p[2] = (R)m[6];
-    g.p[3] = (R)m[7];
+    case QCS_GATE_CPHASE: op = ref ? TO_NONE : TO_PHASE; cond_tgt = true; break;
+    default: break;  // identity
   }
   if (ctl) place(o.control, g.r_cond, g.t_cond, g.id_cond);
   if (cond_tgt) place(o.target, g.r_cond, g.t_cond, g.id_cond);
-  int reg = bit_of[o.target] >= 0 ? reg_of[bit_of[o.target]] : -1;
-  if (form == TF_DIAG && reg < 0) {
-    form = TF_DIAG_OUT;
-    unsigned char none = 0;
+  const int reg = bit_of[o.target] >= 0 ? reg_of[bit_of[o.target]] : -1;
+  if (op == TO_DIAG && reg < 0) {
+    op = TO_DIAG_OUT;
+    unsigned char no_reg = 0;
     uint32_t id = 0;  // id_tgt is set above
-    place(o.target, none, g.t_tgt, id);
+    place(o.target, no_reg, g.t_tgt, id);
   }
-  const bool on_reg = form <= TF_DIAG || form == TF_COPY;
-  g.op = (unsigned char)(form * 8 + (on_reg ? reg : 0));
+  fill_const(g, op, m);
+  static const unsigned char conds[11] = {0, 1, 2, 3, 4, 5, 6, 8, 9, 10, 12};
+  if (op == TO_PHASE) op += (int)(std::find(conds, conds + 11, g.r_cond) - conds);
+  if (op == TO_DIAG || op == TO_REAL || op == TO_RX || op == TO_Y || op == TO_HAD || op == TO_COPY)
+    op += reg;
+  g.op = (unsigned char)op;
 }
 
 template <typename C>
@@ -678,7 +647,7 @@ static int launch_pass(qcs_cuda_state *s, const qcs_cuda_op *ops, const TileStre
   P.ngates = st.last - st.first;
   int map[kTileMaxBits];  // column b: what tile bit b adds to the position
   for (int b = 0; b < P.nt; b++) map[b] = tile_pos(1 << b, kind);
-  int nseq = 0, nflip = 0, flip0 = 0;
+  int nrun = 0, nrest = P.ngates, nflip = 0, flip0 = 0;
   auto move = [&](const qcs_cuda_op &o) {  // X or CNOT: see the head of the file
     const int t = bit_of[o.target];
     if (o.kind == QCS_GATE_CNOT && bit_of[o.control] >= 0) {
@@ -718,26 +687,29 @@ static int launch_pass(qcs_cuda_state *s, const qcs_cuda_op *ops, const TileStre
       std::fill(thread_of, thread_of + kTileMaxBits, -1);
       for (int j = 0; j < P.nt; j++) {
         const int b = order[j];
-        if (j < RB) {
-          G.reg[j] = (unsigned short)map[b];
-          reg_of[b] = j;
+        if (j < RB) {  // the least used one is the pair bit (tile_regs.cuh)
+          G.reg[RB - 1 - j] = (unsigned short)map[b];
+          reg_of[b] = RB - 1 - j;
         } else {
           const int t = P.nt - 1 - j;  // the last, least used ones are the lanes
           G.col[t] = (unsigned short)map[b];
           thread_of[b] = t;
         }
       }
-      G.gate0 = (unsigned char)nseq;
+      G.gate0 = (unsigned char)nrun;
       for (int i : gr.gates) {
-        P.seq[nseq] = (unsigned char)(i - st.first);
-        TileGate<R> &g = P.gate[i - st.first];
+        TileGate<R> g;
         fill_gate<R>(s, ops[i], bit_of, id_of, reg_of, thread_of, g);
-        if (g.op != TF_NONE * 8) nseq++;
+        const int at = g.op != TO_NONE ? nrun++ : --nrest;
+        P.gate[at] = g;
+        P.order[i - st.first] = (unsigned char)at;
       }
-      G.gate1 = (unsigned char)nseq;
+      G.gate1 = (unsigned char)nrun;
     }
     for (int i : gr.moves) {
-      fill_gate<R>(s, ops[i], bit_of, id_of, none, none, P.gate[i - st.first]);
+      const int at = --nrest;
+      fill_gate<R>(s, ops[i], bit_of, id_of, none, none, P.gate[at]);
+      P.order[i - st.first] = (unsigned char)at;
       move(ops[i]);
     }
   }
