@@ -11,26 +11,32 @@
 //  * an instance of at most `tile_q` qubits lives entirely in shared memory:
 //    |0...0> is built there, its gates run there, and <Z_0> and the shots
 //    are computed there -- it never touches HBM;
-//  * gates run in register groups: the gates of a stage are partitioned
-//    greedily into groups on at most 4 tile bits, and one pass over shared
-//    memory applies a whole group, each thread holding the 16 amplitudes of
-//    one setting of the other bits in registers (one pass per group instead
-//    of one per gate);
+//  * gates run in register groups: the gates of a stage are cut into groups
+//    on at most 4 or 5 tile bits, and one pass over shared memory applies a
+//    whole group, each thread holding the 16 or 32 amplitudes of one setting
+//    of the other bits in registers (one pass per group instead of one per
+//    gate; tile_regs.cuh);
 //  * a larger instance lives in a per-CTA slot of global memory and runs in
 //    stages: a stage is a set of tile_q qubits and the gates acting inside
 //    it; for every tile (one setting of the other qubits) the CTA gathers the
 //    2^tile_q amplitudes into shared memory with coalesced runs, applies the
 //    stage's gates there and scatters them back, so a stage costs one read
 //    and one write of the state however many gates it holds;
-//  * <Z_0> is accumulated in FP64 (FP32 partials over 8 amplitudes) and each
-//    shot is drawn from a counter-based generator (splitmix64 of seed,
-//    instance, shot), mapped to an index with an FP64 warp scan.
+//  * <Z_0> is accumulated in FP64 (of FP32 squares) and each shot is drawn
+//    from a counter-based generator (splitmix64 of seed, instance, shot) and
+//    mapped to an index by binary searches over running sums in FP64, then
+//    the amplitudes of the block found.
 //
 // The run is captured once into a CUDA graph (queue reset, kernel, result
 // copies) and replayed; new angles only rewrite the pinned gate table the
 // graph's upload node reads.  The schedule (threads per CTA, tile size,
 // CTAs per SM, instance order) comes from qcs_cuda_batch_autotune, which
 // times the candidates on the batch itself.
+//
+// Measured (default schedule, 1024 shots): 384 instances of 10-22 qubits, 4-16
+// layers 100 -> 64 ms against the kernel that kept a thread's amplitudes in
+// C++ variables, read its gates from global memory and scanned 4096 amplitudes
+// a shot; 608 of 13 qubits 33 -> 0.7 ms (the scans were all of it).
 #include <math.h>
 #include <stdio.h>
 #include <string.h>
@@ -41,6 +47,7 @@
 
 #include "common.cuh"
 #include "fusion.h"
+#include "tile_regs.cuh"
 
 namespace qcs {
 
@@ -51,8 +58,6 @@ struct BInst {
   int group;  // CTAs that share the instance's stages (1: one CTA)
 };
 
-// Bounded spin of one thread on a counter another CTA raises: ~2 s.
-
 struct BStage {
   int group0;
   int ngroups;
@@ -61,22 +66,36 @@ struct BStage {
   signed char q[24];  // local bit m -> global qubit (ascending)
 };
 
-// Up to kGroupQ tile bits whose gates run in one pass: each thread holds the
-// 2^r amplitudes of one setting of the other bits in registers and applies
-// the group's gates to them in order.
+// A stage's gates run in groups of consecutive gates on a few tile bits: one
+// pass over shared memory applies a group, each thread holding the amplitudes
+// of one setting of the other bits in registers.  Register bit j is tile bit
+// q[j]; bits the gates leave free are filled with others.  Register bit 0 (the
+// pair bit, tile_regs.cuh) is the one with the fewest 2x2 gates.
+// CTAs of 256 threads hold 2^5 amplitudes a thread: against 2^4 that halves
+// the dispatch per amplitude and takes a tenth of the passes away (304
+// instances of 18 qubits, 10 layers: 13.7 -> 12.9 ms; 608 of 13 qubits 0.62 ->
+// 0.50).  Larger CTAs have no registers for it (at 1024 threads 0.84 -> 1.28).
+// The order of the gates comes from a greedy partition into groups on at most
+// kGroupQ qubits, and one-qubit gates fold into one 2x2 within those.
 constexpr int kGroupQ = 4;
-struct BGroup {
+constexpr int kMaxRegQ = 5;
+constexpr int reg_q(int threads) { return threads == 256 ? 5 : 4; }
+struct __align__(16) BGroup {
   int gate0;
   int ngates;
-  int r;                    // group bits
-  signed char q[kGroupQ];   // tile bit of group bit j (ascending)
+  unsigned char q[kMaxRegQ];    // tile bit of register bit j
+  unsigned char asc[kMaxRegQ];  // the same tile bits, ascending
+  unsigned char pad[6];
 };
 
-struct BGate {
-  float2 m[4];
-  int type;  // 0: 2x2 on group bit t; 1: 2x2 on group bit t where bit c is set
-  int t, c;
-  int form;  // 0: dense; 1: exchange (X, CNOT: m = [[0,1],[1,0]]); 2: diagonal
+// A planned gate.  p: a 2x2's four complex entries (dense), its two diagonal
+// ones (diag) or the phase.
+enum { BG_DENSE = 0, BG_EXCH = 8, BG_DIAG = 16, BG_PHASE = 24 };  // + register bit
+struct __align__(16) BGate {
+  float p[8];
+  int op;    // BG_* + target register bit (BG_PHASE: no addition)
+  int cond;  // register bits that must be set (exchange: the control or 0)
+  int pad[2];
 };
 
 struct BatchTune {
@@ -110,7 +129,7 @@ struct qcs_cuda_batch {
   std::vector<int> order;         // instance order
   std::vector<int2> items;        // (instance, member) in queue order
   qcs::BatchTune tune;
-  int planned_tile_q;
+  int planned_tile_q, planned_regs;
   // device
   cudaStream_t stream;
   qcs::DeviceInfo dev;
@@ -179,150 +198,354 @@ __device__ double block_sum(double v, double *red) {
   return r;  // valid in thread 0
 }
 
-// Shared-memory position of tile amplitude i: the low 4 bits are XORed with
-// the next 4, a bijection that spreads a warp's accesses over the banks
-// whichever tile bits a gate group holds (without it, a group on bits 0..3
-// sends all 32 lanes of a warp to one bank).
-__device__ __forceinline__ int swz(int i) { return i ^ ((i >> 4) & 15); }
+// The groups of a stage and their gates, as far as they fit: a window copied to
+// shared memory, where the tiles that stream through L1 do not push them out.
+// A stage that fits whole is copied once for all its tiles; a longer one moves
+// the window along.  (Kept there as packed operands, twelve of them, the
+// constants of a gate did not fit the registers any more: 12.8 -> 14.0 ms for
+// 304 instances of 18 qubits.)
+constexpr int kWinGroups = 64, kWinGates = 256;
+struct BWindow {
+  BGate gate[kWinGates];
+  BGroup group[kWinGroups];
+};
 
-// One 2x2 on register bit TB of the R amplitudes a[] (controlled: only where
-// register bit c is set).  Static indices keep a[] in registers.
-template <int R, int TB>
-__device__ __forceinline__ void reg_gate(float2 (&a)[1 << kGroupQ], const BGate &g) {
-  if (g.form == 1) {  // exchange: no arithmetic
-#pragma unroll
-    for (int e = 0; e < R; e++) {
-      if (e & (1 << TB)) continue;
-      if (g.type && !((e >> g.c) & 1)) continue;
-      const float2 v0 = a[e];
-      a[e] = a[e | (1 << TB)];
-      a[e | (1 << TB)] = v0;
-    }
-  } else if (g.form == 2) {  // diagonal: one complex product per amplitude
-#pragma unroll
-    for (int e = 0; e < R; e++) {
-      if (e & (1 << TB)) continue;
-      if (g.type && !((e >> g.c) & 1)) continue;
-      a[e] = cmul(g.m[0], a[e]);
-      a[e | (1 << TB)] = cmul(g.m[3], a[e | (1 << TB)]);
-    }
-  } else {
-#pragma unroll
-    for (int e = 0; e < R; e++) {
-      if (e & (1 << TB)) continue;
-      if (g.type && !((e >> g.c) & 1)) continue;
-      const float2 v0 = a[e], v1 = a[e | (1 << TB)];
-      a[e] = cadd(cmul(g.m[0], v0), cmul(g.m[1], v1));
-      a[e | (1 << TB)] = cadd(cmul(g.m[2], v0), cmul(g.m[3], v1));
-    }
-  }
+// X on register bit TB under the control mask `cond` (one bit, or none).
+template <int TB, int RB>
+__device__ __forceinline__ void batch_exchange(RegsF32<RB> &a, int cond) {
+  each<RB>([&](auto cc) {
+    constexpr int CB = decltype(cc)::value;
+    if constexpr (CB != TB)
+      if (cond == 1 << CB) a.template exchange<TB, CB>();
+  });
+  if (cond == 0) a.template exchange<TB, -1>();
 }
 
-// Apply one group to a tile of 2^nt amplitudes in shared memory.
-template <int T, int RB>
-__device__ __forceinline__ void smem_group_r(float2 *S, int nt, const BGroup &G,
-                                             const BGate *gates) {
-  constexpr int R = 1 << RB;
-  const int np = 1 << (nt - RB);
-  int qb[kGroupQ];
-#pragma unroll
-  for (int j = 0; j < RB; j++) qb[j] = G.q[j];
-  for (int p = threadIdx.x; p < np; p += T) {
-    int base = p;
-#pragma unroll
-    for (int j = 0; j < RB; j++)  // ascending: insert a zero at tile bit qb[j]
-      base = ((base >> qb[j]) << (qb[j] + 1)) | (base & ((1 << qb[j]) - 1));
-    // offset of register e: base with group bit j of e at tile bit qb[j]
-    auto off = [&](int e) {
-      int o = base;
-#pragma unroll
-      for (int j = 0; j < RB; j++)
-        if ((e >> j) & 1) o |= 1 << qb[j];
-      return o;
-    };
-    float2 a[1 << kGroupQ];
-#pragma unroll
-    for (int e = 0; e < R; e++) a[e] = S[swz(off(e))];
-    for (int gi = 0; gi < G.ngates; gi++) {
-      const BGate g = gates[G.gate0 + gi];
-      switch (g.t) {
-        case 0: reg_gate<R, 0>(a, g); break;
-        case 1: if constexpr (RB > 1) reg_gate<R, 1>(a, g); break;
-        case 2: if constexpr (RB > 2) reg_gate<R, 2>(a, g); break;
-        default: if constexpr (RB > 3) reg_gate<R, 3>(a, g); break;
-      }
+template <int RB>
+__device__ __forceinline__ void batch_gate(RegsF32<RB> &a, const BGate &g) {
+  const float4 x = *reinterpret_cast<const float4 *>(g.p);
+  const float4 y = *reinterpret_cast<const float4 *>(g.p + 4);
+  const float k[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+  const int op = g.op;
+  auto target = [&](auto &&f) {  // f(target bit), as a constant
+    if (RB > 4 && (op & 4)) f(std::integral_constant<int, RB - 1>());
+    else if (op & 2) {
+      if (op & 1) f(std::integral_constant<int, 3>());
+      else f(std::integral_constant<int, 2>());
+    } else {
+      if (op & 1) f(std::integral_constant<int, 1>());
+      else f(std::integral_constant<int, 0>());
     }
+  };
+  if (op < BG_EXCH) target([&](auto tb) { a.template dense<decltype(tb)::value>(k); });
+  else if (op < BG_DIAG) target([&](auto tb) { batch_exchange<decltype(tb)::value>(a, g.cond); });
+  else if (op < BG_PHASE) target([&](auto tb) { a.template diag<decltype(tb)::value>(k); });
+  else a.phase_where(k, g.cond);
+}
+
+// Apply one group to a tile of 2^nt amplitudes (nt >= RB) in shared memory.
+template <int T, int RB>
+__device__ __forceinline__ void smem_group(float *S, int nt, const BGroup &G, const BGate *gates) {
+  constexpr int N = 1 << RB;
+  const int L = 1 << nt, np = L >> RB;
+  const float2 kind = {};
+  int m[RB];
 #pragma unroll
-    for (int e = 0; e < R; e++) S[swz(off(e))] = a[e];
+  for (int j = 0; j < RB; j++) m[j] = tile_pos(1 << G.q[j], kind);
+  for (int p = threadIdx.x; p < np; p += T) {
+    int l = p;  // a zero inserted at each register bit, ascending
+#pragma unroll
+    for (int j = 0; j < RB; j++)
+      l = ((l >> G.asc[j]) << (G.asc[j] + 1)) | (l & ((1 << G.asc[j]) - 1));
+    int at = tile_pos(l, kind);
+    auto place = [&](int (&pos)[N]) {
+      int lo[4], hi[N / 4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) lo[k] = at ^ ((k & 1) ? m[0] : 0) ^ ((k & 2) ? m[1] : 0);
+#pragma unroll
+      for (int k = 0; k < N / 4; k++)
+        hi[k] = ((k & 1) ? m[2] : 0) ^ ((k & 2) ? m[3] : 0) ^ ((k & 4) ? m[RB - 1] : 0);
+#pragma unroll
+      for (int e = 0; e < N; e++) pos[e] = lo[e & 3] ^ hi[e >> 2];
+    };
+    RegsF32<RB> a;
+    {
+      int pos[N];
+      place(pos);
+      a.load(S, L, pos);
+    }
+    for (int gi = 0; gi < G.ngates; gi++) batch_gate(a, gates[gi]);
+    asm volatile("" : "+r"(at));  // the positions are formed anew, not kept
+    {
+      int pos[N];
+      place(pos);
+      a.store(S, L, pos);
+    }
   }
 }
 
 template <int T>
-__device__ __forceinline__ void smem_group(float2 *S, int nt, const BGroup &G, const BGate *gates) {
-  switch (G.r) {
-    case 1: smem_group_r<T, 1>(S, nt, G, gates); break;
-    case 2: smem_group_r<T, 2>(S, nt, G, gates); break;
-    case 3: smem_group_r<T, 3>(S, nt, G, gates); break;
-    default: smem_group_r<T, 4>(S, nt, G, gates); break;
+__device__ __forceinline__ void run_groups(float *S, const BStage &st, BWindow &W, int &w0, int &w1,
+                                           const BGroup *groups, const BGate *gates) {
+  const int end = st.group0 + st.ngroups;
+  for (int gi = st.group0; gi < end; gi++) {
+    if (gi < w0 || gi >= w1) {  // (the same decision in every thread)
+      __syncthreads();
+      const int n = end - gi < kWinGroups ? end - gi : kWinGroups;
+      for (int e = threadIdx.x; e < n; e += T) W.group[e] = groups[gi + e];
+      __syncthreads();
+      const int g0 = W.group[0].gate0;
+      int fit = 1;  // a group has at most kWinGates gates
+      while (fit < n && W.group[fit].gate0 + W.group[fit].ngates - g0 <= kWinGates) fit++;
+      const int count = W.group[fit - 1].gate0 + W.group[fit - 1].ngates - g0;
+      const float4 *src = reinterpret_cast<const float4 *>(gates + g0);
+      float4 *dst = reinterpret_cast<float4 *>(W.gate);
+      for (int e = threadIdx.x; e < 3 * count; e += T) dst[e] = src[e];
+      w0 = gi;
+      w1 = gi + fit;
+      __syncthreads();
+    }
+    const BGroup &G = W.group[gi - w0];
+    smem_group<T, reg_q(T)>(S, st.nt, G, W.gate + (G.gate0 - W.group[0].gate0));
+    __syncthreads();
   }
 }
 
-// Shots of one instance: prefix of tile masses in shared memory, one warp per
-// shot, FP64 scan.  amp(i) reads amplitude i (shared or global).
-template <int T, typename AmpFn>
-__device__ void sample_shots(const double *prefix, int n_tiles, int tile, int shots, u64 seed,
-                             int inst, i64 *out, AmpFn amp) {
+// |a|^2 in FP64 (exact products) and in FP32 (as <Z_0> and the masses use it).
+__device__ __forceinline__ double prob64(float2 a) {
+  return (double)a.x * a.x + (double)a.y * a.y;
+}
+__device__ __forceinline__ float prob32(float2 a) { return a.x * a.x + a.y * a.y; }
+
+// Exclusive prefix of x[0 .. m) in shared memory, the total at x[m], by one
+// warp: each lane sums its run of entries, the warp scans the runs.
+__device__ void warp_prefix(double *x, int m) {
+  const int lane = threadIdx.x & 31;
+  const int per = (m + 31) / 32, i0 = lane * per < m ? lane * per : m;
+  const int i1 = i0 + per < m ? i0 + per : m;
+  double s = 0.0;
+  for (int i = i0; i < i1; i++) s += x[i];
+  double incl = s;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  double run = __shfl_up_sync(0xffffffffu, incl, 1);
+  if (lane == 0) run = 0.0;
+  __syncwarp();
+  for (int i = i0; i < i1; i++) {
+    const double v = x[i];
+    x[i] = run;
+    run += v;
+  }
+  const double total = __shfl_sync(0xffffffffu, incl, 31);
+  if (lane == 0) x[m] = total;
+}
+
+constexpr int kSubTile = 32;  // amplitudes per inner step of the resident sampler
+
+// Read-out of an instance that lives in shared memory (L = 2^n amplitudes of
+// a tile of Lt): the blocks of 32 amplitudes, a thread each, give <Z_0>, the
+// sampling tiles' masses (FP32 squares summed in FP64) and each block's mass
+// in FP64; a shot is one thread's work: its tile, then its block by binary
+// search over the tile's running sums, then the block's amplitudes.  (A warp
+// scanning the tile 32 amplitudes at a time took 64 scans a shot, all of
+// them in the FP64 pipe, two lanes wide.)  Returns <Z_0> in thread 0.
+// scratch: 5 + 2 * L / 32 doubles.
+template <int T>
+__device__ double resident_readout(const float *S, int L, int Lt, double *scratch, double *red,
+                                   int shots, u64 seed, int inst, i64 *out) {
+  const float2 kind = {};
+  auto amp = [&](int i) { return tile_get(S, Lt, tile_pos(i, kind)); };
+  const int sub = L < kSubTile ? L : kSubTile, nsub = L / sub;
+  const int tile = L < kMassTile ? L : kMassTile, n_tiles = L / tile, per = tile / sub;
+  double *prefix = scratch, *incl = scratch + 5, *mass = incl + nsub;
+  double z = 0.0;
+  for (int b = threadIdx.x; b < nsub; b += T) {
+    double even = 0.0, odd = 0.0, m = 0.0;
+    for (int k = 0; k < sub; k += 2) {
+      const float2 x = amp(b * sub + k), y = amp(b * sub + k + 1);
+      even += (double)prob32(x);
+      odd += (double)prob32(y);
+      m += prob64(x);
+      m += prob64(y);
+    }
+    incl[b] = m;
+    mass[b] = even + odd;
+    z += even - odd;
+  }
+  z = block_sum<T>(z, red);
+  __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int t = warp; t < n_tiles; t += T / 32) {
+    double m = 0.0;  // the tile's mass
+    for (int b = lane; b < per; b += 32) m += mass[t * per + b];
+    m = bwarp_sum(m);
+    if (lane == 0) prefix[t] = m;
+    // running sums of the tile's blocks: a run of blocks a lane, then a scan
+    const int run = (per + 31) / 32, b0 = t * per + (lane * run < per ? lane * run : per);
+    const int b1 = b0 + run < (t + 1) * per ? b0 + run : (t + 1) * per;
+    double s = 0.0;
+    for (int b = b0; b < b1; b++) s += incl[b];
+    double up = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double y = __shfl_up_sync(0xffffffffu, up, o);
+      if (lane >= o) up += y;
+    }
+    double before = __shfl_up_sync(0xffffffffu, up, 1);
+    if (lane == 0) before = 0.0;
+    for (int b = b0; b < b1; b++) {
+      before += incl[b];
+      incl[b] = before;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double run = 0.0;
+    for (int t = 0; t < n_tiles; t++) {
+      const double m = prefix[t];
+      prefix[t] = run;
+      run += m;
+    }
+    prefix[n_tiles] = run;
+  }
+  __syncthreads();
+  for (int s = threadIdx.x; s < shots; s += T) {
+    const double r = shot_draw(seed, (u64)inst, (u64)s);
+    i64 result = -1;
+    if (r < prefix[n_tiles]) {
+      int t = 0;
+      while (t + 1 < n_tiles && !(r < prefix[t + 1])) t++;
+      const double base = prefix[t];
+      const int first = t * per, end = first + per;
+      int lo = first, hi = end;  // the first block with r < base + its running sum
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (r < base + incl[mid]) hi = mid;
+        else lo = mid + 1;
+      }
+      int from, to;  // where the last nonzero amplitude is taken from, if none is hit
+      if (lo < end) {
+        double cum = lo > first ? base + incl[lo - 1] : base;
+        from = lo * sub;
+        to = from + sub;
+        for (int i = from; i < to; i++) {
+          const double p = prob64(amp(i));
+          cum += p;
+          if (p > 0.0 && r < cum) {
+            result = i;
+            break;
+          }
+        }
+      } else {
+        from = t * tile;
+        to = from + tile;
+      }
+      if (result < 0) {
+        result = from;
+        for (int i = to - 1; i >= from; i--)
+          if (prob64(amp(i)) > 0.0) {
+            result = i;
+            break;
+          }
+      }
+    }
+    out[s] = result;
+  }
+  return z;
+}
+
+// Read-out of an instance in its global slot: a warp takes a sampling tile
+// (<Z_0>, its mass), then a shot: its tile by binary search, and the tile 128
+// amplitudes a step, four a lane (as k_smp_sample).  Returns <Z_0> in thread 0.
+template <int T>
+__device__ double slot_readout(const float2 *slot, i64 size, double *prefix, double *red,
+                               int shots, u64 seed, int inst, i64 *out) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // at most 1024 sampling tiles
+  i64 mtile = size >> 10 > kMassTile ? size >> 10 : kMassTile;
+  if (mtile > size) mtile = size;  // at least 2^11, above the smallest tile
+  const int n_tiles = (int)(size / mtile);
+  double z = 0.0;
+  for (int t = warp; t < n_tiles; t += T / 32) {
+    const float4 *v = reinterpret_cast<const float4 *>(slot + (i64)t * mtile);
+    double even = 0.0, odd = 0.0;
+    for (i64 i = lane; i < mtile / 2; i += 128) {  // four units in flight
+      float4 x[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) x[k] = v[i + 32 * k];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        even += (double)prob32(make_float2(x[k].x, x[k].y));
+        odd += (double)prob32(make_float2(x[k].z, x[k].w));
+      }
+    }
+    even = bwarp_sum(even);
+    odd = bwarp_sum(odd);
+    if (lane == 0) prefix[t] = even + odd;
+    z += lane == 0 ? even - odd : 0.0;
+  }
+  z = block_sum<T>(z, red);
+  __syncthreads();
+  if (warp == 0) warp_prefix(prefix, n_tiles);
+  __syncthreads();
   for (int s = warp; s < shots; s += T / 32) {
     const double r = shot_draw(seed, (u64)inst, (u64)s);
     i64 result = -1;
     if (r < prefix[n_tiles]) {
       int lo = 0, hi = n_tiles - 1;
       while (lo < hi) {
-        int mid = (lo + hi) >> 1;
+        const int mid = (lo + hi) >> 1;
         if (r < prefix[mid + 1]) hi = mid;
         else lo = mid + 1;
       }
       double cum = prefix[lo];
-      i64 last_nonzero = (i64)lo * tile;
-      for (i64 base = (i64)lo * tile; base < (i64)(lo + 1) * tile && result < 0; base += 32) {
-        double p = 0.0;
-        if (lane < tile) {
-          float2 a = amp(base + lane);
-          p = (double)a.x * a.x + (double)a.y * a.y;
+      const i64 first = (i64)lo * mtile, end = first + mtile;
+      const float4 *v = reinterpret_cast<const float4 *>(slot + first) + 2 * lane;
+      float4 n0 = v[0], n1 = v[1];
+      for (i64 base = first; base < end && result < 0; base += 128) {
+        const float4 a = n0, b = n1;
+        v += 64;
+        if (base + 128 < end) {
+          n0 = v[0];
+          n1 = v[1];
         }
-        double incl = p;
+        double sum[4];
+        sum[0] = prob64(make_float2(a.x, a.y));
+        sum[1] = sum[0] + prob64(make_float2(a.z, a.w));
+        sum[2] = sum[1] + prob64(make_float2(b.x, b.y));
+        sum[3] = sum[2] + prob64(make_float2(b.z, b.w));
+        double incl = sum[3];
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-          double y = __shfl_up_sync(0xffffffffu, incl, o);
+          const double y = __shfl_up_sync(0xffffffffu, incl, o);
           if (lane >= o) incl += y;
         }
-        unsigned hit = __ballot_sync(0xffffffffu, lane < tile && r < cum + incl);
-        unsigned nz = __ballot_sync(0xffffffffu, lane < tile && p > 0.0);
-        if (hit) result = base + __ffs(hit) - 1;
-        else if (nz) last_nonzero = base + 31 - __clz(nz);
+        const unsigned hit = __ballot_sync(0xffffffffu, r < cum + incl);
+        if (hit) {  // in the first lane whose running sum exceeds r
+          const int at = __ffs(hit) - 1;
+          double before = __shfl_up_sync(0xffffffffu, incl, 1);
+          before = lane == 0 ? cum : cum + before;
+          int k = 0;
+          while (k < 3 && !(r < before + sum[k])) k++;
+          while (k > 0 && sum[k] == sum[k - 1]) k--;  // not one of no mass
+          result = base + 4 * at + __shfl_sync(0xffffffffu, k, at);
+        }
         cum += __shfl_sync(0xffffffffu, incl, 31);
       }
-      if (result < 0) result = last_nonzero;
+      if (result < 0) {  // the tile's last nonzero amplitude
+        result = first;
+        for (i64 base = first; base < end; base += 32) {
+          const unsigned m = __ballot_sync(0xffffffffu, prob64(slot[base + lane]) > 0.0);
+          if (m) result = base + 31 - __clz(m);
+        }
+      }
     }
     if (lane == 0) out[s] = result;
   }
-}
-
-// Exclusive prefix of m values in shared memory (m <= 1024), total at [m].
-template <int T>
-__device__ void smem_prefix(double *x, int m) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double run = 0.0;
-    for (int i = 0; i < m; i++) {
-      const double t = x[i];
-      x[i] = run;
-      run += t;
-    }
-    x[m] = run;
-  }
-  __syncthreads();
+  return z;
 }
 
 // Thread 0 waits until *cnt >= target, at most `limit` clock cycles; false
@@ -341,25 +564,28 @@ __device__ bool wait_count(const int *cnt, int target, int *err, int where, long
   return true;
 }
 
-// 64 registers a thread: two CTAs of 512 threads (or one of 1024) fit an SM.
 // Work items are (instance, member): an instance of `group` > 1 is shared by
 // `group` CTAs that split the tiles of each stage and meet at a counter
 // after every stage; the grid never exceeds the CTAs that fit the GPU at
 // once, so every member of a group runs concurrently with the others.
 template <int T>
-__global__ void __launch_bounds__(T, 1024 / T)
+__global__ void __launch_bounds__(T, T == 256 ? 2 : 1)
     k_batch(const BInst *insts, const BStage *stages, const BGroup *groups, const BGate *gates,
             const int2 *items, int n_items, int shots, u64 seed, int tile_q, float2 *slots,
             i64 slot_amps, int *queue, int *stage_done, int *lead, int *err, double *z_out,
             i64 *samples_out, long long wait) {
+  QCS_REGS_F32_DECLARE(1 << (reg_q(T) - 1));
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2 *S = reinterpret_cast<float2 *>(smem_raw);               // 2^tile_q amplitudes
-  double *prefix = reinterpret_cast<double *>(S + (1 << tile_q));  // up to 1025 tile masses
+  float *S = reinterpret_cast<float *>(smem_raw);                      // 2^tile_q amplitudes
+  BWindow &W = *reinterpret_cast<BWindow *>(S + (2 << tile_q));
+  double *scratch = reinterpret_cast<double *>(&W + 1);  // of the read-outs
   __shared__ double red[T / 32];
   __shared__ int s_item;
   __shared__ int s_ok;
-  __shared__ i64 goff_lo[64];
-  __shared__ i64 goff_hi[256];
+  // of the stage: a thread's accesses to a tile, and the tile's base by
+  // nibbles of its number
+  __shared__ i64 step_off[64], nib[4][16];
+  const float2 kind = {};
 
   for (;;) {
     __syncthreads();
@@ -373,6 +599,7 @@ __global__ void __launch_bounds__(T, 1024 / T)
     const int G = I.group;
     const i64 size = 1LL << I.n;
     double z = 0.0;
+    int w0 = 0, w1 = 0;  // groups in the window
     // the instance's amplitudes live in the slot of its member-0 CTA
     float2 *slot = slots + (i64)blockIdx.x * slot_amps;
     if (G > 1) {
@@ -388,86 +615,92 @@ __global__ void __launch_bounds__(T, 1024 / T)
       if (!s_ok) return;
       slot = slots + (i64)(*(volatile int *)&lead[inst] - 1) * slot_amps;
     }
+    i64 *out = samples_out + (i64)inst * shots;
     if (I.n <= tile_q) {
-      // ---- shared-memory resident instance ----
-      const int L = 1 << I.n;
-      for (int i = threadIdx.x; i < L; i += T) S[swz(i)] = make_float2(i == 0 ? 1.f : 0.f, 0.f);
-      __syncthreads();
+      // ---- shared-memory resident instance (a tile of at least 2^kMaxRegQ) ----
       const BStage st = stages[I.stage0];
-      for (int gi = 0; gi < st.ngroups; gi++) {
-        smem_group<T>(S, I.n, groups[st.group0 + gi], gates);
-        __syncthreads();
-      }
-      const int tile = L < kMassTile ? L : kMassTile;
-      const int n_tiles = L / tile;
-      for (int t = 0; t < n_tiles; t++) {
-        double zp = 0.0, mp = 0.0;
-        for (int j = threadIdx.x; j < tile; j += T) {
-          const int i = t * tile + j;
-          const float2 a = S[swz(i)];
-          const float p = a.x * a.x + a.y * a.y;
-          mp += (double)p;
-          zp += (i & 1) ? -(double)p : (double)p;
-        }
-        const double ms = block_sum<T>(mp, red);
-        const double zs = block_sum<T>(zp, red);
-        if (threadIdx.x == 0) {
-          prefix[t] = ms;
-          z += zs;
-        }
-      }
-      smem_prefix<T>(prefix, n_tiles);
-      sample_shots<T>(prefix, n_tiles, tile, shots, seed, inst, samples_out + (i64)inst * shots,
-                      [&](i64 i) { return S[swz((int)i)]; });
+      const int Lt = 1 << st.nt;
+      for (int i = threadIdx.x; i < 2 * Lt; i += T) S[i] = i == 0 ? 1.f : 0.f;  // position 0
+      __syncthreads();
+      run_groups<T>(S, st, W, w0, w1, groups, gates);
+      z = resident_readout<T>(S, (int)size, Lt, scratch, red, shots, seed, inst, out);
     } else {
       // ---- global-slot instance, run in stages ----
       for (int si = 0; si < I.nstages; si++) {
         const BStage st = stages[I.stage0 + si];
-        const int nt = st.nt;
-        const int L = 1 << nt;
-        // offset tables for this stage: local index l = lo | hi << 6
+        const int nt = st.nt, L = 1 << nt;
+        // A thread moves units of two amplitudes (16 bytes; tile bit 0 is
+        // qubit 0): unit t + k T, whose offset is that of t plus that of k T.
+        const int nout = I.n - nt;  // qubits outside the tile: the tile number's bits
+        const int steps = L / 2 > T ? L / 2 / T : 1;
         __syncthreads();
-        for (int e = threadIdx.x; e < 64 + 256; e += T) {
-          const bool is_lo = e < 64;
-          const int v = is_lo ? e : e - 64;
-          i64 o = 0;
-          for (int m = 0; m < nt; m++) {
-            const int bit = is_lo ? m : m - 6;
-            if ((is_lo && m < 6) || (!is_lo && m >= 6))
-              if ((v >> bit) & 1) o |= 1LL << st.q[m];
-          }
-          if (is_lo) goff_lo[v] = o;
-          else goff_hi[v] = o;
-        }
-        __syncthreads();
-        // qubits outside the tile, ascending: the tile id's bits
-        i64 outside[40];
-        int nout = 0;
-        {
-          int k = 0;
-          for (int q = 0; q < I.n; q++) {
-            if (k < nt && st.q[k] == q) {
-              k++;
-              continue;
+        for (int e = threadIdx.x; e < 64 + 64; e += T) {
+          if (e < 64) {
+            i64 o = 0;
+            for (int m = 0; m < nt; m++)
+              if (((e * T * 2) >> m) & 1) o |= 1LL << st.q[m];
+            step_off[e] = o;
+          } else {
+            const int k = (e - 64) >> 4, v = (e - 64) & 15;
+            i64 o = 0;
+            int j = 0, in = 0;
+            for (int q = 0; q < I.n; q++) {
+              if (in < nt && st.q[in] == q) {
+                in++;
+                continue;
+              }
+              if ((j >> 2) == k && ((v >> (j & 3)) & 1)) o |= 1LL << q;
+              j++;
             }
-            outside[nout++] = q;
+            nib[k][v] = o;
           }
         }
-        const i64 n_tiles = 1LL << nout;
-        for (i64 tt = member; tt < n_tiles; tt += G) {
-          i64 base = 0;
-          for (int j = 0; j < nout; j++) base |= ((tt >> j) & 1LL) << outside[j];
-          for (int l = threadIdx.x; l < L; l += T) {
-            const i64 gidx = base + goff_lo[l & 63] + goff_hi[l >> 6];
-            S[swz(l)] = si == 0 ? make_float2(gidx == 0 ? 1.f : 0.f, 0.f) : slot[gidx];
+        const int i0 = 2 * threadIdx.x;  // this thread's first amplitude
+        i64 toff = 0;
+        for (int m = 1; m < nt; m++)
+          if ((i0 >> m) & 1) toff |= 1LL << st.q[m];
+        const int tpos = tile_pos(i0, kind);
+        const bool active = i0 < L;
+        __syncthreads();
+        const int n_tiles = 1 << nout;
+        for (int tt = member; tt < n_tiles; tt += G) {
+          i64 base = nib[0][tt & 15] + nib[1][(tt >> 4) & 15] + nib[2][(tt >> 8) & 15] +
+                     nib[3][(tt >> 12) & 15];
+          float2 *vt = slot + base + toff;
+          if (si == 0) {  // |0...0>
+            for (int i = threadIdx.x; i < 2 * L; i += T) S[i] = tt == 0 && i == 0 ? 1.f : 0.f;
+          } else if (active) {
+            for (int k0 = 0; k0 < steps; k0 += 4) {
+              float4 x[4];
+#pragma unroll
+              for (int k = 0; k < 4; k++)
+                if (k0 + k < steps)
+                  x[k] = __ldcg(reinterpret_cast<const float4 *>(vt + step_off[k0 + k]));
+#pragma unroll
+              for (int k = 0; k < 4; k++) {
+                if (k0 + k >= steps) break;
+                const int at = tpos ^ tile_pos((k0 + k) * T * 2, kind);
+                tile_put(S, L, at, make_float2(x[k].x, x[k].y));
+                tile_put(S, L, at ^ 1, make_float2(x[k].z, x[k].w));
+              }
+            }
           }
           __syncthreads();
-          for (int gi = 0; gi < st.ngroups; gi++) {
-            smem_group<T>(S, nt, groups[st.group0 + gi], gates);
-            __syncthreads();
+          if (si > 0 && active && tt + G < n_tiles) {  // the next tile, towards L2
+            const int t2 = tt + G;
+            const float2 *vn = slot + nib[0][t2 & 15] + nib[1][(t2 >> 4) & 15] +
+                               nib[2][(t2 >> 8) & 15] + nib[3][(t2 >> 12) & 15] + toff;
+            for (int k = 0; k < steps; k++)
+              asm volatile("prefetch.global.L2 [%0];" ::"l"(vn + step_off[k]));
           }
-          for (int l = threadIdx.x; l < L; l += T)
-            slot[base + goff_lo[l & 63] + goff_hi[l >> 6]] = S[swz(l)];
+          run_groups<T>(S, st, W, w0, w1, groups, gates);
+          if (active) {
+            for (int k = 0; k < steps; k++) {
+              const int at = tpos ^ tile_pos(k * T * 2, kind);
+              const float2 x = tile_get(S, L, at), y = tile_get(S, L, at ^ 1);
+              *reinterpret_cast<float4 *>(vt + step_off[k]) = make_float4(x.x, x.y, y.x, y.y);
+            }
+          }
           __syncthreads();
         }
         if (G > 1) {  // every member's tiles of this stage are written
@@ -485,29 +718,7 @@ __global__ void __launch_bounds__(T, 1024 / T)
       if (member != 0) continue;  // member 0 reads out the instance
       __threadfence_block();
       __syncthreads();
-      // <Z_0> and tile masses in one contiguous pass (deterministic order);
-      // at most 1024 sampling tiles
-      const i64 mtile = size >> 10 > kMassTile ? size >> 10 : kMassTile;
-      const int n_tiles = (int)(size / mtile);
-      for (int t = 0; t < n_tiles; t++) {
-        double zp = 0.0, mp = 0.0;
-        for (i64 j = threadIdx.x; j < mtile; j += T) {
-          const i64 i = (i64)t * mtile + j;
-          const float2 a = slot[i];
-          const float p = a.x * a.x + a.y * a.y;
-          mp += (double)p;
-          zp += (i & 1) ? -(double)p : (double)p;
-        }
-        const double ms = block_sum<T>(mp, red);
-        const double zs = block_sum<T>(zp, red);
-        if (threadIdx.x == 0) {
-          prefix[t] = ms;
-          z += zs;
-        }
-      }
-      smem_prefix<T>(prefix, n_tiles);
-      sample_shots<T>(prefix, n_tiles, (int)mtile, shots, seed, inst,
-                      samples_out + (i64)inst * shots, [&](i64 i) { return slot[i]; });
+      z = slot_readout<T>(slot, size, scratch, red, shots, seed, inst, out);
     }
     if (threadIdx.x == 0) z_out[inst] = z;
   }
@@ -517,11 +728,13 @@ __global__ void __launch_bounds__(T, 1024 / T)
 // host side
 // ---------------------------------------------------------------------------
 
-// The gates of one stage (op indices in order) on tile qubits tq (ascending)
-// as register groups of at most kGroupQ tile bits: a greedy partition of the
-// stage's gates (commuting only past gates on disjoint qubits).
+// The gates of one stage (op indices in order) on tile qubits tq (ascending):
+// a greedy partition into groups on at most kGroupQ qubits (commuting only past
+// gates on disjoint qubits) gives their order and the one-qubit gates that
+// fold into one 2x2; the sequence is then cut, in order, into register groups
+// on at most `regs` tile bits (and of as many gates as the window holds).
 static void plan_groups(qcs_cuda_batch *b, const std::vector<int> &stage_ops, int n,
-                        const std::vector<int> &tq, BStage &st) {
+                        const std::vector<int> &tq, int regs, BStage &st) {
   st.group0 = (int)b->groups.size();
   std::vector<qcs_cuda_op> sub(stage_ops.size());
   for (size_t j = 0; j < stage_ops.size(); j++) sub[j] = b->ops[stage_ops[j]];
@@ -535,52 +748,66 @@ static void plan_groups(qcs_cuda_batch *b, const std::vector<int> &stage_ops, in
       if (tq[m] == q) return (int)m;
     return -1;
   };
+  struct Planned {
+    std::vector<int> ops;  // that it folds
+    int t, c;              // tile bits (c: -1 for one-qubit gates)
+  };
+  std::vector<Planned> seq;
   for (const PlanItem &it : items) {
+    // pending[m]: the one-qubit gate on tile bit m that later one-qubit gates
+    // on m fold into, -1 after a two-qubit gate touched m
+    std::vector<int> pending(st.nt, -1);
+    for (int g : it.gates) {
+      const qcs_cuda_op &o = sub[g];
+      const int t = tile_bit(o.target);
+      if (gate_is_controlled(o.kind)) {
+        const int c = tile_bit(o.control);
+        pending[t] = pending[c] = -1;
+        seq.push_back({{stage_ops[g]}, t, c});
+      } else if (pending[t] >= 0) {
+        seq[pending[t]].ops.push_back(stage_ops[g]);
+      } else {
+        pending[t] = (int)seq.size();
+        seq.push_back({{stage_ops[g]}, t, -1});
+      }
+    }
+  }
+  for (size_t first = 0; first < seq.size();) {
+    std::vector<int> bits, uses(st.nt, 0);
+    size_t last = first;
+    for (; last < seq.size(); last++) {
+      const Planned &g = seq[last];
+      std::vector<int> more;
+      for (int m : {g.t, g.c})
+        if (m >= 0 && std::find(bits.begin(), bits.end(), m) == bits.end()) more.push_back(m);
+      if (bits.size() + more.size() > (size_t)regs || last - first == kWinGates) break;
+      bits.insert(bits.end(), more.begin(), more.end());
+      if (g.c < 0) uses[g.t]++;
+    }
+    // register bits: first tile bits that no gate touches (the highest ones, so
+    // that a warp's lanes keep the low ones), then those with the fewest 2x2s
+    std::stable_sort(bits.begin(), bits.end(), [&](int x, int y) { return uses[x] < uses[y]; });
+    for (int m = st.nt - 1; (int)bits.size() < regs; m--)
+      if (std::find(bits.begin(), bits.end(), m) == bits.end()) bits.insert(bits.begin(), m);
     BGroup G;
     memset(&G, 0, sizeof(G));
     G.gate0 = (int)b->gate_tc.size();
-    G.r = (int)it.qubits.size();
-    for (int j = 0; j < G.r; j++) G.q[j] = (signed char)tile_bit(it.qubits[j]);
-    auto group_bit = [&](int q) {
-      for (int j = 0; j < G.r; j++)
-        if (it.qubits[j] == q) return j;
-      return -1;
-    };
-    // gates of the group in order; pending[j]: index (in this group's gate
-    // list) of the one-qubit gate on group bit j that later one-qubit gates
-    // on j fold into, -1 after a two-qubit gate touched j
-    std::vector<std::vector<int>> glist;
-    std::vector<int> gtc;
-    int pending[kGroupQ];
-    for (int j = 0; j < kGroupQ; j++) pending[j] = -1;
-    for (int g : it.gates) {
-      const qcs_cuda_op &o = sub[g];
-      const int t = group_bit(o.target);
-      if (gate_is_controlled(o.kind)) {
-        const int c = group_bit(o.control);
-        pending[t] = pending[c] = -1;
-        glist.push_back({stage_ops[g]});
-        gtc.push_back(t | (c << 8));
-      } else if (pending[t] >= 0) {
-        glist[pending[t]].push_back(stage_ops[g]);
-      } else {
-        pending[t] = (int)glist.size();
-        glist.push_back({stage_ops[g]});
-        gtc.push_back(t | (0xFF << 8));
-      }
-    }
-    for (size_t e = 0; e < glist.size(); e++) {
+    G.ngates = (int)(last - first);
+    for (int j = 0; j < regs; j++) G.q[j] = G.asc[j] = (unsigned char)bits[j];
+    std::sort(G.asc, G.asc + regs);
+    auto reg = [&](int m) { return (int)(std::find(bits.begin(), bits.end(), m) - bits.begin()); };
+    for (; first < last; first++) {
+      const Planned &g = seq[first];
       b->fold_off.push_back((int)b->fold_ops.size());
-      for (int op : glist[e]) b->fold_ops.push_back(op);
-      b->gate_tc.push_back(gtc[e]);
+      b->fold_ops.insert(b->fold_ops.end(), g.ops.begin(), g.ops.end());
+      b->gate_tc.push_back(reg(g.t) | (g.c < 0 ? 0xFF : reg(g.c)) << 8);
     }
-    G.ngates = (int)b->gate_tc.size() - G.gate0;
     b->groups.push_back(G);
   }
   st.ngroups = (int)b->groups.size() - st.group0;
 }
 
-static int batch_plan(qcs_cuda_batch *b, int tile_q) {
+static int batch_plan(qcs_cuda_batch *b, int tile_q, int regs) {
   b->insts.clear();
   b->stages.clear();
   b->groups.clear();
@@ -597,12 +824,12 @@ static int batch_plan(qcs_cuda_batch *b, int tile_q) {
     if (I.n <= tile_q) {
       BStage st;
       memset(&st, 0, sizeof(st));
-      st.nt = I.n;
+      st.nt = std::max(I.n, kMaxRegQ);  // qubits a smaller instance lacks stay 0
       std::vector<int> tq(I.n), stage_ops(nops);
       std::iota(tq.begin(), tq.end(), 0);
       std::iota(stage_ops.begin(), stage_ops.end(), b->op_off[i]);
       for (int m = 0; m < I.n; m++) st.q[m] = (signed char)m;
-      plan_groups(b, stage_ops, I.n, tq, st);
+      plan_groups(b, stage_ops, I.n, tq, regs, st);
       b->stages.push_back(st);
       I.nstages = 1;
     } else {
@@ -635,7 +862,7 @@ static int batch_plan(qcs_cuda_batch *b, int tile_q) {
         for (int m = 0; m < st.nt; m++) st.q[m] = (signed char)tq[m];
         std::vector<int> stage_ops;
         for (int g : it.gates) stage_ops.push_back(b->op_off[i] + g);
-        plan_groups(b, stage_ops, I.n, tq, st);
+        plan_groups(b, stage_ops, I.n, tq, regs, st);
         b->stages.push_back(st);
       }
       I.nstages = (int)plan.size();
@@ -644,6 +871,7 @@ static int batch_plan(qcs_cuda_batch *b, int tile_q) {
   }
   b->fold_off.push_back((int)b->fold_ops.size());
   b->planned_tile_q = tile_q;
+  b->planned_regs = regs;
   return QCS_CUDA_OK;
 }
 
@@ -674,16 +902,32 @@ static void batch_fill_gates(qcs_cuda_batch *b) {
     }
     BGate g;
     memset(&g, 0, sizeof(g));
-    for (int e = 0; e < 4; e++) g.m[e] = make_float2((float)acc[2 * e], (float)acc[2 * e + 1]);
-    g.type = gate_is_controlled(kind) ? 1 : 0;
     // exact zeros decide the form: the exchange and diagonal paths give the
-    // same numbers as the dense one (the skipped terms are products with 0)
+    // same numbers as the dense one (the skipped terms are products with 0),
+    // and a controlled phase leaves the amplitudes its 1 would multiply
     const bool off0 = acc[2] == 0.0 && acc[3] == 0.0 && acc[4] == 0.0 && acc[5] == 0.0;
     const bool swap = acc[0] == 0.0 && acc[1] == 0.0 && acc[6] == 0.0 && acc[7] == 0.0 &&
                       acc[2] == 1.0 && acc[3] == 0.0 && acc[4] == 1.0 && acc[5] == 0.0;
-    g.form = swap ? 1 : (off0 ? 2 : 0);
-    g.t = b->gate_tc[gi] & 0xFF;
-    g.c = g.type ? (b->gate_tc[gi] >> 8) & 0xFF : 0;
+    const int t = b->gate_tc[gi] & 0xFF;
+    const int c = gate_is_controlled(kind) ? (b->gate_tc[gi] >> 8) & 0xFF : -1;
+    if (swap) {
+      g.op = BG_EXCH + t;
+      g.cond = c >= 0 ? 1 << c : 0;
+    } else if (c >= 0) {  // CPHASE
+      g.op = BG_PHASE;
+      g.cond = 1 << t | 1 << c;
+      g.p[0] = (float)acc[6];
+      g.p[1] = (float)acc[7];
+    } else if (off0) {
+      g.op = BG_DIAG + t;
+      g.p[0] = (float)acc[0];
+      g.p[1] = (float)acc[1];
+      g.p[2] = (float)acc[6];
+      g.p[3] = (float)acc[7];
+    } else {
+      g.op = BG_DENSE + t;
+      for (int e = 0; e < 8; e++) g.p[e] = (float)acc[e];
+    }
     b->h_gates[gi] = g;
   }
 }
@@ -705,7 +949,12 @@ static void batch_free_device(qcs_cuda_batch *b) {
   b->d_items = nullptr;
 }
 
-static size_t smem_for(int tile_q) { return ((size_t)8 << tile_q) + 1025 * sizeof(double); }
+// The tile, the window of gates, then scratch of the read-outs: 1025 prefixes of a slot's sampling
+// tiles, or 5 + 2 * 2^tile_q / 32 doubles of a resident instance.
+static size_t smem_for(int tile_q) {
+  const size_t blocks = 5 + 2 * (((size_t)1 << tile_q) / kSubTile);
+  return ((size_t)8 << tile_q) + sizeof(BWindow) + std::max<size_t>(1025, blocks) * sizeof(double);
+}
 
 template <int T>
 static int set_smem_attr(int tile_q) {
@@ -836,7 +1085,8 @@ static int batch_capture(qcs_cuda_batch *b) {
 static int batch_apply_tune(qcs_cuda_batch *b, const BatchTune &t) {
   b->tune = t;
   int rc = QCS_CUDA_OK;
-  if (b->planned_tile_q != t.tile_q) rc = batch_plan(b, t.tile_q);
+  if (b->planned_tile_q != t.tile_q || b->planned_regs != reg_q(t.threads))
+    rc = batch_plan(b, t.tile_q, reg_q(t.threads));
   if (!rc) rc = batch_upload(b);
   if (!rc) rc = batch_capture(b);
   return rc;
@@ -945,7 +1195,7 @@ int qcs_cuda_batch_create(int count, const int *num_qubits, const int *op_offset
     if (!rc) rc = check_cuda(cudaMallocHost((void **)&b->h_samples, (size_t)count * shots * sizeof(i64)), "cudaMallocHost(batch)");
   }
   BatchTune t;
-  t.threads = 512;
+  t.threads = 256;
   t.tile_q = 13;
   t.ctas_per_sm = 2;
   t.order = 0;

@@ -34,6 +34,61 @@ __device__ __forceinline__ u64 both2(float s) { return pack2(s, s); }
 // host knows.  Of a plain packed product and a packed sum the assembler makes
 // one fused operation, with one rounding instead of two, .rn or not.
 
+// Shared-memory position of tile amplitude i: its place in the 128-byte row
+// is XORed with the row's number, so that whichever tile bits are held in
+// registers a warp's lanes spread over the banks.  Linear over XOR.
+// (complex64: of a real or imaginary part.)
+__host__ __device__ __forceinline__ int tile_pos(int i, float2) {
+  return i ^ ((i >> 5) & 31) ^ ((i >> 10) & 31);
+}
+__host__ __device__ __forceinline__ int tile_pos(int i, double2) {
+  return i ^ ((i >> 3) & 7) ^ ((i >> 6) & 7) ^ ((i >> 9) & 7);
+}
+
+// One amplitude of a tile of L in shared memory.
+__device__ __forceinline__ float2 tile_get(const float *S, int L, int at) {
+  return make_float2(S[at], S[L + at]);
+}
+__device__ __forceinline__ void tile_put(float *S, int L, int at, float2 v) {
+  S[at] = v.x;
+  S[L + at] = v.y;
+}
+__device__ __forceinline__ double2 tile_get(const double2 *S, int, int at) { return S[at]; }
+__device__ __forceinline__ void tile_put(double2 *S, int, int at, double2 v) { S[at] = v; }
+
+// A gate's constants as packed operands: where the pair bit is the target (tb
+// == 0) or a condition, the two halves take different ones.
+//   dense  own and other entry's x, y, -y: (k0, k1, k2, k3) each for both
+//          halves, or for tb == 0 (k0 | k3) then (k1 | k2)
+//   diag   x, y, -y of k0, then of k1; for tb == 0 of (k0 | k1)
+//   phase  x, y, -y of the phase; 1 + 0 i in the lower half under the pair bit
+__device__ __forceinline__ void pack_factor(u64 *c, float xl, float yl, float xh, float yh) {
+  c[0] = pack2(xl, xh);
+  c[1] = pack2(yl, yh);
+  c[2] = pack2(-yl, -yh);
+}
+__device__ __forceinline__ void pack_dense(u64 *c, int tb, const float *k) {
+  if (tb == 0) {
+    pack_factor(c, k[0], k[1], k[6], k[7]);
+    pack_factor(c + 3, k[2], k[3], k[4], k[5]);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; e++) pack_factor(c + 3 * e, k[2 * e], k[2 * e + 1], k[2 * e], k[2 * e + 1]);
+  }
+}
+__device__ __forceinline__ void pack_diag(u64 *c, int tb, const float *k) {
+  if (tb == 0) {
+    pack_factor(c, k[0], k[1], k[2], k[3]);
+  } else {
+    pack_factor(c, k[0], k[1], k[0], k[1]);
+    pack_factor(c + 3, k[2], k[3], k[2], k[3]);
+  }
+}
+__device__ __forceinline__ void pack_phase(u64 *c, int cond, const float *k) {
+  const bool p = cond & 1;
+  pack_factor(c, p ? 1.f : k[0], p ? 0.f : k[1], k[0], k[1]);
+}
+
 // f(0), f(1), ... f(N - 1), the argument a constant.
 template <int N, int I = 0, typename F>
 __device__ __forceinline__ void each(F &&f) {
@@ -122,6 +177,87 @@ template <int RB> struct RegsF32 {
     }
   }
 
+  // A 2x2 with the four complex entries k on register bit TB.
+  template <int TB>
+  __device__ __forceinline__ void dense(const float *f) {
+    u64 k[12];
+    pack_dense(k, TB, f);
+    if constexpr (TB == 0) {
+      const u64 ax = k[0], ay = k[1], an = k[2], bx = k[3], by = k[4], bn = k[5];
+      each<U>([&](auto uc) {
+        constexpr int u = decltype(uc)::value;
+        asm volatile(
+            "{\n.reg .b32 l, h;\n.reg .b64 r, i, s, t, v;\n"
+            "mov.b64 {l, h}, qre%0;\nmov.b64 r, {h, l};\n"
+            "mov.b64 {l, h}, qim%0;\nmov.b64 i, {h, l};\n"
+            "mul.rn.f32x2 s, %3, qim%0;\nfma.rn.f32x2 s, %1, qre%0, s;\n"
+            "mul.rn.f32x2 t, %1, qim%0;\nfma.rn.f32x2 t, %2, qre%0, t;\n"
+            "mul.rn.f32x2 v, %6, i;\nfma.rn.f32x2 v, %4, r, v;\nadd.rn.f32x2 qre%0, s, v;\n"
+            "mul.rn.f32x2 v, %4, i;\nfma.rn.f32x2 v, %5, r, v;\nadd.rn.f32x2 qim%0, t, v;\n}"
+            ::"n"(u), "l"(ax), "l"(ay), "l"(an), "l"(bx), "l"(by), "l"(bn));
+      });
+    } else {
+      const u64 ax = k[0], ay = k[1], an = k[2], bx = k[3], by = k[4], bn = k[5];
+      const u64 cx = k[6], cy = k[7], cn = k[8], dx = k[9], dy = k[10], dn = k[11];
+      pairs<TB>([&](auto uc, auto wc) {
+        constexpr int u = decltype(uc)::value, w = decltype(wc)::value;
+        asm volatile(
+            "{\n.reg .b64 s, t, v, x;\n"
+            "mul.rn.f32x2 s, %4, qim%0;\nfma.rn.f32x2 s, %2, qre%0, s;\n"
+            "mul.rn.f32x2 t, %2, qim%0;\nfma.rn.f32x2 t, %3, qre%0, t;\n"
+            "mul.rn.f32x2 v, %7, qim%1;\nfma.rn.f32x2 v, %5, qre%1, v;\nadd.rn.f32x2 s, s, v;\n"
+            "mul.rn.f32x2 v, %5, qim%1;\nfma.rn.f32x2 v, %6, qre%1, v;\nadd.rn.f32x2 t, t, v;\n"
+            "mul.rn.f32x2 v, %10, qim%0;\nfma.rn.f32x2 v, %8, qre%0, v;\n"
+            "mul.rn.f32x2 x, %8, qim%0;\nfma.rn.f32x2 x, %9, qre%0, x;\n"
+            "mov.b64 qre%0, s;\nmov.b64 qim%0, t;\n"
+            "mul.rn.f32x2 s, %13, qim%1;\nfma.rn.f32x2 s, %11, qre%1, s;\n"
+            "mul.rn.f32x2 t, %11, qim%1;\nfma.rn.f32x2 t, %12, qre%1, t;\n"
+            "add.rn.f32x2 qre%1, v, s;\nadd.rn.f32x2 qim%1, x, t;\n}" ::"n"(u), "n"(w), "l"(ax),
+            "l"(ay), "l"(an), "l"(bx), "l"(by), "l"(bn), "l"(cx), "l"(cy), "l"(cn), "l"(dx),
+            "l"(dy), "l"(dn));
+      });
+    }
+  }
+
+  // X on register bit TB, where register bit CB (-1: none) is set
+  template <int TB, int CB>
+  __device__ __forceinline__ void exchange() {
+    static_assert(TB != CB, "control equals target");
+    if constexpr (TB == 0) {
+      each<U>([&](auto uc) {
+        constexpr int u = decltype(uc)::value;
+        if constexpr (CB < 0 || (u >> (CB < 1 ? 0 : CB - 1)) & 1)
+          asm volatile("{\n.reg .b32 l, h;\nmov.b64 {l, h}, qre%0;\nmov.b64 qre%0, {h, l};\n"
+                       "mov.b64 {l, h}, qim%0;\nmov.b64 qim%0, {h, l};\n}" ::"n"(u));
+      });
+    } else {
+      pairs<TB>([&](auto uc, auto wc) {
+        constexpr int u = decltype(uc)::value, w = decltype(wc)::value;
+        if constexpr (CB == 0)  // the upper halves
+          asm volatile("{\n.reg .b32 a, b, c, d;\n"
+                       "mov.b64 {a, b}, qre%0;\nmov.b64 {c, d}, qre%1;\n"
+                       "mov.b64 qre%0, {a, d};\nmov.b64 qre%1, {c, b};\n"
+                       "mov.b64 {a, b}, qim%0;\nmov.b64 {c, d}, qim%1;\n"
+                       "mov.b64 qim%0, {a, d};\nmov.b64 qim%1, {c, b};\n}" ::"n"(u), "n"(w));
+        else if constexpr (CB < 0 || (u >> (CB < 1 ? 0 : CB - 1)) & 1)
+          asm volatile("{\n.reg .b64 s;\nmov.b64 s, qre%0;\nmov.b64 qre%0, qre%1;\n"
+                       "mov.b64 qre%1, s;\nmov.b64 s, qim%0;\nmov.b64 qim%0, qim%1;\n"
+                       "mov.b64 qim%1, s;\n}" ::"n"(u), "n"(w));
+      });
+    }
+  }
+
+  // The phase f0 + i f1 where the register bits `cond` are set.
+  __device__ __forceinline__ void phase_where(const float *f, int cond) {
+    u64 k[3];
+    pack_phase(k, cond, f);
+    const u64 xx = k[0], yy = k[1], ny = k[2];
+    each<U>([&](auto uc) {
+      constexpr int u = decltype(uc)::value;
+      if ((u & (cond >> 1)) == (cond >> 1)) turn<u>(xx, yy, ny);
+    });
+  }
+
   // k = c, s: [[c, i s], [i s, c]]
   template <int TB>
   __device__ __forceinline__ void rx(const float *k, u64 z) {
@@ -189,13 +325,14 @@ template <int RB> struct RegsF32 {
 
   // diag(k0 + i k1, k2 + i k3) on register bit TB
   template <int TB>
-  __device__ __forceinline__ void diag(const float *k) {
+  __device__ __forceinline__ void diag(const float *f) {
+    u64 k[6];
+    pack_diag(k, TB, f);
     if constexpr (TB == 0) {
-      const u64 x = pack2(k[0], k[2]), y = pack2(k[1], k[3]), ny = pack2(-k[1], -k[3]);
+      const u64 x = k[0], y = k[1], ny = k[2];
       each<U>([&](auto uc) { turn<decltype(uc)::value>(x, y, ny); });
     } else {
-      const u64 x0 = both2(k[0]), y0 = both2(k[1]), n0 = both2(-k[1]);
-      const u64 x1 = both2(k[2]), y1 = both2(k[3]), n1 = both2(-k[3]);
+      const u64 x0 = k[0], y0 = k[1], n0 = k[2], x1 = k[3], y1 = k[4], n1 = k[5];
       pairs<TB>([&](auto uc, auto wc) {
         turn<decltype(uc)::value>(x0, y0, n0);
         turn<decltype(wc)::value>(x1, y1, n1);
@@ -206,10 +343,10 @@ template <int RB> struct RegsF32 {
   // k0 + i k1 on every amplitude whose register bits COND are set.  With the
   // pair bit among them, the other half takes the factor 1 + 0 i.
   template <int COND>
-  __device__ __forceinline__ void phase(const float *k) {
-    const float x = k[0], y = k[1];
-    const u64 xx = pack2((COND & 1) ? 1.f : x, x), yy = pack2((COND & 1) ? 0.f : y, y);
-    const u64 ny = pack2((COND & 1) ? 0.f : -y, -y);
+  __device__ __forceinline__ void phase(const float *f) {
+    u64 k[3];
+    pack_phase(k, COND, f);
+    const u64 xx = k[0], yy = k[1], ny = k[2];
     each<U>([&](auto uc) {
       constexpr int u = decltype(uc)::value;
       if constexpr ((u & (COND >> 1)) == (COND >> 1)) turn<u>(xx, yy, ny);

@@ -122,28 +122,6 @@ template <typename R> struct TilePass {
 // device
 // ---------------------------------------------------------------------------
 
-// Shared-memory position of tile amplitude i: its place in the 128-byte row
-// is XORed with the row's number, so that whichever tile bits are held in
-// registers a warp's lanes spread over the banks.  Linear over XOR.
-// (complex64: of a real or imaginary part.)
-__host__ __device__ __forceinline__ int tile_pos(int i, float2) {
-  return i ^ ((i >> 5) & 31) ^ ((i >> 10) & 31);
-}
-__host__ __device__ __forceinline__ int tile_pos(int i, double2) {
-  return i ^ ((i >> 3) & 7) ^ ((i >> 6) & 7) ^ ((i >> 9) & 7);
-}
-
-// One amplitude of a tile of L in shared memory.
-__device__ __forceinline__ float2 tile_get(const float *S, int L, int at) {
-  return make_float2(S[at], S[L + at]);
-}
-__device__ __forceinline__ void tile_put(float *S, int L, int at, float2 v) {
-  S[at] = v.x;
-  S[L + at] = v.y;
-}
-__device__ __forceinline__ double2 tile_get(const double2 *S, int, int at) { return S[at]; }
-__device__ __forceinline__ void tile_put(double2 *S, int, int at, double2 v) { S[at] = v; }
-
 // Collects whether an amplitude was an infinity or a NaN: 0 * x is NaN for
 // those alone (and FP32 products cost no integer slot); FP64, whose products
 // are dear, looks at the exponent.

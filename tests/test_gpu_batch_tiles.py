@@ -1,0 +1,54 @@
+"""The batched kernel at the edges of its tiles and windows: instances smaller
+than a thread's registers, exactly one tile, one qubit more (the smallest that
+run in stages), more gates than the window of gates in shared memory holds
+(256) and than one group may have, every gate kind, and every CTA size (which
+also changes the registers a thread holds).
+
+<Z_0> against the FP64 oracle to 1e-5, the bar of the other batch tests; the
+results of one schedule equal another's bit for bit at the same tile size."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from qcs_gb300 import capi
+from qcs_gb300 import workloads as W
+from tests.test_gpu_tiles import every_kind
+
+pytestmark = pytest.mark.gpu
+
+
+def many_kinds(n, seed, count):
+    if n > 1:
+        return every_kind(n, seed, count, p_move=0.4)
+    g = W.GateList()
+    rng = W.Rng(seed)
+    for _ in range(count):
+        k = W.ONE_QUBIT_SET[rng.below(len(W.ONE_QUBIT_SET))]
+        g.add(k, 0, -1, rng.angle() if k in W.PARAMETRIC else 0.0)
+    return g
+
+
+def test_batch_tile_edges_every_schedule():
+    inst = [(n, many_kinds(n, n, 40 + 7 * n)) for n in (1, 2, 3, 4, 5, 6, 10, 11, 12, 13, 14)]
+    # many gates on two qubits (one long group), and a long mixed list
+    long_group = W.GateList()
+    for i in range(700):
+        long_group.add(W.CNOT if i % 2 else W.RX, 1, 0 if i % 2 else -1, 0.1 + 0.01 * i)
+    inst += [(11, long_group), (12, many_kinds(12, 99, 900)), (4, W.GateList()), (15, W.GateList())]
+    want = []
+    for n, g in inst:
+        with O.OracleState(n) as o:
+            o.run(g)
+            want.append(o.expect_z(0))
+    seen = {}
+    with capi.Batch(inst, shots=300, seed=9) as b:
+        for schedule in ((256, 10, 2, 0), (512, 10, 1, 1), (1024, 10, 1, 0), (256, 12, 4, 0),
+                         (512, 12, 2, 0), (1024, 13, 1, 0), (256, 13, 2, 0), (512, 14, 1, 0)):
+            b.config(*schedule)
+            z, samples, _ = b.run()
+            np.testing.assert_allclose(z, want, atol=1e-5)
+            for (n, _), s in zip(inst, samples):
+                assert s.min() >= 0 and s.max() < 1 << n
+            first = seen.setdefault(schedule[1], (z, samples))
+            assert np.array_equal(samples, first[1]), schedule
+            np.testing.assert_allclose(z, first[0], rtol=0, atol=1e-13)
