@@ -16,12 +16,13 @@
 //    whole group, each thread holding the 16 or 32 amplitudes of one setting
 //    of the other bits in registers (one pass per group instead of one per
 //    gate; tile_regs.cuh);
-//  * a larger instance lives in a per-CTA slot of global memory and runs in
+//  * a larger instance lives in a slot of global memory and runs in
 //    stages: a stage is a set of tile_q qubits and the gates acting inside
 //    it; for every tile (one setting of the other qubits) the CTA gathers the
 //    2^tile_q amplitudes into shared memory with coalesced runs, applies the
 //    stage's gates there and scatters them back, so a stage costs one read
-//    and one write of the state however many gates it holds;
+//    and one write of the state however many gates it holds; the tiles are
+//    handed out by tickets to every CTA that comes free;
 //  * <Z_0> is accumulated in FP64 (of FP32 squares) and each shot is drawn
 //    from a counter-based generator (splitmix64 of seed, instance, shot) and
 //    mapped to an index by binary searches over running sums in FP64, then
@@ -55,7 +56,7 @@ struct BInst {
   int n;
   int stage0;
   int nstages;
-  int group;  // CTAs that share the instance's stages (1: one CTA)
+  int group;  // times it is queued: CTAs that start on it
 };
 
 struct BStage {
@@ -103,7 +104,7 @@ struct BatchTune {
   int tile_q;       // 12, 13 or 14
   int ctas_per_sm;  // 1, 2 or 4 (as many as shared memory and registers allow)
   int order;        // 0: largest first, 1: given order
-  int split_q;      // instances above split_q qubits run on 2^(n - split_q) CTAs
+  int split_q;      // instances above split_q qubits are queued for 2^(n - split_q) CTAs
 };
 
 }  // namespace qcs
@@ -139,9 +140,10 @@ struct qcs_cuda_batch {
   qcs::BGate *d_gates;
   qcs::BGate *h_gates;  // pinned; the graph's upload node reads it
   int2 *d_items;
-  int *d_queue;
-  int *d_stage_done;  // per instance: member stage completions this launch
-  int *d_lead;        // per instance: 1 + CTA of member 0 (its slot holds the state)
+  // zeroed by every launch: the queue's head, the slots in use, the shared
+  // instances' tickets
+  char *d_counters;
+  size_t counter_bytes;
   double *d_z;
   double *h_z;          // pinned
   qcs::i64 *d_samples;
@@ -475,7 +477,7 @@ __device__ double slot_readout(const float2 *slot, i64 size, double *prefix, dou
     for (i64 i = lane; i < mtile / 2; i += 128) {  // four units in flight
       float4 x[4];
 #pragma unroll
-      for (int k = 0; k < 4; k++) x[k] = v[i + 32 * k];
+      for (int k = 0; k < 4; k++) x[k] = __ldcg(v + i + 32 * k);
 #pragma unroll
       for (int k = 0; k < 4; k++) {
         even += (double)prob32(make_float2(x[k].x, x[k].y));
@@ -504,13 +506,13 @@ __device__ double slot_readout(const float2 *slot, i64 size, double *prefix, dou
       double cum = prefix[lo];
       const i64 first = (i64)lo * mtile, end = first + mtile;
       const float4 *v = reinterpret_cast<const float4 *>(slot + first) + 2 * lane;
-      float4 n0 = v[0], n1 = v[1];
+      float4 n0 = __ldcg(v), n1 = __ldcg(v + 1);
       for (i64 base = first; base < end && result < 0; base += 128) {
         const float4 a = n0, b = n1;
         v += 64;
         if (base + 128 < end) {
-          n0 = v[0];
-          n1 = v[1];
+          n0 = __ldcg(v);
+          n1 = __ldcg(v + 1);
         }
         double sum[4];
         sum[0] = prob64(make_float2(a.x, a.y));
@@ -538,7 +540,7 @@ __device__ double slot_readout(const float2 *slot, i64 size, double *prefix, dou
       if (result < 0) {  // the tile's last nonzero amplitude
         result = first;
         for (i64 base = first; base < end; base += 32) {
-          const unsigned m = __ballot_sync(0xffffffffu, prob64(slot[base + lane]) > 0.0);
+          const unsigned m = __ballot_sync(0xffffffffu, prob64(__ldcg(slot + base + lane)) > 0.0);
           if (m) result = base + 31 - __clz(m);
         }
       }
@@ -564,15 +566,44 @@ __device__ bool wait_count(const int *cnt, int target, int *err, int where, long
   return true;
 }
 
-// Work items are (instance, member): an instance of `group` > 1 is shared by
-// `group` CTAs that split the tiles of each stage and meet at a counter
-// after every stage; the grid never exceeds the CTAs that fit the GPU at
-// once, so every member of a group runs concurrently with the others.
+// Per instance in a global slot, zero before a launch.
+struct BShare {
+  int next;  // the next ticket
+  int done;  // tickets whose tiles are written
+  int slot;  // 1 + the slot that holds the amplitudes
+  int at_it; // CTAs that take its tickets
+};
+
+// How an instance in a global slot is shared.  Its work is a line of tickets,
+// `chunk` tiles of one stage each, stage after stage; any CTA takes the next
+// ticket, waits until every ticket of the earlier stages is done, does its
+// tiles and counts it done; whoever counts the last one reads the instance
+// out.  A CTA waits only for lower tickets, each in the hands of a CTA that
+// works on it, so nothing depends on which CTAs run at the same time or on
+// when they join: an instance is queued `group` times, and CTAs that find the
+// queue empty join the instances that still have tickets.
+// Fixed members that met after every stage idled until the last of them had
+// come free, and left the rest of the GPU idle at the end of the batch: 96
+// instances of 10-20 qubits 34 -> 11.5 ms, 24 of 12-22 36 -> 16.3, 8 of 18-22
+// 29 -> 12.4, 384 of 10-22 85 -> 72.  64 tickets a stage: a ticket costs two
+// barriers and two atomics, and a stage of few large tickets ends ragged.
+struct BTickets {
+  int chunk, per_stage, total;
+};
+__device__ __forceinline__ BTickets batch_tickets(const BInst &I, int tile_q) {
+  const int n_tiles = 1 << (I.n - tile_q);
+  BTickets k;
+  k.chunk = n_tiles > 64 ? n_tiles / 64 : 1;
+  k.per_stage = n_tiles / k.chunk;
+  k.total = k.per_stage * I.nstages;
+  return k;
+}
+
 template <int T>
 __global__ void __launch_bounds__(T, T == 256 ? 2 : 1)
     k_batch(const BInst *insts, const BStage *stages, const BGroup *groups, const BGate *gates,
             const int2 *items, int n_items, int shots, u64 seed, int tile_q, float2 *slots,
-            i64 slot_amps, int *queue, int *stage_done, int *lead, int *err, double *z_out,
+            i64 slot_amps, int *queue, BShare *share, int *slot_busy, int *err, double *z_out,
             i64 *samples_out, long long wait) {
   QCS_REGS_F32_DECLARE(1 << (reg_q(T) - 1));
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -580,8 +611,8 @@ __global__ void __launch_bounds__(T, T == 256 ? 2 : 1)
   BWindow &W = *reinterpret_cast<BWindow *>(S + (2 << tile_q));
   double *scratch = reinterpret_cast<double *>(&W + 1);  // of the read-outs
   __shared__ double red[T / 32];
-  __shared__ int s_item;
-  __shared__ int s_ok;
+  __shared__ int s_pick, s_ticket, s_slot, s_ok;
+  __shared__ u64 s_best;
   // of the stage: a thread's accesses to a tile, and the tile's base by
   // nibbles of its number
   __shared__ i64 step_off[64], nib[4][16];
@@ -589,32 +620,46 @@ __global__ void __launch_bounds__(T, T == 256 ? 2 : 1)
 
   for (;;) {
     __syncthreads();
-    if (threadIdx.x == 0) s_item = atomicAdd(queue, 1);
+    if (threadIdx.x == 0) s_pick = atomicAdd(queue, 1);
     __syncthreads();
-    const int qi = s_item;
-    if (qi >= n_items) break;
-    const int inst = items[qi].x;
-    const int member = items[qi].y;
+    int inst;
+    const bool joined = s_pick >= n_items;
+    if (!joined) {
+      inst = items[s_pick].x;
+    } else {
+      // the queue is empty: join the instance with the most tiles left per CTA
+      // at it.  A CTA that joins changes at_it, so of those that chose the same
+      // instance one gets it and the others look again.
+      do {
+        __syncthreads();
+        if (threadIdx.x == 0) s_best = 0;
+        __syncthreads();
+        for (int e = threadIdx.x; e < n_items; e += T) {
+          const int2 it = items[e];
+          if (it.y != 0 || it.x >= 1 << 24) continue;
+          const BInst J = insts[it.x];
+          if (J.n <= tile_q) continue;
+          const BTickets k = batch_tickets(J, tile_q);
+          const int left = k.total - *(volatile int *)&share[it.x].next;
+          const int at_it = *(volatile int *)&share[it.x].at_it;
+          if (left <= 0 || at_it >= k.per_stage) continue;
+          const int each = min(left * k.chunk / (at_it + 1) + 1, 0xffffff);
+          atomicMax(&s_best, (u64)each << 40 | (u64)at_it << 24 | it.x);
+        }
+        __syncthreads();
+        inst = s_best ? (int)(s_best & 0xffffff) : -1;
+        if (threadIdx.x == 0 && inst >= 0) {
+          const int at_it = (int)(s_best >> 24) & 0xffff;
+          s_ok = atomicCAS(&share[inst].at_it, at_it, at_it + 1) == at_it;
+        }
+        __syncthreads();
+      } while (inst >= 0 && !s_ok);
+      if (inst < 0) break;
+    }
     const BInst I = insts[inst];
-    const int G = I.group;
     const i64 size = 1LL << I.n;
     double z = 0.0;
     int w0 = 0, w1 = 0;  // groups in the window
-    // the instance's amplitudes live in the slot of its member-0 CTA
-    float2 *slot = slots + (i64)blockIdx.x * slot_amps;
-    if (G > 1) {
-      if (threadIdx.x == 0) {
-        s_ok = 1;
-        if (member == 0) {
-          atomicExch(&lead[inst], blockIdx.x + 1);
-        } else {
-          s_ok = wait_count(&lead[inst], 1, err, 1, wait) ? 1 : 0;
-        }
-      }
-      __syncthreads();
-      if (!s_ok) return;
-      slot = slots + (i64)(*(volatile int *)&lead[inst] - 1) * slot_amps;
-    }
     i64 *out = samples_out + (i64)inst * shots;
     if (I.n <= tile_q) {
       // ---- shared-memory resident instance (a tile of at least 2^kMaxRegQ) ----
@@ -624,28 +669,77 @@ __global__ void __launch_bounds__(T, T == 256 ? 2 : 1)
       __syncthreads();
       run_groups<T>(S, st, W, w0, w1, groups, gates);
       z = resident_readout<T>(S, (int)size, Lt, scratch, red, shots, seed, inst, out);
-    } else {
-      // ---- global-slot instance, run in stages ----
-      for (int si = 0; si < I.nstages; si++) {
-        const BStage st = stages[I.stage0 + si];
-        const int nt = st.nt, L = 1 << nt;
+      if (threadIdx.x == 0) z_out[inst] = z;
+      continue;
+    }
+    // ---- global-slot instance, run in stages ----
+    const BTickets K = batch_tickets(I, tile_q);
+    BShare *sh = share + inst;
+    BStage st;
+    int stage = -1;
+    // of the stage, for this thread (see below)
+    i64 toff = 0;
+    const int i0 = 2 * threadIdx.x;  // its first amplitude
+    const int tpos = tile_pos(i0, kind);
+    const int L = 1 << tile_q;
+    const int steps = L / 2 > T ? L / 2 / T : 1;
+    const bool active = i0 < L;
+    // The next ticket is taken before the tiles of this one, so that its first
+    // tile is known early enough to be fetched.
+    if (threadIdx.x == 0) {
+      if (!joined) atomicAdd(&sh->at_it, 1);
+      s_ticket = atomicAdd(&sh->next, 1);
+    }
+    __syncthreads();
+    int ticket = s_ticket;
+    float2 *slot = nullptr;
+    while (ticket < K.total) {
+      const int si = ticket / K.per_stage;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        s_ok = 1;
+        if (ticket == 0) {  // this CTA opens the instance: a free slot
+          // (at most one instance is open per CTA of the grid)
+          int k = blockIdx.x, tries = 0;
+          while (atomicCAS(&slot_busy[k], 0, 1) != 0 && tries < (1 << 16)) {
+            k = k + 1 < (int)gridDim.x ? k + 1 : 0;
+            tries++;
+          }
+          if (tries < (1 << 16)) {
+            atomicExch(&sh->slot, k + 1);
+          } else {  // after a wait that ran out: its instances keep their slots
+            atomicCAS(err, 0, 3);
+            s_ok = 0;
+          }
+        } else if (slot == nullptr) {
+          s_ok = wait_count(&sh->slot, 1, err, 1, wait) ? 1 : 0;
+        }
+        if (s_ok && si != stage && si > 0)
+          s_ok = wait_count(&sh->done, si * K.per_stage, err, 2, wait) ? 1 : 0;
+        s_slot = *(volatile int *)&sh->slot - 1;
+        s_ticket = atomicAdd(&sh->next, 1);
+      }
+      __syncthreads();
+      if (!s_ok) return;
+      slot = slots + (i64)s_slot * slot_amps;
+      const int next = s_ticket;
+      if (si != stage) {
+        stage = si;
+        st = stages[I.stage0 + si];
         // A thread moves units of two amplitudes (16 bytes; tile bit 0 is
         // qubit 0): unit t + k T, whose offset is that of t plus that of k T.
-        const int nout = I.n - nt;  // qubits outside the tile: the tile number's bits
-        const int steps = L / 2 > T ? L / 2 / T : 1;
-        __syncthreads();
         for (int e = threadIdx.x; e < 64 + 64; e += T) {
           if (e < 64) {
             i64 o = 0;
-            for (int m = 0; m < nt; m++)
+            for (int m = 0; m < tile_q; m++)
               if (((e * T * 2) >> m) & 1) o |= 1LL << st.q[m];
             step_off[e] = o;
-          } else {
+          } else {  // qubits outside the tile, ascending: the tile number's bits
             const int k = (e - 64) >> 4, v = (e - 64) & 15;
             i64 o = 0;
             int j = 0, in = 0;
             for (int q = 0; q < I.n; q++) {
-              if (in < nt && st.q[in] == q) {
+              if (in < tile_q && st.q[in] == q) {
                 in++;
                 continue;
               }
@@ -655,72 +749,71 @@ __global__ void __launch_bounds__(T, T == 256 ? 2 : 1)
             nib[k][v] = o;
           }
         }
-        const int i0 = 2 * threadIdx.x;  // this thread's first amplitude
-        i64 toff = 0;
-        for (int m = 1; m < nt; m++)
+        toff = 0;
+        for (int m = 1; m < tile_q; m++)
           if ((i0 >> m) & 1) toff |= 1LL << st.q[m];
-        const int tpos = tile_pos(i0, kind);
-        const bool active = i0 < L;
         __syncthreads();
-        const int n_tiles = 1 << nout;
-        for (int tt = member; tt < n_tiles; tt += G) {
-          i64 base = nib[0][tt & 15] + nib[1][(tt >> 4) & 15] + nib[2][(tt >> 8) & 15] +
-                     nib[3][(tt >> 12) & 15];
-          float2 *vt = slot + base + toff;
-          if (si == 0) {  // |0...0>
-            for (int i = threadIdx.x; i < 2 * L; i += T) S[i] = tt == 0 && i == 0 ? 1.f : 0.f;
-          } else if (active) {
-            for (int k0 = 0; k0 < steps; k0 += 4) {
-              float4 x[4];
-#pragma unroll
-              for (int k = 0; k < 4; k++)
-                if (k0 + k < steps)
-                  x[k] = __ldcg(reinterpret_cast<const float4 *>(vt + step_off[k0 + k]));
-#pragma unroll
-              for (int k = 0; k < 4; k++) {
-                if (k0 + k >= steps) break;
-                const int at = tpos ^ tile_pos((k0 + k) * T * 2, kind);
-                tile_put(S, L, at, make_float2(x[k].x, x[k].y));
-                tile_put(S, L, at ^ 1, make_float2(x[k].z, x[k].w));
-              }
-            }
-          }
-          __syncthreads();
-          if (si > 0 && active && tt + G < n_tiles) {  // the next tile, towards L2
-            const int t2 = tt + G;
-            const float2 *vn = slot + nib[0][t2 & 15] + nib[1][(t2 >> 4) & 15] +
-                               nib[2][(t2 >> 8) & 15] + nib[3][(t2 >> 12) & 15] + toff;
-            for (int k = 0; k < steps; k++)
-              asm volatile("prefetch.global.L2 [%0];" ::"l"(vn + step_off[k]));
-          }
-          run_groups<T>(S, st, W, w0, w1, groups, gates);
-          if (active) {
-            for (int k = 0; k < steps; k++) {
-              const int at = tpos ^ tile_pos(k * T * 2, kind);
-              const float2 x = tile_get(S, L, at), y = tile_get(S, L, at ^ 1);
-              *reinterpret_cast<float4 *>(vt + step_off[k]) = make_float4(x.x, x.y, y.x, y.y);
-            }
-          }
-          __syncthreads();
-        }
-        if (G > 1) {  // every member's tiles of this stage are written
-          __threadfence();  // each thread's slot writes, before the count
-          __syncthreads();
-          if (threadIdx.x == 0) {
-            __threadfence();
-            atomicAdd(&stage_done[inst], 1);
-            s_ok = wait_count(&stage_done[inst], G * (si + 1), err, 2, wait) ? 1 : 0;
-          }
-          __syncthreads();
-          if (!s_ok) return;
-        }
       }
-      if (member != 0) continue;  // member 0 reads out the instance
-      __threadfence_block();
+      auto tile_at = [&](int tt) {  // this thread's first unit of a tile
+        return slot + nib[0][tt & 15] + nib[1][(tt >> 4) & 15] + nib[2][(tt >> 8) & 15] +
+               nib[3][(tt >> 12) & 15] + toff;
+      };
+      const int t0 = (ticket - si * K.per_stage) * K.chunk;
+      for (int tt = t0; tt < t0 + K.chunk; tt++) {
+        float2 *vt = tile_at(tt);
+        if (si == 0) {  // |0...0>
+          for (int i = threadIdx.x; i < 2 * L; i += T) S[i] = tt == 0 && i == 0 ? 1.f : 0.f;
+        } else if (active) {
+          for (int k0 = 0; k0 < steps; k0 += 4) {
+            float4 x[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+              if (k0 + k < steps)
+                x[k] = __ldcg(reinterpret_cast<const float4 *>(vt + step_off[k0 + k]));
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+              if (k0 + k >= steps) break;
+              const int at = tpos ^ tile_pos((k0 + k) * T * 2, kind);
+              tile_put(S, L, at, make_float2(x[k].x, x[k].y));
+              tile_put(S, L, at ^ 1, make_float2(x[k].z, x[k].w));
+            }
+          }
+        }
+        __syncthreads();
+        const int after = tt + 1 < t0 + K.chunk ? tt + 1
+                          : next / K.per_stage == si ? (next - si * K.per_stage) * K.chunk : -1;
+        if (si > 0 && active && after >= 0) {  // the next tile, towards L2
+          const float2 *vn = tile_at(after);
+          for (int k = 0; k < steps; k++)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(vn + step_off[k]));
+        }
+        run_groups<T>(S, st, W, w0, w1, groups, gates);
+        if (active) {
+          for (int k = 0; k < steps; k++) {
+            const int at = tpos ^ tile_pos(k * T * 2, kind);
+            const float2 x = tile_get(S, L, at), y = tile_get(S, L, at ^ 1);
+            *reinterpret_cast<float4 *>(vt + step_off[k]) = make_float4(x.x, x.y, y.x, y.y);
+          }
+        }
+        __syncthreads();
+      }
+      __threadfence();  // each thread's slot writes, before the count
       __syncthreads();
-      z = slot_readout<T>(slot, size, scratch, red, shots, seed, inst, out);
+      if (threadIdx.x == 0) {
+        __threadfence();
+        s_ok = atomicAdd(&sh->done, 1) == K.total - 1;
+        __threadfence();
+      }
+      __syncthreads();
+      if (s_ok) {  // the last one: the whole state is written
+        z = slot_readout<T>(slot, size, scratch, red, shots, seed, inst, out);
+        if (threadIdx.x == 0) z_out[inst] = z;
+        __syncthreads();
+        if (threadIdx.x == 0) atomicExch(&slot_busy[s_slot], 0);
+      }
+      ticket = next;
     }
-    if (threadIdx.x == 0) z_out[inst] = z;
+    if (threadIdx.x == 0) atomicSub(&sh->at_it, 1);
   }
 }
 
@@ -972,8 +1065,8 @@ static int batch_upload(qcs_cuda_batch *b) {
   if (!rc) rc = check_cuda(cudaMallocHost((void **)&b->h_gates, std::max<size_t>(1, b->gate_tc.size()) * sizeof(BGate)), "cudaMallocHost(batch)");
   if (rc) return rc;
   batch_fill_gates(b);
-  // grid: CTAs per SM from the tune, but never more than fit the GPU at once
-  // (members of a group wait for each other); every CTA owns a global slot
+  // grid: CTAs per SM from the tune, but never more than fit the GPU at once;
+  // a global slot for each
   int fit = 0;
   switch (b->tune.threads) {
     case 256: rc = set_smem_attr<256>(b->tune.tile_q); break;
@@ -989,8 +1082,11 @@ static int batch_upload(qcs_cuda_batch *b) {
   if (rc) return rc;
   if (fit < 1) return set_error(QCS_CUDA_EUNSUP, "batch kernel does not fit an SM");
   const int grid = b->dev.num_sms * std::min(b->tune.ctas_per_sm, fit);
-  // group sizes: 2^(n - split_q) CTAs above split_q qubits (never below the
-  // tile, at most half the grid)
+  // CTAs that start on an instance: 2^(n - split_q) above split_q qubits (never
+  // below the tile, at most half the grid).  With CTAs joining at the end the
+  // choice matters little: 384 instances of 10-22 qubits 75 / 72 / 73 / 79 ms
+  // at split_q 27 / 19 / 17 / 16 (more CTAs than tickets a stage wait), 24 of
+  // 12-22 16.4 / 16.4 / 16.2 / 13.7.
   for (int i = 0; i < b->count; i++) {
     BInst &I = b->insts[i];
     int G = 1;
@@ -1036,17 +1132,17 @@ static int batch_enqueue(qcs_cuda_batch *b) {
   const size_t gbytes = std::max<size_t>(1, b->gate_tc.size()) * sizeof(BGate);
   int rc = check_cuda(cudaMemcpyAsync(b->d_gates, b->h_gates, gbytes, cudaMemcpyHostToDevice, b->stream),
                       "batch gate upload");
-  if (!rc) rc = check_cuda(cudaMemsetAsync(b->d_queue, 0, sizeof(int), b->stream), "batch queue reset");
-  if (!rc) rc = check_cuda(cudaMemsetAsync(b->d_stage_done, 0, b->count * sizeof(int), b->stream), "batch counters");
-  if (!rc) rc = check_cuda(cudaMemsetAsync(b->d_lead, 0, b->count * sizeof(int), b->stream), "batch counters");
+  if (!rc) rc = check_cuda(cudaMemsetAsync(b->d_counters, 0, b->counter_bytes, b->stream), "batch counters");
   if (!rc) rc = check_cuda(cudaMemsetAsync(b->d_err, 0, sizeof(int), b->stream), "batch error flag");
   if (rc) return rc;
   const size_t smem = smem_for(b->tune.tile_q);
   const int tq = b->tune.tile_q;
+  BShare *share = (BShare *)b->d_counters;
+  int *queue = (int *)(share + b->count), *busy = queue + 1;
 #define QCS_LAUNCH_BATCH(T)                                                                       \
   k_batch<T><<<b->grid, T, smem, b->stream>>>(                                                    \
       b->d_insts, b->d_stages, b->d_groups, b->d_gates, b->d_items, (int)b->items.size(),           \
-      b->shots, b->seed, tq, b->d_slots, (i64)b->slot_amps, b->d_queue, b->d_stage_done, b->d_lead, \
+      b->shots, b->seed, tq, b->d_slots, (i64)b->slot_amps, queue, share, busy,                     \
       b->d_err, b->d_z, b->d_samples, b->wait_captured)
   switch (b->tune.threads) {
     case 256: QCS_LAUNCH_BATCH(256); break;
@@ -1124,9 +1220,7 @@ static void batch_destroy(qcs_cuda_batch *b) {
   if (!b) return;
   if (b->stream) cudaStreamSynchronize(b->stream);
   batch_free_device(b);
-  cudaFree(b->d_queue);
-  cudaFree(b->d_stage_done);
-  cudaFree(b->d_lead);
+  cudaFree(b->d_counters);
   cudaFree(b->d_z);
   cudaFree(b->d_samples);
   cudaFree(b->d_slots);
@@ -1184,9 +1278,9 @@ int qcs_cuda_batch_create(int count, const int *num_qubits, const int *op_offset
   int rc = check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
   if (!rc) rc = device_info(dev, &b->dev);
   if (!rc) rc = check_cuda(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking), "cudaStreamCreate");
-  if (!rc) rc = check_cuda(cudaMalloc((void **)&b->d_queue, sizeof(int)), "cudaMalloc(batch)");
-  if (!rc) rc = check_cuda(cudaMalloc((void **)&b->d_stage_done, count * sizeof(int)), "cudaMalloc(batch)");
-  if (!rc) rc = check_cuda(cudaMalloc((void **)&b->d_lead, count * sizeof(int)), "cudaMalloc(batch)");
+  // as many slots as CTAs can be resident, four to an SM at most
+  b->counter_bytes = count * sizeof(BShare) + (1 + 4 * (size_t)b->dev.num_sms) * sizeof(int);
+  if (!rc) rc = check_cuda(cudaMalloc((void **)&b->d_counters, b->counter_bytes), "cudaMalloc(batch)");
   if (!rc) rc = check_cuda(cudaMalloc((void **)&b->d_err, sizeof(int)), "cudaMalloc(batch)");
   if (!rc) rc = check_cuda(cudaMalloc((void **)&b->d_z, count * sizeof(double)), "cudaMalloc(batch)");
   if (!rc) rc = check_cuda(cudaMallocHost((void **)&b->h_z, count * sizeof(double)), "cudaMallocHost(batch)");

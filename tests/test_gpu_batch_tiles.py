@@ -52,3 +52,28 @@ def test_batch_tile_edges_every_schedule():
             first = seen.setdefault(schedule[1], (z, samples))
             assert np.array_equal(samples, first[1]), schedule
             np.testing.assert_allclose(z, first[0], rtol=0, atol=1e-13)
+
+
+@pytest.mark.parametrize("count", [1, 3, 40])
+def test_batch_tickets_any_sharing_same_bits(count):
+    # stages of 2 to 512 tiles (64 tickets at most) taken by one CTA, by queued
+    # groups and by every CTA that comes free; more instances than one, and
+    # fewer than CTAs
+    inst = W.variational_batch(count, seed=7 + count, n_range=(11, 19), depth_range=(1, 5))
+    inst[0] = (14, inst[0][1] if inst[0][0] <= 14 else many_kinds(14, 3, 60))
+    with capi.Batch(inst, shots=200, seed=2) as b:
+        for schedule, splits in (((256, 10, 2, 0), (27, 18, 10)), ((256, 13, 2, 1), (27, 15, 13))):
+            for split in splits:
+                b.config(*schedule)
+                b.split(split)
+                for repeat in range(2):
+                    z, samples, _ = b.run()
+                    key = (z.tobytes(), samples.tobytes())
+                    if split == splits[0] and repeat == 0:
+                        first = key
+                    assert key == first, (schedule, split)
+            for i in range(min(count, 3)):
+                n, g = inst[i]
+                with O.OracleState(n) as o:
+                    o.run(g)
+                    assert abs(o.expect_z(0) - z[i]) < 1e-5
