@@ -35,9 +35,9 @@
 // times the candidates on the batch itself.
 //
 // Measured (default schedule, 1024 shots): 384 instances of 10-22 qubits, 4-16
-// layers 100 -> 64 ms against the kernel that kept a thread's amplitudes in
-// C++ variables, read its gates from global memory and scanned 4096 amplitudes
-// a shot; 608 of 13 qubits 33 -> 0.7 ms (the scans were all of it).
+// layers 110 -> 48 ms against the kernel that kept a thread's amplitudes in
+// C++ variables, read its gates from global memory, shared an instance among
+// fixed CTAs and scanned 4096 amplitudes a shot; 608 of 13 qubits 33 -> 0.7 ms.
 #include <math.h>
 #include <stdio.h>
 #include <string.h>
@@ -57,6 +57,7 @@ struct BInst {
   int stage0;
   int nstages;
   int group;  // times it is queued: CTAs that start on it
+  int tickets;  // of a stage, at most
 };
 
 struct BStage {
@@ -148,7 +149,8 @@ struct qcs_cuda_batch {
   double *h_z;          // pinned
   qcs::i64 *d_samples;
   qcs::i64 *h_samples;  // pinned
-  float2 *d_slots;      // one global slot per CTA for instances above tile_q
+  float2 *d_slots;      // as many global slots as CTAs, for instances above tile_q
+  double *d_sums;       // their read-outs' block sums
   int *d_err;
   long long wait_captured;  // wait limit the captured graph's kernel carries
   size_t slot_amps;
@@ -313,11 +315,81 @@ __device__ __forceinline__ void run_groups(float *S, const BStage &st, BWindow &
   }
 }
 
-// |a|^2 in FP64 (exact products) and in FP32 (as <Z_0> and the masses use it).
-__device__ __forceinline__ double prob64(float2 a) {
-  return (double)a.x * a.x + (double)a.y * a.y;
-}
+// ---- read-outs ----------------------------------------------------------
+// <Z_0> and the sampling tiles' masses are FP64 sums of FP32 squares; inside a
+// tile a shot follows running sums of exact squares in FP64.  All of it is
+// bound by the FP64 pipe (two lanes per clock and SM), which also does the
+// conversions from float, so those are made with integer operations (exact
+// for zeros and normal numbers; others are converted), the squares go straight
+// into the sums by FMA, and no amplitude is summed twice: every block of 32 or
+// more amplitudes is summed once, by whichever CTA is free, and a shot (a
+// thread) searches the running sums and then one block.  Against a scan of the
+// shot's tile, 4096 amplitudes or more, by a warp of the instance's one CTA: 384
+// instances of 12-16 qubits 10.5 -> 1.6 ms, 96 of 10-20 11.5 -> 2.9, 384 of
+// 10-22 72 -> 63, 8 of 18-22 12.4 -> 4.1 (with more tickets a stage).
+
 __device__ __forceinline__ float prob32(float2 a) { return a.x * a.x + a.y * a.y; }
+__device__ __forceinline__ bool nonzero(float2 a) { return a.x != 0.f || a.y != 0.f; }
+
+// |x| as a double; PLAIN: of a zero or a normal number, by its bits.
+template <bool PLAIN>
+__device__ __forceinline__ double to64(float x) {
+  if (!PLAIN) return fabs((double)x);
+  const unsigned w = __float_as_uint(x) << 1;
+  return __hiloint2double(w ? (int)((w >> 4) + 0x38000000u) : 0, (int)(w << 28));
+}
+
+// Whether all of the numbers seen are zero or normal.
+struct PlainTest {
+  unsigned lo = 0xffffffffu, hi = 0;  // of the bits without the sign, less one
+  __device__ __forceinline__ void see(float x) {
+    const unsigned w = (__float_as_uint(x) << 1) - 1u;  // zero: the largest
+    lo = min(lo, w);
+    hi = max(hi, w + 1u);
+  }
+  __device__ __forceinline__ bool plain() const { return lo >= 0xffffffu && hi < 0xff000000u; }
+};
+
+// cum[k] = c + the squares of a[0 .. k].
+template <bool PLAIN>
+__device__ __forceinline__ void running8(const float2 (&a)[8], double c, double (&cum)[8]) {
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const double x = to64<PLAIN>(a[k].x), y = to64<PLAIN>(a[k].y);
+    c = fma(x, x, c);
+    c = fma(y, y, c);
+    cum[k] = c;
+  }
+}
+
+// The sums of a block: FP32 squares of its even and odd amplitudes, and FP64 squares.
+struct BlockSums {
+  double even = 0.0, odd = 0.0, exact = 0.0;
+  template <bool PLAIN>
+  __device__ __forceinline__ void add(const float2 (&a)[8], const float (&p)[8]) {
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+      even += to64<PLAIN>(p[k]);
+      odd += to64<PLAIN>(p[k + 1]);
+    }
+    double c[8];
+    running8<PLAIN>(a, exact, c);
+    exact = c[7];
+  }
+  __device__ __forceinline__ void add(const float2 (&a)[8]) {  // a[0]: an even amplitude
+    float p[8];
+    PlainTest t;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      p[k] = prob32(a[k]);
+      t.see(p[k]);
+      t.see(a[k].x);
+      t.see(a[k].y);
+    }
+    if (t.plain()) add<true>(a, p);
+    else add<false>(a, p);
+  }
+};
 
 // Exclusive prefix of x[0 .. m) in shared memory, the total at x[m], by one
 // warp: each lane sums its run of entries, the warp scans the runs.
@@ -345,208 +417,219 @@ __device__ void warp_prefix(double *x, int m) {
   if (lane == 0) x[m] = total;
 }
 
-constexpr int kSubTile = 32;  // amplitudes per inner step of the resident sampler
+constexpr int kBlock = 32;        // amplitudes of a block, at least
+constexpr int kMaxBlocks = 8192;  // blocks of an instance
+constexpr int kMaxTiles = 1024;   // sampling tiles of an instance
 
-// Read-out of an instance that lives in shared memory (L = 2^n amplitudes of
-// a tile of Lt): the blocks of 32 amplitudes, a thread each, give <Z_0>, the
-// sampling tiles' masses (FP32 squares summed in FP64) and each block's mass
-// in FP64; a shot is one thread's work: its tile, then its block by binary
-// search over the tile's running sums, then the block's amplitudes.  (A warp
-// scanning the tile 32 amplitudes at a time took 64 scans a shot, all of
-// them in the FP64 pipe, two lanes wide.)  Returns <Z_0> in thread 0.
-// scratch: 5 + 2 * L / 32 doubles.
-template <int T>
-__device__ double resident_readout(const float *S, int L, int Lt, double *scratch, double *red,
-                                   int shots, u64 seed, int inst, i64 *out) {
-  const float2 kind = {};
-  auto amp = [&](int i) { return tile_get(S, Lt, tile_pos(i, kind)); };
-  const int sub = L < kSubTile ? L : kSubTile, nsub = L / sub;
-  const int tile = L < kMassTile ? L : kMassTile, n_tiles = L / tile, per = tile / sub;
-  double *prefix = scratch, *incl = scratch + 5, *mass = incl + nsub;
-  double z = 0.0;
-  for (int b = threadIdx.x; b < nsub; b += T) {
-    double even = 0.0, odd = 0.0, m = 0.0;
-    for (int k = 0; k < sub; k += 2) {
-      const float2 x = amp(b * sub + k), y = amp(b * sub + k + 1);
-      even += (double)prob32(x);
-      odd += (double)prob32(y);
-      m += prob64(x);
-      m += prob64(y);
-    }
-    incl[b] = m;
-    mass[b] = even + odd;
-    z += even - odd;
-  }
-  z = block_sum<T>(z, red);
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int t = warp; t < n_tiles; t += T / 32) {
-    double m = 0.0;  // the tile's mass
-    for (int b = lane; b < per; b += 32) m += mass[t * per + b];
-    m = bwarp_sum(m);
-    if (lane == 0) prefix[t] = m;
-    // running sums of the tile's blocks: a run of blocks a lane, then a scan
-    const int run = (per + 31) / 32, b0 = t * per + (lane * run < per ? lane * run : per);
-    const int b1 = b0 + run < (t + 1) * per ? b0 + run : (t + 1) * per;
-    double s = 0.0;
-    for (int b = b0; b < b1; b++) s += incl[b];
+struct ReadShape {
+  i64 block, tile;  // amplitudes
+  int n_blocks, n_tiles, per;  // per: blocks of a tile
+};
+__host__ __device__ inline ReadShape read_shape(i64 size) {
+  ReadShape r;
+  r.block = size / kMaxBlocks > kBlock ? size / kMaxBlocks : kBlock;
+  r.tile = size / kMaxTiles > kMassTile ? size / kMaxTiles : kMassTile;
+  if (r.tile > size) r.tile = size;
+  if (r.block > size) r.block = size;
+  r.n_blocks = (int)(size / r.block);
+  r.n_tiles = (int)(size / r.tile);
+  r.per = (int)(r.tile / r.block);
+  return r;
+}
+
+// From the blocks' sums: prefix[0 .. n_tiles], the tiles' running masses, and
+// incl[b], the running sum of exact squares within b's tile (incl may be
+// `exact`).  1 to 32 lanes a tile, a run of its blocks each.  GLOBAL: the sums
+// are in global memory, written by several CTAs.
+template <int T, bool GLOBAL>
+__device__ void running_sums(const ReadShape &R, const double *mass, const double *exact,
+                             double *incl, double *prefix) {
+  const int g = R.per < 8 ? 1 : R.per / 8 < 32 ? R.per / 8 : 32, run = R.per / g;
+  for (int u0 = 0; u0 < R.n_tiles * g; u0 += T) {  // full warps: they shuffle
+    const int u = u0 + threadIdx.x;
+    const bool valid = u < R.n_tiles * g;
+    const int j = u & (g - 1), b0 = u * run;
+    double m = 0.0, s = 0.0;
+    if (valid)
+      for (int k = 0; k < run; k++) {
+        m += GLOBAL ? __ldcg(mass + b0 + k) : mass[b0 + k];
+        s += GLOBAL ? __ldcg(exact + b0 + k) : exact[b0 + k];
+      }
     double up = s;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
+    for (int o = 1; o < g; o <<= 1) {
+      m += __shfl_xor_sync(0xffffffffu, m, o);
       const double y = __shfl_up_sync(0xffffffffu, up, o);
-      if (lane >= o) up += y;
+      if (j >= o) up += y;
     }
     double before = __shfl_up_sync(0xffffffffu, up, 1);
-    if (lane == 0) before = 0.0;
-    for (int b = b0; b < b1; b++) {
-      before += incl[b];
-      incl[b] = before;
+    if (j == 0) before = 0.0;
+    if (!valid) continue;
+    if (j == 0) prefix[u / g] = m;
+    for (int k = 0; k < run; k++) {
+      before += GLOBAL ? __ldcg(exact + b0 + k) : exact[b0 + k];
+      incl[b0 + k] = before;
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double run = 0.0;
-    for (int t = 0; t < n_tiles; t++) {
-      const double m = prefix[t];
-      prefix[t] = run;
-      run += m;
-    }
-    prefix[n_tiles] = run;
-  }
+  if (threadIdx.x < 32) warp_prefix(prefix, R.n_tiles);
   __syncthreads();
+}
+
+// The shots, a thread each: its tile and its block by binary search over
+// running sums, then the block's amplitudes; load8(i, a) gives amplitudes
+// i .. i+7 (those from the instance's size on are 0).
+template <int T, class Load8>
+__device__ __forceinline__ void pick_shots(const ReadShape &R, const double *prefix,
+                                           const double *incl, int shots, u64 seed, int inst,
+                                           i64 *out, const Load8 &load8) {
   for (int s = threadIdx.x; s < shots; s += T) {
     const double r = shot_draw(seed, (u64)inst, (u64)s);
     i64 result = -1;
-    if (r < prefix[n_tiles]) {
-      int t = 0;
-      while (t + 1 < n_tiles && !(r < prefix[t + 1])) t++;
+    if (r < prefix[R.n_tiles]) {
+      int t = 0, last = R.n_tiles - 1;
+      while (t < last) {
+        const int mid = (t + last) >> 1;
+        if (r < prefix[mid + 1]) last = mid;
+        else t = mid + 1;
+      }
       const double base = prefix[t];
-      const int first = t * per, end = first + per;
+      const int first = t * R.per, end = first + R.per;
       int lo = first, hi = end;  // the first block with r < base + its running sum
       while (lo < hi) {
         const int mid = (lo + hi) >> 1;
         if (r < base + incl[mid]) hi = mid;
         else lo = mid + 1;
       }
-      int from, to;  // where the last nonzero amplitude is taken from, if none is hit
+      i64 from = t * R.tile, to = from + R.tile;  // where the last nonzero one is taken
       if (lo < end) {
         double cum = lo > first ? base + incl[lo - 1] : base;
-        from = lo * sub;
-        to = from + sub;
-        for (int i = from; i < to; i++) {
-          const double p = prob64(amp(i));
-          cum += p;
-          if (p > 0.0 && r < cum) {
-            result = i;
-            break;
+        from = lo * R.block;
+        to = from + R.block;
+        for (i64 i = from; i < to && result < 0; i += 8) {
+          float2 a[8];
+          load8(i, a);
+          PlainTest test;
+#pragma unroll
+          for (int k = 0; k < 8; k++) {
+            test.see(a[k].x);
+            test.see(a[k].y);
           }
+          double c[8];
+          if (test.plain()) running8<true>(a, cum, c);
+          else running8<false>(a, cum, c);
+          cum = c[7];
+          if (!(r < cum)) continue;
+#pragma unroll
+          for (int k = 7; k >= 0; k--)
+            if (nonzero(a[k]) && r < c[k]) result = i + k;
         }
-      } else {
-        from = t * tile;
-        to = from + tile;
       }
       if (result < 0) {
         result = from;
-        for (int i = to - 1; i >= from; i--)
-          if (prob64(amp(i)) > 0.0) {
-            result = i;
-            break;
-          }
+        for (i64 i = (to - 1) & ~(i64)7; i >= from && result == from; i -= 8) {
+          float2 a[8];
+          load8(i, a);
+#pragma unroll
+          for (int k = 0; k < 8; k++)
+            if (nonzero(a[k])) result = i + k;
+        }
       }
     }
     out[s] = result;
   }
-  return z;
 }
 
-// Read-out of an instance in its global slot: a warp takes a sampling tile
-// (<Z_0>, its mass), then a shot: its tile by binary search, and the tile 128
-// amplitudes a step, four a lane (as k_smp_sample).  Returns <Z_0> in thread 0.
+// Read-out of an instance that lives in shared memory (L = 2^n amplitudes of
+// a tile of Lt; those from L on are 0).  Returns <Z_0> in thread 0.
+// scratch: 5 + 2 * L / 32 doubles.
 template <int T>
-__device__ double slot_readout(const float2 *slot, i64 size, double *prefix, double *red,
-                               int shots, u64 seed, int inst, i64 *out) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // at most 1024 sampling tiles
-  i64 mtile = size >> 10 > kMassTile ? size >> 10 : kMassTile;
-  if (mtile > size) mtile = size;  // at least 2^11, above the smallest tile
-  const int n_tiles = (int)(size / mtile);
+__device__ double resident_readout(const float *S, int L, int Lt, double *scratch, double *red,
+                                   int shots, u64 seed, int inst, i64 *out) {
+  const float2 kind = {};
+  const ReadShape R = read_shape(L);
+  double *prefix = scratch, *exact = scratch + 5, *mass = exact + R.n_blocks;
+  auto load8 = [&](i64 i, float2 (&a)[8]) {
+#pragma unroll
+    for (int k = 0; k < 8; k++) a[k] = tile_get(S, Lt, tile_pos((int)i + k, kind));
+  };
   double z = 0.0;
-  for (int t = warp; t < n_tiles; t += T / 32) {
-    const float4 *v = reinterpret_cast<const float4 *>(slot + (i64)t * mtile);
-    double even = 0.0, odd = 0.0;
-    for (i64 i = lane; i < mtile / 2; i += 128) {  // four units in flight
-      float4 x[4];
-#pragma unroll
-      for (int k = 0; k < 4; k++) x[k] = __ldcg(v + i + 32 * k);
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        even += (double)prob32(make_float2(x[k].x, x[k].y));
-        odd += (double)prob32(make_float2(x[k].z, x[k].w));
-      }
+  for (int b = threadIdx.x; b < R.n_blocks; b += T) {
+    BlockSums sums;
+    for (int k = 0; k < (int)R.block; k += 8) {
+      float2 a[8];
+      load8(b * R.block + k, a);
+      sums.add(a);
     }
-    even = bwarp_sum(even);
-    odd = bwarp_sum(odd);
-    if (lane == 0) prefix[t] = even + odd;
-    z += lane == 0 ? even - odd : 0.0;
+    exact[b] = sums.exact;
+    mass[b] = sums.even + sums.odd;
+    z += sums.even - sums.odd;
   }
   z = block_sum<T>(z, red);
   __syncthreads();
-  if (warp == 0) warp_prefix(prefix, n_tiles);
-  __syncthreads();
-  for (int s = warp; s < shots; s += T / 32) {
-    const double r = shot_draw(seed, (u64)inst, (u64)s);
-    i64 result = -1;
-    if (r < prefix[n_tiles]) {
-      int lo = 0, hi = n_tiles - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (r < prefix[mid + 1]) hi = mid;
-        else lo = mid + 1;
-      }
-      double cum = prefix[lo];
-      const i64 first = (i64)lo * mtile, end = first + mtile;
-      const float4 *v = reinterpret_cast<const float4 *>(slot + first) + 2 * lane;
-      float4 n0 = __ldcg(v), n1 = __ldcg(v + 1);
-      for (i64 base = first; base < end && result < 0; base += 128) {
-        const float4 a = n0, b = n1;
-        v += 64;
-        if (base + 128 < end) {
-          n0 = __ldcg(v);
-          n1 = __ldcg(v + 1);
-        }
-        double sum[4];
-        sum[0] = prob64(make_float2(a.x, a.y));
-        sum[1] = sum[0] + prob64(make_float2(a.z, a.w));
-        sum[2] = sum[1] + prob64(make_float2(b.x, b.y));
-        sum[3] = sum[2] + prob64(make_float2(b.z, b.w));
-        double incl = sum[3];
+  running_sums<T, false>(R, mass, exact, exact, prefix);
+  pick_shots<T>(R, prefix, exact, shots, seed, inst, out, load8);
+  return z;
+}
+
+// Read-out of an instance in its global slot.  The block sums are tickets:
+// part `part` of `parts`, four lanes a block; sums: mass, even - odd and exact
+// square sum of each block.
+template <int T>
+__device__ void slot_sums(const float2 *slot, i64 size, int part, int parts, double *sums) {
+  const ReadShape R = read_shape(size);
+  const int n = R.n_blocks / parts;  // at least 2^tile_q / 32
+  const int j = threadIdx.x & 3;
+  for (int b0 = 0; b0 < n; b0 += T / 4) {  // full warps: they shuffle
+    const int b = part * n + b0 + threadIdx.x / 4;
+    const bool valid = b0 + threadIdx.x / 4 < n;
+    BlockSums s;
+    if (valid) {
+      const float4 *v = reinterpret_cast<const float4 *>(slot + b * R.block) + j;
+      for (i64 i = 0; i < R.block; i += 32, v += 16) {
+        float2 a[8];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const double y = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += y;
+        for (int k = 0; k < 4; k++) {
+          const float4 x = __ldcg(v + 4 * k);
+          a[2 * k] = make_float2(x.x, x.y);
+          a[2 * k + 1] = make_float2(x.z, x.w);
         }
-        const unsigned hit = __ballot_sync(0xffffffffu, r < cum + incl);
-        if (hit) {  // in the first lane whose running sum exceeds r
-          const int at = __ffs(hit) - 1;
-          double before = __shfl_up_sync(0xffffffffu, incl, 1);
-          before = lane == 0 ? cum : cum + before;
-          int k = 0;
-          while (k < 3 && !(r < before + sum[k])) k++;
-          while (k > 0 && sum[k] == sum[k - 1]) k--;  // not one of no mass
-          result = base + 4 * at + __shfl_sync(0xffffffffu, k, at);
-        }
-        cum += __shfl_sync(0xffffffffu, incl, 31);
-      }
-      if (result < 0) {  // the tile's last nonzero amplitude
-        result = first;
-        for (i64 base = first; base < end; base += 32) {
-          const unsigned m = __ballot_sync(0xffffffffu, prob64(__ldcg(slot + base + lane)) > 0.0);
-          if (m) result = base + 31 - __clz(m);
-        }
+        s.add(a);
       }
     }
-    if (lane == 0) out[s] = result;
+    double mass = s.even + s.odd, diff = s.even - s.odd;
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+      mass += __shfl_xor_sync(0xffffffffu, mass, o);
+      diff += __shfl_xor_sync(0xffffffffu, diff, o);
+      s.exact += __shfl_xor_sync(0xffffffffu, s.exact, o);
+    }
+    if (valid && j < 3) sums[(i64)j * R.n_blocks + b] = j == 0 ? mass : j == 1 ? diff : s.exact;
   }
+}
+
+// The rest, once all sums are there.  room: space for `room_blocks` doubles in
+// shared memory.  Returns <Z_0> in thread 0.
+template <int T>
+__device__ double slot_readout(const float2 *slot, i64 size, double *sums, double *room,
+                               int room_blocks, double *prefix, double *red, int shots, u64 seed,
+                               int inst, i64 *out) {
+  const ReadShape R = read_shape(size);
+  const double *mass = sums, *diff = sums + R.n_blocks;
+  double *exact = sums + 2 * (i64)R.n_blocks;
+  double *incl = R.n_blocks <= room_blocks ? room : exact;
+  double z = 0.0;
+  for (int b = threadIdx.x; b < R.n_blocks; b += T) z += __ldcg(diff + b);
+  z = block_sum<T>(z, red);
+  __syncthreads();
+  running_sums<T, true>(R, mass, exact, incl, prefix);
+  pick_shots<T>(R, prefix, incl, shots, seed, inst, out, [&](i64 i, float2 (&a)[8]) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const float4 x = __ldcg(reinterpret_cast<const float4 *>(slot + i) + k);
+      a[2 * k] = make_float2(x.x, x.y);
+      a[2 * k + 1] = make_float2(x.z, x.w);
+    }
+  });
   return z;
 }
 
@@ -585,17 +668,16 @@ struct BShare {
 // Fixed members that met after every stage idled until the last of them had
 // come free, and left the rest of the GPU idle at the end of the batch: 96
 // instances of 10-20 qubits 34 -> 11.5 ms, 24 of 12-22 36 -> 16.3, 8 of 18-22
-// 29 -> 12.4, 384 of 10-22 85 -> 72.  64 tickets a stage: a ticket costs two
-// barriers and two atomics, and a stage of few large tickets ends ragged.
+// 29 -> 12.4, 384 of 10-22 85 -> 72.
 struct BTickets {
   int chunk, per_stage, total;
 };
 __device__ __forceinline__ BTickets batch_tickets(const BInst &I, int tile_q) {
   const int n_tiles = 1 << (I.n - tile_q);
   BTickets k;
-  k.chunk = n_tiles > 64 ? n_tiles / 64 : 1;
+  k.chunk = n_tiles > I.tickets ? n_tiles / I.tickets : 1;
   k.per_stage = n_tiles / k.chunk;
-  k.total = k.per_stage * I.nstages;
+  k.total = k.per_stage * (I.nstages + 1);  // the read-out's sums are the last stage
   return k;
 }
 
@@ -603,7 +685,7 @@ template <int T>
 __global__ void __launch_bounds__(T, T == 256 ? 2 : 1)
     k_batch(const BInst *insts, const BStage *stages, const BGroup *groups, const BGate *gates,
             const int2 *items, int n_items, int shots, u64 seed, int tile_q, float2 *slots,
-            i64 slot_amps, int *queue, BShare *share, int *slot_busy, int *err, double *z_out,
+            i64 slot_amps, double *slot_sum, i64 sums_of_slot, int *queue, BShare *share, int *slot_busy, int *err, double *z_out,
             i64 *samples_out, long long wait) {
   QCS_REGS_F32_DECLARE(1 << (reg_q(T) - 1));
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -722,8 +804,11 @@ __global__ void __launch_bounds__(T, T == 256 ? 2 : 1)
       __syncthreads();
       if (!s_ok) return;
       slot = slots + (i64)s_slot * slot_amps;
+      double *sums = slot_sum + (i64)s_slot * sums_of_slot;
       const int next = s_ticket;
-      if (si != stage) {
+      if (si == I.nstages) {
+        slot_sums<T>(slot, size, ticket - si * K.per_stage, K.per_stage, sums);
+      } else if (si != stage) {
         stage = si;
         st = stages[I.stage0 + si];
         // A thread moves units of two amplitudes (16 bytes; tile bit 0 is
@@ -759,7 +844,7 @@ __global__ void __launch_bounds__(T, T == 256 ? 2 : 1)
                nib[3][(tt >> 12) & 15] + toff;
       };
       const int t0 = (ticket - si * K.per_stage) * K.chunk;
-      for (int tt = t0; tt < t0 + K.chunk; tt++) {
+      for (int tt = t0; si < I.nstages && tt < t0 + K.chunk; tt++) {
         float2 *vt = tile_at(tt);
         if (si == 0) {  // |0...0>
           for (int i = threadIdx.x; i < 2 * L; i += T) S[i] = tt == 0 && i == 0 ? 1.f : 0.f;
@@ -806,7 +891,8 @@ __global__ void __launch_bounds__(T, T == 256 ? 2 : 1)
       }
       __syncthreads();
       if (s_ok) {  // the last one: the whole state is written
-        z = slot_readout<T>(slot, size, scratch, red, shots, seed, inst, out);
+        z = slot_readout<T>(slot, size, sums, reinterpret_cast<double *>(S), L, scratch, red, shots,
+                            seed, inst, out);
         if (threadIdx.x == 0) z_out[inst] = z;
         __syncthreads();
         if (threadIdx.x == 0) atomicExch(&slot_busy[s_slot], 0);
@@ -1045,7 +1131,7 @@ static void batch_free_device(qcs_cuda_batch *b) {
 // The tile, the window of gates, then scratch of the read-outs: 1025 prefixes of a slot's sampling
 // tiles, or 5 + 2 * 2^tile_q / 32 doubles of a resident instance.
 static size_t smem_for(int tile_q) {
-  const size_t blocks = 5 + 2 * (((size_t)1 << tile_q) / kSubTile);
+  const size_t blocks = 5 + 2 * (((size_t)1 << tile_q) / kBlock);
   return ((size_t)8 << tile_q) + sizeof(BWindow) + std::max<size_t>(1025, blocks) * sizeof(double);
 }
 
@@ -1054,6 +1140,11 @@ static int set_smem_attr(int tile_q) {
   return check_cuda(cudaFuncSetAttribute(k_batch<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem_for(tile_q)),
                     "cudaFuncSetAttribute(batch)");
+}
+
+// Doubles of a slot's block sums.
+static size_t sums_of_slot(const qcs_cuda_batch *b) {
+  return 3 * (size_t)read_shape((i64)b->slot_amps).n_blocks;
 }
 
 static int batch_upload(qcs_cuda_batch *b) {
@@ -1084,9 +1175,9 @@ static int batch_upload(qcs_cuda_batch *b) {
   const int grid = b->dev.num_sms * std::min(b->tune.ctas_per_sm, fit);
   // CTAs that start on an instance: 2^(n - split_q) above split_q qubits (never
   // below the tile, at most half the grid).  With CTAs joining at the end the
-  // choice matters little: 384 instances of 10-22 qubits 75 / 72 / 73 / 79 ms
-  // at split_q 27 / 19 / 17 / 16 (more CTAs than tickets a stage wait), 24 of
-  // 12-22 16.4 / 16.4 / 16.2 / 13.7.
+  // choice matters little: 384 instances of 10-22 qubits 62.8 / 62.7 / 69.8 ms
+  // at split_q 27 / 19 / 16 (CTAs that wait at the stages' ends), 24 of 12-22
+  // 8.8 / 8.8 / 8.6.
   for (int i = 0; i < b->count; i++) {
     BInst &I = b->insts[i];
     int G = 1;
@@ -1096,6 +1187,11 @@ static int batch_upload(qcs_cuda_batch *b) {
       G = std::min(G, std::max(1, grid / 2));
     }
     I.group = G;
+    // A ticket costs two barriers and two atomics, and CTAs wait at the end of a
+    // stage that leaves some of them without one: 384 instances of 10-22 qubits
+    // 62.8 / 62.8 / 63.9 ms with 64 / 128 / 256 tickets, 24 of 12-22 10.5 / 8.8
+    // / 8.6, 8 of 18-22 6.2 / 4.8 / 4.1, two of 21-22 3.0 / 1.8 / 1.5.
+    I.tickets = b->count < grid ? 256 : 128;
   }
   // instance order
   b->order.resize(b->count);
@@ -1123,7 +1219,13 @@ static int batch_upload(qcs_cuda_batch *b) {
     const size_t slot = b->max_n > 12 ? ((size_t)1 << b->max_n) : 4096;
     b->slot_amps = slot;
     rc = check_cuda(cudaMalloc((void **)&b->d_slots, slot * grid * sizeof(float2)), "cudaMalloc(batch slots)");
-    if (rc) return rc;
+    cudaFree(b->d_sums);
+    b->d_sums = nullptr;
+    if (!rc) rc = check_cuda(cudaMalloc((void **)&b->d_sums, sums_of_slot(b) * grid * sizeof(double)), "cudaMalloc(batch sums)");
+    if (rc) {
+      b->grid = 0;  // the next schedule allocates again
+      return rc;
+    }
   }
   return rc;
 }
@@ -1142,7 +1244,8 @@ static int batch_enqueue(qcs_cuda_batch *b) {
 #define QCS_LAUNCH_BATCH(T)                                                                       \
   k_batch<T><<<b->grid, T, smem, b->stream>>>(                                                    \
       b->d_insts, b->d_stages, b->d_groups, b->d_gates, b->d_items, (int)b->items.size(),           \
-      b->shots, b->seed, tq, b->d_slots, (i64)b->slot_amps, queue, share, busy,                     \
+      b->shots, b->seed, tq, b->d_slots, (i64)b->slot_amps, b->d_sums,           \
+      (i64)sums_of_slot(b), queue, share, busy,                                                    \
       b->d_err, b->d_z, b->d_samples, b->wait_captured)
   switch (b->tune.threads) {
     case 256: QCS_LAUNCH_BATCH(256); break;
@@ -1223,6 +1326,7 @@ static void batch_destroy(qcs_cuda_batch *b) {
   cudaFree(b->d_counters);
   cudaFree(b->d_z);
   cudaFree(b->d_samples);
+  cudaFree(b->d_sums);
   cudaFree(b->d_slots);
   cudaFree(b->d_err);
   if (b->h_z) cudaFreeHost(b->h_z);

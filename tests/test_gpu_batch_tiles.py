@@ -77,3 +77,38 @@ def test_batch_tickets_any_sharing_same_bits(count):
                 with O.OracleState(n) as o:
                     o.run(g)
                     assert abs(o.expect_z(0) - z[i]) < 1e-5
+
+
+def test_batch_readout_of_every_size_and_value():
+    # blocks of 32, 64, ... amplitudes, one sampling tile to many; amplitudes
+    # that are zero, below the smallest normal float, and all on one index
+    small = W.GateList()
+    for _ in range(3):
+        small.add(W.RX, 3, -1, 2e-14)  # |a|^2 of the odd branches: 1e-28, 1e-56, ...
+    small.add(W.RX, 0, -1, 1e-19)
+    small.add(W.RX, 7, -1, 1e-22)
+    inst = []
+    for n in (1, 3, 5, 8, 13, 14, 15, 17, 19, 20):
+        ones, spread = W.GateList(), W.GateList()
+        for q in range(n):
+            ones.add(W.X, q)
+            spread.add(W.H, q)
+        spread.add(W.RY, n - 1, -1, 0.7)
+        inst += [(n, ones), (n, spread)]
+    inst += [(9, small), (14, small), (16, small)]
+    shots = 2000
+    with capi.Batch(inst, shots=shots, seed=21) as b:
+        z, samples, _ = b.run()
+    for i, (n, g) in enumerate(inst):
+        with O.OracleState(n) as o:
+            o.run(g)
+            assert abs(o.expect_z(0) - z[i]) < 1e-5, i
+        s = samples[i]
+        assert s.min() >= 0 and s.max() < 1 << n
+        if g is small:
+            assert not s.any()
+        elif i % 2 == 0:
+            assert (s == (1 << n) - 1).all()
+        else:  # each low bit is fair: 6 standard deviations
+            for q in range(n - 1):
+                assert abs((s >> q & 1).mean() - 0.5) < 6 * 0.5 / np.sqrt(shots), (n, q)
