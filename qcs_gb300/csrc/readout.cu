@@ -21,6 +21,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "measure.h"
 #include "sampler.cuh"
 
 namespace qcs {
@@ -308,6 +309,101 @@ __global__ void __launch_bounds__(kReduceThreads)
       }
     }
   }
+}
+
+// Every qubit of a small state measured in one block, the state in shared
+// memory: per qubit P(0) and P(1) (FP32 squares of two adjacent amplitudes,
+// summed in FP64; complex128 in FP64), the outcome of its draw, the collapse.
+// A thread keeps its pairs of amplitudes, so a qubit's collapse and the next
+// one's sums are one pass.  Bound by the FP64 pipe's latency and width (two
+// lanes per clock: hence few warps, and sums that split the lanes between P(0)
+// and P(1)).  10 qubits: 25 us with the wait; a measurement that
+// returns to the host for its outcome takes a reduction, a wait and a
+// collapse, 18 us a qubit.  Above 128 KB one SM no longer holds the state.
+constexpr int kMeasureMaxBytes = 128 << 10;
+constexpr int kMeasureMaxQubits = 14;
+constexpr int kMeasureThreads = 512;
+struct MeasureDraws { double r[kMeasureMaxQubits]; };
+
+// Lanes 0-15 get the warp's sum of a, the others that of b.
+__device__ __forceinline__ double warp_sum2(double a, double b) {
+  const bool up = (threadIdx.x & 16) != 0;
+  double x = (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+
+template <typename C>
+__global__ void __launch_bounds__(kMeasureThreads)
+    k_measure_all(C *v, int n, const __grid_constant__ MeasureDraws draws, double *outcomes) {
+  using R = decltype(C::x);
+  constexpr int kWarps = kMeasureThreads / 32;  // 16: a lane each for P(0) and P(1)
+  extern __shared__ __align__(16) unsigned char measure_smem[];
+  C *S = reinterpret_cast<C *>(measure_smem);
+  __shared__ double part[2][kWarps];
+  __shared__ R s_scale;
+  __shared__ int s_out;
+  const int size = 1 << n, T = blockDim.x, warps = T / 32;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  int bits = 0;  // thread 0: the outcomes so far
+  int o = 0;     // the last qubit's outcome and scale
+  R s = (R)1;
+  for (int q = 0; q <= n; q++) {
+    double A = 0.0, B = 0.0;
+    for (int i = 2 * threadIdx.x; i < size; i += 2 * T) {  // n >= 1
+      C x, y;
+      if (q == 0) {
+        x = v[i];
+        y = v[i + 1];
+      } else {  // collapsed
+        x = S[i];
+        y = S[i + 1];
+        const bool kx = ((i >> (q - 1)) & 1) == o, ky = (((i + 1) >> (q - 1)) & 1) == o;
+        x.x = kx ? x.x * s : (R)0;
+        x.y = kx ? x.y * s : (R)0;
+        y.x = ky ? y.x * s : (R)0;
+        y.y = ky ? y.y * s : (R)0;
+      }
+      if (q == n) {
+        v[i] = x;
+        v[i + 1] = y;
+        continue;
+      }
+      S[i] = x;
+      S[i + 1] = y;
+      const R px = x.x * x.x + x.y * x.y, py = y.x * y.x + y.y * y.y;
+      if (q == 0) {
+        A += (double)px;
+        B += (double)py;
+      } else if ((i >> q) & 1) {
+        B += (double)(px + py);
+      } else {
+        A += (double)(px + py);
+      }
+    }
+    if (q == n) break;
+    const double sum = warp_sum2(A, B);
+    if ((l & 15) == 0) part[l >> 4][w] = sum;
+    __syncthreads();
+    if (w == 0) {
+      double x = (l & 15) < warps ? part[l >> 4][l & 15] : 0.0;
+#pragma unroll
+      for (int k = kWarps / 2; k > 0; k >>= 1) x += __shfl_xor_sync(0xffffffffu, x, k);
+      const double other = __shfl_xor_sync(0xffffffffu, x, 16);
+      if (l == 0) {
+        const int out = draws.r[q] <= x ? 0 : 1;
+        const double kept = out ? other : x;
+        s_scale = kept > 1e-12 && kept != 1.0 ? (R)(1.0 / sqrt(kept)) : (R)1;
+        s_out = out;
+        bits |= out << q;
+      }
+    }
+    __syncthreads();
+    o = s_out;
+    s = s_scale;
+  }
+  if (threadIdx.x == 0) outcomes[0] = (double)bits;
 }
 
 template <typename C, typename R>
@@ -624,6 +720,40 @@ int qcs_cuda_measure(qcs_cuda_state *s, int qubit, double random_val, int *outco
                 "measure collapse");
   if (rc) return rc;
   *outcome = o;
+  return QCS_CUDA_OK;
+}
+
+int qcs_measure_all(qcs_cuda_state *s, const double *random_vals, int *outcomes) {
+  QCS_CHECK_STATE(s);
+  const bool c128 = s->prec == QCS_CUDA_C128;
+  const size_t bytes = (size_t)s->size * (c128 ? 16 : 8);
+  if (s->n > kMeasureMaxQubits || bytes > (size_t)kMeasureMaxBytes) return QCS_CUDA_EUNSUP;
+  MeasureDraws draws = {};
+  for (int q = 0; q < s->n; q++) draws.r[q] = random_vals[q];
+  const int pairs = (int)(s->size / 2);
+  // four pairs a thread: fewer warps share the FP64 pipe
+  const int threads = pairs < 128 ? 32 : pairs < 4 * kMeasureThreads ? pairs / 4 : kMeasureThreads;
+  int rc = QCS_CUDA_OK;
+  if (bytes > (48 << 10)) {  // the launch's default limit
+    const void *k = c128 ? (const void *)k_measure_all<double2> : (const void *)k_measure_all<float2>;
+    rc = check_cuda(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         kMeasureMaxBytes),
+                    "cudaFuncSetAttribute(measure)");
+  }
+  if (rc) return rc;
+  prof_begin(s);
+  if (c128)
+    k_measure_all<double2><<<1, threads, bytes, s->stream>>>((double2 *)s->vec, s->n, draws,
+                                                             s->h_result_dev);
+  else
+    k_measure_all<float2><<<1, threads, bytes, s->stream>>>((float2 *)s->vec, s->n, draws,
+                                                            s->h_result_dev);
+  invalidate_sum(s);
+  rc = launched(s, KC_COLLAPSE, 2.0 * bytes, "measure all");
+  if (!rc) rc = wait_result(s, sizeof(double), "measure sync");
+  if (rc) return rc;
+  const int bits = (int)s->h_result[0];
+  for (int q = 0; q < s->n; q++) outcomes[q] = (bits >> q) & 1;
   return QCS_CUDA_OK;
 }
 
