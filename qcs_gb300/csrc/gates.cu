@@ -31,6 +31,7 @@ constexpr int kSweepBlocksPerSM = 8;
 template <typename C>
 __global__ void __launch_bounds__(kSweepThreads)
     k_dense1q(C *dst, const C *src, i64 npairs, int t, Mat2<C> m) {
+  grid_wait();
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   const i64 tb = 1LL << t;
   i64 p = (i64)blockIdx.x * blockDim.x + threadIdx.x;
@@ -62,6 +63,7 @@ __global__ void __launch_bounds__(kSweepThreads)
 template <typename C>
 __global__ void __launch_bounds__(kSweepThreads)
     k_diag1q(C *v, i64 size, int t, C d0, C d1) {
+  grid_wait();
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   for (; i + (kUnroll - 1) * nthr < size; i += kUnroll * nthr) {
@@ -82,6 +84,7 @@ __global__ void __launch_bounds__(kSweepThreads)
 template <typename C>
 __global__ void __launch_bounds__(kSweepThreads)
     k_phase_mask(C *v, i64 count, int blo, int bhi, i64 setmask, C phase) {
+  grid_wait();
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   i64 p = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   for (; p + (kUnroll - 1) * nthr < count; p += kUnroll * nthr) {
@@ -111,6 +114,7 @@ __global__ void __launch_bounds__(kSweepThreads)
 // blo-1 (and bhi-1), or'ed with setmask >> 1.  Four units in flight.
 __global__ void __launch_bounds__(kSweepThreads)
     k_phase_mask_v2(float4 *v, i64 units, int blo, int bhi, i64 setmask, float2 phase) {
+  grid_wait();
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   i64 p = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   for (; p < units; p += kUnroll * nthr) {
@@ -139,6 +143,7 @@ __global__ void __launch_bounds__(kSweepThreads)
 // sectors the touched amplitudes lie in.
 __global__ void __launch_bounds__(kSweepThreads)
     k_phase_mask_odd(float4 *v, i64 units, int bhi, float2 phase) {
+  grid_wait();
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   const i64 set = bhi >= 1 ? 1LL << (bhi - 1) : 0;
   i64 p = (i64)blockIdx.x * blockDim.x + threadIdx.x;
@@ -164,6 +169,7 @@ __global__ void __launch_bounds__(kSweepThreads)
 template <typename C>
 __global__ void __launch_bounds__(kSweepThreads)
     k_ctrl1q(C *v, i64 npairs, int blo, int bhi, i64 cmask, int t, Mat2<C> m) {
+  grid_wait();
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   const i64 tb = 1LL << t;
   i64 p = (i64)blockIdx.x * blockDim.x + threadIdx.x;
@@ -195,6 +201,7 @@ __global__ void __launch_bounds__(kSweepThreads)
 // control and target bits.  Same per-amplitude arithmetic as k_ctrl1q.
 __global__ void __launch_bounds__(kSweepThreads)
     k_ctrl1q_v2(float4 *v, i64 npairs, int blo, int bhi, i64 cmask, int t, Mat2<float2> m) {
+  grid_wait();
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   const i64 tb = 1LL << (t - 1);
   i64 p = (i64)blockIdx.x * blockDim.x + threadIdx.x;
@@ -233,6 +240,7 @@ __global__ void __launch_bounds__(kSweepThreads)
 template <typename C, bool CTRL>
 __global__ void __launch_bounds__(kSweepThreads)
     k_exch1q(C *v, i64 npairs, int blo, int bhi, i64 cmask, int t, C m01, C m10) {
+  grid_wait();
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   const i64 tb = 1LL << t;
   i64 p = (i64)blockIdx.x * blockDim.x + threadIdx.x;
@@ -266,6 +274,7 @@ __global__ void __launch_bounds__(kSweepThreads)
 template <typename C, int FORM>
 __global__ void __launch_bounds__(kSweepThreads)
     k_ctrl1q_reference(C *dst, const C *src, i64 npairs, int t, i64 cmask, Mat2<C> m) {
+  grid_wait();
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   const i64 tb = 1LL << t;
   for (i64 p = (i64)blockIdx.x * blockDim.x + threadIdx.x; p < npairs; p += nthr) {
@@ -287,6 +296,7 @@ __global__ void __launch_bounds__(kSweepThreads)
 template <typename C, int FORM>
 __global__ void __launch_bounds__(kSweepThreads)
     k_oop1q(C *dst, const C *src, i64 npairs, int t, Mat2<C> m) {
+  grid_wait();
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   const i64 tb = 1LL << t;
   i64 p = (i64)blockIdx.x * blockDim.x + threadIdx.x;
@@ -316,6 +326,7 @@ __global__ void __launch_bounds__(kSweepThreads)
 // comes from the current one (src/q_gates.c:311-316).
 template <typename C>
 __global__ void k_flip(C *dst, const C *src, i64 index, double *sum) {
+  grid_wait();
   C a = src[index];
   dst[index] = make_c<C>(-(double)a.x, -(double)a.y);
   if (sum) {
@@ -333,22 +344,28 @@ static void swap_buffers(qcs_cuda_state *s) {
   s->scratch = t;
 }
 
+// A sweep over `work` items, kUnroll in flight a thread.
+template <typename... P, typename... A>
+static void launch_sweep(qcs_cuda_state *s, void (*kernel)(P...), i64 work, A &&...args) {
+  const int grid = grid_for(work, kSweepThreads * kUnroll, s->dev, kSweepBlocksPerSM);
+  launch_next(sweep_early(s, grid), kernel, grid, kSweepThreads, 0, s->stream,
+              static_cast<A &&>(args)...);
+}
+
 template <typename C>
 static int apply_1q_t(qcs_cuda_state *s, const double m[8], int t) {
-  const DeviceInfo &d = s->dev;
   const double Ns = (double)s->size * sizeof(C);
   Mat2<C> g = to_mat2<C>(m);
   C *v = (C *)s->vec;
   if (s->sem == QCS_CUDA_REFERENCE) {
     i64 np = s->size / 2;
-    const int gr = grid_for(np, kSweepThreads * kUnroll, d, kSweepBlocksPerSM);
     prof_begin(s);
     if (is_zero(m + 2) && is_zero(m + 4))
-      k_oop1q<C, 1><<<gr, kSweepThreads, 0, s->stream>>>((C *)s->scratch, v, np, t, g);
+      launch_sweep(s, k_oop1q<C, 1>, np, (C *)s->scratch, v, np, t, g);
     else if (is_zero(m) && is_zero(m + 6))
-      k_oop1q<C, 2><<<gr, kSweepThreads, 0, s->stream>>>((C *)s->scratch, v, np, t, g);
+      launch_sweep(s, k_oop1q<C, 2>, np, (C *)s->scratch, v, np, t, g);
     else
-      k_dense1q<C><<<gr, kSweepThreads, 0, s->stream>>>((C *)s->scratch, v, np, t, g);
+      launch_sweep(s, k_dense1q<C>, np, (C *)s->scratch, v, np, t, g);
     int rc = launched(s, KC_DENSE1Q, 2 * Ns, "apply_1q");
     if (rc) return rc;
     swap_buffers(s);
@@ -360,38 +377,31 @@ static int apply_1q_t(qcs_cuda_state *s, const double m[8], int t) {
     i64 cnt = s->size / 2;
     prof_begin(s);
     if (std::is_same<C, float2>::value && t >= 1)
-      k_phase_mask_v2<<<grid_for(cnt / 2, kSweepThreads * kUnroll, d, kSweepBlocksPerSM),
-                        kSweepThreads, 0, s->stream>>>((float4 *)v, cnt / 2, t, -1, 1LL << t,
-                                                       make_float2((float)m[6], (float)m[7]));
+      launch_sweep(s, k_phase_mask_v2, cnt / 2, (float4 *)v, cnt / 2, t, -1, 1LL << t,
+                   make_float2((float)m[6], (float)m[7]));
     else if (std::is_same<C, float2>::value)  // t == 0
-      k_phase_mask_odd<<<grid_for(cnt, kSweepThreads * kUnroll, d, kSweepBlocksPerSM),
-                         kSweepThreads, 0, s->stream>>>((float4 *)v, cnt, -1,
-                                                        make_float2((float)m[6], (float)m[7]));
+      launch_sweep(s, k_phase_mask_odd, cnt, (float4 *)v, cnt, -1,
+                   make_float2((float)m[6], (float)m[7]));
     else
-      k_phase_mask<C><<<grid_for(cnt, kSweepThreads * kUnroll, d, kSweepBlocksPerSM),
-                        kSweepThreads, 0, s->stream>>>(v, cnt, t, -1, 1LL << t, g.g[3]);
+      launch_sweep(s, k_phase_mask<C>, cnt, v, cnt, t, -1, 1LL << t, g.g[3]);
     return launched(s, KC_PHASE_MASK, Ns, "apply_1q (phase)");
   }
   if (diag) {
     prof_begin(s);
-    k_diag1q<C><<<grid_for(s->size, kSweepThreads * kUnroll, d, kSweepBlocksPerSM), kSweepThreads,
-                  0, s->stream>>>(v, s->size, t, g.g[0], g.g[3]);
+    launch_sweep(s, k_diag1q<C>, s->size, v, s->size, t, g.g[0], g.g[3]);
     return launched(s, KC_DIAG1Q, 2 * Ns, "apply_1q (diagonal)");
   }
   i64 np = s->size / 2;
   prof_begin(s);
   if (std::is_same<C, double2>::value && is_zero(m) && is_zero(m + 6))  // X, Y
-    k_exch1q<C, false><<<grid_for(np, kSweepThreads * kUnroll, d, kSweepBlocksPerSM),
-                         kSweepThreads, 0, s->stream>>>(v, np, -1, -1, 0, t, g.g[1], g.g[2]);
+    launch_sweep(s, k_exch1q<C, false>, np, v, np, -1, -1, 0, t, g.g[1], g.g[2]);
   else
-    k_dense1q<C><<<grid_for(np, kSweepThreads * kUnroll, d, kSweepBlocksPerSM), kSweepThreads,
-                   0, s->stream>>>(v, v, np, t, g);
+    launch_sweep(s, k_dense1q<C>, np, v, v, np, t, g);
   return launched(s, KC_DENSE1Q, 2 * Ns, "apply_1q");
 }
 
 template <typename C>
 static int apply_ctrl_t(qcs_cuda_state *s, const double m[8], int c, int t) {
-  const DeviceInfo &d = s->dev;
   const double Ns = (double)s->size * sizeof(C);
   Mat2<C> g = to_mat2<C>(m);
   C *v = (C *)s->vec;
@@ -399,16 +409,12 @@ static int apply_ctrl_t(qcs_cuda_state *s, const double m[8], int c, int t) {
   if (s->sem == QCS_CUDA_REFERENCE) {
     i64 np = s->size / 2;
     prof_begin(s);
-    const int gr = grid_for(np, kSweepThreads, d, kSweepBlocksPerSM);
     if (is_zero(m + 2))
-      k_ctrl1q_reference<C, 1><<<gr, kSweepThreads, 0, s->stream>>>((C *)s->scratch, v, np, t,
-                                                                     cmask, g);
+      launch_sweep(s, k_ctrl1q_reference<C, 1>, np * kUnroll, (C *)s->scratch, v, np, t, cmask, g);
     else if (is_zero(m))
-      k_ctrl1q_reference<C, 2><<<gr, kSweepThreads, 0, s->stream>>>((C *)s->scratch, v, np, t,
-                                                                     cmask, g);
+      launch_sweep(s, k_ctrl1q_reference<C, 2>, np * kUnroll, (C *)s->scratch, v, np, t, cmask, g);
     else
-      k_ctrl1q_reference<C, 0><<<gr, kSweepThreads, 0, s->stream>>>((C *)s->scratch, v, np, t,
-                                                                     cmask, g);
+      launch_sweep(s, k_ctrl1q_reference<C, 0>, np * kUnroll, (C *)s->scratch, v, np, t, cmask, g);
     int rc = launched(s, KC_CTRL1Q, 2 * Ns, "apply_controlled");
     if (rc) return rc;
     swap_buffers(s);
@@ -421,31 +427,24 @@ static int apply_ctrl_t(qcs_cuda_state *s, const double m[8], int c, int t) {
     i64 cnt = s->size / 4;
     prof_begin(s);
     if (std::is_same<C, float2>::value && blo >= 1)
-      k_phase_mask_v2<<<grid_for(cnt / 2, kSweepThreads * kUnroll, d, kSweepBlocksPerSM),
-                        kSweepThreads, 0, s->stream>>>((float4 *)v, cnt / 2, blo, bhi,
-                                                       cmask | (1LL << t),
-                                                       make_float2((float)m[6], (float)m[7]));
+      launch_sweep(s, k_phase_mask_v2, cnt / 2, (float4 *)v, cnt / 2, blo, bhi, cmask | (1LL << t),
+                   make_float2((float)m[6], (float)m[7]));
     else if (std::is_same<C, float2>::value)  // blo == 0: units with bit bhi set
-      k_phase_mask_odd<<<grid_for(cnt, kSweepThreads * kUnroll, d, kSweepBlocksPerSM),
-                         kSweepThreads, 0, s->stream>>>((float4 *)v, cnt, bhi,
-                                                        make_float2((float)m[6], (float)m[7]));
+      launch_sweep(s, k_phase_mask_odd, cnt, (float4 *)v, cnt, bhi,
+                   make_float2((float)m[6], (float)m[7]));
     else
-      k_phase_mask<C><<<grid_for(cnt, kSweepThreads * kUnroll, d, kSweepBlocksPerSM),
-                        kSweepThreads, 0, s->stream>>>(v, cnt, blo, bhi, cmask | (1LL << t),
-                                                       g.g[3]);
+      launch_sweep(s, k_phase_mask<C>, cnt, v, cnt, blo, bhi, cmask | (1LL << t), g.g[3]);
     return launched(s, KC_PHASE_MASK, Ns / 2, "apply_controlled (phase)");
   }
   i64 np = s->size / 4;
   prof_begin(s);
   if (std::is_same<C, float2>::value && blo >= 1)
-    k_ctrl1q_v2<<<grid_for(np / 2, kSweepThreads * kUnroll, d, kSweepBlocksPerSM), kSweepThreads,
-                  0, s->stream>>>((float4 *)v, np / 2, blo, bhi, cmask, t, to_mat2<float2>(m));
+    launch_sweep(s, k_ctrl1q_v2, np / 2, (float4 *)v, np / 2, blo, bhi, cmask, t,
+                 to_mat2<float2>(m));
   else if (std::is_same<C, double2>::value && is_zero(m) && is_zero(m + 6))  // CNOT
-    k_exch1q<C, true><<<grid_for(np, kSweepThreads * kUnroll, d, kSweepBlocksPerSM),
-                        kSweepThreads, 0, s->stream>>>(v, np, blo, bhi, cmask, t, g.g[1], g.g[2]);
+    launch_sweep(s, k_exch1q<C, true>, np, v, np, blo, bhi, cmask, t, g.g[1], g.g[2]);
   else
-    k_ctrl1q<C><<<grid_for(np, kSweepThreads * kUnroll, d, kSweepBlocksPerSM), kSweepThreads, 0,
-                  s->stream>>>(v, np, blo, bhi, cmask, t, g);
+    launch_sweep(s, k_ctrl1q<C>, np, v, np, blo, bhi, cmask, t, g);
   return launched(s, KC_CTRL1Q, Ns, "apply_controlled");
 }
 
@@ -479,9 +478,11 @@ int phase_flip(qcs_cuda_state *s, i64 index) {
   }
   prof_begin(s);
   if (s->prec == QCS_CUDA_C128)
-    k_flip<double2><<<1, 1, 0, s->stream>>>((double2 *)dst, (const double2 *)src, index, sum);
+    launch_next(true, k_flip<double2>, 1, 1, 0, s->stream, (double2 *)dst, (const double2 *)src,
+                index, sum);
   else
-    k_flip<float2><<<1, 1, 0, s->stream>>>((float2 *)dst, (const float2 *)src, index, sum);
+    launch_next(true, k_flip<float2>, 1, 1, 0, s->stream, (float2 *)dst, (const float2 *)src, index,
+                sum);
   if (s->sem == QCS_CUDA_REFERENCE) invalidate_sum(s);
   return launched(s, KC_OTHER, s->prec == QCS_CUDA_C128 ? 32.0 : 16.0, "phase_flip");
 }

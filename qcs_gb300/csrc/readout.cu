@@ -133,6 +133,7 @@ template <int OP>
 __global__ void __launch_bounds__(kReduceThreads)
     k_reduce_c64(const float4 *v, i64 units, int q, ReduceSlot *slots, unsigned *count,
                  double *result) {
+  grid_wait();
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   double A = 0.0, B = 0.0;
   for (i64 u = (i64)blockIdx.x * blockDim.x + threadIdx.x; u < units; u += 4 * nthr) {
@@ -166,6 +167,7 @@ template <int OP>
 __global__ void __launch_bounds__(kReduceThreads)
     k_reduce_c128(const double2 *v, i64 size, int q, ReduceSlot *slots, unsigned *count,
                   double *result) {
+  grid_wait();
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   double A = 0.0, B = 0.0;
   for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < size; i += nthr) {
@@ -345,6 +347,7 @@ __global__ void __launch_bounds__(kMeasureThreads)
   __shared__ int s_out;
   const int size = 1 << n, T = blockDim.x, warps = T / 32;
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  grid_wait();
   int bits = 0;  // thread 0: the outcomes so far
   int o = 0;     // the last qubit's outcome and scale
   R s = (R)1;
@@ -560,11 +563,11 @@ static int reduce(qcs_cuda_state *s, int op, int q, double *res, int nres) {
   auto go = [&](auto opc) {
     constexpr int OP = decltype(opc)::value;
     if (c128)
-      k_reduce_c128<OP><<<grid, kReduceThreads, 0, s->stream>>>(
-          (const double2 *)s->vec, work, q, s->d_partials, s->d_count, dst);
+      launch_next(sweep_early(s, grid), k_reduce_c128<OP>, grid, kReduceThreads, 0, s->stream,
+                  (const double2 *)s->vec, work, q, s->d_partials, s->d_count, dst);
     else
-      k_reduce_c64<OP><<<grid, kReduceThreads, 0, s->stream>>>(
-          (const float4 *)s->vec, work, q, s->d_partials, s->d_count, dst);
+      launch_next(sweep_early(s, grid), k_reduce_c64<OP>, grid, kReduceThreads, 0, s->stream,
+                  (const float4 *)s->vec, work, q, s->d_partials, s->d_count, dst);
   };
   if (op == OP_NORM) go(std::integral_constant<int, OP_NORM>());
   else if (op == OP_MASK) go(std::integral_constant<int, OP_MASK>());
@@ -745,11 +748,11 @@ int qcs_measure_all(qcs_cuda_state *s, const double *random_vals, int *outcomes)
   if (rc) return rc;
   prof_begin(s);
   if (c128)
-    k_measure_all<double2><<<1, threads, bytes, s->stream>>>((double2 *)s->vec, s->n, draws,
-                                                             s->h_result_dev);
+    launch_next(true, k_measure_all<double2>, 1, threads, bytes, s->stream, (double2 *)s->vec, s->n,
+                draws, s->h_result_dev);
   else
-    k_measure_all<float2><<<1, threads, bytes, s->stream>>>((float2 *)s->vec, s->n, draws,
-                                                            s->h_result_dev);
+    launch_next(true, k_measure_all<float2>, 1, threads, bytes, s->stream, (float2 *)s->vec, s->n,
+                draws, s->h_result_dev);
   invalidate_sum(s);
   rc = launched(s, KC_COLLAPSE, 2.0 * bytes, "measure all");
   if (!rc) rc = wait_result(s, sizeof(double), "measure sync");

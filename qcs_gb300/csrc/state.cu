@@ -90,6 +90,7 @@ __global__ void k_set_one(C *v, i64 index) {
 // the index.
 template <typename C>
 __global__ void __launch_bounds__(kSweepThreads) k_basis(float4 *v, i64 units, i64 index) {
+  grid_wait();
   constexpr int UNIT = 16 / sizeof(C);
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   for (i64 u = (i64)blockIdx.x * blockDim.x + threadIdx.x; u < units; u += nthr) {
@@ -444,9 +445,11 @@ int qcs_cuda_set_basis(qcs_cuda_state *s, long long index) {
     const int grid = grid_for(units, kSweepThreads, s->dev, 8);
     prof_begin(s);
     if (s->prec == QCS_CUDA_C128)
-      k_basis<double2><<<grid, kSweepThreads, 0, s->stream>>>((float4 *)s->vec, units, index);
+      launch_next(true, k_basis<double2>, grid, kSweepThreads, 0, s->stream, (float4 *)s->vec, units,
+                  index);
     else
-      k_basis<float2><<<grid, kSweepThreads, 0, s->stream>>>((float4 *)s->vec, units, index);
+      launch_next(true, k_basis<float2>, grid, kSweepThreads, 0, s->stream, (float4 *)s->vec, units,
+                  index);
     return launched(s, KC_OTHER, (double)bytes, "set_basis");
   }
   int rc = check_cuda(cudaMemsetAsync(s->vec, 0, bytes, s->stream), "cudaMemset(state)");

@@ -334,6 +334,7 @@ __global__ void __launch_bounds__(1 << (TileTraits<C>::max_bits - kTileRegBits),
       if ((k >> j) & 1) o ^= P.store[sb + j];
     return o;
   };
+  grid_wait();
   for (i64 tile = blockIdx.x; tile < P.n_tiles; tile += gridDim.x) {
     i64 base = 0;
     for (int j = 0; j < P.nout; j++) base |= ((tile >> j) & 1LL) << P.out[j];
@@ -701,7 +702,13 @@ static int launch_pass(qcs_cuda_state *s, const qcs_cuda_op *ops, const TileStre
   const int grid = (int)std::min<i64>(P.n_tiles, cap);
   s->h2d_bytes += (long long)(offsetof(TilePass<R>, gate) + P.ngates * sizeof(TileGate<R>));
   prof_begin(s);
-  k_tile<C><<<grid, threads, smem, s->stream>>>((C *)s->vec, P);
+  // Started early (launch_next) where every tile finds an SM of its own, and
+  // for complex64 but not at one to three tiles an SM: new angles every run,
+  // 16 qubits (32 tiles) 99 -> 76 us, 18 (128) 108 -> 89, 20 (512) 186 -> 153;
+  // 19 (256), replayed, 105 -> 125; complex128, 18 qubits (256) 610 -> 1101.
+  const int sms = s->dev.num_sms;
+  const bool early = 2 * grid <= sms || (sizeof(C) == 8 && (grid <= sms || grid > 3 * sms));
+  launch_next(early, k_tile<C>, grid, threads, smem, s->stream, (C *)s->vec, P);
   invalidate_sum(s);
   return launched(s, KC_TILE, 2.0 * s->size * sizeof(C), "gate tile pass");
 }
