@@ -12,8 +12,9 @@
 // takes the Adam step in place.  A gradient is summed over the rows in slots
 // of 64, each in row order, and over the slots in order, so it does not
 // depend on how the work is cut.  Latency bounds both: 64 steps on 256 rows
-// take 1.3 ms, where one CTA per 64 rows for everything, a kernel for the sum
-// of the slots and one for Adam took 21.7 ms.
+// take 1.16 ms (1.32 when a kernel starts only after the end of the one before
+// it), where one CTA per 64 rows for everything, a kernel for the sum of the
+// slots and one for Adam took 21.7 ms.
 #include <atomic>
 #include <math.h>
 #include <string.h>
@@ -127,6 +128,12 @@ __global__ void __launch_bounds__(kMlpRowThreads)
   const int tid = threadIdx.x;
   const int r0 = blockIdx.x * kMlpRows;
   const int s = tid >> 4, j = 4 * (tid & 15), row = r0 + s;
+  for (int e = tid; e < kMlpRows * F; e += kMlpRowThreads) {
+    if (r0 + e / F < n) copy4(x + e, X + (size_t)r0 * F + e);
+    else x[e] = 0.f;
+  }
+  const float yr = Y && row < n ? Y[row] : 0.f;
+  grid_wait();  // the parameters are the kernel before's, the records are not
   for (int e = tid; e < (F + 2 * H) * (H / 4); e += kMlpRowThreads) {
     const int i = e / (H / 4), c = 4 * (e % (H / 4));  // rows of w1, w2, w3
     const int off = i < F ? S.off_w1 + i * H : i < F + H ? S.off_w2 + (i - F) * H
@@ -138,12 +145,7 @@ __global__ void __launch_bounds__(kMlpRowThreads)
     const int off = k == 0 ? S.off_b1 : k == 1 ? S.off_b2 : k == 2 ? S.off_b3 : S.off_w4;
     copy16(b1 + k * H + c, params + off + c);
   }
-  for (int e = tid; e < kMlpRows * F; e += kMlpRowThreads) {
-    if (r0 + e / F < n) copy4(x + e, X + (size_t)r0 * F + e);
-    else x[e] = 0.f;
-  }
   const float b4 = params[S.off_b4];
-  const float yr = Y && row < n ? Y[row] : 0.f;
   copy_commit();
   copy_wait<0>();
   __syncthreads();
@@ -289,6 +291,7 @@ __global__ void __launch_bounds__(kMlpGradThreads)
     }
     copy_commit();
   };
+  grid_wait();
   for (int c = 0; c < kMlpStages - 1; c++) load(c);
   const int off_w = layer == 0 ? S.off_w1 : layer == 1 ? S.off_w2 : layer == 2 ? S.off_w3 : S.off_w4;
   const bool mine = last ? i == 0 : i <= K;  // a layer's bias follows its weights
@@ -438,15 +441,17 @@ static int cm_grad_device(qcs_cuda_costmodel *m, const float *x, const float *y,
   MlpActs acts;
   acts.p = m->d_acts;
   acts.rows = (size_t)m->cap_grad;
-  k_mlp_rows<<<(n + kMlpRows - 1) / kMlpRows, kMlpRowThreads, mlp_smem(m->F), m->stream>>>(
-      m->d_params, m->F, x, y, n, 1.f / n, acts, m->d_loss_rows, nullptr);
+  launch_next(true, k_mlp_rows, (n + kMlpRows - 1) / kMlpRows, kMlpRowThreads, mlp_smem(m->F),
+              m->stream, m->d_params, m->F, x, y, n, 1.f / n, acts, m->d_loss_rows,
+              (float *)nullptr);
   int rc = check_launch("cost model rows");
   if (rc) return rc;
   MlpAdam none;
   memset(&none, 0, sizeof(none));
   if (n <= kMlpDirectRows) {
-    k_mlp_grad<<<mlp_grad_blocks(m->F), kMlpGradThreads, kMlpStages * sizeof(MlpChunk), m->stream>>>(
-        m->F, x, n, acts, m->d_grad, adam ? *adam : none);
+    launch_next(true, k_mlp_grad, mlp_grad_blocks(m->F), kMlpGradThreads,
+                kMlpStages * sizeof(MlpChunk), m->stream, m->F, x, n, acts, m->d_grad,
+                adam ? *adam : none);
     return check_launch("cost model gradient");
   }
   const int nslots = (n + kMlpSlot - 1) / kMlpSlot;
