@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   float *epi = reinterpret_cast<float *>(smem + S::OFF_EPI);
   const uint32_t bar0 = smem_u32(smem + S::OFF_BAR);  // 8-byte barriers:
   // 0,1 a_full[stage]  2,3 mma_done[stage]  4,5 acc_empty[stage]  6 drain
-  // 7..10 sq_full[slot]: a tile's column norms are in colsq[slot]
+  // 7..10 sq_full[slot]: a tile's column norms are in colsq[slot]  11 image
   auto bar = [&](int i) { return bar0 + 8u * (uint32_t)i; };
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + S::OFF_MISC);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + S::OFF_MISC + 4);
@@ -240,15 +240,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     mbar_init(bar(5), kTcEpiThreads);
     mbar_init(bar(6), 1);
     for (int k = 0; k < kSqSlots; k++) mbar_init(bar(7 + k), kTcProdThreads);
+    mbar_init(bar(11), 1);
     *abort_flag = 0;
     fence_barrier_init();
+    bulk_load(smem_u32(sB), bimg, S::IMG_BYTES, bar(11));
   }
   for (int i = tid; i < kTcM; i += kTcThreads) col_off[i] = g.col_off[i];
   for (int i = tid; i < KA; i += kTcThreads) blk_off[i] = g.blk_off[i];
-  {
-    uint4 *dst = reinterpret_cast<uint4 *>(sB);
-    for (int i = tid; i < S::IMG_BYTES / 16; i += kTcThreads) dst[i] = bimg[i];
-  }
   // Diffusion fused in front of the block (diffuse_sum != null): the block
   // reads psi but must act on 2m - psi, m = sum * inv_n; since
   // U (2m 1 - psi) = 2m (U 1) - U psi, the epilogue writes beta - U psi with
@@ -263,7 +261,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       beta[i] = make_float2(tr * r.x - ti * r.y, tr * r.y + ti * r.x);
     }
   }
-  fence_async_shared();  // the block matrix is read by the tensor cores
   if (warp == kTcMmaWarp) {
     tmem_alloc(smem_u32(tmem_slot), S::TMEM_COLS);
     tmem_relinquish();
@@ -432,7 +429,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       constexpr uint32_t idesc = idesc_bf16(kTcM, S::N);
       const uint32_t a0 = smem_u32(sA), b_hi = smem_u32(sB), b_lo = b_hi + S::B_BYTES;
       const TileWalk w = tile_walk(g);
-      for (int it = 0; it < w.count; ++it) {
+      const bool image = wait_bar(bar(11), 0, abort_flag, err, 7, wait);
+      for (int it = 0; image && it < w.count; ++it) {
         const int stage = it & 1;
         if (!wait_bar(bar(stage), (it >> 1) & 1, abort_flag, err, 2, wait)) break;
         if (it >= 2 && !wait_bar(bar(4 + stage), ((it - 2) >> 1) & 1, abort_flag, err, 3, wait))
@@ -451,10 +449,11 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         }
         umma_commit(bar(2 + stage));
       }
-      // every MMA issued above must finish before TMEM is released
+      // every MMA issued above must finish before TMEM is released, and the
+      // image be there before the CTA ends
       umma_commit(bar(6));
       long long t0 = clock64();
-      while (!mbar_try_wait(bar(6), 0)) {
+      while (!mbar_try_wait(bar(6), 0) || !mbar_try_wait(bar(11), 0)) {
         if (clock64() - t0 > kWaitCycles) {
           atomicExch(err, 4);
           break;
@@ -652,6 +651,7 @@ __global__ void __launch_bounds__(Tc7::THREADS, 1)
   const uint32_t bar0 = smem_u32(smem + S::OFF_BAR);  // 8-byte barriers:
   // 0,1 chunk_full[stage]  2,3 chunk_free[stage]  4,5 acc_full[acc]
   // 6,7 acc_empty[acc]  8 drain  9..12 sq_full[slot]: a tile's column norms
+  // 13 image
   auto bar = [&](int i) { return bar0 + 8u * (uint32_t)i; };
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + S::OFF_MISC);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + S::OFF_MISC + 4);
@@ -669,15 +669,13 @@ __global__ void __launch_bounds__(Tc7::THREADS, 1)
     mbar_init(bar(7), kTcEpiThreads);
     mbar_init(bar(8), 1);
     for (int k = 0; k < kSqSlots; k++) mbar_init(bar(9 + k), S::PROD_THREADS);
+    mbar_init(bar(13), 1);
     *abort_flag = 0;
     fence_barrier_init();
+    bulk_load(smem_u32(sB), bimg, S::IMG_BYTES, bar(13));
   }
   for (int i = tid; i < kTcM; i += S::THREADS) col_off[i] = g.col_off[i];
   for (int i = tid; i < S::KA; i += S::THREADS) blk_off[i] = g.blk_off[i];
-  {
-    uint4 *dst = reinterpret_cast<uint4 *>(sB);
-    for (int i = tid; i < S::IMG_BYTES / 16; i += S::THREADS) dst[i] = bimg[i];
-  }
   float2 *beta = reinterpret_cast<float2 *>(smem + S::OFF_BETA);
   if (FUSED && diffuse_sum) {  // as in k_block_tc: beta[a] = 2m * (row sum a of U)
     const float tr = (float)(2.0 * (diffuse_sum[0] * inv_n));
@@ -688,7 +686,6 @@ __global__ void __launch_bounds__(Tc7::THREADS, 1)
       beta[i] = make_float2(tr * r.x - ti * r.y, tr * r.y + ti * r.x);
     }
   }
-  fence_async_shared();
   if (warp == S::MMA_WARP) {
     tmem_alloc(smem_u32(tmem_slot), S::TMEM_COLS);
     tmem_relinquish();
@@ -870,7 +867,7 @@ __global__ void __launch_bounds__(Tc7::THREADS, 1)
       constexpr uint32_t idesc_neg = idesc | (1u << 14);  // negate B
       const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
       const TileWalk w = tile_walk(g);
-      bool ok = true;
+      bool ok = wait_bar(bar(13), 0, abort_flag, err, 7, wait);
       for (i64 it = 0; ok && it < w.count; ++it) {
         const int acc_st = (int)(it & 1);
         if (it >= 2 &&
@@ -919,7 +916,7 @@ __global__ void __launch_bounds__(Tc7::THREADS, 1)
       }
       umma_commit(bar(8));
       long long t0 = clock64();
-      while (!mbar_try_wait(bar(8), 0)) {
+      while (!mbar_try_wait(bar(8), 0) || !mbar_try_wait(bar(13), 0)) {
         if (clock64() - t0 > kWaitCycles) {
           atomicExch(err, 4);
           break;
