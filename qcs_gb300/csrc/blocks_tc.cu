@@ -159,10 +159,11 @@ struct TcGeom {
   int nruns;          // prefetch pieces of a tile (at most 128)
   int run_bytes;      // bytes per piece (>= 512 B: the tile holds qubits 0..6)
   int pf_ahead;       // tiles ahead whose pieces are prefetched
-  signed char freeq[40];
-  i64 col_off[kTcM];  // column m -> offset (bits of m on the column qubits)
-  i64 blk_off[128];   // block index a -> offset (bit j of a on qubits[j])
-  i64 run_off[128];   // piece j -> offset of its first amplitude
+  // qubits of the bits of a column's, a block row's and a piece's number; the
+  // kernels spread them into tables themselves (as tables of 1 KB in the
+  // parameters, lanes read different places of cold lines: 41 blocks on 20 qubits
+  // 234 -> 226 us, Grover on 26 14.7 -> 14.4 ms)
+  signed char colq[8], blkq[8], runq[8];
   i64 nib[10][16];    // tile id nibble k with value v -> its part of the tile's offset
 };
 
@@ -176,6 +177,14 @@ struct TcGeom {
 // four placements at 28 qubits (mean), 1 tile ahead 0.79, none 0.71.
 static int pf_ahead(int k) { return k == 7 ? 1 : 2; }
 static int pf_piece_bits() { return 16; }
+
+// The offset of number x < 128: its bits on the qubits q.
+__device__ __forceinline__ i64 spread(int x, const signed char (&q)[8]) {
+  i64 o = 0;
+#pragma unroll
+  for (int b = 0; b < 7; b++) o |= (i64)((x >> b) & 1) << q[b];
+  return o;
+}
 
 // The tile's offset: its id's bits scattered onto the free qubits, four
 // bits per table lookup (the index is the same across a warp, so the
@@ -245,8 +254,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     fence_barrier_init();
     bulk_load(smem_u32(sB), bimg, S::IMG_BYTES, bar(11));
   }
-  for (int i = tid; i < kTcM; i += kTcThreads) col_off[i] = g.col_off[i];
-  for (int i = tid; i < KA; i += kTcThreads) blk_off[i] = g.blk_off[i];
+  for (int i = tid; i < kTcM; i += kTcThreads) col_off[i] = spread(i, g.colq);
+  for (int i = tid; i < KA; i += kTcThreads) blk_off[i] = spread(i, g.blkq);
   // Diffusion fused in front of the block (diffuse_sum != null): the block
   // reads psi but must act on 2m - psi, m = sum * inv_n; since
   // U (2m 1 - psi) = 2m (U 1) - U psi, the epilogue writes beta - U psi with
@@ -370,7 +379,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       // the pieces of the tile pf_ahead ahead go to L2 now, so that the
       // register loads issued for later tiles find them there
       if (p < g.nruns && it + g.pf_ahead < w.count)  // nruns <= 128 < 256 producers
-        prefetch_l2(v + tile_base(w.at(it + g.pf_ahead), g) + g.run_off[p],
+        prefetch_l2(v + tile_base(w.at(it + g.pf_ahead), g) + spread(p, g.runq),
                     (uint32_t)g.run_bytes);
       // in low mode every lane of a warp takes the same decision: the norm
       // exchange below is a full-warp shuffle
@@ -674,8 +683,8 @@ __global__ void __launch_bounds__(Tc7::THREADS, 1)
     fence_barrier_init();
     bulk_load(smem_u32(sB), bimg, S::IMG_BYTES, bar(13));
   }
-  for (int i = tid; i < kTcM; i += S::THREADS) col_off[i] = g.col_off[i];
-  for (int i = tid; i < S::KA; i += S::THREADS) blk_off[i] = g.blk_off[i];
+  for (int i = tid; i < kTcM; i += S::THREADS) col_off[i] = spread(i, g.colq);
+  for (int i = tid; i < S::KA; i += S::THREADS) blk_off[i] = spread(i, g.blkq);
   float2 *beta = reinterpret_cast<float2 *>(smem + S::OFF_BETA);
   if (FUSED && diffuse_sum) {  // as in k_block_tc: beta[a] = 2m * (row sum a of U)
     const float tr = (float)(2.0 * (diffuse_sum[0] * inv_n));
@@ -831,7 +840,7 @@ __global__ void __launch_bounds__(Tc7::THREADS, 1)
       const i64 it = q / S::CHUNKS;
       const int c = (int)(q % S::CHUNKS);
       if (c == 0 && p < g.nruns && it + g.pf_ahead < w.count)
-        prefetch_l2(v + tile_base(w.at(it + g.pf_ahead), g) + g.run_off[p],
+        prefetch_l2(v + tile_base(w.at(it + g.pf_ahead), g) + spread(p, g.runq),
                     (uint32_t)g.run_bytes);
       // stage b is free once the MMAs of chunk q - 2 are done
       if (q >= 2) {
@@ -1233,28 +1242,19 @@ static void tc_prepare(const qcs_cuda_state *s, int k, const int *qubits_in, con
       role[q] = -2;
       colq.push_back(q);
     }
+  int freeq[40];
   for (int q = 0; q < s->n; q++)
-    if (role[q] == -1) g.freeq[g.nfree++] = (signed char)q;
+    if (role[q] == -1) freeq[g.nfree++] = q;
   for (int k = 0; 4 * k < g.nfree; k++)
     for (int v = 0; v < 16; v++) {
       i64 o = 0;
       for (int b = 0; b < 4 && 4 * k + b < g.nfree; b++)
-        if ((v >> b) & 1) o |= 1LL << g.freeq[4 * k + b];
+        if ((v >> b) & 1) o |= 1LL << freeq[4 * k + b];
       g.nib[k][v] = o;
     }
   g.n_tiles = 1LL << g.nfree;
-  for (int m = 0; m < kTcM; m++) {
-    i64 o = 0;
-    for (int b = 0; b < 7; b++)
-      if ((m >> b) & 1) o |= 1LL << colq[b];
-    g.col_off[m] = o;
-  }
-  for (int a = 0; a < KA; a++) {
-    i64 o = 0;
-    for (int j = 0; j < k; j++)
-      if ((a >> j) & 1) o |= 1LL << qubits[j];
-    g.blk_off[a] = o;
-  }
+  for (int b = 0; b < 7; b++) g.colq[b] = (signed char)colq[b];
+  for (int j = 0; j < k; j++) g.blkq[j] = (signed char)qubits[j];
   {
     // the tile's qubits ascending; the lowest R of them are 0..R-1 (R >= 7),
     // so the tile is 2^(k+7-R) runs of 2^R adjacent amplitudes
@@ -1270,14 +1270,9 @@ static void tc_prepare(const qcs_cuda_state *s, int k, const int *qubits_in, con
     while (piece > pf_piece_bits() && nrun_bits + (R - piece) < 7) piece--;
     g.nruns = 1 << (nrun_bits + (R - piece));
     g.run_bytes = (int)(8LL << piece);
-    for (int j = 0; j < g.nruns; j++) {
-      const int sub = j & ((1 << (R - piece)) - 1);  // piece within its run
-      const int run = j >> (R - piece);
-      i64 o = (i64)sub << piece;
-      for (int b = R; b < nt; b++)
-        if ((run >> (b - R)) & 1) o |= 1LL << tq[b];
-      g.run_off[j] = o;
-    }
+    // a piece's number: its place in its run, then the run's qubits
+    for (int b = 0; b < nrun_bits + R - piece; b++)
+      g.runq[b] = (signed char)(b < R - piece ? piece + b : tq[b + piece]);
     g.pf_ahead = pf_ahead(k);
   }
   bool low = true;  // the block is exactly qubits 0..k-1
