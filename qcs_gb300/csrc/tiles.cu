@@ -49,8 +49,9 @@ namespace qcs {
 
 int apply_op(qcs_cuda_state *s, const qcs_cuda_op &o);
 
-constexpr int kTileRegBits = 4;     // 16 amplitudes a thread
+constexpr int kTileRegBits = 4;     // 16 amplitudes a thread at most
 constexpr int kTileMaxBits = 11;    // tile amplitudes: 2^11 at most
+constexpr int kTileMaxThreadBits = 8;
 constexpr int kTileMaxGates = 128;  // per pass (they ride in the kernel parameters)
 constexpr int kTileMaxGroups = 32;
 constexpr int kTileMaxFlips = 32;
@@ -95,7 +96,7 @@ template <typename R> struct TileGate {
 struct TileGroup {
   unsigned char gate0, gate1, flip0, flip1;
   unsigned short reg[kTileRegBits];
-  unsigned short col[kTileMaxBits - kTileRegBits];
+  unsigned short col[kTileMaxThreadBits];
 };
 struct TileFlip {
   unsigned short mask;  // XORed into the constant
@@ -151,27 +152,29 @@ template <> struct TileTraits<float2> {
   typedef float R;
   typedef float Elem;  // of the tile in shared memory
   typedef FiniteF32 Finite;
-  typedef RegsF32<kTileRegBits> Regs;
+  template <int RB> using Regs = RegsF32<RB>;
   static constexpr int max_bits = 11, low = 4, blocks = 7;
 };
 template <> struct TileTraits<double2> {
   typedef double R;
   typedef double2 Elem;
   typedef FiniteF64 Finite;
-  typedef RegsF64<kTileRegBits> Regs;
+  template <int RB> using Regs = RegsF64<RB>;
   static constexpr int max_bits = 10, low = 3, blocks = 8;
 };
 
 #define QCS_TILE_TARGET(CALL)                                               \
-  if (op & 2) {                                                             \
-    if (op & 1) { constexpr int TB = 3; CALL; }                             \
-    else { constexpr int TB = 2; CALL; }                                    \
+  if (Regs::N > 4 && (op & 2)) {                                            \
+    if (Regs::N > 8 && (op & 1)) { constexpr int TB = Regs::N > 8 ? 3 : 0; CALL; } \
+    else { constexpr int TB = Regs::N > 4 ? 2 : 0; CALL; }                  \
   } else {                                                                  \
     if (op & 1) { constexpr int TB = 1; CALL; }                             \
     else { constexpr int TB = 0; CALL; }                                    \
   }
-#define QCS_TILE_PHASE(I, COND) \
-  case TO_PHASE + I: a.template phase<COND>(g.p); break;
+#define QCS_TILE_PHASE(I, COND)                   \
+  case TO_PHASE + I:                              \
+    if constexpr (COND < Regs::N) a.template phase<COND>(g.p); \
+    break;
 
 // One gate on the amplitudes of thread t.  (The compiler makes no jump table of
 // a switch here but a tree of comparisons over all the forms, seven branches
@@ -293,12 +296,12 @@ __device__ __noinline__ void general_tile(E *S, const TilePass<R> &P, uint32_t t
 
 // One thread per TileTraits::regs amplitudes of the tile; CTAs are persistent
 // over their tiles.
-template <typename C>
-__global__ void __launch_bounds__(1 << (TileTraits<C>::max_bits - kTileRegBits),
-                                  TileTraits<C>::blocks)
+template <typename C, int RB>
+__global__ void __launch_bounds__(1 << (TileTraits<C>::max_bits - RB),
+                                  TileTraits<C>::blocks >> (kTileRegBits - RB))
     k_tile(C *v, const __grid_constant__ TilePass<typename TileTraits<C>::R> P) {
   typedef typename TileTraits<C>::Elem E;
-  constexpr int RB = kTileRegBits, REGS = 1 << RB;
+  constexpr int REGS = 1 << RB;
   constexpr int UNIT = 16 / sizeof(C);  // amplitudes per 16-byte access
   constexpr int STEPS = REGS / UNIT;    // accesses per thread and tile
   constexpr int STEP_BITS = UNIT == 2 ? RB - 1 : RB;
@@ -380,16 +383,17 @@ __global__ void __launch_bounds__(1 << (TileTraits<C>::max_bits - kTileRegBits),
         for (int j = 0; j < TileTraits<C>::max_bits - RB; j++)
           if ((t >> j) & 1) at ^= G.col[j];
         auto place = [&](int (&pos)[REGS]) {  // register e: its bits' columns
-          int lo[4], hi[4];
+          int lo[4], hi[REGS / 4];
 #pragma unroll
-          for (int k = 0; k < 4; k++) {
+          for (int k = 0; k < 4; k++)
             lo[k] = at ^ ((k & 1) ? G.reg[0] : 0) ^ ((k & 2) ? G.reg[1] : 0);
+#pragma unroll
+          for (int k = 0; k < REGS / 4; k++)
             hi[k] = ((k & 1) ? G.reg[2] : 0) ^ ((k & 2) ? G.reg[3] : 0);
-          }
 #pragma unroll
           for (int e = 0; e < REGS; e++) pos[e] = lo[e & 3] ^ hi[e >> 2];
         };
-        typename TileTraits<C>::Regs a;
+        typename TileTraits<C>::template Regs<RB> a;
         {
           int pos[REGS];
           place(pos);
@@ -441,7 +445,7 @@ static bool moves_only(const qcs_cuda_op &o, bool reference) {
 // the current group; a later gate may still join the group if it commutes
 // with the waiting moves exactly: on other qubits, or diagonal on their
 // controls.  Stops early (s.last) when the pass is full.
-static void cut_groups(const qcs_cuda_op *ops, bool reference, TileStretch &s) {
+static void cut_groups(const qcs_cuda_op *ops, bool reference, int regs, TileStretch &s) {
   typedef unsigned long long Mask;
   Mask moved = 0, ctl = 0;  // targets and controls of the waiting moves
   TileStretch::Group g;
@@ -474,7 +478,7 @@ static void cut_groups(const qcs_cuda_op *ops, bool reference, TileStretch &s) {
     }
     const int q = needed_qubit(o);
     const bool held = q < 0 || ((g.qubits >> q) & 1);
-    const bool full = !held && __builtin_popcountll(g.qubits) == kTileRegBits;
+    const bool full = !held && __builtin_popcountll(g.qubits) == regs;
     // a condition of the gate on a moved qubit, or its target on a control
     const bool clash = ((t | c) & moved) || (q >= 0 && (t & ctl));
     if ((full || clash) && !close(i)) break;
@@ -485,7 +489,7 @@ static void cut_groups(const qcs_cuda_op *ops, bool reference, TileStretch &s) {
 }
 
 std::vector<TileStretch> tile_stretches(const qcs_cuda_op *ops, int count, int n, int nt, int low,
-                                        bool reference) {
+                                        bool reference, int regs) {
   std::vector<TileStretch> plan;
   for (int i = 0; i < count;) {
     TileStretch s;
@@ -506,7 +510,7 @@ std::vector<TileStretch> tile_stretches(const qcs_cuda_op *ops, int count, int n
       }
     s.last = i;
     s.qubits = set;
-    cut_groups(ops, reference, s);
+    cut_groups(ops, reference, regs, s);
     i = s.last;
     plan.push_back(s);
   }
@@ -603,10 +607,9 @@ static void fill_gate(const qcs_cuda_state *s, const qcs_cuda_op &o, const int *
   g.op = (unsigned char)op;
 }
 
-template <typename C>
+template <typename C, int RB>
 static int launch_pass(qcs_cuda_state *s, const qcs_cuda_op *ops, const TileStretch &st) {
   typedef typename TileTraits<C>::R R;
-  constexpr int RB = kTileRegBits;
   const C kind = {};
   TilePass<R> P;
   memset(&P, 0, offsetof(TilePass<R>, gate));
@@ -708,26 +711,37 @@ static int launch_pass(qcs_cuda_state *s, const qcs_cuda_op *ops, const TileStre
   // 19 (256), replayed, 105 -> 125; complex128, 18 qubits (256) 610 -> 1101.
   const int sms = s->dev.num_sms;
   const bool early = 2 * grid <= sms || (sizeof(C) == 8 && (grid <= sms || grid > 3 * sms));
-  launch_next(early, k_tile<C>, grid, threads, smem, s->stream, (C *)s->vec, P);
+  launch_next(early, k_tile<C, RB>, grid, threads, smem, s->stream, (C *)s->vec, P);
   invalidate_sum(s);
   return launched(s, KC_TILE, 2.0 * s->size * sizeof(C), "gate tile pass");
 }
 
-template <typename C>
-static int run_tiles_t(qcs_cuda_state *s, const qcs_cuda_op *ops, int count) {
-  const int nt = std::min(TileTraits<C>::max_bits, s->n);
+template <typename C, int RB>
+static int run_tiles_t(qcs_cuda_state *s, const qcs_cuda_op *ops, int count, int bits) {
+  const int nt = std::min(bits, s->n);
   for (const TileStretch &st : tile_stretches(ops, count, s->n, nt, TileTraits<C>::low,
-                                              s->sem == QCS_CUDA_REFERENCE)) {
+                                              s->sem == QCS_CUDA_REFERENCE, RB)) {
     const int rc = st.last - st.first == 1 ? apply_op(s, ops[st.first])
-                                           : launch_pass<C>(s, ops, st);
+                                           : launch_pass<C, RB>(s, ops, st);
     if (rc) return rc;
   }
   return QCS_CUDA_OK;
 }
 
+// Each quarter of an SM has an FP64 pipe of its own, which takes 64 cycles an
+// instruction of a warp, and tiles of 64 threads leave half of them idle where
+// an SM has one tile: there a complex128 tile has 4 warps, of 8 amplitudes a
+// thread, or of 4 with half the tile where that gives more SMs one.
+// Sweeps of 4 layers of RY, RZ and a CNOT ladder, 16 amplitudes a thread against
+// this: 12 qubits 337 -> 122 us, 16 (128 tiles of 2^9) 454 -> 177, 17 (128 of
+// 2^10) 493 -> 308; from 18 qubits on an SM has two tiles and more.
 int run_tiles(qcs_cuda_state *s, const qcs_cuda_op *ops, int count) {
-  return s->prec == QCS_CUDA_C128 ? run_tiles_t<double2>(s, ops, count)
-                                  : run_tiles_t<float2>(s, ops, count);
+  if (s->prec == QCS_CUDA_C64)
+    return run_tiles_t<float2, kTileRegBits>(s, ops, count, TileTraits<float2>::max_bits);
+  const i64 sms = s->dev.num_sms;
+  if (s->size >> 9 <= sms) return run_tiles_t<double2, 2>(s, ops, count, 9);
+  if (s->size >> 10 <= sms) return run_tiles_t<double2, 3>(s, ops, count, 10);
+  return run_tiles_t<double2, 4>(s, ops, count, 10);
 }
 
 // A state smaller than one thread's registers stays with the sweeps.

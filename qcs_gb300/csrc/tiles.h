@@ -11,7 +11,7 @@ namespace qcs {
 
 // Consecutive gates ops[first .. last) run in one pass over the state, on the
 // tile qubits `qubits` (a bit mask).  A group applies `gates` in order, whose
-// non-diagonal targets lie on at most 4 qubits (its mask), then `moves` (X,
+// non-diagonal targets lie on at most `regs` qubits (its mask), then `moves` (X,
 // CNOT).
 struct TileStretch {
   struct Group {
@@ -27,7 +27,7 @@ struct TileStretch {
 // always hold the `low` lowest qubits.  The gates keep their order (but for
 // moves that commute exactly).
 std::vector<TileStretch> tile_stretches(const qcs_cuda_op *ops, int count, int n, int nt, int low,
-                                        bool reference);
+                                        bool reference, int regs);
 
 // Applies a list of gates (no phase flips or diffusions) in place.
 int run_tiles(qcs_cuda_state *s, const qcs_cuda_op *ops, int count);

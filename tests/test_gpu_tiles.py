@@ -112,3 +112,23 @@ def test_flips_and_diffusions_between_gates(prec, sem):
 def test_infinities_and_nans_spread_as_in_the_sweeps(n, prec, sem):
     compare(n, prec, sem, every_kind(n, 31, 12), start(n, 5, bad=True))
     compare(n, prec, sem, every_kind(n, 32, 60), start(n, 6, bad=True))
+
+
+@pytest.mark.parametrize("sem", [capi.PHYSICAL, capi.REFERENCE])
+@pytest.mark.parametrize("n", [4, 8, 9, 16, 17, 18])
+def test_every_split_of_a_complex128_tile(n, sem):
+    """4, 8 and 16 amplitudes a thread, tiles of 2^9 and 2^10; groups of few
+    qubits (more groups than a pass takes), phases with conditions on every
+    pair of register bits, and tiles with an infinity or a NaN."""
+    wide = W.GateList()
+    for rep in range(12):
+        for q in range(n):
+            wide.add(W.RY, q, -1, 0.3 + 0.1 * rep + 0.01 * q)
+    for q in range(n):
+        for p in range(n):
+            if p != q:
+                wide.add(W.CPHASE, q, p, 0.2 + 0.03 * q + 0.005 * p)
+                wide.add(W.RX, p, -1, 0.4)
+    compare(n, capi.C128, sem, every_kind(n, 500 + n, 400), start(n, n))
+    compare(n, capi.C128, sem, wide, start(n, n + 1))
+    compare(n, capi.C128, sem, every_kind(n, 600 + n, 150), start(n, n + 2, bad=True))
