@@ -735,10 +735,18 @@ static int run_tiles_t(qcs_cuda_state *s, const qcs_cuda_op *ops, int count, int
 // Sweeps of 4 layers of RY, RZ and a CNOT ladder, 16 amplitudes a thread against
 // this: 12 qubits 337 -> 122 us, 16 (128 tiles of 2^9) 454 -> 177, 17 (128 of
 // 2^10) 493 -> 308; from 18 qubits on an SM has two tiles and more.
+// complex64 gates wait for their own latency where an SM has one or two tiles,
+// which 8 warps of 8 amplitudes hide better than 4 of 16, and smaller tiles spread
+// (300 random gates; 4, 8 amplitudes a thread in 2^10, 8 and 16 in 2^11): 13
+// qubits 67, 71, 72, 83 us; 16 91, 95, 95, 115; 17 103, 100, 101, 120; 19 210,
+// 143, 130, 147; 20 332, 230, 239, 192.  4 a thread gains little where it gains.
 int run_tiles(qcs_cuda_state *s, const qcs_cuda_op *ops, int count) {
-  if (s->prec == QCS_CUDA_C64)
-    return run_tiles_t<float2, kTileRegBits>(s, ops, count, TileTraits<float2>::max_bits);
   const i64 sms = s->dev.num_sms;
+  if (s->prec == QCS_CUDA_C64) {
+    if (s->size >> 10 <= sms / 2) return run_tiles_t<float2, 3>(s, ops, count, 10);
+    if (s->size >> 11 <= 2 * sms) return run_tiles_t<float2, 3>(s, ops, count, 11);
+    return run_tiles_t<float2, 4>(s, ops, count, 11);
+  }
   if (s->size >> 9 <= sms) return run_tiles_t<double2, 2>(s, ops, count, 9);
   if (s->size >> 10 <= sms) return run_tiles_t<double2, 3>(s, ops, count, 10);
   return run_tiles_t<double2, 4>(s, ops, count, 10);

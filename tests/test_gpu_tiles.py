@@ -132,3 +132,10 @@ def test_every_split_of_a_complex128_tile(n, sem):
     compare(n, capi.C128, sem, every_kind(n, 500 + n, 400), start(n, n))
     compare(n, capi.C128, sem, wide, start(n, n + 1))
     compare(n, capi.C128, sem, every_kind(n, 600 + n, 150), start(n, n + 2, bad=True))
+
+
+@pytest.mark.parametrize("n", [10, 16, 17, 19, 20])
+def test_every_split_of_a_complex64_tile(n):
+    """8 amplitudes a thread in tiles of 2^10 and 2^11, and 16."""
+    compare(n, capi.C64, capi.PHYSICAL, every_kind(n, 700 + n, 400), start(n, n))
+    compare(n, capi.C64, capi.PHYSICAL, every_kind(n, 800 + n, 150), start(n, n + 2, bad=True))
