@@ -49,6 +49,7 @@
 #include "common.cuh"
 #include "fusion.h"
 #include "tile_regs.cuh"
+#include "widen.cuh"
 
 namespace qcs {
 
@@ -318,10 +319,8 @@ __device__ __forceinline__ void run_groups(float *S, const BStage &st, BWindow &
 // ---- read-outs ----------------------------------------------------------
 // <Z_0> and the sampling tiles' masses are FP64 sums of FP32 squares; inside a
 // tile a shot follows running sums of exact squares in FP64.  All of it is
-// bound by the FP64 pipe (two lanes per clock and SM), which also does the
-// conversions from float, so those are made with integer operations (exact
-// for zeros and normal numbers; others are converted), the squares go straight
-// into the sums by FMA, and no amplitude is summed twice: every block of 32 or
+// bound by the FP64 pipe, so floats are widened with integer operations
+// (widen.cuh), the squares go straight into the sums by FMA, and no amplitude is summed twice: every block of 32 or
 // more amplitudes is summed once, by whichever CTA is free, and a shot (a
 // thread) searches the running sums and then one block.  Against a scan of the
 // shot's tile, 4096 amplitudes or more, by a warp of the instance's one CTA: 384
@@ -330,25 +329,6 @@ __device__ __forceinline__ void run_groups(float *S, const BStage &st, BWindow &
 
 __device__ __forceinline__ float prob32(float2 a) { return a.x * a.x + a.y * a.y; }
 __device__ __forceinline__ bool nonzero(float2 a) { return a.x != 0.f || a.y != 0.f; }
-
-// |x| as a double; PLAIN: of a zero or a normal number, by its bits.
-template <bool PLAIN>
-__device__ __forceinline__ double to64(float x) {
-  if (!PLAIN) return fabs((double)x);
-  const unsigned w = __float_as_uint(x) << 1;
-  return __hiloint2double(w ? (int)((w >> 4) + 0x38000000u) : 0, (int)(w << 28));
-}
-
-// Whether all of the numbers seen are zero or normal.
-struct PlainTest {
-  unsigned lo = 0xffffffffu, hi = 0;  // of the bits without the sign, less one
-  __device__ __forceinline__ void see(float x) {
-    const unsigned w = (__float_as_uint(x) << 1) - 1u;  // zero: the largest
-    lo = min(lo, w);
-    hi = max(hi, w + 1u);
-  }
-  __device__ __forceinline__ bool plain() const { return lo >= 0xffffffu && hi < 0xff000000u; }
-};
 
 // cum[k] = c + the squares of a[0 .. k].
 template <bool PLAIN>

@@ -27,12 +27,6 @@ namespace qcs {
 
 enum { OP_NORM = 0, OP_MASK = 1, OP_SUM = 2 };
 
-__device__ __forceinline__ double warp_sum(double x) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  return x;
-}
-
 // Called by every thread of every block, after thread 0 has written the
 // block's partial: true in the block that gets here last, which then sees
 // every block's.  Leaves the counter at zero for the next launch.
@@ -50,66 +44,57 @@ __device__ __forceinline__ bool last_block(unsigned *count) {
   return last;
 }
 
-// Sum four FP64 values over the block; thread 0 writes `out`.
-__device__ void block_sum4(double a, double b, double c, double d, ReduceSlot *out) {
-  __shared__ double sh[4][kReduceThreads / 32];
-  a = warp_sum(a);
-  b = warp_sum(b);
-  c = warp_sum(c);
-  d = warp_sum(d);
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) {
-    sh[0][w] = a;
-    sh[1][w] = b;
-    sh[2][w] = c;
-    sh[3][w] = d;
-  }
-  __syncthreads();
-  if (w == 0) {
-    const int nw = blockDim.x >> 5;
-    a = l < nw ? sh[0][l] : 0.0;
-    b = l < nw ? sh[1][l] : 0.0;
-    c = l < nw ? sh[2][l] : 0.0;
-    d = l < nw ? sh[3][l] : 0.0;
-    a = warp_sum(a);
-    b = warp_sum(b);
-    c = warp_sum(c);
-    d = warp_sum(d);
-    if (l == 0) {
-      out->a = a;
-      out->b = b;
-      out->c = c;
-      out->d = d;
-    }
-  }
+// Lanes 0-15 get the warp's sum of a, the others that of b.
+__device__ __forceinline__ double warp_sum2(double a, double b) {
+  const bool up = (threadIdx.x & 16) != 0;
+  double x = (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
 }
 
-// The block adds nblocks partials in a fixed order; thread 0 writes four sums.
+// Two FP64 sums over the block; in warp 0, lane 0 gets that of a and lane 16
+// that of b.  (Half the lanes for each: 8 additions in a row, where summing
+// both, and two unused values, in every lane took 40 in the FP64 pipe: <Z> on
+// 16 qubits 17.9 -> 14.0 us a call.)
+__device__ __forceinline__ double block_sum2(double a, double b) {
+  constexpr int kWarps = kReduceThreads / 32;
+  static_assert(kWarps <= 16, "a lane of each half per warp");
+  __shared__ double sh[2][kWarps];
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  double x = warp_sum2(a, b);
+  if ((l & 15) == 0) sh[l >> 4][w] = x;
+  __syncthreads();
+  x = 0.0;
+  if (w == 0) {
+    x = (l & 15) < kWarps ? sh[l >> 4][l & 15] : 0.0;
+#pragma unroll
+    for (int o = kWarps / 2; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  }
+  return x;
+}
+
+// The block adds nblocks partials in a fixed order and writes the two sums.
 __device__ void sum_slots(const ReduceSlot *p, int nblocks, double *result) {
-  double a = 0.0, b = 0.0, c = 0.0, d = 0.0;
+  double a = 0.0, b = 0.0;
   for (int i = threadIdx.x; i < nblocks; i += blockDim.x) {
-    const double2 *s = reinterpret_cast<const double2 *>(p + i);
-    const double2 x = __ldcg(s), y = __ldcg(s + 1);
+    const double2 x = __ldcg(reinterpret_cast<const double2 *>(p + i));
     a += x.x;
     b += x.y;
-    c += y.x;
-    d += y.y;
   }
   __syncthreads();
-  ReduceSlot r;
-  block_sum4(a, b, c, d, &r);
-  if (threadIdx.x == 0) {
-    result[0] = r.a;
-    result[1] = r.b;
-    result[2] = r.c;
-    result[3] = r.d;
-  }
+  const double x = block_sum2(a, b);
+  if (threadIdx.x == 0) result[0] = x;
+  if (threadIdx.x == 16) result[1] = x;
 }
 
 // Ends a reduction: the block's partial, then (last block) the total.
 __device__ __forceinline__ void reduce_end(double a, double b, ReduceSlot *slots, unsigned *count,
                                            double *result) {
-  block_sum4(a, b, 0.0, 0.0, slots + blockIdx.x);
+  const double x = block_sum2(a, b);
+  if (threadIdx.x == 0) slots[blockIdx.x].a = x;
+  if (threadIdx.x == 16) slots[blockIdx.x].b = x;
+  __syncwarp();  // lane 16's partial, before thread 0 counts the block
   if (last_block(count)) sum_slots(slots, gridDim.x, result);
 }
 
@@ -128,9 +113,11 @@ __device__ __forceinline__ void accum(i64 idx, R re, R im, int q, R &pa, R &pb) 
 }
 
 // complex64: units of two amplitudes (one 16-byte load), four units per
-// step, FP32 within a step, FP64 across steps.
+// step, FP32 within a step, FP64 across steps.  (Four blocks an SM is the grid;
+// said so, the compiler keeps a step's four loads in flight: with 32 registers a
+// pass over 28 qubits took 5 % longer.)
 template <int OP>
-__global__ void __launch_bounds__(kReduceThreads)
+__global__ void __launch_bounds__(kReduceThreads, 4)
     k_reduce_c64(const float4 *v, i64 units, int q, ReduceSlot *slots, unsigned *count,
                  double *result) {
   grid_wait();
@@ -325,15 +312,6 @@ constexpr int kMeasureMaxBytes = 128 << 10;
 constexpr int kMeasureMaxQubits = 14;
 constexpr int kMeasureThreads = 512;
 struct MeasureDraws { double r[kMeasureMaxQubits]; };
-
-// Lanes 0-15 get the warp's sum of a, the others that of b.
-__device__ __forceinline__ double warp_sum2(double a, double b) {
-  const bool up = (threadIdx.x & 16) != 0;
-  double x = (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
-#pragma unroll
-  for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  return x;
-}
 
 template <typename C>
 __global__ void __launch_bounds__(kMeasureThreads)
