@@ -51,7 +51,7 @@ def parse():
                     choices=["auto", "simt", "tensor"])
     ap.add_argument("--plain-steps", type=int, default=None,
                     help="timed steps of the plain form (default: --steps, at most 3: "
-                         "one plain step is ~10 s)")
+                         "one plain step is about 1 s)")
     ap.add_argument("--parity-qubits", type=int, default=24)
     ap.add_argument("--no-parity", action="store_true")
     ap.add_argument("--cpu-sample-gates", type=int, default=48)
@@ -71,7 +71,7 @@ def parse():
                     help="batch: largest instance (qubit counts uniform in [10, this]); "
                          "smaller values give small profiling cases")
     ap.add_argument("--no-autotune", action="store_true",
-                    help="batch: keep the default schedule (512 threads, tile 2^13, 2 CTAs/SM)")
+                    help="batch: keep the default schedule (256 threads, tile 2^13, 2 CTAs/SM)")
     ap.add_argument("--shots", type=int, default=1024)
     return ap.parse_args()
 
@@ -612,27 +612,24 @@ def run_sweeps(args, dist):
 
 
 def fp64_ops_physical(gates, n: int) -> float:
-    """FP64 operations of a gate list's complex128 sweeps in PHYSICAL
-    semantics, counted per kernel: a complex product is 6 operations (4
-    multiplies, 2 adds, no FMA: the reference's order), a sum 2.  Dense 2x2
-    (H, RX, RY): 2 products + 1 sum per output, 28 per pair; exchange (X, Y,
-    CNOT): 1 product per output, 12 per pair; diagonal (RZ): 1 product per
-    amplitude; phase (Z, P, CPHASE): 1 product per touched amplitude."""
+    """FP64 operations of a gate list on a complex128 state in PHYSICAL
+    semantics, as the tile passes do them (no FMA: the reference's order): RX,
+    RY 8 multiplies and 4 adds a pair, H 4 and 4 (its products serve both
+    outputs); a complex product of 6 an amplitude for RZ and an amplitude that
+    P or CPHASE touches; X, Y, Z and CNOT move amplitudes or flip signs."""
     from qcs_gb300 import workloads as W
     N = float(1 << n)
     ops = 0.0
     for k in gates.kinds:
         k = int(k)
-        if k in (W.H, W.RX, W.RY):
-            ops += 28 * N / 2
-        elif k in (W.X, W.Y):
+        if k in (W.RX, W.RY):
             ops += 12 * N / 2
+        elif k == W.H:
+            ops += 8 * N / 2
         elif k == W.RZ:
             ops += 6 * N
-        elif k in (W.Z, W.P):
+        elif k == W.P:
             ops += 6 * N / 2
-        elif k == W.CNOT:
-            ops += 12 * N / 4
         elif k == W.CPHASE:
             ops += 6 * N / 4
     return ops
@@ -644,8 +641,8 @@ FP64_NOMINAL_OPS = 0.625e12
 
 
 def run_random20(args, dist):
-    """20 qubits, complex128, random basis state, QFT, 200 random gates, one
-    kernel per gate.  REFERENCE semantics must equal the reference's
+    """20 qubits, complex128, random basis state, QFT, 200 random gates, gate
+    by gate.  REFERENCE semantics must equal the reference's
     sequential rule (oracle COMPAT mode) bit for bit; PHYSICAL semantics must
     equal the oracle's physical mode bit for bit."""
     from oracle import oracle as O
@@ -695,8 +692,8 @@ def run_random20(args, dist):
                 "frac": fops / (ms / 1e3) / FP64_NOMINAL_OPS,
                 "peak_source": "nominal (1.25 TFLOP/s with FMA counted as 2; not measured "
                                "on this pool)",
-                "note": "the 16 MB (complex128) state stays in L2; the sweeps are bound by "
-                        "FP64 issue, plus one launch per gate"}
+                "note": "the 16 MB (complex128) state stays in L2; the tile passes, several "
+                        "gates each, are bound by FP64 issue"}
         out[name] = {"gate_apps_per_s": len(full) / (ms / 1e3), "ms_per_circuit": ms,
                      "bit_exact": bool(np.array_equal(a.view(np.float64), ref.view(np.float64))),
                      "max_abs_err": float(np.max(np.abs(a - ref))),

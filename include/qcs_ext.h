@@ -21,7 +21,7 @@ extern "C" {
 void qc_cphase(t_q_circuit *circuit, int control, int target, double angle);
 
 /* Circuit with explicit precision (QCS_CUDA_C64/C128), semantics
- * (QCS_CUDA_PHYSICAL/REFERENCE) and fusion width (0: one kernel per gate).
+ * (QCS_CUDA_PHYSICAL/REFERENCE) and fusion width (0: gate by gate).
  * qc_create reads the same settings from QCS_CUDA_PRECISION ("c64",
  * "c128"), QCS_CUDA_SEMANTICS ("physical", "reference") and QCS_CUDA_FUSION
  * (an integer k) and defaults to c64 / physical / 0. */
