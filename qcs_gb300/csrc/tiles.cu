@@ -144,9 +144,9 @@ struct FiniteF64 {
 // ms on 27 qubits (brick, 752 gates), 87 and 101 us on 13, where the threads
 // of the tiles are all the parallelism there is; 10 against 11 (complex128,
 // 20 qubits, 417 gates): 2.13 and 2.32 ms.  Likewise 16 amplitudes a thread
-// against 32: 27.7 and 28.9 ms, 87 and 122 us.
+// against 32: 27.7 and 28.9 ms, 87 and 122 us.  (By number of tiles: run_tiles.)
 // low: qubits every tile holds, so that it is read in runs of 128 bytes.
-// blocks: CTAs an SM holds (72 registers a thread for complex64).
+// blocks: CTAs an SM holds at 16 amplitudes a thread (72 registers, complex64).
 template <typename C> struct TileTraits;
 template <> struct TileTraits<float2> {
   typedef float R;
@@ -294,7 +294,7 @@ __device__ __noinline__ void general_tile(E *S, const TilePass<R> &P, uint32_t t
   }
 }
 
-// One thread per TileTraits::regs amplitudes of the tile; CTAs are persistent
+// One thread per 2^RB amplitudes of the tile; CTAs are persistent
 // over their tiles.
 template <typename C, int RB>
 __global__ void __launch_bounds__(1 << (TileTraits<C>::max_bits - RB),
@@ -700,8 +700,13 @@ static int launch_pass(qcs_cuda_state *s, const qcs_cuda_op *ops, const TileStre
   for (int b = 0; b < P.nt; b++) P.store[b] = (unsigned short)map[b];
   const int threads = 1 << (P.nt - RB);
   const size_t smem = sizeof(C) << P.nt;
-  const i64 cap = (i64)s->dev.num_sms * std::min(32, TileTraits<C>::blocks
-                                                         << (TileTraits<C>::max_bits - P.nt));
+  // Several times the CTAs that an SM holds: CTAs that end and begin fall out of
+  // step, so the loads of some run under the gates of others, and the last tiles
+  // are spread.  As many as it holds (7), 28, 64, 100: 27 qubits (complex64, 752
+  // gates) 27.7, 25.7, 25.1, 24.9 ms alone, but 23.9, 24.0, 24.3 a run where
+  // three states run at once, which has the same effect; 24 qubits 3.13, 2.89,
+  // 2.97, 2.97.  complex128, 24 qubits (8, 28, 100) 33.8, 32.4, 31.9.
+  const i64 cap = (i64)s->dev.num_sms * (sizeof(C) == 8 ? 28 : 64);
   const int grid = (int)std::min<i64>(P.n_tiles, cap);
   s->h2d_bytes += (long long)(offsetof(TilePass<R>, gate) + P.ngates * sizeof(TileGate<R>));
   prof_begin(s);
@@ -730,11 +735,13 @@ static int run_tiles_t(qcs_cuda_state *s, const qcs_cuda_op *ops, int count, int
 
 // Each quarter of an SM has an FP64 pipe of its own, which takes 64 cycles an
 // instruction of a warp, and tiles of 64 threads leave half of them idle where
-// an SM has one tile: there a complex128 tile has 4 warps, of 8 amplitudes a
-// thread, or of 4 with half the tile where that gives more SMs one.
+// an SM has one tile: a complex128 tile has 4 warps, of 8 amplitudes a thread,
+// or of 4 with half the tile where that gives more SMs one.
 // Sweeps of 4 layers of RY, RZ and a CNOT ladder, 16 amplitudes a thread against
 // this: 12 qubits 337 -> 122 us, 16 (128 tiles of 2^9) 454 -> 177, 17 (128 of
-// 2^10) 493 -> 308; from 18 qubits on an SM has two tiles and more.
+// 2^10) 493 -> 308; from 18 qubits on an SM has two tiles and more,
+// and 4 warps a tile still spread better (18, 20, 24 qubits, QFT and 200 gates,
+// 16 amplitudes against 8: 701, 2166, 34748 us, 607, 1975, 34251).
 // complex64 gates wait for their own latency where an SM has one or two tiles,
 // which 8 warps of 8 amplitudes hide better than 4 of 16, and smaller tiles spread
 // (300 random gates; 4, 8 amplitudes a thread in 2^10, 8 and 16 in 2^11): 13
@@ -748,8 +755,7 @@ int run_tiles(qcs_cuda_state *s, const qcs_cuda_op *ops, int count) {
     return run_tiles_t<float2, 4>(s, ops, count, 11);
   }
   if (s->size >> 9 <= sms) return run_tiles_t<double2, 2>(s, ops, count, 9);
-  if (s->size >> 10 <= sms) return run_tiles_t<double2, 3>(s, ops, count, 10);
-  return run_tiles_t<double2, 4>(s, ops, count, 10);
+  return run_tiles_t<double2, 3>(s, ops, count, 10);
 }
 
 // A state smaller than one thread's registers stays with the sweeps.

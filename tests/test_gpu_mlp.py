@@ -2,7 +2,7 @@
 (8), gradient slots (64), the size above which the slots are summed by a
 kernel of their own (1024), and the smallest and largest feature counts.
 
-Gradients against the FP64 checker to 1e-4 of the largest, the bar of the
+Gradients against the FP64 oracle to 1e-4 of the largest, the bar of the
 other cost-model tests: FP32 sums of up to 1100 terms, each layer's rounding
 passed on to the next.  One Adam step against the formula on the device's own
 gradient to 2e-7: the step is at most lr = 1e-3 with a few FP32 roundings, and
