@@ -255,16 +255,17 @@ int qcs_cuda_batch_run(qcs_cuda_batch *b, double *expect_z0,
                        long long *samples, double *ms);
 /* Times every schedule (threads per CTA 256/512/1024, tile 2^12..2^14,
  * 1, 2 or 4 CTAs per SM as fit, largest-first or given order) on this batch, then how
- * widely large instances spread (an instance above split_q qubits is shared
- * by 2^(n - split_q) CTAs, split_q in 17..20 or never), and keeps the
+ * widely large instances spread (2^(n - split_q) CTAs start on an instance above
+ * split_q qubits, split_q in 17..20 or one always), and keeps the
  * fastest; chosen (4 ints) receives threads, tile qubits, CTAs per SM and
  * order. */
 int qcs_cuda_batch_autotune(qcs_cuda_batch *b, int repeats, int *chosen);
 /* The schedule in force (5 ints): threads, tile qubits, CTAs per SM that
  * actually run, order, split_q. */
 int qcs_cuda_batch_schedule(qcs_cuda_batch *b, int *schedule);
-/* Instances above split_q qubits (and above the tile) are shared by
- * 2^(n - split_q) CTAs, at most half the grid; 27 never splits. */
+/* 2^(n - split_q) CTAs, at most half the grid, start on an instance above
+ * split_q qubits (and above the tile), one at 27; CTAs that come free at the
+ * end of the batch join.  Results do not depend on it. */
 int qcs_cuda_batch_split(qcs_cuda_batch *b, int split_q);
 /* Algorithmic HBM bytes of one run under the schedule in force: for every
  * instance above the tile (kept in a global slot), one write of its 2^n

@@ -313,6 +313,17 @@ __global__ void __launch_bounds__(kReduceThreads)
   }
 }
 
+// One amplitude, to the host (8 us a call, and 3 less behind
+// another kernel, than a copy and the stream's end: 9 and 13).
+template <typename C>
+__global__ void k_peek(const C *v, i64 index, double *result) {
+  grid_wait();
+  const C x = v[index];
+  result[0] = x.x;
+  result[1] = x.y;
+  report(result);
+}
+
 // Every qubit of a small state measured in one block, the state in shared
 // memory: per qubit P(0) and P(1) (FP32 squares of two adjacent amplitudes,
 // summed in FP64; complex128 in FP64), the outcome of its draw, the collapse.
@@ -786,18 +797,20 @@ int qcs_cuda_probability(qcs_cuda_state *s, long long index, double *p) {
     *p = 0.0;  // qc_get_probability returns 0.0 out of range (src/qcs.c:392-393)
     return QCS_CUDA_OK;
   }
-  size_t bytes = s->prec == QCS_CUDA_C128 ? 16 : 8;
-  int rc = copy_d2h(s, s->h_result, (char *)s->vec + (size_t)index * bytes, bytes,
-                    "probability readback");
-  if (!rc) rc = check_cuda(cudaStreamSynchronize(s->stream), "probability sync");
+  const size_t bytes = s->prec == QCS_CUDA_C128 ? 16 : 8;
+  expect_report(s);
+  prof_begin(s);
+  if (s->prec == QCS_CUDA_C128)
+    launch_next(true, k_peek<double2>, 1, 1, 0, s->stream, (const double2 *)s->vec, (i64)index,
+                s->h_result_dev);
+  else
+    launch_next(true, k_peek<float2>, 1, 1, 0, s->stream, (const float2 *)s->vec, (i64)index,
+                s->h_result_dev);
+  int rc = launched(s, KC_OTHER, (double)bytes, "probability");
+  if (!rc) rc = wait_report(s, bytes, "probability sync");
   if (rc) return rc;
-  if (s->prec == QCS_CUDA_C128) {
-    double re = s->h_result[0], im = s->h_result[1];
-    *p = (re * re) + (im * im);
-  } else {
-    const float *f = (const float *)s->h_result;
-    *p = ((double)f[0] * (double)f[0]) + ((double)f[1] * (double)f[1]);
-  }
+  const double re = s->h_result[0], im = s->h_result[1];
+  *p = (re * re) + (im * im);
   return QCS_CUDA_OK;
 }
 
