@@ -89,6 +89,7 @@ struct qcs_cuda_state {
   double *d_result;    // 8 doubles
   double *h_result;    // pinned, 8 doubles
   double *h_result_dev;  // its device address: kernels write results there
+  qcs::i64 calls;        // read-outs so far: the number the last one waits for
   // cached sum of amplitudes (complex, FP64) for Grover iterations; valid
   // while sum_valid != 0 (kept on the device in d_result[4..5])
   int sum_valid;

@@ -74,19 +74,21 @@ __device__ __forceinline__ double block_sum2(double a, double b) {
   return x;
 }
 
-// The host waits for result[kReady], written after everything else (by one
-// thread, in step with those that wrote it): the kernel's end and the stream's
-// take microseconds more to reach it.
+// The host waits for its call's number in result[kReady], written after
+// everything else (by one thread, in step with those that wrote it): the
+// kernel's end and the stream's take microseconds more to reach it.  The number
+// tells this kernel's result from that of one before it whose call returned
+// early, with an error.
 constexpr int kReady = 7;
-__device__ __forceinline__ void report(double *result) {
+__device__ __forceinline__ void report(double *result, i64 call) {
   __threadfence_system();
-  *(volatile double *)(result + kReady) = 1.0;
+  *(volatile i64 *)(result + kReady) = call;
 }
 
 // The block adds nblocks partials in a fixed order and writes the two sums.
 // HOST: to the pinned buffer that the host reads.
 template <bool HOST>
-__device__ void sum_slots(const ReduceSlot *p, int nblocks, double *result) {
+__device__ void sum_slots(const ReduceSlot *p, int nblocks, double *result, i64 call) {
   double a = 0.0, b = 0.0;
   for (int i = threadIdx.x; i < nblocks; i += blockDim.x) {
     const double2 x = __ldcg(reinterpret_cast<const double2 *>(p + i));
@@ -98,18 +100,18 @@ __device__ void sum_slots(const ReduceSlot *p, int nblocks, double *result) {
   if (threadIdx.x == 0) result[0] = x;
   if (threadIdx.x == 16) result[1] = x;
   __syncwarp();
-  if (HOST && threadIdx.x == 0) report(result);
+  if (HOST && threadIdx.x == 0) report(result, call);
 }
 
 // Ends a reduction: the block's partial, then (last block) the total.
 template <bool HOST>
 __device__ __forceinline__ void reduce_end(double a, double b, ReduceSlot *slots, unsigned *count,
-                                           double *result) {
+                                           double *result, i64 call) {
   const double x = block_sum2(a, b);
   if (threadIdx.x == 0) slots[blockIdx.x].a = x;
   if (threadIdx.x == 16) slots[blockIdx.x].b = x;
   __syncwarp();  // lane 16's partial, before thread 0 counts the block
-  if (last_block(count)) sum_slots<HOST>(slots, gridDim.x, result);
+  if (last_block(count)) sum_slots<HOST>(slots, gridDim.x, result, call);
 }
 
 template <int OP, typename R>
@@ -133,7 +135,7 @@ __device__ __forceinline__ void accum(i64 idx, R re, R im, int q, R &pa, R &pb) 
 template <int OP>
 __global__ void __launch_bounds__(kReduceThreads, 4)
     k_reduce_c64(const float4 *v, i64 units, int q, ReduceSlot *slots, unsigned *count,
-                 double *result) {
+                 double *result, i64 call) {
   grid_wait();
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   double A = 0.0, B = 0.0;
@@ -161,13 +163,13 @@ __global__ void __launch_bounds__(kReduceThreads, 4)
     A += (double)pa;
     B += (double)pb;
   }
-  reduce_end<OP != OP_SUM>(A, B, slots, count, result);
+  reduce_end<OP != OP_SUM>(A, B, slots, count, result, call);
 }
 
 template <int OP>
 __global__ void __launch_bounds__(kReduceThreads)
     k_reduce_c128(const double2 *v, i64 size, int q, ReduceSlot *slots, unsigned *count,
-                  double *result) {
+                  double *result, i64 call) {
   grid_wait();
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   double A = 0.0, B = 0.0;
@@ -175,13 +177,13 @@ __global__ void __launch_bounds__(kReduceThreads)
     double2 x = v[i];
     accum<OP, double>(i, x.x, x.y, q, A, B);
   }
-  reduce_end<OP != OP_SUM>(A, B, slots, count, result);
+  reduce_end<OP != OP_SUM>(A, B, slots, count, result, call);
 }
 
 // One block combines partials that another kernel left.
 __global__ void __launch_bounds__(kReduceThreads)
     k_finalize(const ReduceSlot *p, int nblocks, double *result) {
-  sum_slots<false>(p, nblocks, result);
+  sum_slots<false>(p, nblocks, result, 0);
 }
 
 // Physical diffusion psi := 2*(S/N) - psi, fused with the sum of the new
@@ -215,7 +217,7 @@ __global__ void __launch_bounds__(kReduceThreads)
     A += (double)pa;
     B += (double)pb;
   }
-  reduce_end<false>(A, B, slots, count, S);  // every block has read S by now
+  reduce_end<false>(A, B, slots, count, S, 0);  // every block has read S by now
 }
 
 __global__ void __launch_bounds__(kReduceThreads)
@@ -232,7 +234,7 @@ __global__ void __launch_bounds__(kReduceThreads)
     A += y.x;
     B += y.y;
   }
-  reduce_end<false>(A, B, slots, count, S);
+  reduce_end<false>(A, B, slots, count, S, 0);
 }
 
 // The reference's diffusion (src/q_gates.c:334-355): mean := S/|S| when
@@ -316,12 +318,12 @@ __global__ void __launch_bounds__(kReduceThreads)
 // One amplitude, to the host (8 us a call, and 3 less behind
 // another kernel, than a copy and the stream's end: 9 and 13).
 template <typename C>
-__global__ void k_peek(const C *v, i64 index, double *result) {
+__global__ void k_peek(const C *v, i64 index, double *result, i64 call) {
   grid_wait();
   const C x = v[index];
   result[0] = x.x;
   result[1] = x.y;
-  report(result);
+  report(result, call);
 }
 
 // Every qubit of a small state measured in one block, the state in shared
@@ -340,7 +342,8 @@ struct MeasureDraws { double r[kMeasureMaxQubits]; };
 
 template <typename C>
 __global__ void __launch_bounds__(kMeasureThreads)
-    k_measure_all(C *v, int n, const __grid_constant__ MeasureDraws draws, double *outcomes) {
+    k_measure_all(C *v, int n, const __grid_constant__ MeasureDraws draws, double *outcomes,
+                  i64 call) {
   using R = decltype(C::x);
   constexpr int kWarps = kMeasureThreads / 32;  // 16: a lane each for P(0) and P(1)
   extern __shared__ __align__(16) unsigned char measure_smem[];
@@ -411,7 +414,7 @@ __global__ void __launch_bounds__(kMeasureThreads)
   __syncthreads();  // the state is written
   if (threadIdx.x == 0) {
     outcomes[0] = (double)bits;
-    report(outcomes);
+    report(outcomes, call);
   }
 }
 
@@ -466,7 +469,7 @@ __device__ __forceinline__ void block_best(R &bv, i64 &bi) {
 // Ends an argmax: the block's best, then (last block) the best of all.
 template <typename R>
 __device__ __forceinline__ void argmax_end(R bv, i64 bi, ReduceSlot *slots, unsigned *count,
-                                           double *result) {
+                                           double *result, i64 call) {
   block_best(bv, bi);
   if (threadIdx.x == 0) {
     slots[blockIdx.x].a = (double)bv;
@@ -486,13 +489,13 @@ __device__ __forceinline__ void argmax_end(R bv, i64 bi, ReduceSlot *slots, unsi
   if (threadIdx.x == 0) {
     result[0] = v;
     result[1] = (double)at;
-    report(result);
+    report(result, call);
   }
 }
 
 template <typename C, typename R>
 __global__ void __launch_bounds__(kReduceThreads)
-    k_argmax(const C *v, i64 size, ReduceSlot *slots, unsigned *count, double *result) {
+    k_argmax(const C *v, i64 size, ReduceSlot *slots, unsigned *count, double *result, i64 call) {
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   R bv = (R)-1;
   i64 bi = size;
@@ -504,7 +507,7 @@ __global__ void __launch_bounds__(kReduceThreads)
       bi = i;
     }
   }
-  argmax_end(bv, bi, slots, count, result);
+  argmax_end(bv, bi, slots, count, result, call);
 }
 
 // complex64: units of two amplitudes (one 16-byte load), four in flight per
@@ -512,7 +515,7 @@ __global__ void __launch_bounds__(kReduceThreads)
 // independent of which thread saw which amplitude.
 __global__ void __launch_bounds__(kReduceThreads)
     k_argmax_c64(const float4 *v, i64 units, ReduceSlot *slots, unsigned *count,
-                 double *result) {
+                 double *result, i64 call) {
   const i64 nthr = (i64)gridDim.x * blockDim.x;
   float bv = -1.f;
   i64 bi = 2 * units;
@@ -539,7 +542,7 @@ __global__ void __launch_bounds__(kReduceThreads)
       }
     }
   }
-  argmax_end(bv, bi, slots, count, result);
+  argmax_end(bv, bi, slots, count, result, call);
 }
 
 // ---- shot sampling: sampler.cuh -------------------------------------------------
@@ -560,17 +563,16 @@ static int wait_result(qcs_cuda_state *s, size_t bytes, const char *what) {
   return check_cuda(cudaStreamSynchronize(s->stream), what);
 }
 
-// The same for a kernel that ends with report(): by watching for it, a few
-// microseconds sooner than the stream is known to be done (<Z> on 16 qubits 14.0
-// -> 12.2 us a call).  expect_report goes before the launch.  (A profiled launch's closing event is waited for too.)
-static void expect_report(qcs_cuda_state *s) {
-  __atomic_store_n((long long *)(s->h_result + kReady), 0LL, __ATOMIC_SEQ_CST);
-}
-static int wait_report(qcs_cuda_state *s, size_t bytes, const char *what) {
+// The same for a kernel that ends with report(): by watching for its call's
+// number, a few microseconds sooner than the stream is known to be done (<Z> on 16
+// qubits 14.0 -> 12.2 us a call).  (A profiled launch's closing event is waited
+// for too.)
+static i64 next_call(qcs_cuda_state *s) { return ++s->calls; }
+static int wait_report(qcs_cuda_state *s, i64 call, size_t bytes, const char *what) {
   if (!s->prof) {
-    const long long *ready = (const long long *)(s->h_result + kReady);
+    const i64 *ready = (const i64 *)(s->h_result + kReady);
     for (int i = 0; i < (1 << 20); i++)  // tens of milliseconds
-      if (__atomic_load_n(ready, __ATOMIC_ACQUIRE)) {
+      if (__atomic_load_n(ready, __ATOMIC_ACQUIRE) == call) {
         s->d2h_bytes += (long long)bytes;
         return QCS_CUDA_OK;
       }
@@ -585,23 +587,25 @@ static int reduce(qcs_cuda_state *s, int op, int q, double *res, int nres) {
   double *dst = op == OP_SUM ? s->d_result + 4 : s->h_result_dev;
   const i64 work = c128 ? s->size : s->size / 2;
   const int grid = reduce_grid(s, work);
-  if (op != OP_SUM) expect_report(s);
+  const i64 call = next_call(s);
   prof_begin(s);
   auto go = [&](auto opc) {
     constexpr int OP = decltype(opc)::value;
     if (c128)
       launch_next(sweep_early(s, grid), k_reduce_c128<OP>, grid, kReduceThreads, 0, s->stream,
-                  (const double2 *)s->vec, work, q, s->d_partials, s->d_count, dst);
+                  (const double2 *)s->vec, work, q, s->d_partials, s->d_count, dst,
+                  call);
     else
       launch_next(sweep_early(s, grid), k_reduce_c64<OP>, grid, kReduceThreads, 0, s->stream,
-                  (const float4 *)s->vec, work, q, s->d_partials, s->d_count, dst);
+                  (const float4 *)s->vec, work, q, s->d_partials, s->d_count, dst,
+                  call);
   };
   if (op == OP_NORM) go(std::integral_constant<int, OP_NORM>());
   else if (op == OP_MASK) go(std::integral_constant<int, OP_MASK>());
   else go(std::integral_constant<int, OP_SUM>());
   int rc = launched(s, KC_REDUCE, Ns, "reduce");
   if (rc || !res) return rc;
-  rc = wait_report(s, 4 * sizeof(double), "reduce sync");
+  rc = wait_report(s, call, 4 * sizeof(double), "reduce sync");
   if (rc) return rc;
   for (int i = 0; i < nres; i++) res[i] = s->h_result[i];
   return QCS_CUDA_OK;
@@ -772,18 +776,21 @@ int qcs_measure_all(qcs_cuda_state *s, const double *random_vals, int *outcomes)
                                          kMeasureMaxBytes),
                     "cudaFuncSetAttribute(measure)");
   }
+  // It collapses the state: not launched while an error is pending that
+  // launched() would report as its own.
+  if (!rc) rc = check_launch("measure all");
   if (rc) return rc;
-  expect_report(s);
+  const i64 call = next_call(s);
   prof_begin(s);
   if (c128)
     launch_next(true, k_measure_all<double2>, 1, threads, bytes, s->stream, (double2 *)s->vec, s->n,
-                draws, s->h_result_dev);
+                draws, s->h_result_dev, call);
   else
     launch_next(true, k_measure_all<float2>, 1, threads, bytes, s->stream, (float2 *)s->vec, s->n,
-                draws, s->h_result_dev);
+                draws, s->h_result_dev, call);
   invalidate_sum(s);
   rc = launched(s, KC_COLLAPSE, 2.0 * bytes, "measure all");
-  if (!rc) rc = wait_report(s, sizeof(double), "measure sync");
+  if (!rc) rc = wait_report(s, call, sizeof(double), "measure sync");
   if (rc) return rc;
   const int bits = (int)s->h_result[0];
   for (int q = 0; q < s->n; q++) outcomes[q] = (bits >> q) & 1;
@@ -798,16 +805,16 @@ int qcs_cuda_probability(qcs_cuda_state *s, long long index, double *p) {
     return QCS_CUDA_OK;
   }
   const size_t bytes = s->prec == QCS_CUDA_C128 ? 16 : 8;
-  expect_report(s);
+  const i64 call = next_call(s);
   prof_begin(s);
   if (s->prec == QCS_CUDA_C128)
     launch_next(true, k_peek<double2>, 1, 1, 0, s->stream, (const double2 *)s->vec, (i64)index,
-                s->h_result_dev);
+                s->h_result_dev, call);
   else
     launch_next(true, k_peek<float2>, 1, 1, 0, s->stream, (const float2 *)s->vec, (i64)index,
-                s->h_result_dev);
+                s->h_result_dev, call);
   int rc = launched(s, KC_OTHER, (double)bytes, "probability");
-  if (!rc) rc = wait_report(s, bytes, "probability sync");
+  if (!rc) rc = wait_report(s, call, bytes, "probability sync");
   if (rc) return rc;
   const double re = s->h_result[0], im = s->h_result[1];
   *p = (re * re) + (im * im);
@@ -819,17 +826,17 @@ int qcs_cuda_argmax(qcs_cuda_state *s, long long *index, double *prob) {
   if (!index) return set_error(QCS_CUDA_EINVAL, "null out");
   const bool pairs = s->prec == QCS_CUDA_C64;  // n >= 1: at least one pair
   const int grid = reduce_grid(s, pairs ? s->size / 2 : s->size);
-  expect_report(s);
+  const i64 call = next_call(s);
   prof_begin(s);
   if (pairs)
     k_argmax_c64<<<grid, kReduceThreads, 0, s->stream>>>(
-        (const float4 *)s->vec, s->size / 2, s->d_partials, s->d_count, s->h_result_dev);
+        (const float4 *)s->vec, s->size / 2, s->d_partials, s->d_count, s->h_result_dev, call);
   else
     k_argmax<double2, double><<<grid, kReduceThreads, 0, s->stream>>>(
-        (const double2 *)s->vec, s->size, s->d_partials, s->d_count, s->h_result_dev);
+        (const double2 *)s->vec, s->size, s->d_partials, s->d_count, s->h_result_dev, call);
   int rc = launched(s, KC_REDUCE, (double)s->size * (s->prec == QCS_CUDA_C128 ? 16 : 8),
                     "argmax");
-  if (!rc) rc = wait_report(s, 2 * sizeof(double), "argmax sync");
+  if (!rc) rc = wait_report(s, call, 2 * sizeof(double), "argmax sync");
   if (rc) return rc;
   *index = (long long)s->h_result[1];
   if (prob) return qcs_cuda_probability(s, *index, prob);

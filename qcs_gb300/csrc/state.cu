@@ -368,6 +368,7 @@ int qcs_cuda_state_create(int num_qubits, int precision, int semantics,
   if (!rc) rc = check_cuda(cudaMemsetAsync(s->d_err, 0, sizeof(int), s->stream), "cudaMemset(err)");
   if (!rc) rc = host_buffer((void **)&s->h_result, (void **)&s->h_result_dev, 8 * sizeof(double),
                             "cudaMallocHost(result)");
+  if (!rc) memset(s->h_result, 0, 8 * sizeof(double));
   if (!rc) rc = dmalloc((void **)&s->d_count, sizeof(unsigned), "cudaMalloc(block counter)");
   if (!rc) rc = check_cuda(cudaMemsetAsync(s->d_count, 0, sizeof(unsigned), s->stream),
                            "cudaMemset(block counter)");
