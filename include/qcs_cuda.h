@@ -375,6 +375,8 @@ int qcs_cuda_sample(qcs_cuda_state *s, const double *random_vals, int shots,
  * (shots doubles) and `samples` (shots 64-bit indices, -1 when a draw is not
  * below the total).  Work is queued on `stream` (a cudaStream_t, NULL for the
  * default stream); the call does not wait for it.
+ * `amplitudes` is aligned to 16 bytes; a complex64 state of fewer than 4096
+ * amplitudes may be aligned to 8 (else QCS_CUDA_EINVAL).
  * Limit: count must be a power of two no larger than 2^28 amplitudes; the
  * scratch is a fixed array of about 544 KB inside the library, held on every GPU that
  * loads it until the process exits.  The first call on a device looks up

@@ -120,6 +120,11 @@ extern "C" int qcs_cuda_sample_noalloc(const void *amplitudes, long long count, 
                      count, kNoAllocMaxTiles, kNoAllocTile);
   if (shots < 0 || (shots > 0 && (!draws || !samples)))
     return set_error(QCS_CUDA_EINVAL, "sample_noalloc: bad shot arguments");
+  // full tiles are read 16 bytes at a time; a complex64 state below one, by
+  // amplitudes where it has to be
+  const uintptr_t align = precision == QCS_CUDA_C64 && count < kNoAllocTile ? 8 : 16;
+  if (reinterpret_cast<uintptr_t>(amplitudes) % align)
+    return set_error(QCS_CUDA_EINVAL, "sample_noalloc: amplitudes not aligned to %d bytes", (int)align);
   double *prefix = nullptr;
   int rc = noalloc_scratch(&prefix);
   if (rc) return rc;

@@ -281,6 +281,8 @@ __global__ void k_smp_sample(const C *v, i64 tile, i64 n_tiles, i64 per, const d
                              const double *boff, int G, const double *draws, int shots, i64 *out) {
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  // a caller's own complex64 state may lie on 8 bytes; wider loads ask for 16
+  const bool wide = (reinterpret_cast<uintptr_t>(v) & 15) == 0;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   for (int s = warp; s < shots; s += nwarps) {
     const double r = draws[s];
@@ -307,7 +309,7 @@ __global__ void k_smp_sample(const C *v, i64 tile, i64 n_tiles, i64 per, const d
       C next[4];  // the group after this one, in flight
       auto load = [&](i64 base, C (&x)[4]) {
         const i64 i = base + 4 * lane;
-        if (i + 4 <= end) {
+        if (wide && i + 4 <= end) {
           smp_load4(v + i, x);
         } else {
 #pragma unroll
