@@ -133,6 +133,27 @@ template <int RB> struct RegsF32 {
     });
   }
 
+  // The same; whether an amplitude is an infinity or a NaN: 0 x is a NaN for those
+  // alone.
+  __device__ __forceinline__ bool store_finite(float *S, int L, const int (&pos)[N]) const {
+    float z[4] = {0.f, 0.f, 0.f, 0.f};  // as many chains
+    each<U>([&](auto uc) {
+      constexpr int u = decltype(uc)::value;
+      float a, b, c, d;
+      asm volatile("mov.b64 {%0, %1}, qre%4;\nmov.b64 {%2, %3}, qim%4;"
+                   : "=f"(a), "=f"(b), "=f"(c), "=f"(d) : "n"(u));
+      S[pos[2 * u]] = a;
+      S[pos[2 * u + 1]] = b;
+      S[L + pos[2 * u]] = c;
+      S[L + pos[2 * u + 1]] = d;
+      z[0] = fmaf(a, 0.f, z[0]);
+      z[1] = fmaf(b, 0.f, z[1]);
+      z[2] = fmaf(c, 0.f, z[2]);
+      z[3] = fmaf(d, 0.f, z[3]);
+    });
+    return (z[0] + z[1]) + (z[2] + z[3]) != 0.f;
+  }
+
   // f(u, w) for the register pairs that differ in register bit TB >= 1
   template <int TB, typename F>
   static __device__ __forceinline__ void pairs(F &&f) {

@@ -13,7 +13,8 @@
 // products and sums as in the sweeps, so the results are the sweeps' bit for
 // bit; only products with an entry that is exactly 0 or 1 are left out, which
 // changes no finite value (at most the sign of a zero).  A tile that holds an
-// infinity or a NaN takes every product the sweeps take (general_tile).
+// infinity or a NaN, or comes to hold one, begins again and takes every product
+// the sweeps take (general_tile).
 //
 // Inside a tile the gates run in register groups: the stretch is cut, again
 // in order, into groups whose targets lie on at most 4 tile bits; a thread
@@ -28,7 +29,7 @@
 // groups and the final store read through the map.
 //
 // Measured against one sweep per gate: 27 qubits complex64, brick, 752 gates
-// 241 -> 24.5 ms; 13 qubits, QFT and 200 random gates 212 -> 34 us a run;
+// 241 -> 22.5 ms; 13 qubits, QFT and 200 random gates 212 -> 34 us a run;
 // complex128, 20 qubits, the same circuit 3.98 -> 1.78 ms.  What bounds it:
 // on large complex64 states the instructions of the gate loop (a pass of 36
 // rotations issues 0.57 of the slots, two fifths of them packed arithmetic,
@@ -93,9 +94,10 @@ template <typename R> struct TileGate {
 // A group: gates [gate0, gate1) on registers e, where bit j of e adds
 // reg[j], bit j of the thread index col[j], to the shared-memory position
 // (XOR).  Before it, flips [flip0, flip1) change the constant.
+// (reg: 32 bits wide because with 16 one build of k_tile took reg[3] for 0.)
 struct TileGroup {
   unsigned char gate0, gate1, flip0, flip1;
-  unsigned short reg[kTileRegBits];
+  int reg[kTileRegBits];
   unsigned short col[kTileMaxThreadBits];
 };
 struct TileFlip {
@@ -343,7 +345,17 @@ __global__ void __launch_bounds__(1 << (TileTraits<C>::max_bits - RB),
     for (int j = 0; j < P.nout; j++) base |= ((tile >> j) & 1LL) << P.out[j];
     C *const vt = v + base + toff;
     const uint32_t id = (uint32_t)tile;
-    typename TileTraits<C>::Finite fin;
+    // Of an infinity, in the tile from the start or come up on the way, the
+    // products with zeros that are left out here are NaNs in the sweeps.  Some
+    // amplitude is an infinity or a NaN to the end then (nothing but the
+    // reference's CNOT drops one, and that drops the same ones in the sweeps), so
+    // one look after the last gate finds it, while the tile is still in memory to
+    // begin again.  The look is taken where it costs least: large states, bound by
+    // instructions, in the registers of the last group (27 qubits 24.1 -> 22.5 ms
+    // against a look at every amplitude that is read, in the units of the store
+    // 24.8), small ones, bound by latency, in the units of the store (16 qubits
+    // 189 -> 186 us a run with its read-outs, in the registers 191).
+    bool bad = false;
     {
       uint4 x[STEPS];
 #pragma unroll
@@ -353,62 +365,73 @@ __global__ void __launch_bounds__(1 << (TileTraits<C>::max_bits - RB),
         const C *y = reinterpret_cast<const C *>(&x[k]);
         const int at = tload ^ tile_pos(k << sb, kind);
 #pragma unroll
-        for (int j = 0; j < UNIT; j++) {
-          fin.see(y[j]);
-          tile_put(S, L, at ^ j, y[j]);
-        }
+        for (int j = 0; j < UNIT; j++) tile_put(S, L, at ^ j, y[j]);
       }
     }
-    const bool bad = __syncthreads_or(fin.bad());
+    __syncthreads();
     int c = 0;  // the map's constant
     auto flips = [&](int f0, int f1) {
       for (int f = f0; f < f1; f++)
         if (P.flip[f].id_bit < 0 || ((id >> P.flip[f].id_bit) & 1)) c ^= P.flip[f].mask;
     };
-    if (bad) {
-      general_tile<C>(S, P, id);
+    for (int gr = 0; gr < P.ngroups; gr++) {
+      const TileGroup &G = P.group[gr];
+      flips(G.flip0, G.flip1);
+      int at = c;
+#pragma unroll
+      for (int j = 0; j < TileTraits<C>::max_bits - RB; j++)
+        if ((t >> j) & 1) at ^= G.col[j];
+      auto place = [&](int (&pos)[REGS]) {  // register e: its bits' columns
+        int lo[4], hi[REGS / 4];
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          lo[k] = at ^ ((k & 1) ? G.reg[0] : 0) ^ ((k & 2) ? G.reg[1] : 0);
+#pragma unroll
+        for (int k = 0; k < REGS / 4; k++)
+          hi[k] = ((k & 1) ? G.reg[2] : 0) ^ ((k & 2) ? G.reg[3] : 0);
+#pragma unroll
+        for (int e = 0; e < REGS; e++) pos[e] = lo[e & 3] ^ hi[e >> 2];
+      };
+      typename TileTraits<C>::template Regs<RB> a;
+      {
+        int pos[REGS];
+        place(pos);
+        a.load(S, L, pos);
+      }
+      for (int i = G.gate0; i < G.gate1; i++) tile_apply(a, P.gate[i], (uint32_t)t, id, z);
+      asm volatile("" : "+r"(at));  // the positions are formed anew, not kept
+      int pos[REGS];
+      place(pos);
+      if constexpr (RB == kTileRegBits) {
+        if (gr + 1 == P.ngroups) {
+          bad = __syncthreads_or(a.store_finite(S, L, pos));
+          break;
+        }
+      }
+      a.store(S, L, pos);
+      __syncthreads();
+    }
+    flips(P.flip0, P.flip1);
+    if constexpr (RB < kTileRegBits) {
+      uint4 x[STEPS];
+      typename TileTraits<C>::Finite fin;
+#pragma unroll
       for (int k = 0; k < STEPS; k++) {
-        uint4 x;
-        C *y = reinterpret_cast<C *>(&x);
-        for (int j = 0; j < UNIT; j++)
-          y[j] = tile_get(S, L, tload ^ tile_pos((k << sb) | j, kind));
-        *reinterpret_cast<uint4 *>(vt + step_off(k)) = x;
-      }
-    } else {
-      for (int gr = 0; gr < P.ngroups; gr++) {
-        const TileGroup &G = P.group[gr];
-        flips(G.flip0, G.flip1);
-        int at = c;
+        C *y = reinterpret_cast<C *>(&x[k]);
+        const int at = c ^ tstore ^ step_store(k);
 #pragma unroll
-        for (int j = 0; j < TileTraits<C>::max_bits - RB; j++)
-          if ((t >> j) & 1) at ^= G.col[j];
-        auto place = [&](int (&pos)[REGS]) {  // register e: its bits' columns
-          int lo[4], hi[REGS / 4];
-#pragma unroll
-          for (int k = 0; k < 4; k++)
-            lo[k] = at ^ ((k & 1) ? G.reg[0] : 0) ^ ((k & 2) ? G.reg[1] : 0);
-#pragma unroll
-          for (int k = 0; k < REGS / 4; k++)
-            hi[k] = ((k & 1) ? G.reg[2] : 0) ^ ((k & 2) ? G.reg[3] : 0);
-#pragma unroll
-          for (int e = 0; e < REGS; e++) pos[e] = lo[e & 3] ^ hi[e >> 2];
-        };
-        typename TileTraits<C>::template Regs<RB> a;
-        {
-          int pos[REGS];
-          place(pos);
-          a.load(S, L, pos);
+        for (int j = 0; j < UNIT; j++) {
+          y[j] = tile_get(S, L, j ? at ^ P.store[0] : at);
+          fin.see(y[j]);
         }
-        for (int i = G.gate0; i < G.gate1; i++) tile_apply(a, P.gate[i], (uint32_t)t, id, z);
-        asm volatile("" : "+r"(at));  // the positions are formed anew, not kept
-        {
-          int pos[REGS];
-          place(pos);
-          a.store(S, L, pos);
-        }
-        __syncthreads();
       }
-      flips(P.flip0, P.flip1);
+      bad = __syncthreads_or(fin.bad());
+      if (!bad) {
+#pragma unroll
+        for (int k = 0; k < STEPS; k++) *reinterpret_cast<uint4 *>(vt + step_off(k)) = x[k];
+        continue;  // no access to shared memory since the barrier
+      }
+    } else if (!bad) {
 #pragma unroll
       for (int k = 0; k < STEPS; k++) {
         uint4 x;
@@ -416,6 +439,22 @@ __global__ void __launch_bounds__(1 << (TileTraits<C>::max_bits - RB),
         const int at = c ^ tstore ^ step_store(k);
 #pragma unroll
         for (int j = 0; j < UNIT; j++) y[j] = tile_get(S, L, j ? at ^ P.store[0] : at);
+        *reinterpret_cast<uint4 *>(vt + step_off(k)) = x;
+      }
+    }
+    if (bad) {
+      for (int k = 0; k < STEPS; k++) {
+        const uint4 x = *reinterpret_cast<const uint4 *>(vt + step_off(k));
+        const C *y = reinterpret_cast<const C *>(&x);
+        for (int j = 0; j < UNIT; j++) tile_put(S, L, tload ^ tile_pos((k << sb) | j, kind), y[j]);
+      }
+      __syncthreads();
+      general_tile<C>(S, P, id);
+      for (int k = 0; k < STEPS; k++) {
+        uint4 x;
+        C *y = reinterpret_cast<C *>(&x);
+        for (int j = 0; j < UNIT; j++)
+          y[j] = tile_get(S, L, tload ^ tile_pos((k << sb) | j, kind));
         *reinterpret_cast<uint4 *>(vt + step_off(k)) = x;
       }
     }
@@ -670,7 +709,7 @@ static int launch_pass(qcs_cuda_state *s, const qcs_cuda_op *ops, const TileStre
       for (int j = 0; j < P.nt; j++) {
         const int b = order[j];
         if (j < RB) {  // the least used one is the pair bit (tile_regs.cuh)
-          G.reg[RB - 1 - j] = (unsigned short)map[b];
+          G.reg[RB - 1 - j] = map[b];
           reg_of[b] = RB - 1 - j;
         } else {
           const int t = P.nt - 1 - j;  // the last, least used ones are the lanes
@@ -693,6 +732,13 @@ static int launch_pass(qcs_cuda_state *s, const qcs_cuda_op *ops, const TileStre
       fill_gate<R>(s, ops[i], bit_of, id_of, none, none, P.gate[at]);
       P.order[i - st.first] = (unsigned char)at;
       move(ops[i]);
+    }
+  }
+  if (RB == kTileRegBits && P.ngroups == 0) {  // moves alone: the look takes a group
+    TileGroup &G = P.group[P.ngroups++];
+    for (int j = 0; j < P.nt; j++) {
+      if (j < RB) G.reg[RB - 1 - j] = map[P.nt - 1 - j];
+      else G.col[P.nt - 1 - j] = (unsigned short)map[P.nt - 1 - j];
     }
   }
   P.flip0 = (unsigned char)flip0;
