@@ -767,13 +767,67 @@ static int launch_pass(qcs_cuda_state *s, const qcs_cuda_op *ops, const TileStre
   return launched(s, KC_TILE, 2.0 * s->size * sizeof(C), "gate tile pass");
 }
 
+// Whether the sweeps of a stretch's gates cost less than its pass: a sweep leaves
+// out what its gate leaves alone, the whole of an identity's, three quarters of a
+// controlled phase's, half of a phase's or a CNOT's.  A pass reads and writes
+// everything once.  Work is counted in sixteenths of a pass; a condition on a
+// qubit so low that its amplitudes lie in the same 32 bytes as the others saves
+// nothing, in the same 128 bytes part of it.  The reference's sweeps go out of
+// place, over everything.
+// complex64, us by sweeps against us by a pass: two controlled phases on 20, 22, 23,
+// 24, 27, 30 qubits 8, 9, 12, 17, 175, 1299 against 5, 11, 21, 47, 335, 2660; four 17,
+// 20, 25, 40, 350, 2597 against 5, 12, 23, 46, 340, 2650; two phases 8, 12, 17, 33,
+// 335, 2596 against the same.  Below 32 MB the launches decide, above 64 the bytes
+// (that lie in L2 in part: 128 MB), between them both.
+// complex128: the FP64 pipe bounds both ways, and a pass has its reads and writes on
+// top; but it takes signs and moves without that pipe, and is better at all else.
+// Two controlled phases on 18, 20, 22, 27 qubits 12, 14, 33, 784 against 10, 17, 43,
+// 1058, on the lowest qubits of 21, 23, 27 21, 72, 1129 against 24, 81, 1060; four 25,
+// 29, 66, 1568 against 12, 27, 67, 1740; three phases 19, 31, 86, 2331 against 13, 26,
+// 81, 2450; two CNOTs 16, 21, 57, 1556 against 5, 8, 18, 638.
+static bool sweeps_cost_less(const qcs_cuda_state *s, const qcs_cuda_op *ops, int count) {
+  if (s->sem == QCS_CUDA_REFERENCE) return false;
+  const bool c64 = s->prec == QCS_CUDA_C64;
+  const i64 bytes = s->size * (c64 ? 8 : 16);
+  const int sector = c64 ? 2 : 1;  // qubits within 32 bytes
+  int sweeps = 0, work = 0;
+  for (int i = 0; i < count && work <= 32; i++) {
+    const qcs_cuda_op &o = ops[i];
+    double m[8];
+    gate_matrix(o.kind, o.angle, m);
+    auto is = [&](int e, double v) { return m[2 * e] == v && m[2 * e + 1] == 0.0; };
+    const bool diag = is(1, 0.0) && is(2, 0.0), ctl = gate_is_controlled(o.kind);
+    if (diag && is(0, 1.0) && is(3, 1.0)) continue;  // an identity: no sweep
+    if (!c64 && !diag) return false;
+    if (!c64 && o.kind == QCS_GATE_Z) return false;
+    int w = 16;
+    auto condition = [&](int q) { w = q < sector ? w : q < sector + 2 ? w * 3 / 4 : w / 2; };
+    if (ctl) condition(o.control);
+    if (diag && is(0, 1.0)) condition(o.target);
+    work += w;
+    sweeps++;
+  }
+  if (sweeps <= 1) return true;
+  if (c64) {
+    if (bytes < (32 << 20)) return false;
+    if (bytes <= (64 << 20)) return 4 * sweeps + work <= (bytes <= (32 << 20) ? 20 : 28);
+    return work <= 16;
+  }
+  if (bytes < (16 << 20)) return false;
+  if (sweeps == 2 && bytes >= (32 << 20) && bytes <= (128 << 20)) return work <= 24;
+  return work <= (bytes < (64 << 20) ? 12 : bytes < (128 << 20) ? 16 : 20);
+}
+
 template <typename C, int RB>
 static int run_tiles_t(qcs_cuda_state *s, const qcs_cuda_op *ops, int count, int bits) {
   const int nt = std::min(bits, s->n);
   for (const TileStretch &st : tile_stretches(ops, count, s->n, nt, TileTraits<C>::low,
                                               s->sem == QCS_CUDA_REFERENCE, RB)) {
-    const int rc = st.last - st.first == 1 ? apply_op(s, ops[st.first])
-                                           : launch_pass<C, RB>(s, ops, st);
+    int rc = QCS_CUDA_OK;
+    if (st.last - st.first == 1 || sweeps_cost_less(s, ops + st.first, st.last - st.first))
+      for (int i = st.first; !rc && i < st.last; i++) rc = apply_op(s, ops[i]);
+    else
+      rc = launch_pass<C, RB>(s, ops, st);
     if (rc) return rc;
   }
   return QCS_CUDA_OK;
