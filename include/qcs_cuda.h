@@ -254,7 +254,7 @@ int qcs_cuda_batch_set_angles(qcs_cuda_batch *b, const double *angles);
 int qcs_cuda_batch_run(qcs_cuda_batch *b, double *expect_z0,
                        long long *samples, double *ms);
 /* Times every schedule (threads per CTA 256/512/1024, tile 2^12..2^14,
- * 1, 2 or 4 CTAs per SM as fit, largest-first or given order) on this batch, then how
+ * 1, 2 or 4 CTAs per SM where as many fit, largest-first or given order) on this batch, then how
  * widely large instances spread (2^(n - split_q) CTAs start on an instance above
  * split_q qubits, split_q in 17..20 or one always), and keeps the
  * fastest; chosen (4 ints) receives threads, tile qubits, CTAs per SM and
@@ -274,7 +274,8 @@ int qcs_cuda_batch_split(qcs_cuda_batch *b, int split_q);
  * (8 bytes per instance and 8 per shot).  Instances that fit the tile live
  * in shared memory and move no state bytes. */
 int qcs_cuda_batch_traffic(qcs_cuda_batch *b, double *hbm_bytes);
-/* Sets one schedule explicitly (split_q is kept). */
+/* Sets one schedule explicitly (split_q is kept).  Of ctas_per_sm, as many run as
+ * fit an SM: qcs_cuda_batch_schedule tells how many that are. */
 int qcs_cuda_batch_config(qcs_cuda_batch *b, int threads, int tile_q,
                           int ctas_per_sm, int order);
 

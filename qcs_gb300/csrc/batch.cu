@@ -104,7 +104,7 @@ struct __align__(16) BGate {
 struct BatchTune {
   int threads;      // 256, 512 or 1024
   int tile_q;       // 12, 13 or 14
-  int ctas_per_sm;  // 1, 2 or 4 (as many as shared memory and registers allow)
+  int ctas_per_sm;  // 1, 2 or 4 (as many run as shared memory and registers allow)
   int order;        // 0: largest first, 1: given order
   int split_q;      // instances above split_q qubits are queued for 2^(n - split_q) CTAs
 };
@@ -1115,11 +1115,22 @@ static size_t smem_for(int tile_q) {
   return ((size_t)8 << tile_q) + sizeof(BWindow) + std::max<size_t>(1025, blocks) * sizeof(double);
 }
 
+// CTAs that an SM holds at once: by registers 2 of 256 threads and 1 of 512 or
+// 1024, by shared memory fewer.
 template <int T>
-static int set_smem_attr(int tile_q) {
-  return check_cuda(cudaFuncSetAttribute(k_batch<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem_for(tile_q)),
-                    "cudaFuncSetAttribute(batch)");
+static int batch_fit_t(int tile_q, int *fit) {
+  int rc = check_cuda(cudaFuncSetAttribute(k_batch<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)smem_for(tile_q)),
+                      "cudaFuncSetAttribute(batch)");
+  if (!rc)
+    rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(fit, k_batch<T>, T,
+                                                                  smem_for(tile_q)),
+                    "occupancy");
+  return rc;
+}
+static int batch_fit(int threads, int tile_q, int *fit) {
+  return threads == 256 ? batch_fit_t<256>(tile_q, fit)
+         : threads == 512 ? batch_fit_t<512>(tile_q, fit) : batch_fit_t<1024>(tile_q, fit);
 }
 
 // Doubles of a slot's block sums.
@@ -1139,17 +1150,7 @@ static int batch_upload(qcs_cuda_batch *b) {
   // grid: CTAs per SM from the tune, but never more than fit the GPU at once;
   // a global slot for each
   int fit = 0;
-  switch (b->tune.threads) {
-    case 256: rc = set_smem_attr<256>(b->tune.tile_q); break;
-    case 512: rc = set_smem_attr<512>(b->tune.tile_q); break;
-    default: rc = set_smem_attr<1024>(b->tune.tile_q); break;
-  }
-  if (rc) return rc;
-  switch (b->tune.threads) {
-    case 256: rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_batch<256>, 256, smem_for(b->tune.tile_q)), "occupancy"); break;
-    case 512: rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_batch<512>, 512, smem_for(b->tune.tile_q)), "occupancy"); break;
-    default: rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_batch<1024>, 1024, smem_for(b->tune.tile_q)), "occupancy"); break;
-  }
+  rc = batch_fit(b->tune.threads, b->tune.tile_q, &fit);
   if (rc) return rc;
   if (fit < 1) return set_error(QCS_CUDA_EUNSUP, "batch kernel does not fit an SM");
   const int grid = b->dev.num_sms * std::min(b->tune.ctas_per_sm, fit);
@@ -1447,25 +1448,27 @@ int qcs_cuda_batch_autotune(qcs_cuda_batch *b, int repeats, int *chosen) {
   BatchTune best = b->tune;
   float best_ms = 1e30f;
   for (int th : threads)
-    for (int tq : tiles)
+    for (int tq : tiles) {
+      int fit = 0;
+      int rc = batch_fit(th, tq, &fit);
+      if (rc) return rc;
       for (int cp : ctas)
         for (int ord = 0; ord < 2; ord++) {
-          // the CTAs of an SM must fit its shared memory, and four only
-          // with 256 threads (64 registers a thread)
-          if (smem_for(tq) * cp > 220 * 1024 || th * cp > 1024) continue;
+          if (cp > fit) continue;  // it would run as a schedule of fewer
           BatchTune t = b->tune;
           t.threads = th;
           t.tile_q = tq;
           t.ctas_per_sm = cp;
           t.order = ord;
           float ms = 0.f;
-          int rc = time_tune(t, &ms);
+          rc = time_tune(t, &ms);
           if (rc) return rc;
           if (ms < best_ms) {
             best_ms = ms;
             best = t;
           }
         }
+    }
   // then how far large instances spread over CTAs (27: never)
   const int splits[] = {17, 18, 19, 20, 27};
   const BatchTune base = best;
