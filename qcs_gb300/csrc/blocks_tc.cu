@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     mbar_init(bar(11), 1);
     *abort_flag = 0;
     fence_barrier_init();
-    bulk_load(smem_u32(sB), bimg, S::IMG_BYTES, bar(11));
+    bulk_load<S::IMG_BYTES>(smem_u32(sB), bimg, bar(11));
   }
   for (int i = tid; i < kTcM; i += kTcThreads) col_off[i] = spread(i, g.colq);
   for (int i = tid; i < KA; i += kTcThreads) blk_off[i] = spread(i, g.blkq);
@@ -681,7 +681,7 @@ __global__ void __launch_bounds__(Tc7::THREADS, 1)
     mbar_init(bar(13), 1);
     *abort_flag = 0;
     fence_barrier_init();
-    bulk_load(smem_u32(sB), bimg, S::IMG_BYTES, bar(13));
+    bulk_load<S::IMG_BYTES>(smem_u32(sB), bimg, bar(13));
   }
   for (int i = tid; i < kTcM; i += S::THREADS) col_off[i] = spread(i, g.colq);
   for (int i = tid; i < S::KA; i += S::THREADS) blk_off[i] = spread(i, g.blkq);

@@ -41,18 +41,20 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
 __device__ __forceinline__ void prefetch_l2(const void *p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
-// Copies `bytes` (a multiple of 16 KB) from global to shared memory (both
-// 16-byte aligned), 16 KB at a time; `bar`, initialised by this thread for one
-// arrival, completes its phase when all of it is there.
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes,
-                                          uint32_t bar) {
+// Copies BYTES from global to shared memory (both 16-byte aligned), 16 KB at a
+// time; `bar`, initialised by this thread for one arrival, completes its phase when
+// all of it is there.
+template <uint32_t BYTES>
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bar) {
+  constexpr uint32_t PIECE = 16384;
+  static_assert(BYTES % PIECE == 0, "bulk copies in whole pieces");
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(BYTES)
                : "memory");
-  for (uint32_t o = 0; o < bytes; o += 16384)
+  for (uint32_t o = 0; o < BYTES; o += PIECE)
     asm volatile(
         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-        ::"r"(dst + o), "l"(reinterpret_cast<const uint8_t *>(src) + o), "r"(16384u), "r"(bar)
+        ::"r"(dst + o), "l"(reinterpret_cast<const uint8_t *>(src) + o), "r"(PIECE), "r"(bar)
         : "memory");
 }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
