@@ -21,7 +21,10 @@
 #include "../../include/qcs.h"
 #include "../../include/qcs_cuda.h"
 #include "../../include/qcs_ext.h"
-#include "../csrc/measure_all.h"
+
+/* All qubits of a small state measured in one launch (csrc/readout.cu). */
+int qcs_measure_all(qcs_cuda_state *s, const double *random_vals,
+                    int *outcomes);
 
 struct t_q_circuit {
   int num_qubits;
