@@ -352,6 +352,11 @@ int qcs_cuda_prob_zero(qcs_cuda_state *s, int qubit, double *p0);
  * outcome 0 when random_val <= p0; collapse and renormalise. */
 int qcs_cuda_measure(qcs_cuda_state *s, int qubit, double random_val,
                      int *outcome);
+/* For qc_measure_all: what qcs_cuda_measure of qubits 0 .. n-1 in turn does,
+ * with one draw each, in one launch.  QCS_CUDA_EUNSUP, and nothing done, for a
+ * state of more than 128 KB. */
+int qcs_measure_all(qcs_cuda_state *s, const double *random_vals,
+                    int *outcomes);
 /* qc_get_probability (src/qcs.c:391-395), 64-bit index. */
 int qcs_cuda_probability(qcs_cuda_state *s, long long index, double *p);
 /* qc_find_most_likely_state (src/qcs.c:464-478): first index of the

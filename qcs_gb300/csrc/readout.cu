@@ -756,9 +756,6 @@ int qcs_cuda_measure(qcs_cuda_state *s, int qubit, double random_val, int *outco
   return QCS_CUDA_OK;
 }
 
-// For qc_measure_all: what qcs_cuda_measure of qubits 0 .. n-1 in turn does, with
-// one draw each.  QCS_CUDA_EUNSUP, and nothing done, for a state of more than
-// 128 KB.
 int qcs_measure_all(qcs_cuda_state *s, const double *random_vals, int *outcomes) {
   QCS_CHECK_STATE(s);
   const bool c128 = s->prec == QCS_CUDA_C128;

@@ -22,10 +22,6 @@
 #include "../../include/qcs_cuda.h"
 #include "../../include/qcs_ext.h"
 
-/* All qubits of a small state measured in one launch (csrc/readout.cu). */
-int qcs_measure_all(qcs_cuda_state *s, const double *random_vals,
-                    int *outcomes);
-
 struct t_q_circuit {
   int num_qubits;
   int num_gates;
