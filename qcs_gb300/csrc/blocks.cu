@@ -338,9 +338,9 @@ struct PlanCache {
 // while their total stays under this many bytes.
 constexpr size_t kPlanCacheMatBytes = 64u << 20;
 
-// A plain run (one kernel per op) kept as a CUDA graph.  Small states run
-// circuits of short kernels whose launches, one per gate, take as long as
-// the kernels (a 20-qubit complex128 QFT phase: ~3 us of work).  The same op
+// A plain run (no fusion) kept as a CUDA graph.  Small states run circuits of
+// short kernels, tile passes and sweeps, whose launches take as long as the
+// kernels (a 20-qubit complex128 QFT phase: ~3 us of work).  The same op
 // list, byte for byte, is captured into a graph on its second run in a row
 // and replayed from then on: one graph launch per circuit.  The cached
 // amplitude sum is reset before the capture and before every replay, so the

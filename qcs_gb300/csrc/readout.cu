@@ -571,7 +571,9 @@ static i64 next_call(qcs_cuda_state *s) { return ++s->calls; }
 static int wait_report(qcs_cuda_state *s, i64 call, size_t bytes, const char *what) {
   if (!s->prof) {
     const i64 *ready = (const i64 *)(s->h_result + kReady);
-    for (int i = 0; i < (1 << 20); i++)  // tens of milliseconds
+    // 0.34 ms on the Grace host of a GB300, 1 to 2 ms on x86 hosts; a longer wait is
+    // left to the stream
+    for (int i = 0; i < (1 << 20); i++)
       if (__atomic_load_n(ready, __ATOMIC_ACQUIRE) == call) {
         s->d2h_bytes += (long long)bytes;
         return QCS_CUDA_OK;

@@ -29,11 +29,11 @@
 // groups and the final store read through the map.
 //
 // Measured against one sweep per gate: 27 qubits complex64, brick, 752 gates
-// 241 -> 22.5 ms; 13 qubits, QFT and 200 random gates 212 -> 34 us a run;
+// 241 -> 22.5 ms; 13 qubits, QFT and 200 random gates 212 -> 28 us a run;
 // complex128, 20 qubits, the same circuit 3.98 -> 1.78 ms.  What bounds it:
 // on large complex64 states the instructions of the gate loop (a pass of 36
-// rotations issues 0.57 of the slots, two fifths of them packed arithmetic,
-// with DRAM at 0.19; a pass of CNOTs alone runs at 0.9 of HBM); on complex128
+// rotations issues 0.69 of the slots, two fifths of them packed arithmetic,
+// with DRAM at 0.39; a pass of CNOTs alone runs at 0.9 of HBM); on complex128
 // the FP64 pipe (84 % busy); on small states the latency of a pass.
 #include <stddef.h>
 #include <string.h>
@@ -148,7 +148,10 @@ struct FiniteF64 {
 // 20 qubits, 417 gates): 2.13 and 2.32 ms.  Likewise 16 amplitudes a thread
 // against 32: 27.7 and 28.9 ms, 87 and 122 us.  (By number of tiles: run_tiles.)
 // low: qubits every tile holds, so that it is read in runs of 128 bytes.
-// blocks: CTAs an SM holds at 16 amplitudes a thread (72 registers, complex64).
+// blocks: CTAs an SM holds at 16 amplitudes a thread.  complex64: 72 registers, for
+// which 140 bytes a thread are spilled outside the loop over gates (2.6 M of a 26-qubit
+// pass's 290 M warp instructions); the bound was chosen when the grid was what the GPU
+// holds at once.
 template <typename C> struct TileTraits;
 template <> struct TileTraits<float2> {
   typedef float R;
