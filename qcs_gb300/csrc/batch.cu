@@ -130,7 +130,8 @@ struct qcs_cuda_batch {
   std::vector<int> fold_ops;
   std::vector<int> gate_tc;       // its group-local target | control << 8 (control 0xFF: none)
   std::vector<int> order;         // instance order
-  std::vector<int2> items;        // (instance, member) in queue order
+  std::vector<int2> items;        // (instance, member) in queue order, then those in slots
+  int n_items;                    // of the queue
   qcs::BatchTune tune;
   int planned_tile_q, planned_regs;
   // device
@@ -397,7 +398,7 @@ __device__ void warp_prefix(double *x, int m) {
   if (lane == 0) x[m] = total;
 }
 
-constexpr int kBlock = 32;        // amplitudes of a block, at least
+constexpr int kBlock = 32;        // amplitudes of a block in a slot, at least
 constexpr int kMaxBlocks = 8192;  // blocks of an instance
 constexpr int kMaxTiles = 1024;   // sampling tiles of an instance
 
@@ -405,9 +406,9 @@ struct ReadShape {
   i64 block, tile;  // amplitudes
   int n_blocks, n_tiles, per;  // per: blocks of a tile
 };
-__host__ __device__ inline ReadShape read_shape(i64 size) {
+__host__ __device__ inline ReadShape read_shape(i64 size, int block = kBlock) {
   ReadShape r;
-  r.block = size / kMaxBlocks > kBlock ? size / kMaxBlocks : kBlock;
+  r.block = size / kMaxBlocks > block ? size / kMaxBlocks : block;
   r.tile = size / kMaxTiles > kMassTile ? size / kMaxTiles : kMassTile;
   if (r.tile > size) r.tile = size;
   if (r.block > size) r.block = size;
@@ -521,12 +522,15 @@ __device__ __forceinline__ void pick_shots(const ReadShape &R, const double *pre
 
 // Read-out of an instance that lives in shared memory (L = 2^n amplitudes of
 // a tile of Lt; those from L on are 0).  Returns <Z_0> in thread 0.
-// scratch: 5 + 2 * L / 32 doubles.
+// A block's sums are chains of FP64 additions in one thread, so small instances
+// have blocks of fewer than 32 amplitudes, up to 256 of them (20000 of 5 qubits, 20
+// gates, 16 shots: 1144 -> 775 us).
+// scratch: 5 + 2 * (L / 32 or 256) doubles.
 template <int T>
 __device__ double resident_readout(const float *S, int L, int Lt, double *scratch, double *red,
                                    int shots, u64 seed, int inst, i64 *out) {
   const float2 kind = {};
-  const ReadShape R = read_shape(L);
+  const ReadShape R = read_shape(L, L >= 256 * kBlock ? kBlock : L >= 4096 ? L / 256 : 8);
   double *prefix = scratch, *exact = scratch + 5, *mass = exact + R.n_blocks;
   auto load8 = [&](i64 i, float2 (&a)[8]) {
 #pragma unroll
@@ -545,6 +549,7 @@ __device__ double resident_readout(const float *S, int L, int Lt, double *scratc
     z += sums.even - sums.odd;
   }
   z = block_sum<T>(z, red);
+  if (shots == 0) return z;
   __syncthreads();
   running_sums<T, false>(R, mass, exact, exact, prefix);
   pick_shots<T>(R, prefix, exact, shots, seed, inst, out, load8);
@@ -664,7 +669,7 @@ __device__ __forceinline__ BTickets batch_tickets(const BInst &I, int tile_q) {
 template <int T>
 __global__ void __launch_bounds__(T, T == 256 ? 2 : 1)
     k_batch(const BInst *insts, const BStage *stages, const BGroup *groups, const BGate *gates,
-            const int2 *items, int n_items, int shots, u64 seed, int tile_q, float2 *slots,
+            const int2 *items, int n_items, int n_slot, int shots, u64 seed, int tile_q, float2 *slots,
             i64 slot_amps, double *slot_sum, i64 sums_of_slot, int *queue, BShare *share, int *slot_busy, int *err, double *z_out,
             i64 *samples_out, long long wait) {
   QCS_REGS_F32_DECLARE(1 << (reg_q(T) - 1));
@@ -688,19 +693,25 @@ __global__ void __launch_bounds__(T, T == 256 ? 2 : 1)
     const bool joined = s_pick >= n_items;
     if (!joined) {
       inst = items[s_pick].x;
+    } else if (n_slot == 0) {
+      break;
     } else {
       // the queue is empty: join the instance with the most tiles left per CTA
-      // at it.  A CTA that joins changes at_it, so of those that chose the same
-      // instance one gets it and the others look again.
+      // at it (those in slots are listed after the queue).  A CTA that joins
+      // changes at_it, so of those that chose the same instance one gets it and
+      // the others look again.
+      // (The upper half of the grid, whose CTAs lie beside one of the lower half on
+      // an SM, lets that go first: one instance of 16 qubits, eight CTAs, takes 388
+      // us where they have eight SMs and 535 where two share one.)
+      if (2 * blockIdx.x >= gridDim.x) __nanosleep(4000);
       do {
         __syncthreads();
         if (threadIdx.x == 0) s_best = 0;
         __syncthreads();
-        for (int e = threadIdx.x; e < n_items; e += T) {
-          const int2 it = items[e];
-          if (it.y != 0 || it.x >= 1 << 24) continue;
+        for (int e = threadIdx.x; e < n_slot; e += T) {
+          const int2 it = items[n_items + e];
+          if (it.x >= 1 << 24) continue;
           const BInst J = insts[it.x];
-          if (J.n <= tile_q) continue;
           const BTickets k = batch_tickets(J, tile_q);
           const int left = k.total - *(volatile int *)&share[it.x].next;
           const int at_it = *(volatile int *)&share[it.x].at_it;
@@ -1109,7 +1120,8 @@ static void batch_free_device(qcs_cuda_batch *b) {
 }
 
 // The tile, the window of gates, then scratch of the read-outs: 1025 prefixes of a slot's sampling
-// tiles, or 5 + 2 * 2^tile_q / 32 doubles of a resident instance.
+// tiles, or 5 + 2 * 2^tile_q / 32 doubles of a resident instance (5 + 2 * 256 of one
+// below 2^13 amplitudes).
 static size_t smem_for(int tile_q) {
   const size_t blocks = 5 + 2 * (((size_t)1 << tile_q) / kBlock);
   return ((size_t)8 << tile_q) + sizeof(BWindow) + std::max<size_t>(1025, blocks) * sizeof(double);
@@ -1190,6 +1202,9 @@ static int batch_upload(qcs_cuda_batch *b) {
   b->items.clear();
   for (int inst : b->order)
     for (int g = 0; g < b->insts[inst].group; g++) b->items.push_back(make_int2(inst, g));
+  b->n_items = (int)b->items.size();
+  for (int inst : b->order)
+    if (b->insts[inst].n > b->tune.tile_q) b->items.push_back(make_int2(inst, 0));
   if (!rc) rc = check_cuda(cudaMalloc((void **)&b->d_items, b->items.size() * sizeof(int2)), "cudaMalloc(batch)");
   if (!rc) rc = check_cuda(cudaMemcpy(b->d_items, b->items.data(), b->items.size() * sizeof(int2), cudaMemcpyHostToDevice), "upload");
   if (rc) return rc;
@@ -1224,7 +1239,8 @@ static int batch_enqueue(qcs_cuda_batch *b) {
   int *queue = (int *)(share + b->count), *busy = queue + 1;
 #define QCS_LAUNCH_BATCH(T)                                                                       \
   k_batch<T><<<b->grid, T, smem, b->stream>>>(                                                    \
-      b->d_insts, b->d_stages, b->d_groups, b->d_gates, b->d_items, (int)b->items.size(),           \
+      b->d_insts, b->d_stages, b->d_groups, b->d_gates, b->d_items, b->n_items,                     \
+      (int)b->items.size() - b->n_items,                                                           \
       b->shots, b->seed, tq, b->d_slots, (i64)b->slot_amps, b->d_sums,           \
       (i64)sums_of_slot(b), queue, share, busy,                                                    \
       b->d_err, b->d_z, b->d_samples, b->wait_captured)
